@@ -65,6 +65,17 @@ int upload_side(const SideSchedule& sc, int B, const SegMatrix& A, unsigned* tic
 
 }  // namespace
 
+std::vector<uint8_t> segment_lanes(const SideSchedule& sc, int nseg) {
+    std::vector<uint8_t> lanes((size_t)nseg, 1);
+    for (const Task& t : sc.tasks)  // light tasks first: the list tasks then take the segments they skip
+        if (!(t.flags & kTaskList))
+            std::fill(lanes.begin() + t.seg_begin, lanes.begin() + t.seg_end, (uint8_t)task_lanes(t.flags));
+    for (const Task& t : sc.tasks)
+        if (t.flags & kTaskList)
+            for (int h = t.seg_begin; h < t.seg_end; ++h) lanes[sc.list_idx[h]] = (uint8_t)task_lanes(t.flags);
+    return lanes;
+}
+
 int TaskLayout::build(const std::vector<int>& csr_ptr, const std::vector<int>& csc_ptr, const std::vector<int>& roff,
                       const std::vector<int>& coff, const SegMatrix& rows_A, const SegMatrix& cols_A, int task_nnz,
                       bool all_active, cudaStream_t s, int row_lanes, int col_lanes, int max_segs) {

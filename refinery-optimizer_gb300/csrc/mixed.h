@@ -3,6 +3,7 @@
 // for one LP or a batch of LPs; see mixed.cu for the algorithm.
 #pragma once
 
+#include <memory>
 #include <vector>
 
 #include "common.cuh"
@@ -106,6 +107,9 @@ struct SideSchedule {
 void make_schedule(const std::vector<int>& ptr, const std::vector<int>& inst_off, int task_nnz, SideSchedule& out,
                    int light_lanes = 0, int max_segs = kTaskSegs);
 
+// Lanes per segment that a schedule gives to each of nseg segments.
+std::vector<uint8_t> segment_lanes(const SideSchedule& sc, int nseg);
+
 // Device task layout of a block-diagonal (batched) matrix for the task engine
 // (warp.cuh): per side (rows = CSR for A x, columns = CSC for A^T y) the SpMV
 // tasks, their reduction groups, partial slots, tickets and active list; the
@@ -144,9 +148,11 @@ struct Vecs {
     int pow_n;
 };
 
+class ResidentPlan;  // resident.h
+
 class MixedSolver {
   public:
-    MixedSolver() = default;
+    MixedSolver();
     MixedSolver(const MixedSolver&) = delete;
     MixedSolver& operator=(const MixedSolver&) = delete;
     ~MixedSolver();
@@ -189,6 +195,7 @@ class MixedSolver {
     int setup_persistent();
     int set_form(int form);
     int setup_packed();
+    int setup_resident();
     int apply_shape(const sih_pdhg_launch_shape& sh);
     int time_block(double* seconds);
 
@@ -227,6 +234,8 @@ class MixedSolver {
     // lanes per segment of the light tasks (0 = length rule), staged prefixes
     // the rule chose (the tuner may switch them off), tuned flag
     int lanes_r_ = 0, lanes_c_ = 0, stage_x_rule_ = 0, stage_y_rule_ = 0, tuned_ = 0;
+    // the steps of one LP or a batch in the shared memory of a cluster per instance
+    std::unique_ptr<ResidentPlan> resident_;
     int packed_ = 0;  // options.packed: two kernels per step on packed column records
     Vecs V_{};
     std::vector<Inst> host_inst_;

@@ -1,0 +1,880 @@
+// Resident step form: the steps between two evaluations of an LP whose matrix,
+// vectors and controller state all fit in the shared memory of one thread-block
+// cluster (one block for the smallest), a cluster per instance of a batch.
+//
+// Small LPs are bound by latency: in the other forms every step crosses the
+// whole chip two or three times (kernel boundaries or grid barriers, 1.5 us
+// each) and every gather goes to L2.  Here a step touches no global memory:
+// the block's share of both sides of the matrix stays in shared memory for the
+// whole launch, every block of the cluster holds a copy of x' and y' that it
+// gathers from, owners push their new entries to all copies through
+// distributed shared memory, and the phases are separated by the hardware
+// cluster barrier.  (Gathering from another block's shared memory instead was
+// measured at a quarter of the L2 gather rate; pushing costs one remote store
+// per entry and block and needs no answer.)
+//
+// Arithmetic: each segment is summed by the same lanes in the same order as in
+// the task engine (kBatch FMA chains per lane, the lane group's shuffle tree),
+// and every element update is the same expression, so iterates agree with the
+// other forms up to the order of the compensated norms, whose FP64 totals
+// differ in the last bits at most.
+//
+// What bounds it (cycle counters around each phase, 2,000 x 5,000 LP on 16
+// blocks, 14,100 cycles = 6.8 us per step): the x' phase 1,050, its barrier with
+// the average updates 2,100, A x' 2,200, barrier 1,150, A^T y' 3,250, barrier
+// 1,400, the controller 2,550 (of which one FP64 division 550 and a dozen
+// dependent FP64 operations of 65 each).  The phases are chains of dependent
+// instructions on one or two passes per warp; the entries themselves are a
+// small part.  Measured per step, whole solves: 317 x 803 13.7 -> 5.2 us (1, 2, 4, 8
+// blocks: 8.7, 6.6, 5.2, 5.2), 2,000 x 5,000 13.7 -> 7.4 us (8 blocks: 9.9), 64 of
+// the latter as a batch 84 -> 43 us.
+#include <algorithm>
+#include <cstring>
+
+#include "eval.cuh"
+#include "resident.h"
+
+namespace sihg {
+
+namespace {
+
+constexpr int kResThreads = 1024;  // launch bound of a block (64 registers; 672 threads used at most)
+constexpr int kColWords = 9;       // per column: x (2), K^T y (2), c, l, u, average (2)
+constexpr int kRowWords = 8;       // per row: y (2), K x (2), rl, ru, average (2)
+
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+
+// The cluster barrier in two halves, so that work on a block's own data fits
+// between them.
+__device__ __forceinline__ void cluster_arrive() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Shared-window address of `p` in block `rank` of the cluster.
+__device__ __forceinline__ unsigned map_rank(const void* p, int rank) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+
+__device__ __forceinline__ void st_rank(unsigned addr, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+
+__device__ __forceinline__ void st_rank2(unsigned addr, float a, float b) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(a), "f"(b) : "memory");
+}
+
+// Stores v at *p in every block of the cluster; the lanes of a segment's group
+// share the blocks.
+__device__ __forceinline__ void push(float* p, float v, int sub, int L, int cluster) {
+    if (cluster == 1) {
+        if (sub == 0) *p = v;
+        return;
+    }
+#pragma unroll 4
+    for (int r = sub; r < cluster; r += L) st_rank(map_rank(p, r), v);
+}
+
+// Dot products of one pass: lane (group, sub) sums its entries with `vec`; the
+// sum s + e (e: the compensation) is valid in each group's first lane.  The phases are bound by the latency
+// and the number of these instructions, not by shared-memory bandwidth: two
+// batches of entries are read before the first is summed, and rows past the
+// pass's width add 0 * 0 (a branch over them costs more).
+template <bool COMP>
+__device__ __forceinline__ void pass_sums(const int2* __restrict__ rows, int width, int lg,
+                                          const float* __restrict__ vec, float& s, float& e) {
+    constexpr int kU = 2 * kBatch;
+    float acc[kBatch] = {0.f, 0.f, 0.f, 0.f};
+    s = e = 0.f;
+    const int2* p = rows + (threadIdx.x & 31);
+    for (int k = 0; k < width; k += kU, p += 32 * kU) {
+        int2 w[kU];
+        float g[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) w[u] = k + u < width ? p[32 * u] : make_int2(-1, 0);
+#pragma unroll
+        for (int u = 0; u < kU; ++u) g[u] = w[u].x >= 0 ? vec[w[u].x] : 0.f;
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            if (COMP) {
+                float pr, pe, ss, se;
+                two_prod(__int_as_float(w[u].y), g[u], pr, pe);
+                two_sum(s, pr, ss, se);
+                s = ss;
+                e = __fadd_rn(e, __fadd_rn(pe, se));
+            } else {
+                acc[u % kBatch] = fmaf(__int_as_float(w[u].y), g[u], acc[u % kBatch]);
+            }
+        }
+    }
+    if (!COMP) s = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    // the group's tree (the group's first lane adds as group_sum / group_sum2 do)
+    for (int o = (1 << lg) >> 1; o > 0; o >>= 1) {
+        const float s2 = __shfl_xor_sync(FULL_MASK, s, o);
+        if (COMP) {
+            const float e2 = __shfl_xor_sync(FULL_MASK, e, o);
+            float t, te;
+            two_sum(s, s2, t, te);
+            s = t;
+            e = __fadd_rn(e, __fadd_rn(e2, te));
+        } else {
+            s += s2;
+        }
+    }
+}
+
+// The same rounded to float, in every lane of the group.
+template <bool COMP>
+__device__ __forceinline__ float pass_dot(const int2* __restrict__ rows, int width, int lg,
+                                          const float* __restrict__ vec) {
+    float s, e;
+    pass_sums<COMP>(rows, width, lg, vec, s, e);
+    if (!COMP) return s;
+    return __shfl_sync(FULL_MASK, __fadd_rn(s, e), (threadIdx.x & 31) >> lg << lg);
+}
+
+// What a step needs of the controller's state (FP32), published to the block.
+struct StepPub {
+    int cur, avg, done;
+    float w, tau, sigma;
+};
+
+// One pass as a warp sees it: the segment of this lane's group.
+struct Pass {
+    const int2* rows;
+    int width, lg, sub, seg, local;  // seg: in the instance, local: in the block
+    bool on;                         // the group has a segment
+    __device__ __forceinline__ Pass(const int4& t, const int2* side_rows) {
+        const int lane = threadIdx.x & 31;
+        rows = side_rows + (size_t)t.x * 32;
+        width = t.y & 0xffffff;
+        lg = t.y >> 24;
+        const int g = lane >> lg;
+        sub = lane & ((1 << lg) - 1);
+        seg = t.z + g;
+        local = (t.w & 0xffffff) + g;
+        on = g < (t.w >> 24);
+    }
+};
+
+// Rows: K x' and the dual update (the operations of DualStepEpi::apply).
+template <bool COMP>
+__device__ __forceinline__ void dual_phase(const int4* pass, int passes, const int2* rows, float* R, int nl, int cur,
+                                           const float* xs, float* ys, float sigma, int cluster, Acc& dy2) {
+    const int nw = (blockDim.x >> 5) - 1;
+    for (int p = threadIdx.x >> 5; p < passes; p += nw) {
+        const Pass t(pass[p], rows);
+        const float kxp = pass_dot<COMP>(t.rows, t.width, t.lg, xs);
+        if (t.on) {
+            const float* r = R + t.local;
+            const float yo = r[cur * nl], kx = r[(2 + cur) * nl], rl = r[4 * nl], ru = r[5 * nl];
+            const float wv = (2.0f * kxp - kx) + yo / sigma;
+            const float yv = sigma * (wv - fminf(fmaxf(wv, rl), ru));
+            push(ys + t.seg, yv, t.sub, 1 << t.lg, cluster);
+            if (t.sub == 0) {
+                R[(2 + (cur ^ 1)) * nl + t.local] = kxp;
+                R[(cur ^ 1) * nl + t.local] = yv;
+                const float dy = yv - yo;
+                dy2.add(dy * dy);
+            }
+        }
+    }
+}
+
+// Columns: K^T y', interaction and movement (the operations of KtyStepEpi::apply).
+template <bool COMP>
+__device__ __forceinline__ void kty_phase(const int4* pass, int passes, const int2* rows, float* C, int nl, int cur,
+                                          const float* ys, Acc& inter, Acc& dx2) {
+    const int nw = (blockDim.x >> 5) - 1;
+    for (int p = threadIdx.x >> 5; p < passes; p += nw) {
+        const Pass t(pass[p], rows);
+        const float k = pass_dot<COMP>(t.rows, t.width, t.lg, ys);
+        if (t.on && t.sub == 0) {
+            const float* c = C + t.local;
+            const float dx = c[(cur ^ 1) * nl] - c[cur * nl];
+            C[(2 + (cur ^ 1)) * nl + t.local] = k;
+            inter.add(dx * (k - c[(2 + cur) * nl]));
+            dx2.add(dx * dx);
+        }
+    }
+}
+
+// Sums a, b and c over the warp: a and b share one butterfly (the halves of
+// the warp swap first: the lower lanes end with the total of a, the upper ones
+// with that of b, both in `a`), c has its own beside it.
+__device__ __forceinline__ void warp_reduce_three(Acc& a, Acc& b, Acc& c) {
+    const bool up = (threadIdx.x & 16) != 0;
+    Acc keep = up ? b : a, give = up ? a : b, got;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        got.s = __shfl_xor_sync(FULL_MASK, o == 16 ? give.s : keep.s, o);
+        got.c = __shfl_xor_sync(FULL_MASK, o == 16 ? give.c : keep.c, o);
+        keep = acc_plus(keep, got);
+        got.s = __shfl_xor_sync(FULL_MASK, c.s, o);
+        got.c = __shfl_xor_sync(FULL_MASK, c.c, o);
+        c = acc_plus(c, got);
+    }
+    a = keep;
+}
+
+// The partial sums {inter, |dx|^2, |dy|^2} of a warp or a block.
+struct Sums {
+    float2 inter, dx2, dy2;
+};
+
+// Loads n (at most 32) of them, one per lane, and sums them over the warp (as
+// warp_reduce_three).
+__device__ __forceinline__ void reduce_sums(const Sums* p, int n, Acc& a, Acc& c) {
+    const int lane = threadIdx.x & 31;
+    Acc b;
+    a.reset();
+    c.reset();
+    if (lane < n) {
+        a.s = p[lane].inter.x;
+        a.c = p[lane].inter.y;
+        b.s = p[lane].dx2.x;
+        b.c = p[lane].dx2.y;
+        c.s = p[lane].dy2.x;
+        c.c = p[lane].dy2.y;
+    }
+    warp_reduce_three(a, b, c);
+}
+constexpr int kEvalQ = 18;  // reductions of an evaluation: 8 of the rows, 10 of the columns
+
+// Sums of a side's segments with the first candidate point, to s and e by local segment.
+__device__ __forceinline__ void eval_sums(bool comp, const int4* pass, int passes, const int2* rows, const float* vec,
+                                          float* s_out, float* e_out) {
+    const int nw = (blockDim.x >> 5) - 1;
+    for (int p = threadIdx.x >> 5; p < passes; p += nw) {
+        const Pass t(pass[p], rows);
+        float s, e;
+        if (comp)
+            pass_sums<true>(t.rows, t.width, t.lg, vec, s, e);
+        else
+            pass_sums<false>(t.rows, t.width, t.lg, vec, s, e);
+        if (t.on && t.sub == 0) {
+            s_out[t.local] = s;
+            e_out[t.local] = e;
+        }
+    }
+}
+
+// The evaluation epilogue of a side's segments: first candidate's sums from s
+// and e, the second's from `vec`; `first` is the instance's first segment.
+template <class Epi>
+__device__ __forceinline__ void eval_apply(bool comp, const int4* pass, int passes, const int2* rows, const float* vec,
+                                           const float* s_in, const float* e_in, int first, Epi& epi) {
+    const int nw = (blockDim.x >> 5) - 1;
+    for (int p = threadIdx.x >> 5; p < passes; p += nw) {
+        const Pass t(pass[p], rows);
+        SegDot<2> d;
+        if (comp)
+            pass_sums<true>(t.rows, t.width, t.lg, vec, d.s[1], d.e[1]);
+        else
+            pass_sums<false>(t.rows, t.width, t.lg, vec, d.s[1], d.e[1]);
+        if (t.on && t.sub == 0) {
+            d.s[0] = s_in[t.local];
+            d.e[0] = e_in[t.local];
+            epi.apply(first + t.seg, d, epi.pre(first + t.seg));
+        }
+    }
+}
+
+// Total of n (at most 32) partials of reduction i, in every lane.
+__device__ __forceinline__ Acc eval_total(const float2* p, int n, int i) {
+    const int lane = threadIdx.x & 31;
+    Acc v[1];
+    if (lane < n) {
+        v[0].s = p[lane].x;
+        v[0].c = p[lane].y;
+    }
+    const bool is_max = i == 2 || i == 3 || i == 10 || i == 11;
+    warp_reduce_acc<1>(v, is_max ? 1u : 0u);
+    return v[0];
+}
+
+}  // namespace
+
+// Blocks: all warps but the last own passes; the last warp runs the step
+// controller (every block its own copy, from the same partials, so that no
+// answer has to come back).
+__global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, int nsteps, int periods, Vecs V, Inst* st, unsigned* done_count) {
+    extern __shared__ char sm[];
+    __shared__ Inst S;  // the controller's copy (its first lane's)
+    __shared__ StepPub pub;
+    __shared__ int flag;
+    __shared__ unsigned ignored;  // done count of the other blocks' controller copies
+    const int inst = blockIdx.x / A.cluster, cluster = A.cluster;
+    if (st[inst].done) return;  // the whole cluster
+    const int rank = cluster > 1 ? (int)cluster_rank() : 0;
+    const ResBlock& blk = A.blocks[blockIdx.x];
+    const int4 io = A.inst[inst];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x >> 5) - 1;
+    const bool ctrl = warp == nw;
+    int4* rpass = reinterpret_cast<int4*>(sm + A.sm.pass[0]);
+    int4* cpass = reinterpret_cast<int4*>(sm + A.sm.pass[1]);
+    int2* rrows = reinterpret_cast<int2*>(sm + A.sm.rows[0]);
+    int2* crows = reinterpret_cast<int2*>(sm + A.sm.rows[1]);
+    float* xs = reinterpret_cast<float*>(sm + A.sm.xs);
+    float* ys = reinterpret_cast<float*>(sm + A.sm.ys);
+    float* C = reinterpret_cast<float*>(sm + A.sm.col);  // x x' | K^T y K^T y' | c l u | average hi lo
+    float* R = reinterpret_cast<float*>(sm + A.sm.row);  // y y' | K x K x' | rl ru | average hi lo
+    Sums* wsum = reinterpret_cast<Sums*>(sm + A.sm.red);  // of every warp of this block
+    Sums* bsum = wsum + 32;                               // of every block of the cluster
+    const int ncl = A.sm.locals[1], nrl = A.sm.locals[0];
+    const int rp = blk.side[0].passes, cp = blk.side[1].passes;
+    for (int k = threadIdx.x; k < rp; k += blockDim.x) rpass[k] = A.passes[blk.side[0].pass_begin + k];
+    for (int k = threadIdx.x; k < cp; k += blockDim.x) cpass[k] = A.passes[blk.side[1].pass_begin + k];
+    for (int h = 0; h < 2; ++h) {
+        const int4* src = reinterpret_cast<const int4*>(A.rows + (size_t)blk.side[h].row_begin * 32);
+        int4* dst = reinterpret_cast<int4*>(h ? crows : rrows);
+        for (int k = threadIdx.x; k < blk.side[h].rows * 16; k += blockDim.x) dst[k] = __ldg(src + k);
+    }
+    if (threadIdx.x == 0) {
+        S = st[inst];
+        const StepScalars sc = step_scalars(S);
+        pub = StepPub{sc.cur, sc.avg, 0, sc.w, sc.tau, (float)(S.eta * S.omega)};
+    }
+    __syncthreads();
+    if (!ctrl) {  // owners' data
+        const int cur = pub.cur;
+        for (int p = warp; p < cp; p += nw) {
+            const Pass t(cpass[p], crows);
+            if (t.on && t.sub == 0) {
+                const int j = io.x + t.seg;
+                float* c = C + t.local;
+                c[cur * ncl] = pick(V.x0, V.x1, cur)[j];
+                c[(2 + cur) * ncl] = pick(V.kty0, V.kty1, cur)[j];
+                c[4 * ncl] = V.c[j];
+                c[5 * ncl] = V.l[j];
+                c[6 * ncl] = V.u[j];
+                const float2 a = V.x_acc[j];
+                c[7 * ncl] = a.x;
+                c[8 * ncl] = a.y;
+            }
+        }
+        for (int p = warp; p < rp; p += nw) {
+            const Pass t(rpass[p], rrows);
+            if (t.on && t.sub == 0) {
+                const int j = io.z + t.seg;
+                float* r = R + t.local;
+                r[cur * nrl] = pick(V.y0, V.y1, cur)[j];
+                r[(2 + cur) * nrl] = pick(V.kx0, V.kx1, cur)[j];
+                r[4 * nrl] = V.rl[j];
+                r[5 * nrl] = V.ru[j];
+                const float2 a = V.y_acc[j];
+                r[6 * nrl] = a.x;
+                r[7 * nrl] = a.y;
+            }
+        }
+    }
+    cluster_arrive();  // every block of the cluster runs before the first remote store
+    cluster_wait();
+    for (int period = 0; period < periods && !pub.done; ++period) {
+    const bool comp = S.refine != 0;
+    for (int k = 0; k < nsteps && !pub.done; ++k) {
+        const int cur = pub.cur;
+        const bool avg = pub.avg != 0;
+        const float w = pub.w, tau = pub.tau, sg = pub.sigma;
+        // x' = clip(x - tau (c + K^T y), l, u)
+        if (!ctrl) {
+            for (int p = warp; p < cp; p += nw) {
+                const Pass t(cpass[p], crows);
+                if (t.on) {
+                    const float* c = C + t.local;
+                    const float v = fmaf(-tau, c[4 * ncl] + c[(2 + cur) * ncl], c[cur * ncl]);
+                    const float xp = fminf(fmaxf(v, c[5 * ncl]), c[6 * ncl]);
+                    if (t.sub == 0) C[(cur ^ 1) * ncl + t.local] = xp;
+                    push(xs + t.seg, xp, t.sub, 1 << t.lg, cluster);
+                }
+            }
+        }
+        cluster_arrive();
+        if (ctrl) {
+            if (lane == 0) schedule_pows(S, V);
+        } else if (avg) {  // the pending average updates, while the other blocks arrive
+            for (int k2 = threadIdx.x; k2 < blk.side[1].locals; k2 += nw * 32) {
+                const float2 a = ff_axpy(make_float2(C[7 * ncl + k2], C[8 * ncl + k2]), w, C[cur * ncl + k2]);
+                C[7 * ncl + k2] = a.x;
+                C[8 * ncl + k2] = a.y;
+            }
+            for (int k2 = threadIdx.x; k2 < blk.side[0].locals; k2 += nw * 32) {
+                const float2 a = ff_axpy(make_float2(R[6 * nrl + k2], R[7 * nrl + k2]), w, R[cur * nrl + k2]);
+                R[6 * nrl + k2] = a.x;
+                R[7 * nrl + k2] = a.y;
+            }
+        }
+        cluster_wait();
+        Acc dy2;
+        if (!ctrl) {
+            if (comp)
+                dual_phase<true>(rpass, rp, rrows, R, nrl, cur, xs, ys, sg, cluster, dy2);
+            else
+                dual_phase<false>(rpass, rp, rrows, R, nrl, cur, xs, ys, sg, cluster, dy2);
+        }
+        cluster_arrive();
+        cluster_wait();
+        // Everything of the controller that does not need this phase's sums
+        // runs beside it, and what is left after it is one chain of FP64
+        // operations, which are slow here (65 cycles an addition or
+        // multiplication, 550 a division): a lane each for eta_bar, the next
+        // eta and its tau and sigma, one division for all of them.
+        double coef = 1.0, grow = 0.0, om = 0.0, inv_om = 0.0, eta = 0.0, W1 = 0.0, avg_w = 0.0, total_dy2 = 0.0;
+        bool nan = false, accept = false;
+        if (!ctrl) {
+            Acc inter, dx2;
+            if (comp)
+                kty_phase<true>(cpass, cp, crows, C, ncl, cur, ys, inter, dx2);
+            else
+                kty_phase<false>(cpass, cp, crows, C, ncl, cur, ys, inter, dx2);
+            warp_reduce_three(inter, dx2, dy2);  // inter: |dx|^2 in the upper lanes
+            if (lane == 0) {
+                wsum[warp].inter = make_float2(inter.s, inter.c);
+                wsum[warp].dy2 = make_float2(dy2.s, dy2.c);
+            }
+            if (lane == 16) wsum[warp].dx2 = make_float2(inter.s, inter.c);
+        } else {
+            om = S.omega;
+            eta = S.eta;
+            W1 = S.W + eta;
+            const double quot = (lane == 1 ? eta : 1.0) / (lane == 1 ? W1 : om);
+            inv_om = __shfl_sync(FULL_MASK, quot, 0);
+            avg_w = __shfl_sync(FULL_MASK, quot, 1);
+            const double per = lane == 2 ? inv_om : (lane == 3 ? om : 1.0);
+            grow = (1.0 + S.pow06) * eta * per;
+            coef = lane == 0 ? 1.0 : (1.0 - S.pow03) * per;
+        }
+        __syncthreads();
+        if (ctrl) {  // the block's sums to every block: lane r (inter, |dy|^2) and 16 + r (|dx|^2) to block r
+            Acc a, c;
+            reduce_sums(wsum, nw, a, c);
+            if ((lane & 15) < cluster) {
+                st_rank2(map_rank(lane < 16 ? &bsum[rank].inter : &bsum[rank].dx2, lane & 15), a.s, a.c);
+                if (lane < 16) st_rank2(map_rank(&bsum[rank].dy2, lane), c.s, c.c);
+            }
+        }
+        cluster_arrive();
+        cluster_wait();
+        if (ctrl) {
+            Acc two, d[1];
+            reduce_sums(bsum, cluster, two, d[0]);
+            const double mine = (double)two.s + (double)two.c, dy2 = (double)d[0].s + (double)d[0].c;
+            const double inter = __shfl_sync(FULL_MASK, mine, 0), dx2 = __shfl_sync(FULL_MASK, mine, 16);
+            // step_controller: lane 0 eta_bar, lane 1 (1 - k^-0.3) eta_bar, lanes
+            // 2 and 3 the same / and * omega.  Non-negative FP64 numbers compare
+            // as integers (FP64 compares have the latency of FP64 sums); a NaN
+            // compares above infinity.
+            const double movement = om * dx2 + dy2 * inv_om;
+            const double ai = fabs(inter);
+            const double quot = __double_as_longlong(ai) != 0 ? coef * movement / (2.0 * ai) : INFINITY;
+            const long long qb = __double_as_longlong(quot), inf = 0x7ff0000000000000ll;
+            const bool less = __shfl_sync(FULL_MASK, (int)(qb < __double_as_longlong(grow)), 1) != 0;
+            const double next = less ? quot : grow;
+            nan = __double_as_longlong(fabs(movement)) > inf || __double_as_longlong(ai) > inf;
+            accept = !nan && __double_as_longlong(eta) <= qb && qb <= inf;  // lane 0
+            if (nan) {
+                if (lane == 0) pub.done = 3;
+            } else {
+                if (lane == 2) pub.tau = (float)next;
+                if (lane == 3) pub.sigma = (float)next;
+                if (lane == 0) {
+                    pub.avg = accept;
+                    if (accept) {
+                        pub.cur = cur ^ 1;
+                        pub.w = (float)avg_w;
+                    }
+                }
+                eta = __shfl_sync(FULL_MASK, next, 1);
+            }
+            total_dy2 = dy2;
+        }
+        __syncthreads();
+        if (ctrl && lane == 0) {  // the instance's counters, beside the next phase
+            S.attempts += 1;
+            if (nan) {
+                S.done = 3;
+            } else {
+                S.dy2 = total_dy2;
+                S.eta = eta;
+                S.avg_pending = accept;
+                if (accept) {
+                    S.cur ^= 1;
+                    S.steps += 1;
+                    S.since_restart += 1;
+                    S.W = W1;
+                    S.avg_w = avg_w;
+                } else {
+                    S.rejections += 1;
+                }
+            }
+        }
+    }
+    // The evaluation (as k_flush_avg, k_eval_rows, k_eval_cols and k_restart):
+    // the copies hold the current point, then the average one; the epilogues
+    // read their segments' data from global memory, where the owners put the
+    // current point first.
+    const int cur = pub.cur;
+    const bool avg = pub.avg != 0;
+    const bool failed = pub.done != 0;  // a step of this period: nothing to evaluate, and no store to a block that may have ended
+    const float w = pub.w;
+    if (!ctrl) {
+        for (int p = warp; p < cp; p += nw) {
+            const Pass t(cpass[p], crows);
+            if (t.on) {
+                const int j = io.x + t.seg;
+                float* c = C + t.local;
+                const float x = c[cur * ncl];
+                if (!failed) push(xs + t.seg, x, t.sub, 1 << t.lg, cluster);
+                if (t.sub == 0) {
+                    float2 a = make_float2(c[7 * ncl], c[8 * ncl]);
+                    if (avg) a = ff_axpy(a, w, x);
+                    c[7 * ncl] = a.x;
+                    c[8 * ncl] = a.y;
+                    pick(V.x0, V.x1, cur)[j] = x;
+                    pick(V.kty0, V.kty1, cur)[j] = c[(2 + cur) * ncl];
+                    V.x_acc[j] = a;
+                    V.x_avg[j] = __fadd_rn(a.x, a.y);
+                }
+            }
+        }
+        for (int p = warp; p < rp; p += nw) {
+            const Pass t(rpass[p], rrows);
+            if (t.on) {
+                const int j = io.z + t.seg;
+                float* r = R + t.local;
+                const float y = r[cur * nrl];
+                if (!failed) push(ys + t.seg, y, t.sub, 1 << t.lg, cluster);
+                if (t.sub == 0) {
+                    float2 a = make_float2(r[6 * nrl], r[7 * nrl]);
+                    if (avg) a = ff_axpy(a, w, y);
+                    r[6 * nrl] = a.x;
+                    r[7 * nrl] = a.y;
+                    pick(V.y0, V.y1, cur)[j] = y;
+                    pick(V.kx0, V.kx1, cur)[j] = r[(2 + cur) * nrl];
+                    V.y_acc[j] = a;
+                    V.y_avg[j] = __fadd_rn(a.x, a.y);
+                }
+            }
+        }
+    }
+    if (failed) {
+        if (rank == 0 && ctrl && lane == 0) st[inst] = S;
+        return;
+    }
+    cluster_arrive();
+    cluster_wait();
+    if (!ctrl) {  // the current point's sums, kept where the candidate point was
+        eval_sums(comp, rpass, rp, rrows, xs, R + (cur ^ 1) * nrl, R + (2 + (cur ^ 1)) * nrl);
+        eval_sums(comp, cpass, cp, crows, ys, C + (cur ^ 1) * ncl, C + (2 + (cur ^ 1)) * ncl);
+    }
+    cluster_arrive();
+    cluster_wait();
+    if (!ctrl) {
+        for (int p = warp; p < cp; p += nw) {
+            const Pass t(cpass[p], crows);
+            if (t.on)
+                push(xs + t.seg, __fadd_rn(C[7 * ncl + t.local], C[8 * ncl + t.local]), t.sub, 1 << t.lg, cluster);
+        }
+        for (int p = warp; p < rp; p += nw) {
+            const Pass t(rpass[p], rrows);
+            if (t.on)
+                push(ys + t.seg, __fadd_rn(R[6 * nrl + t.local], R[7 * nrl + t.local]), t.sub, 1 << t.lg, cluster);
+        }
+    }
+    cluster_arrive();
+    cluster_wait();
+    float2* ewarp = reinterpret_cast<float2*>(sm + A.sm.eval);  // [kEvalQ][32] of the block's warps
+    float2* eblock = ewarp + kEvalQ * 32;                       // [kEvalQ][16] of the cluster's blocks
+    double* etot = reinterpret_cast<double*>(eblock + kEvalQ * 16);
+    if (!ctrl) {
+        EvalRowsEpi er{V};
+        er.begin(S);
+        Acc q[8];
+        eval_apply(comp, rpass, rp, rrows, xs, R + (cur ^ 1) * nrl, R + (2 + (cur ^ 1)) * nrl, io.z, er);
+        er.values(q);
+        warp_reduce_acc<8>(q, 0x0Cu);
+        if (lane == 0)
+            for (int i = 0; i < 8; ++i) ewarp[i * 32 + warp] = make_float2(q[i].s, q[i].c);
+    }
+    if (!ctrl) {
+        EvalColsEpi ec{V, nullptr};
+        ec.begin(S);
+        Acc q[10];
+        eval_apply(comp, cpass, cp, crows, ys, C + (cur ^ 1) * ncl, C + (2 + (cur ^ 1)) * ncl, io.x, ec);
+        ec.values(q);
+        warp_reduce_acc<10>(q, 0x0Cu);
+        if (lane == 0)
+            for (int i = 0; i < 10; ++i) ewarp[(8 + i) * 32 + warp] = make_float2(q[i].s, q[i].c);
+    }
+    __syncthreads();
+    for (int i = warp; i < kEvalQ; i += nw + 1) {
+        const Acc v = eval_total(ewarp + i * 32, nw, i);
+        if (lane < cluster) st_rank2(map_rank(eblock + i * 16 + rank, lane), v.s, v.c);
+    }
+    cluster_arrive();
+    cluster_wait();
+    for (int i = warp; i < kEvalQ; i += nw + 1) {
+        const Acc v = eval_total(eblock + i * 16, cluster, i);
+        if (lane == 0) etot[i] = (double)v.s + (double)v.c;
+    }
+    __syncthreads();
+    if (ctrl && lane == 0) {
+        for (int i = 0; i < 8; ++i) S.row_eval[i] = etot[i];
+        S.col_eval_dist[0] = etot[16];
+        S.col_eval_dist[1] = etot[17];
+        eval_controller(S, etot + 8, rank == 0 ? done_count : &ignored);
+        const StepScalars sc = step_scalars(S);
+        pub = StepPub{sc.cur, 0, S.done, sc.w, sc.tau, (float)(S.eta * S.omega)};
+        flag = S.restart_flag;
+    }
+    __syncthreads();
+    if (!ctrl && flag != 0) {  // restart at the current (1) or the average point (2)
+        for (int p = warp; p < cp; p += nw) {
+            const Pass t(cpass[p], crows);
+            if (t.on && t.sub == 0) {
+                const int j = io.x + t.seg;
+                float* c = C + t.local;
+                if (flag == 2) {
+                    pick(V.x0, V.x1, cur)[j] = c[cur * ncl] = V.x_avg[j];
+                    pick(V.kty0, V.kty1, cur)[j] = c[(2 + cur) * ncl] = V.kty_eval[j];
+                }
+                const float x = c[cur * ncl];
+                V.x_last[j] = x;
+                V.x_acc[j] = make_float2(x, 0.f);
+                c[7 * ncl] = x;
+                c[8 * ncl] = 0.f;
+            }
+        }
+        for (int p = warp; p < rp; p += nw) {
+            const Pass t(rpass[p], rrows);
+            if (t.on && t.sub == 0) {
+                const int j = io.z + t.seg;
+                float* r = R + t.local;
+                if (flag == 2) {
+                    pick(V.y0, V.y1, cur)[j] = r[cur * nrl] = V.y_avg[j];
+                    pick(V.kx0, V.kx1, cur)[j] = r[(2 + cur) * nrl] = V.kx_eval[j];
+                }
+                const float y = r[cur * nrl];
+                V.y_last[j] = y;
+                V.y_acc[j] = make_float2(y, 0.f);
+                r[6 * nrl] = y;
+                r[7 * nrl] = 0.f;
+            }
+        }
+    }
+    }
+    if (rank == 0 && ctrl && lane == 0) st[inst] = S;
+}
+
+namespace {
+
+// Entries of every pass from the (renumbered, scaled) matrix: a warp per pass.
+__global__ void k_resident_fill(int npass, const int4* __restrict__ place, SegMatrix R, SegMatrix C,
+                                int2* __restrict__ rows) {
+    // place: {first row of entries, width | log2 L << 24 | side << 30, first segment in the batch | -, segments | -},
+    // followed by the other side's first index in the next int4
+    const int lane = threadIdx.x & 31;
+    const int nw = gridDim.x * (blockDim.x >> 5);
+    for (int p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); p < npass; p += nw) {
+        const int4 t = place[2 * p];
+        const int4 o = place[2 * p + 1];
+        const SegMatrix& A = o.y ? C : R;
+        const int L = o.z, sub = lane & (L - 1), g = lane / L;
+        int k = 0, e = 0;
+        if (g < t.w) {
+            k = A.ptr[t.z + g] + sub;
+            e = A.ptr[t.z + g + 1];
+        }
+        for (int r = 0; r < t.y; ++r, k += L) {
+            int2 v = make_int2(-1, 0);
+            if (k < e) {
+                v = A.pairs[k];
+                v.x -= o.x;
+            }
+            rows[((size_t)t.x + r) * 32 + lane] = v;
+        }
+    }
+}
+
+int align16(int v) { return (v + 15) & ~15; }
+
+}  // namespace
+
+void ResidentPlan::release() {
+    ready_ = false;
+    tab_.release();
+    rows_.release();
+}
+
+int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>& csc_ptr, const std::vector<int>& roff,
+                        const std::vector<int>& coff, const std::vector<uint8_t>& row_lanes,
+                        const std::vector<uint8_t>& col_lanes, int sm_count, cudaStream_t s) {
+    release();
+    const int B = (int)roff.size() - 1;
+    instances_ = B;
+    int dev = 0, optin = 0;
+    SIHG_CUDA(cudaGetDevice(&dev));
+    SIHG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    cudaFuncAttributes fa{};
+    SIHG_CUDA(cudaFuncGetAttributes(&fa, k_resident_steps));
+    const int budget = optin - (int)fa.sharedSizeBytes;
+    const std::vector<int>* ptrs[2] = {&csr_ptr, &csc_ptr};
+    const std::vector<int>* offs[2] = {&roff, &coff};
+    const std::vector<uint8_t>* lanes[2] = {&row_lanes, &col_lanes};
+    // the smallest instance bound: both copies and both sides of the matrix
+    // over 16 blocks must fit; most batches end here
+    for (int b = 0; b < B; ++b) {
+        const double nnz = csr_ptr[roff[b + 1]] - csr_ptr[roff[b]], m = roff[b + 1] - roff[b], n = coff[b + 1] - coff[b];
+        if (4.0 * (m + n) + (16.0 * nnz + 4.0 * (kColWords * n + kRowWords * m)) / 16.0 > budget) return SIH_PDHG_OK;
+    }
+    std::vector<ResBlock> blocks;
+    std::vector<int4> passes, place, inst(B);
+    for (int b = 0; b < B; ++b) inst[b] = make_int4(coff[b], coff[b + 1] - coff[b], roff[b], roff[b + 1] - roff[b]);
+    ResSmem sm{};
+    auto plan = [&](int C, int& most) -> long long {  // rows of entries; `most`: passes of a block
+        blocks.assign((size_t)B * C, ResBlock{});
+        passes.clear();
+        place.clear();
+        long long row = 0;
+        int mrows[2] = {0, 0}, mpass[2] = {0, 0}, mloc[2] = {0, 0}, mn = 0, mm = 0;
+        for (int b = 0; b < B; ++b) {
+            mn = std::max(mn, inst[b].y);
+            mm = std::max(mm, inst[b].w);
+            for (int h = 0; h < 2; ++h) {
+                const std::vector<int>& ptr = *ptrs[h];
+                const int s0 = (*offs[h])[b], s1 = (*offs[h])[b + 1];
+                const int other = (*offs[1 - h])[b];
+                std::vector<std::vector<int4>> mine(C), where(C);
+                std::vector<int> nrow(C, 0), nloc(C, 0);
+                int turn = 0;
+                for (int seg = s0; seg < s1; ++turn) {
+                    const int L = (*lanes[h])[seg];
+                    int e = seg, width = 0, lg = 0;
+                    while ((1 << lg) < L) ++lg;
+                    while (e < s1 && e - seg < 32 / L && (*lanes[h])[e] == L) {
+                        width = std::max(width, (ptr[e + 1] - ptr[e] + L - 1) / L);
+                        ++e;
+                    }
+                    // the passes run by descending length: dealt out back and forth
+                    const int q = turn % (2 * C), r = q < C ? q : 2 * C - 1 - q;
+                    mine[r].push_back(make_int4(nrow[r], width | (lg << 24), seg - s0, nloc[r] | ((e - seg) << 24)));
+                    where[r].push_back(make_int4(nrow[r], width, seg, e - seg));
+                    where[r].push_back(make_int4(other, h, L, 0));
+                    nrow[r] += width;
+                    nloc[r] += e - seg;
+                    seg = e;
+                }
+                for (int r = 0; r < C; ++r) {
+                    ResSide& sd = blocks[(size_t)b * C + r].side[h];
+                    sd = ResSide{(int)passes.size(), (int)mine[r].size(), (int)row, nrow[r], nloc[r]};
+                    for (size_t k = 0; k < where[r].size(); k += 2) where[r][k].x += (int)row;
+                    passes.insert(passes.end(), mine[r].begin(), mine[r].end());
+                    place.insert(place.end(), where[r].begin(), where[r].end());
+                    row += nrow[r];
+                    mrows[h] = std::max(mrows[h], nrow[r]);
+                    mpass[h] = std::max(mpass[h], sd.passes);
+                    mloc[h] = std::max(mloc[h], nloc[r]);
+                }
+            }
+        }
+        most = std::max(mpass[0], mpass[1]);
+        long long at = 0;
+        auto put = [&](long long bytes) {
+            const long long a = at;
+            at = (at + bytes + 15) & ~15ll;
+            return (int)std::min<long long>(a, INT32_MAX);
+        };
+        for (int h = 0; h < 2; ++h) sm.rows[h] = put(256ll * mrows[h]);
+        for (int h = 0; h < 2; ++h) sm.pass[h] = put(16ll * mpass[h]);
+        sm.xs = put(4ll * mn);
+        sm.ys = put(4ll * mm);
+        sm.locals[0] = mloc[0];
+        sm.locals[1] = mloc[1];
+        sm.col = put(4ll * kColWords * mloc[1]);
+        sm.row = put(4ll * kRowWords * mloc[0]);
+        sm.red = put((long long)sizeof(Sums) * (32 + 16));
+        sm.eval = put(kEvalQ * (8ll * 32 + 8ll * 16 + 8));
+        sm.total = (int)std::min<long long>(at, INT32_MAX);
+        return row;
+    };
+    // The smallest cluster that holds an instance; a larger one while SMs are
+    // left over and a block has more than 8 passes a side (two warps per
+    // scheduler): beyond that the barriers and pushes of more blocks cost what
+    // the shorter phases save (317 x 803: 4 blocks of 9 passes and 8 of 5 are
+    // equal).
+    int C = 1, most = 0;
+    long long rows = plan(C, most);
+    while (C < 16 && sm.total > budget) rows = plan(C *= 2, most);
+    if (sm.total > budget) return SIH_PDHG_OK;
+    while (C < 16 && (long long)B * 2 * C <= sm_count && most > 8) rows = plan(C *= 2, most);
+    // 20 warps with passes at most (31: 3 % slower on the batch of 64, whose blocks have 39 passes)
+    const int nw = std::max(1, std::min(20, most));
+    threads_ = 32 * (nw + 1);
+    npass_ = (int)passes.size();
+    SIHG_CUDA(cudaFuncSetAttribute(k_resident_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
+    SIHG_CUDA(cudaFuncSetAttribute(k_resident_steps, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    if (C > 1) {
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim = {(unsigned)C, 1, 1};
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)(B * C));
+        cfg.blockDim = dim3((unsigned)threads_);
+        cfg.dynamicSmemBytes = (size_t)sm.total;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, k_resident_steps, &cfg) != cudaSuccess || clusters < 1) {
+            (void)cudaGetLastError();
+            return SIH_PDHG_OK;
+        }
+    }
+    const size_t nb = sizeof(ResBlock) * blocks.size(), ni = sizeof(int4) * inst.size(),
+                 np = sizeof(int4) * passes.size(), nl = sizeof(int4) * place.size();
+    const size_t o_i = align16((int)nb), o_p = o_i + ni, o_l = o_p + np;
+    std::vector<char> buf(o_l + nl);
+    std::memcpy(buf.data(), blocks.data(), nb);
+    std::memcpy(buf.data() + o_i, inst.data(), ni);
+    std::memcpy(buf.data() + o_p, passes.data(), np);
+    std::memcpy(buf.data() + o_l, place.data(), nl);
+    SIHG_TRY(tab_.alloc(buf.size()));
+    SIHG_CUDA(cudaMemcpyAsync(tab_.as<void>(), buf.data(), buf.size(), cudaMemcpyHostToDevice, s));
+    SIHG_TRY(rows_.alloc(256 * (size_t)std::max<long long>(1, rows)));
+    char* d = tab_.as<char>();
+    args_ = ResArgs{(const ResBlock*)d, (const int4*)(d + o_i), (const int4*)(d + o_p), rows_.as<int2>(), sm, C};
+    ready_ = true;
+    return SIH_PDHG_OK;
+}
+
+int ResidentPlan::fill(const SegMatrix& rows_A, const SegMatrix& cols_A, cudaStream_t s) {
+    const int4* place = args_.passes + npass_;
+    k_resident_fill<<<std::max(1, std::min(1216, (npass_ + 7) / 8)), 256, 0, s>>>(npass_, place, rows_A, cols_A,
+                                                                                rows_.as<int2>());
+    SIHG_LAUNCH_CHECK();
+    return SIH_PDHG_OK;
+}
+
+int ResidentPlan::launch(int nsteps, int periods, const Vecs& V, Inst* st, unsigned* done_count,
+                         cudaStream_t s) const {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {(unsigned)args_.cluster, 1, 1};
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(instances_ * args_.cluster));
+    cfg.blockDim = dim3((unsigned)threads_);
+    cfg.dynamicSmemBytes = (size_t)args_.sm.total;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    SIHG_CUDA(cudaLaunchKernelEx(&cfg, k_resident_steps, args_, nsteps, periods, V, st, done_count));
+    return SIH_PDHG_OK;
+}
+
+}  // namespace sihg

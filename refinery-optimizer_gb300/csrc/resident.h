@@ -1,0 +1,62 @@
+// Resident step form: LPs whose matrix fits in the shared memory of one
+// thread-block cluster (see resident.cu).
+#pragma once
+
+#include <vector>
+
+#include "mixed.h"
+
+namespace sihg {
+
+// Passes of one side held by one block (32 / L segments of L lanes each) and
+// where its share of the layout lies.
+struct ResSide {
+    int pass_begin, passes;  // in the pass table
+    int row_begin, rows;     // rows of 32 entries
+    int locals;              // segments of the side this block owns
+};
+
+struct ResBlock {
+    ResSide side[2];  // 0 rows of A (A x), 1 columns (A^T y)
+};
+
+// Where a block keeps what, in bytes of dynamic shared memory; the same in
+// every block of a launch.
+struct ResSmem {
+    int pass[2], rows[2], xs, ys, col, row, red, eval, locals[2], total;
+};
+
+struct ResArgs {
+    const ResBlock* blocks;  // [instances x cluster]
+    const int4* inst;        // {first column, columns, first row, rows} of each instance
+    // pass: {first row of entries in its block, width | log2 L << 24, first
+    // segment in the instance, first local segment | segments << 24}
+    const int4* passes;
+    const int2* rows;        // entries {index in the instance, value}; empty {-1, 0}
+    ResSmem sm;
+    int cluster;
+};
+
+class ResidentPlan {
+  public:
+    // Plans the form for these instances (segment pointers of the batch, lanes
+    // per segment of both sides); ready() says whether they fit.
+    int build(const std::vector<int>& csr_ptr, const std::vector<int>& csc_ptr, const std::vector<int>& roff,
+              const std::vector<int>& coff, const std::vector<uint8_t>& row_lanes,
+              const std::vector<uint8_t>& col_lanes, int sm_count, cudaStream_t s);
+    // Copies the scaled entries into the layout.
+    int fill(const SegMatrix& rows_A, const SegMatrix& cols_A, cudaStream_t s);
+    // `periods` times nsteps steps and an evaluation of every running instance.
+    int launch(int nsteps, int periods, const Vecs& V, Inst* st, unsigned* done_count, cudaStream_t s) const;
+    bool ready() const { return ready_; }
+    int grid() const { return args_.cluster * instances_; }
+    void release();
+
+  private:
+    bool ready_ = false;
+    int instances_ = 0, threads_ = 0, npass_ = 0;
+    ResArgs args_{};
+    DevMem tab_, rows_;
+};
+
+}  // namespace sihg

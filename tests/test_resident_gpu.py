@@ -1,0 +1,107 @@
+"""Resident step form (csrc/resident.cu): LPs whose matrix, vectors and state
+fit in the shared memory of one thread-block cluster.
+
+The form does the operations of the other forms on every segment and element;
+only the compensated norms are added in another order, with FP64 totals that
+differ in the last bits.  One rounding of the FP32 step sizes may flip from
+that (6e-8 relative), so that after 128 steps the points agree to 128 x 6e-8 <
+1e-5 of their scale; after a solve both meet the tolerance at the same
+optimum."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def sih():
+    import sih_pdhg
+
+    if not sih_pdhg.GpuSolver.is_cuda_available():
+        pytest.fail("GPU test run without a CUDA device")
+    return sih_pdhg
+
+
+def _dense_row_lp(sih, m, n, seed):
+    """One row over every column (longer than a warp's rows of entries), the rest with few."""
+    rng = np.random.default_rng(seed)
+    rows = np.concatenate([np.zeros(n, int), rng.integers(1, m, 3 * n)])
+    cols = np.concatenate([np.arange(n), np.repeat(np.arange(n), 3)])
+    A = sih.SparseMatrix.from_triplets(m, n, rows, cols, rng.standard_normal(4 * n))
+    x0 = rng.uniform(0, 1, n)
+    ax = A.mat_vec(x0)
+    y0 = -np.abs(rng.standard_normal(m))
+    c = A.mat_trans_vec(y0) + rng.uniform(0, 1, n)
+    return sih.Problem.from_arrays(A, c, np.zeros(n), np.full(n, 2.0), np.full(m, -np.inf), ax + 0.1)
+
+
+def _problem(sih, kind):
+    from sih_pdhg.generators import mixed_bounds_lp, small_random_lp, zipf_lp
+
+    if kind == "dense_row":
+        return _dense_row_lp(sih, 120, 1500, 0)
+    if kind == "every_bound":
+        return mixed_bounds_lp(seed=2)
+    if kind == "zipf":
+        return zipf_lp(900, 2000, 16000, seed=1)
+    m, n, k = kind
+    return small_random_lp(m, n, k, 1)
+
+
+# one block; two; a full portable cluster; 16 blocks; lengths at and past a batch and a lane group
+KINDS = [(2, 3, 1), (33, 64, 1), (50, 120, 4), (200, 500, 8), (700, 1500, 9), (1999, 4999, 8), (2500, 6000, 11),
+         (40, 45, 33), "every_bound", "dense_row", "zipf"]
+
+
+@pytest.mark.parametrize("kind", KINDS, ids=str)
+def test_steps_equal_the_kernel_per_phase_form(sih, kind):
+    p = _problem(sih, kind)
+    cfg = sih.GpuPdhgConfig(max_iterations=128, tol_primal=1e-12, tol_dual=1e-12, tol_gap=1e-12)
+    a = sih.solve_gpu_mixed(p, cfg, persistent=0)
+    b = sih.solve_gpu_mixed(p, cfg)
+    assert a.simplex_iterations == b.simplex_iterations and a.restarts == b.restarts
+    assert a.step_rejections == b.step_rejections
+    for u, v in ((a.x, b.x), (a.row_duals, b.row_duals)):
+        assert np.max(np.abs(u - v), initial=0.0) <= 1e-5 * max(1.0, np.max(np.abs(u), initial=0.0))
+    assert b.kernel_launches < a.kernel_launches / 10  # the whole period is one launch
+
+
+@pytest.mark.parametrize("compensated", [0, 2])
+def test_solves_to_the_same_optimum(sih, compensated):
+    p = _problem(sih, (300, 700, 6))
+    cfg = sih.GpuPdhgConfig(max_iterations=200000)
+    a = sih.solve_gpu_mixed(p, cfg, persistent=0, compensated=compensated)
+    b = sih.solve_gpu_mixed(p, cfg, compensated=compensated)
+    assert a.is_optimal() and b.is_optimal()
+    assert max(b.rel_primal, b.rel_dual, b.rel_gap) <= 1e-4
+    assert abs(a.primal_objective - b.primal_objective) <= 4e-4 * (1 + abs(a.primal_objective))
+
+
+def test_batch_of_unequal_instances(sih):
+    """Instances that need other cluster shares and stop at other evaluations,
+    and the same batch with one that does not fit (every instance then runs in
+    the other forms)."""
+    from sih_pdhg.generators import refinery_lp
+
+    ps = [_problem(sih, k) for k in ((200, 500, 8), (2, 3, 1), (1999, 4999, 8), "every_bound", (700, 1500, 9))]
+    cfg = sih.GpuPdhgConfig(max_iterations=20000)
+    for extra in ([], [refinery_lp(24, 1)]):
+        a = sih.solve_batch(ps + extra, cfg, persistent=0, autotune=0)
+        b = sih.solve_batch(ps + extra, cfg, autotune=0)
+        for u, v in zip(a, b):
+            assert u.status == v.status
+            assert abs(u.primal_objective - v.primal_objective) <= 4e-4 * (1 + abs(u.primal_objective))
+
+
+def test_run_again_and_warm_start(sih):
+    p = _problem(sih, (700, 1500, 9))
+    with sih.PdhgHandle(p, sih.GpuPdhgConfig(max_iterations=20000), algorithm=sih.ALGO_MIXED) as h:
+        h.run()
+        a = h.result(0)
+        h.run()
+        b = h.result(0)
+        assert a.is_optimal() and np.array_equal(a.x, b.x) and a.simplex_iterations == b.simplex_iterations
+        h.set_start(0, a.x, a.row_duals, a.final_primal_weight)
+        h.run()
+        c = h.result(0)
+    assert c.is_optimal() and c.simplex_iterations <= 64
