@@ -21,6 +21,7 @@
 #include <chrono>
 
 #include "plain.h"
+#include "resident.h"
 #include "spmv.cuh"
 #include "warp.cuh"
 
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(256, 8) plain_check_cols_kernel(SegMatrix At, 
     if (threadIdx.x == 0 && b > 0.f) atomicMax(&st->max_d_bits, __float_as_uint(b));
 }
 
-// The host part of the reference check (gpu_solver.cpp:252-268), one thread.
+// The host part of the reference check, one thread.
 __global__ void plain_check_finish_kernel(PlainState* st) {
     if (st->done) {
         st->copy_best = 0;
@@ -157,22 +158,7 @@ __global__ void plain_check_finish_kernel(PlainState* st) {
     const float max_p = __uint_as_float(st->max_p_bits), max_d = __uint_as_float(st->max_d_bits);
     st->max_p_bits = 0u;
     st->max_d_bits = 0u;
-    const float np = max_p / st->max_abs_b, nd = max_d / st->max_abs_c;
-    const float comb = (np < nd) ? nd : np;
-    const int it = min(st->next_check, st->max_iterations);
-    st->next_check += st->check_frequency;
-    st->checks += 1;
-    st->last_norm_p = np;
-    st->last_norm_d = nd;
-    st->copy_best = 0;
-    if (comb < st->best_combined) {
-        st->best_combined = comb;
-        st->copy_best = 1;
-    }
-    if (np <= st->tol_p && nd <= st->tol_d) {
-        st->done = 1;
-        st->iterations = it;
-    }
+    plain_check(*st, max_p, max_d);
 }
 
 __global__ void plain_copy_best_kernel(int n, const float* __restrict__ x, float* __restrict__ best,
@@ -193,6 +179,8 @@ __global__ void abs_sum_step_kernel(int nseg, const int* __restrict__ ptr, const
 }
 
 // ---------------------------------------------------------------- host driver
+PlainSolver::PlainSolver() : resident_(std::make_unique<ResidentPlan>()) {}
+
 int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const sih_pdhg_options& opts) {
     hp_ = &hp;
     cfg_ = cfg;
@@ -260,11 +248,20 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
         SIHG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, plain_primal_tasks, kThreads, 0));
         task_grid_ = sm_count_ * std::max(1, occ);
         const long long warps = (long long)task_grid_ * (kThreads / 32);
-        const int task_nnz = opts.tile_nnz > 0
-                                 ? opts.tile_nnz
-                                 : (int)std::max(128LL, std::min(2048LL, (long long)nnz / std::max(1LL, 3 * warps)));
+        task_nnz_ = opts.tile_nnz > 0
+                        ? opts.tile_nnz
+                        : (int)std::max(128LL, std::min(2048LL, (long long)nnz / std::max(1LL, 3 * warps)));
         SIHG_TRY(layout_.build(hp.csr_ptr, hp.csc_ptr, std::vector<int>{0, m}, std::vector<int>{0, n}, A_, At_,
-                               task_nnz, true, s));
+                               task_nnz_, true, s));
+    }
+
+    if (layout_.rows.ntasks > 0 && opts.use_graph) {  // LPs that fit: every iteration in one cluster
+        SideSchedule rs, cs;
+        make_schedule(hp.csr_ptr, std::vector<int>{0, m}, task_nnz_, rs);
+        make_schedule(hp.csc_ptr, std::vector<int>{0, n}, task_nnz_, cs);
+        SIHG_TRY(resident_->build(hp.csr_ptr, hp.csc_ptr, std::vector<int>{0, m}, std::vector<int>{0, n},
+                                  segment_lanes(rs, m), segment_lanes(cs, n), sm_count_, s, true));
+        if (resident_->ready()) SIHG_TRY(resident_->fill(A_, At_, s));
     }
 
     // step sizes on the device, in the reference's summation order
@@ -350,7 +347,7 @@ int PlainSolver::record_block(int iters, cudaGraphExec_t* exec) {
 }
 
 int PlainSolver::record_graphs() {
-    if (!opts_.use_graph) return SIH_PDHG_OK;
+    if (!opts_.use_graph || resident_->ready()) return SIH_PDHG_OK;
     const int cf = cfg_.check_frequency;
     const int maxit = cfg_.max_iterations;
     if (maxit >= cf) SIHG_TRY(record_block(cf, &block_exec_));
@@ -406,14 +403,27 @@ int PlainSolver::iterate() {
         cudaStream_t s = stream_;
         cudaEventRecord(ev_start_, s);
         bool done = false;
-        for (int b = 0; b < nblocks + (tail ? 1 : 0) && !done && rc == SIH_PDHG_OK; ++b) {
-            const int slot = b % kWindow;
-            if (b >= kWindow) {
+        // a launch of the resident form runs several blocks of iterations and checks
+        constexpr int kChecks = 8;
+        for (int b = 0, turn = 0; b < nblocks + (tail ? 1 : 0) && !done && rc == SIH_PDHG_OK; ++turn) {
+            const int slot = turn % kWindow;
+            if (turn >= kWindow) {
                 cudaError_t e = cudaEventSynchronize(ev[slot]);
                 if (e != cudaSuccess) { rc = cuda_fail(e, "cudaEventSynchronize", __FILE__, __LINE__); break; }
                 if (h_done[slot]) { done = true; break; }
             }
             const bool is_tail = b == nblocks;
+            if (resident_->ready()) {
+                const int checks = is_tail ? 1 : std::min(kChecks, nblocks - b);
+                launches_ += 1;
+                rc = resident_->launch_plain(is_tail ? tail : cf, checks, vec_, state_.as<PlainState>(), s);
+                if (rc != SIH_PDHG_OK) break;
+                b += checks;
+                cudaMemcpyAsync(&h_done[slot], &state_.as<PlainState>()->done, sizeof(int), cudaMemcpyDeviceToHost, s);
+                cudaEventRecord(ev[slot], s);
+                continue;
+            }
+            ++b;
             launches_ += 2ull * (is_tail ? tail : cf) + 4ull;
             if (opts_.use_graph) {
                 cudaError_t e = cudaGraphLaunch(is_tail ? tail_exec_ : block_exec_, s);

@@ -1,6 +1,7 @@
 // Plain FP32 PDHG (the reference's algorithm) on the device.
 #pragma once
 
+#include <memory>
 #include <vector>
 
 #include "common.cuh"
@@ -31,14 +32,37 @@ struct PlainState {
     int refine;          // task-engine flag (compensated SpMVs): always 0 here
 };
 
+// The host part of the reference check (gpu_solver.cpp:252-268) for the largest
+// row violation and column measure, one thread.
+__device__ __forceinline__ void plain_check(PlainState& S, float max_p, float max_d) {
+    const float np = max_p / S.max_abs_b, nd = max_d / S.max_abs_c;
+    const float comb = (np < nd) ? nd : np;
+    const int it = min(S.next_check, S.max_iterations);
+    S.next_check += S.check_frequency;
+    S.checks += 1;
+    S.last_norm_p = np;
+    S.last_norm_d = nd;
+    S.copy_best = 0;
+    if (comb < S.best_combined) {
+        S.best_combined = comb;
+        S.copy_best = 1;
+    }
+    if (np <= S.tol_p && nd <= S.tol_d) {
+        S.done = 1;
+        S.iterations = it;
+    }
+}
+
 struct PlainVecs {
     const float *c, *l, *u, *tau, *rl, *ru, *sigma;
     float *x, *xbar, *y, *best_x;
 };
 
+class ResidentPlan;  // resident.h
+
 class PlainSolver {
   public:
-    PlainSolver() = default;
+    PlainSolver();
     PlainSolver(const PlainSolver&) = delete;
     PlainSolver& operator=(const PlainSolver&) = delete;
     ~PlainSolver();
@@ -78,7 +102,8 @@ class PlainSolver {
     cudaGraphExec_t block_exec_ = nullptr, tail_exec_ = nullptr;
     DevMem csc_ptr_, csr_ptr_, csc_pairs_, csr_pairs_, colvec_, rowvec_, state_, heavy_;
     TaskLayout layout_;   // task engine of the fast (non-exact) iteration kernels
-    int task_grid_ = 1;
+    int task_grid_ = 1, task_nnz_ = 0;
+    std::unique_ptr<ResidentPlan> resident_;  // LPs that fit in a cluster: iterations and checks there
     SegMatrix A_{}, At_{};
     SpmvPlan plan_csr_{}, plan_csc_{};
     PlainVecs vec_{};

@@ -32,6 +32,7 @@
 #include <cstring>
 
 #include "eval.cuh"
+#include "plain.h"
 #include "resident.h"
 
 namespace sihg {
@@ -41,6 +42,8 @@ namespace {
 constexpr int kResThreads = 1024;  // launch bound of a block (64 registers; 672 threads used at most)
 constexpr int kColWords = 9;       // per column: x (2), K^T y (2), c, l, u, average (2)
 constexpr int kRowWords = 8;       // per row: y (2), K x (2), rl, ru, average (2)
+constexpr int kPlainColWords = 6;  // plain algorithm, per column: x, c, l, u, tau, best x
+constexpr int kPlainRowWords = 4;  // per row: y, rl, ru, sigma
 
 __device__ __forceinline__ unsigned cluster_rank() {
     unsigned r;
@@ -163,6 +166,18 @@ struct Pass {
         on = g < (t.w >> 24);
     }
 };
+
+// Copies this block's passes and entries of both sides to shared memory.
+__device__ __forceinline__ void load_block(const ResArgs& A, const ResBlock& blk, char* sm) {
+    for (int h = 0; h < 2; ++h) {
+        const ResSide& sd = blk.side[h];
+        int4* pass = reinterpret_cast<int4*>(sm + A.sm.pass[h]);
+        for (int k = threadIdx.x; k < sd.passes; k += blockDim.x) pass[k] = A.passes[sd.pass_begin + k];
+        const int4* src = reinterpret_cast<const int4*>(A.rows + (size_t)sd.row_begin * 32);
+        int4* dst = reinterpret_cast<int4*>(sm + A.sm.rows[h]);
+        for (int k = threadIdx.x; k < sd.rows * 16; k += blockDim.x) dst[k] = __ldg(src + k);
+    }
+}
 
 // Rows: K x' and the dual update (the operations of DualStepEpi::apply).
 template <bool COMP>
@@ -330,13 +345,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
     Sums* bsum = wsum + 32;                               // of every block of the cluster
     const int ncl = A.sm.locals[1], nrl = A.sm.locals[0];
     const int rp = blk.side[0].passes, cp = blk.side[1].passes;
-    for (int k = threadIdx.x; k < rp; k += blockDim.x) rpass[k] = A.passes[blk.side[0].pass_begin + k];
-    for (int k = threadIdx.x; k < cp; k += blockDim.x) cpass[k] = A.passes[blk.side[1].pass_begin + k];
-    for (int h = 0; h < 2; ++h) {
-        const int4* src = reinterpret_cast<const int4*>(A.rows + (size_t)blk.side[h].row_begin * 32);
-        int4* dst = reinterpret_cast<int4*>(h ? crows : rrows);
-        for (int k = threadIdx.x; k < blk.side[h].rows * 16; k += blockDim.x) dst[k] = __ldg(src + k);
-    }
+    load_block(A, blk, sm);
     if (threadIdx.x == 0) {
         S = st[inst];
         const StepScalars sc = step_scalars(S);
@@ -673,6 +682,165 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
     if (rank == 0 && ctrl && lane == 0) st[inst] = S;
 }
 
+// Plain algorithm (the reference's FP32 PDHG): `checks` times `iterations`
+// iterations and the reference's convergence check, on one cluster.  Two
+// phases an iteration, no reduction and no controller between checks.  The
+// element updates are those of plain_primal_tasks / plain_dual_tasks; the
+// check takes its maxima over the same sums.
+__global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, int iterations, int checks, PlainVecs v,
+                                                                   PlainState* st) {
+    extern __shared__ char sm[];
+    __shared__ PlainState S;  // every block's copy
+    __shared__ float wmax[2][32];
+    __shared__ float bmax[2][16];
+    const int cluster = A.cluster;
+    if (st->done) return;  // the whole cluster
+    const int rank = cluster > 1 ? (int)cluster_rank() : 0;
+    const ResBlock& blk = A.blocks[blockIdx.x];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    int4* rpass = reinterpret_cast<int4*>(sm + A.sm.pass[0]);
+    int4* cpass = reinterpret_cast<int4*>(sm + A.sm.pass[1]);
+    int2* rrows = reinterpret_cast<int2*>(sm + A.sm.rows[0]);
+    int2* crows = reinterpret_cast<int2*>(sm + A.sm.rows[1]);
+    float* xs = reinterpret_cast<float*>(sm + A.sm.xs);  // x_bar; x in a check
+    float* ys = reinterpret_cast<float*>(sm + A.sm.ys);
+    float* C = reinterpret_cast<float*>(sm + A.sm.col);  // x | c | l | u | tau | best x
+    float* R = reinterpret_cast<float*>(sm + A.sm.row);  // y | rl | ru | sigma
+    const int ncl = A.sm.locals[1], nrl = A.sm.locals[0];
+    const int rp = blk.side[0].passes, cp = blk.side[1].passes;
+    load_block(A, blk, sm);
+    if (threadIdx.x == 0) S = *st;
+    for (int k = threadIdx.x; k < A.inst[0].w; k += blockDim.x) ys[k] = v.y[k];
+    __syncthreads();
+    for (int p = warp; p < cp; p += nw) {
+        const Pass t(cpass[p], crows);
+        if (t.on && t.sub == 0) {
+            float* c = C + t.local;
+            c[0] = v.x[t.seg];
+            c[ncl] = v.c[t.seg];
+            c[2 * ncl] = v.l[t.seg];
+            c[3 * ncl] = v.u[t.seg];
+            c[4 * ncl] = v.tau[t.seg];
+            c[5 * ncl] = v.best_x[t.seg];
+        }
+    }
+    for (int p = warp; p < rp; p += nw) {
+        const Pass t(rpass[p], rrows);
+        if (t.on && t.sub == 0) {
+            float* r = R + t.local;
+            r[0] = v.y[t.seg];
+            r[nrl] = v.rl[t.seg];
+            r[2 * nrl] = v.ru[t.seg];
+            r[3 * nrl] = v.sigma[t.seg];
+        }
+    }
+    cluster_arrive();  // every block of the cluster runs before the first remote store
+    cluster_wait();
+    for (int check = 0; check < checks && !S.done; ++check) {
+        for (int it = 0; it < iterations; ++it) {
+            for (int p = warp; p < cp; p += nw) {
+                const Pass t(cpass[p], crows);
+                const float aty = pass_dot<false>(t.rows, t.width, t.lg, ys);
+                float x_new = 0.f;
+                if (t.on) {
+                    const float* c = C + t.local;
+                    const float x = c[0], l = c[2 * ncl], u = c[3 * ncl];
+                    x_new = __fsub_rn(x, __fmul_rn(c[4 * ncl], __fadd_rn(c[ncl], aty)));
+                    if (x_new < l) x_new = l;
+                    if (x_new > u) x_new = u;
+                    push(xs + t.seg, __fsub_rn(__fmul_rn(2.0f, x_new), x), t.sub, 1 << t.lg, cluster);
+                }
+                __syncwarp();  // every lane of the group has read x
+                if (t.on && t.sub == 0) C[t.local] = x_new;
+            }
+            cluster_arrive();
+            cluster_wait();
+            for (int p = warp; p < rp; p += nw) {
+                const Pass t(rpass[p], rrows);
+                const float axbar = pass_dot<false>(t.rows, t.width, t.lg, xs);
+                float y = 0.f;
+                if (t.on) {
+                    const float* r = R + t.local;
+                    const float sig = r[3 * nrl];
+                    const float w = __fadd_rn(axbar, r[0] / sig);
+                    float q = w;
+                    if (q < r[nrl]) q = r[nrl];
+                    if (q > r[2 * nrl]) q = r[2 * nrl];
+                    y = __fmul_rn(sig, __fsub_rn(w, q));
+                    push(ys + t.seg, y, t.sub, 1 << t.lg, cluster);
+                }
+                __syncwarp();
+                if (t.on && t.sub == 0) R[t.local] = y;
+            }
+            cluster_arrive();
+            cluster_wait();
+        }
+        // the check (plain_check_rows / _cols / _finish / _copy_best kernels)
+        for (int p = warp; p < cp; p += nw) {
+            const Pass t(cpass[p], crows);
+            if (t.on) push(xs + t.seg, C[t.local], t.sub, 1 << t.lg, cluster);
+        }
+        cluster_arrive();
+        float most[2] = {0.f, 0.f};
+        for (int p = warp; p < cp; p += nw) {
+            const Pass t(cpass[p], crows);
+            const float aty = pass_dot<false>(t.rows, t.width, t.lg, ys);
+            if (t.on) {
+                const float* c = C + t.local;
+                const float x = c[0], tau = c[4 * ncl];
+                float proj = __fsub_rn(x, __fmul_rn(tau, __fadd_rn(c[ncl], aty)));
+                if (proj < c[2 * ncl]) proj = c[2 * ncl];
+                if (proj > c[3 * ncl]) proj = c[3 * ncl];
+                most[1] = fmaxf(most[1], fabsf(__fsub_rn(x, proj)) / fmaxf(1e-4f, tau));
+            }
+        }
+        cluster_wait();
+        for (int p = warp; p < rp; p += nw) {
+            const Pass t(rpass[p], rrows);
+            const float ax = pass_dot<false>(t.rows, t.width, t.lg, xs);
+            if (t.on) {
+                const float rl = R[nrl + t.local], ru = R[2 * nrl + t.local];
+                float viol = 0.0f;
+                if (rl > -1e15f && ax < rl) viol = fmaxf(viol, __fsub_rn(rl, ax));
+                if (ru < 1e15f && ax > ru) viol = fmaxf(viol, __fsub_rn(ax, ru));
+                most[0] = fmaxf(most[0], viol);
+            }
+        }
+        for (int h = 0; h < 2; ++h) {
+            const float m = warp_max(most[h]);
+            if (lane == 0) wmax[h][warp] = m;
+        }
+        __syncthreads();
+        if (warp < 2) {
+            const float m = warp_max(lane < nw ? wmax[warp][lane] : 0.f);
+            if (lane < cluster) st_rank(map_rank(&bmax[warp][rank], lane), m);
+        }
+        cluster_arrive();
+        cluster_wait();
+        if (warp == 0) {
+            const float max_p = warp_max(lane < cluster ? bmax[0][lane] : 0.f);
+            const float max_d = warp_max(lane < cluster ? bmax[1][lane] : 0.f);
+            if (lane == 0) plain_check(S, max_p, max_d);
+        }
+        __syncthreads();
+        if (S.copy_best)
+            for (int k = threadIdx.x; k < blk.side[1].locals; k += blockDim.x) C[5 * ncl + k] = C[k];
+        __syncthreads();  // the owners move x in the next iteration
+    }
+    for (int p = warp; p < cp; p += nw) {
+        const Pass t(cpass[p], crows);
+        if (t.on && t.sub == 0) {
+            v.x[t.seg] = C[t.local];
+            v.best_x[t.seg] = C[5 * ncl + t.local];
+        }
+    }
+    for (int p = warp; p < rp; p += nw) {
+        const Pass t(rpass[p], rrows);
+        if (t.on && t.sub == 0) v.y[t.seg] = R[t.local];
+    }
+    if (rank == 0 && threadIdx.x == 0) *st = S;
+}
+
 namespace {
 
 // Entries of every pass from the (renumbered, scaled) matrix: a warp per pass.
@@ -715,15 +883,17 @@ void ResidentPlan::release() {
 
 int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>& csc_ptr, const std::vector<int>& roff,
                         const std::vector<int>& coff, const std::vector<uint8_t>& row_lanes,
-                        const std::vector<uint8_t>& col_lanes, int sm_count, cudaStream_t s) {
+                        const std::vector<uint8_t>& col_lanes, int sm_count, cudaStream_t s, bool plain) {
     release();
+    const void* kernel = plain ? (const void*)k_resident_plain : (const void*)k_resident_steps;
+    const int col_words = plain ? kPlainColWords : kColWords, row_words = plain ? kPlainRowWords : kRowWords;
     const int B = (int)roff.size() - 1;
     instances_ = B;
     int dev = 0, optin = 0;
     SIHG_CUDA(cudaGetDevice(&dev));
     SIHG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     cudaFuncAttributes fa{};
-    SIHG_CUDA(cudaFuncGetAttributes(&fa, k_resident_steps));
+    SIHG_CUDA(cudaFuncGetAttributes(&fa, kernel));
     const int budget = optin - (int)fa.sharedSizeBytes;
     const std::vector<int>* ptrs[2] = {&csr_ptr, &csc_ptr};
     const std::vector<int>* offs[2] = {&roff, &coff};
@@ -732,7 +902,7 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
     // over 16 blocks must fit; most batches end here
     for (int b = 0; b < B; ++b) {
         const double nnz = csr_ptr[roff[b + 1]] - csr_ptr[roff[b]], m = roff[b + 1] - roff[b], n = coff[b + 1] - coff[b];
-        if (4.0 * (m + n) + (16.0 * nnz + 4.0 * (kColWords * n + kRowWords * m)) / 16.0 > budget) return SIH_PDHG_OK;
+        if (4.0 * (m + n) + (16.0 * nnz + 4.0 * (col_words * n + row_words * m)) / 16.0 > budget) return SIH_PDHG_OK;
     }
     std::vector<ResBlock> blocks;
     std::vector<int4> passes, place, inst(B);
@@ -797,8 +967,8 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
         sm.ys = put(4ll * mm);
         sm.locals[0] = mloc[0];
         sm.locals[1] = mloc[1];
-        sm.col = put(4ll * kColWords * mloc[1]);
-        sm.row = put(4ll * kRowWords * mloc[0]);
+        sm.col = put(4ll * col_words * mloc[1]);
+        sm.row = put(4ll * row_words * mloc[0]);
         sm.red = put((long long)sizeof(Sums) * (32 + 16));
         sm.eval = put(kEvalQ * (8ll * 32 + 8ll * 16 + 8));
         sm.total = (int)std::min<long long>(at, INT32_MAX);
@@ -818,8 +988,8 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
     const int nw = std::max(1, std::min(20, most));
     threads_ = 32 * (nw + 1);
     npass_ = (int)passes.size();
-    SIHG_CUDA(cudaFuncSetAttribute(k_resident_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
-    SIHG_CUDA(cudaFuncSetAttribute(k_resident_steps, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    SIHG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
+    SIHG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     if (C > 1) {
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
@@ -831,7 +1001,7 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
         cfg.attrs = at;
         cfg.numAttrs = 1;
         int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, k_resident_steps, &cfg) != cudaSuccess || clusters < 1) {
+        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
             (void)cudaGetLastError();
             return SIH_PDHG_OK;
         }
@@ -861,9 +1031,8 @@ int ResidentPlan::fill(const SegMatrix& rows_A, const SegMatrix& cols_A, cudaStr
     return SIH_PDHG_OK;
 }
 
-int ResidentPlan::launch(int nsteps, int periods, const Vecs& V, Inst* st, unsigned* done_count,
-                         cudaStream_t s) const {
-    cudaLaunchAttribute at[1];
+// The launch configuration of one cluster per instance.
+cudaLaunchConfig_t ResidentPlan::config(cudaLaunchAttribute* at, cudaStream_t s) const {
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim = {(unsigned)args_.cluster, 1, 1};
     cudaLaunchConfig_t cfg{};
@@ -873,7 +1042,21 @@ int ResidentPlan::launch(int nsteps, int periods, const Vecs& V, Inst* st, unsig
     cfg.stream = s;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    return cfg;
+}
+
+int ResidentPlan::launch(int nsteps, int periods, const Vecs& V, Inst* st, unsigned* done_count,
+                         cudaStream_t s) const {
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = config(at, s);
     SIHG_CUDA(cudaLaunchKernelEx(&cfg, k_resident_steps, args_, nsteps, periods, V, st, done_count));
+    return SIH_PDHG_OK;
+}
+
+int ResidentPlan::launch_plain(int iterations, int checks, const PlainVecs& v, PlainState* st, cudaStream_t s) const {
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = config(at, s);
+    SIHG_CUDA(cudaLaunchKernelEx(&cfg, k_resident_plain, args_, iterations, checks, v, st));
     return SIH_PDHG_OK;
 }
 

@@ -37,22 +37,29 @@ struct ResArgs {
     int cluster;
 };
 
+struct PlainVecs;   // plain.h
+struct PlainState;
+
 class ResidentPlan {
   public:
     // Plans the form for these instances (segment pointers of the batch, lanes
-    // per segment of both sides); ready() says whether they fit.
+    // per segment of both sides), of the mixed or the plain algorithm (one
+    // instance); ready() says whether they fit.
     int build(const std::vector<int>& csr_ptr, const std::vector<int>& csc_ptr, const std::vector<int>& roff,
               const std::vector<int>& coff, const std::vector<uint8_t>& row_lanes,
-              const std::vector<uint8_t>& col_lanes, int sm_count, cudaStream_t s);
+              const std::vector<uint8_t>& col_lanes, int sm_count, cudaStream_t s, bool plain = false);
     // Copies the scaled entries into the layout.
     int fill(const SegMatrix& rows_A, const SegMatrix& cols_A, cudaStream_t s);
     // `periods` times nsteps steps and an evaluation of every running instance.
     int launch(int nsteps, int periods, const Vecs& V, Inst* st, unsigned* done_count, cudaStream_t s) const;
+    // `checks` times `iterations` iterations and a check of the plain algorithm.
+    int launch_plain(int iterations, int checks, const PlainVecs& v, PlainState* st, cudaStream_t s) const;
     bool ready() const { return ready_; }
     int grid() const { return args_.cluster * instances_; }
     void release();
 
   private:
+    cudaLaunchConfig_t config(cudaLaunchAttribute* at, cudaStream_t s) const;
     bool ready_ = false;
     int instances_ = 0, threads_ = 0, npass_ = 0;
     ResArgs args_{};

@@ -105,3 +105,31 @@ def test_run_again_and_warm_start(sih):
         h.run()
         c = h.result(0)
     assert c.is_optimal() and c.simplex_iterations <= 64
+
+
+@pytest.mark.parametrize("kind", KINDS, ids=str)
+@pytest.mark.parametrize("iterations", [7, 130, 425])
+def test_plain_iterations_are_those_of_the_task_kernels(sih, kind, iterations):
+    """The plain algorithm in the cluster (iterations and checks, several checks
+    a launch, a shorter last block) against its kernels launched one by one: no
+    sum enters the iterates but the segments', so they are the same bits."""
+    p = _problem(sih, kind)
+    cfg = sih.GpuPdhgConfig(max_iterations=iterations, tol_primal=1e-9, tol_dual=1e-9)
+    a = sih.GpuSolver.solve_ex(p, cfg, use_graph=0)
+    b = sih.solve_gpu_pdhg(p, cfg)
+    assert a.simplex_iterations == b.simplex_iterations and a.status == b.status
+    assert b.kernel_launches < a.kernel_launches / 10
+    np.testing.assert_array_equal(a.row_duals, b.row_duals)
+    np.testing.assert_array_equal(a.x, b.x)
+    # the checks sum with the iteration's lanes: FP32 sums of at most 1,500 terms in another order
+    assert abs(a.ref_primal - b.ref_primal) <= 1e-4 * (1e-3 + a.ref_primal)
+    assert abs(a.ref_dual - b.ref_dual) <= 1e-4 * (1e-3 + a.ref_dual)
+
+
+def test_plain_stops_at_the_same_check(sih):
+    p = _problem(sih, (200, 500, 8))
+    cfg = sih.GpuPdhgConfig(max_iterations=8000)
+    a = sih.GpuSolver.solve_ex(p, cfg, use_graph=0)
+    b = sih.solve_gpu_pdhg(p, cfg)
+    assert a.is_optimal() and b.is_optimal()
+    assert abs(a.simplex_iterations - b.simplex_iterations) <= cfg.check_frequency
