@@ -1420,20 +1420,26 @@ int MixedSolver::setup(const std::vector<const HostProblem*>& probs, const sih_p
     return setup_resident();
 }
 
-// The resident step form where the step form is left to the engine (or form 2
-// is asked for) and every instance fits: its steps take no global memory
-// traffic at all (2,000 x 5,000 LP: 13.7 -> 7.4 us per step, see resident.cu).
+// The resident step forms where the step form is left to the engine (or form 2
+// is asked for): a cluster per instance where every instance fits in one (2,000
+// x 5,000 LP: 13.7 -> 7.4 us per step), else one LP over every SM while its
+// matrix fits in their shared memory (see resident.cu for both).
 int MixedSolver::setup_resident() {
     if (resident_->ready() || packed_ || !(opts_.persistent < 0 || (opts_.persistent == 2 && B_ == 1)))
         return SIH_PDHG_OK;
     if (B_ == 1 && persistent_ != 2) return SIH_PDHG_OK;
+    // (a batch: no cluster holds the mean instance)
+    if (B_ > 1 && 16.0 * (double)nnz_ > 220.0 * 1024.0 * 16.0 * B_) return SIH_PDHG_OK;
     SideSchedule rs, cs;
     const int segs = latency_bound() ? kSoloTaskSegs : kTaskSegs;
-    if (16.0 * (double)nnz_ > 220.0 * 1024.0 * 16.0 * B_) return SIH_PDHG_OK;  // no cluster holds the mean instance
     make_schedule(h_csr_ptr_, row_off_, task_nnz_, rs, lanes_r_, segs);
     make_schedule(h_csc_ptr_, col_off_, task_nnz_, cs, lanes_c_, segs);
-    SIHG_TRY(resident_->build(h_csr_ptr_, h_csc_ptr_, row_off_, col_off_, segment_lanes(rs, M_), segment_lanes(cs, N_),
-                              sm_count_, stream_));
+    const std::vector<uint8_t> rl = segment_lanes(rs, M_), cl = segment_lanes(cs, N_);
+    SIHG_TRY(resident_->build(h_csr_ptr_, h_csc_ptr_, row_off_, col_off_, rl, cl, sm_count_, stream_,
+                              ResidentPlan::kCluster));
+    if (!resident_->ready() && B_ == 1)
+        SIHG_TRY(resident_->build(h_csr_ptr_, h_csc_ptr_, row_off_, col_off_, rl, cl, sm_count_, stream_,
+                                  ResidentPlan::kGrid));
     if (!resident_->ready()) return SIH_PDHG_OK;
     SIHG_TRY(resident_->fill(SegMatrix{M_, csr_ptr_.as<int>(), csr_pairs_.as<int2>()},
                              SegMatrix{N_, csc_ptr_.as<int>(), csc_pairs_.as<int2>()}, stream_));
@@ -1501,6 +1507,28 @@ constexpr double kBarrierLimitSec = 2.0;
 static GridBar make_bar(const DevMem& words, unsigned expected, double limit_sec) {
     unsigned long long* w = words.as<unsigned long long>();
     return GridBar{w, reinterpret_cast<int*>(w + 1), expected, (unsigned long long)(limit_sec * 1e9)};
+}
+
+// One launch of a resident form: `periods` evaluation periods.
+int MixedSolver::launch_resident(cudaStream_t s, int periods) {
+    Inst* st = state_.as<Inst>();
+    unsigned* done = done_count_.as<unsigned>();
+    launches_ += 1;
+    if (resident_->kind() == ResidentPlan::kCluster)
+        return resident_->launch(eval_freq_, periods, V_, st, done, s);
+    const int rc = resident_->launch_grid(eval_freq_, periods, V_, st, done, pack_.as<float4>(), N_,
+                                          make_bar(bar_, (unsigned)pgrid_, kBarrierLimitSec), s);
+    if (rc != SIH_PDHG_ERR_UNSUPPORTED) return rc;
+    // SMs taken by other work: these and all later steps run in form 2's other
+    // kernel, or as kernels per phase (launch_persistent)
+    launches_ -= 1;
+    resident_->release();
+    SIHG_TRY(set_form(2));
+    for (int k = 0; k < periods; ++k) {
+        SIHG_TRY(launch_persistent(s, eval_freq_));
+        SIHG_TRY(launch_eval(s));
+    }
+    return SIH_PDHG_OK;
 }
 
 // One cooperative launch of the persistent step kernel: `nsteps` steps.
@@ -1779,6 +1807,7 @@ int MixedSolver::run() {
     const bool graph = opts_.use_graph && !persistent_;
     if (graph) SIHG_TRY(record_graph());
     if (persistent_) SIHG_CUDA(cudaMemsetAsync(bar_.as<void>(), 0, 4 * sizeof(unsigned), stream_));
+    if (resident_->ready()) SIHG_TRY(resident_->reset(stream_));
     const auto t0 = std::chrono::steady_clock::now();
     launches_ = 0;
     SIHG_TRY(reset_state());
@@ -1818,8 +1847,7 @@ int MixedSolver::run() {
                 }
             }
             if (resident_->ready()) {  // evaluates too
-                launches_ += 1;
-                SIHG_TRY(resident_->launch(eval_freq_, periods, V_, state_.as<Inst>(), done_count_.as<unsigned>(), s));
+                SIHG_TRY(launch_resident(s, periods));
             } else if (persistent_) {
                 SIHG_TRY(launch_persistent(s, eval_freq_));
                 SIHG_TRY(launch_eval(s));

@@ -196,6 +196,7 @@ class MixedSolver {
     int set_form(int form);
     int setup_packed();
     int setup_resident();
+    int launch_resident(cudaStream_t s, int periods);
     int apply_shape(const sih_pdhg_launch_shape& sh);
     int time_block(double* seconds);
 

@@ -260,7 +260,7 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
         make_schedule(hp.csr_ptr, std::vector<int>{0, m}, task_nnz_, rs);
         make_schedule(hp.csc_ptr, std::vector<int>{0, n}, task_nnz_, cs);
         SIHG_TRY(resident_->build(hp.csr_ptr, hp.csc_ptr, std::vector<int>{0, m}, std::vector<int>{0, n},
-                                  segment_lanes(rs, m), segment_lanes(cs, n), sm_count_, s, true));
+                                  segment_lanes(rs, m), segment_lanes(cs, n), sm_count_, s, ResidentPlan::kPlain));
         if (resident_->ready()) SIHG_TRY(resident_->fill(A_, At_, s));
     }
 

@@ -32,6 +32,7 @@
 #include <cstring>
 
 #include "eval.cuh"
+#include "gridsync.cuh"
 #include "plain.h"
 #include "resident.h"
 
@@ -39,7 +40,8 @@ namespace sihg {
 
 namespace {
 
-constexpr int kResThreads = 1024;  // launch bound of a block (64 registers; 672 threads used at most)
+constexpr int kResThreads = 672;   // most threads of a block of a cluster: 20 warps with passes, the controller
+constexpr int kGridThreads = 768;  // threads of a block of the grid form
 constexpr int kColWords = 9;       // per column: x (2), K^T y (2), c, l, u, average (2)
 constexpr int kRowWords = 8;       // per row: y (2), K x (2), rl, ru, average (2)
 constexpr int kPlainColWords = 6;  // plain algorithm, per column: x, c, l, u, tau, best x
@@ -85,15 +87,16 @@ __device__ __forceinline__ void push(float* p, float v, int sub, int L, int clus
     for (int r = sub; r < cluster; r += L) st_rank(map_rank(p, r), v);
 }
 
-// Dot products of one pass: lane (group, sub) sums its entries with `vec`; the
-// sum s + e (e: the compensation) is valid in each group's first lane.  The phases are bound by the latency
-// and the number of these instructions, not by shared-memory bandwidth: two
-// batches of entries are read before the first is summed, and rows past the
-// pass's width add 0 * 0 (a branch over them costs more).
-template <bool COMP>
-__device__ __forceinline__ void pass_sums(const int2* __restrict__ rows, int width, int lg,
-                                          const float* __restrict__ vec, float& s, float& e) {
-    constexpr int kU = 2 * kBatch;
+// Dot products of one pass: lane (group, sub) sums its entries with the values
+// gather(index); the sum s + e (e: the compensation) is valid in each group's
+// first lane.  The phases are bound by the latency and the number of these
+// instructions, not by shared-memory bandwidth: BATCHES batches of entries are
+// read before the first is summed, and rows past the pass's width add 0 * 0 (a
+// branch over them costs more).
+template <bool COMP, int BATCHES, class Gather>
+__device__ __forceinline__ void pass_sums(const int2* __restrict__ rows, int width, int lg, Gather&& gather, float& s,
+                                          float& e) {
+    constexpr int kU = BATCHES * kBatch;
     float acc[kBatch] = {0.f, 0.f, 0.f, 0.f};
     s = e = 0.f;
     const int2* p = rows + (threadIdx.x & 31);
@@ -103,7 +106,7 @@ __device__ __forceinline__ void pass_sums(const int2* __restrict__ rows, int wid
 #pragma unroll
         for (int u = 0; u < kU; ++u) w[u] = k + u < width ? p[32 * u] : make_int2(-1, 0);
 #pragma unroll
-        for (int u = 0; u < kU; ++u) g[u] = w[u].x >= 0 ? vec[w[u].x] : 0.f;
+        for (int u = 0; u < kU; ++u) g[u] = w[u].x >= 0 ? gather(w[u].x) : 0.f;
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
             if (COMP) {
@@ -134,14 +137,45 @@ __device__ __forceinline__ void pass_sums(const int2* __restrict__ rows, int wid
 }
 
 // The same rounded to float, in every lane of the group.
-template <bool COMP>
-__device__ __forceinline__ float pass_dot(const int2* __restrict__ rows, int width, int lg,
-                                          const float* __restrict__ vec) {
+template <bool COMP, int BATCHES, class Gather>
+__device__ __forceinline__ float pass_dot(const int2* __restrict__ rows, int width, int lg, Gather&& gather) {
     float s, e;
-    pass_sums<COMP>(rows, width, lg, vec, s, e);
+    pass_sums<COMP, BATCHES>(rows, width, lg, gather, s, e);
     if (!COMP) return s;
     return __shfl_sync(FULL_MASK, __fadd_rn(s, e), (threadIdx.x & 31) >> lg << lg);
 }
+
+// Gathers from a copy in shared memory.
+struct FromShared {
+    const float* v;
+    __device__ __forceinline__ float operator()(int i) const { return v[i]; }
+};
+
+// Gathers of a vector written earlier in the same launch (coherent loads).
+struct FromGlobal {
+    const float* v;
+    __device__ __forceinline__ float operator()(int i) const {
+        float x;
+        asm volatile("ld.global.f32 %0, [%1];" : "=f"(x) : "l"(v + i));
+        return x;
+    }
+};
+
+// The candidate x' of a column from its record {x, c + K^T y, l, u}.
+__device__ __forceinline__ float x_from_record(const float4& r, float tau) {
+    return fminf(fmaxf(fmaf(-tau, r.y, r.x), r.z), r.w);
+}
+struct FromRecords {
+    const float4* v;
+    float tau;
+    __device__ __forceinline__ float operator()(int i) const {
+        float4 r;
+        asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
+                     : "l"(v + i));
+        return x_from_record(r, tau);
+    }
+};
 
 // What a step needs of the controller's state (FP32), published to the block.
 struct StepPub {
@@ -186,7 +220,7 @@ __device__ __forceinline__ void dual_phase(const int4* pass, int passes, const i
     const int nw = (blockDim.x >> 5) - 1;
     for (int p = threadIdx.x >> 5; p < passes; p += nw) {
         const Pass t(pass[p], rows);
-        const float kxp = pass_dot<COMP>(t.rows, t.width, t.lg, xs);
+        const float kxp = pass_dot<COMP, 2>(t.rows, t.width, t.lg, FromShared{xs});
         if (t.on) {
             const float* r = R + t.local;
             const float yo = r[cur * nl], kx = r[(2 + cur) * nl], rl = r[4 * nl], ru = r[5 * nl];
@@ -210,7 +244,7 @@ __device__ __forceinline__ void kty_phase(const int4* pass, int passes, const in
     const int nw = (blockDim.x >> 5) - 1;
     for (int p = threadIdx.x >> 5; p < passes; p += nw) {
         const Pass t(pass[p], rows);
-        const float k = pass_dot<COMP>(t.rows, t.width, t.lg, ys);
+        const float k = pass_dot<COMP, 2>(t.rows, t.width, t.lg, FromShared{ys});
         if (t.on && t.sub == 0) {
             const float* c = C + t.local;
             const float dx = c[(cur ^ 1) * nl] - c[cur * nl];
@@ -261,6 +295,83 @@ __device__ __forceinline__ void reduce_sums(const Sums* p, int n, Acc& a, Acc& c
     }
     warp_reduce_three(a, b, c);
 }
+// The step controller (step_controller), spread over the lanes of one warp.
+// FP64 is slow here (65 cycles an addition or multiplication, 550 a division):
+// what does not need the step's sums is prepared beside the A^T y' phase, and
+// what does is one chain with one division, a lane each for eta_bar, the next
+// eta and its tau and sigma.
+struct StepCtrl {
+    double coef, grow, om, inv_om, eta, W1, avg_w, dy2;
+    bool nan, accept;
+
+    __device__ __forceinline__ void prepare(const Inst& S) {
+        const int lane = threadIdx.x & 31;
+        om = S.omega;
+        eta = S.eta;
+        W1 = S.W + eta;
+        const double quot = (lane == 1 ? eta : 1.0) / (lane == 1 ? W1 : om);
+        inv_om = __shfl_sync(FULL_MASK, quot, 0);
+        avg_w = __shfl_sync(FULL_MASK, quot, 1);
+        const double per = lane == 2 ? inv_om : (lane == 3 ? om : 1.0);
+        grow = (1.0 + S.pow06) * eta * per;
+        coef = lane == 0 ? 1.0 : (1.0 - S.pow03) * per;
+    }
+    // From n partial sums of the step.
+    __device__ __forceinline__ void decide(const Sums* sums, int n, StepPub& pub) {
+        const int lane = threadIdx.x & 31;
+        Acc two, d;
+        reduce_sums(sums, n, two, d);
+        const double mine = (double)two.s + (double)two.c;
+        dy2 = (double)d.s + (double)d.c;
+        const double inter = __shfl_sync(FULL_MASK, mine, 0), dx2 = __shfl_sync(FULL_MASK, mine, 16);
+        // lane 0 eta_bar, lane 1 (1 - k^-0.3) eta_bar, lanes 2 and 3 the same
+        // / and * omega.  Non-negative FP64 numbers compare as integers (FP64
+        // compares have the latency of FP64 sums); a NaN compares above infinity.
+        const double movement = om * dx2 + dy2 * inv_om;
+        const double ai = fabs(inter);
+        const double quot = __double_as_longlong(ai) != 0 ? coef * movement / (2.0 * ai) : INFINITY;
+        const long long qb = __double_as_longlong(quot), inf = 0x7ff0000000000000ll;
+        const bool less = __shfl_sync(FULL_MASK, (int)(qb < __double_as_longlong(grow)), 1) != 0;
+        const double next = less ? quot : grow;
+        nan = __double_as_longlong(fabs(movement)) > inf || __double_as_longlong(ai) > inf;
+        accept = !nan && __double_as_longlong(eta) <= qb && qb <= inf;  // lane 0
+        if (nan) {
+            if (lane == 0) pub.done = 3;
+            return;
+        }
+        if (lane == 2) pub.tau = (float)next;
+        if (lane == 3) pub.sigma = (float)next;
+        if (lane == 0) {
+            pub.avg = accept;
+            if (accept) {
+                pub.cur ^= 1;
+                pub.w = (float)avg_w;
+            }
+        }
+        eta = __shfl_sync(FULL_MASK, next, 1);
+    }
+    // The instance's state after the step (lane 0, beside the next phase).
+    __device__ __forceinline__ void record(Inst& S) const {
+        S.attempts += 1;
+        if (nan) {
+            S.done = 3;
+            return;
+        }
+        S.dy2 = dy2;
+        S.avg_pending = accept;
+        if (accept) {
+            S.cur ^= 1;
+            S.steps += 1;
+            S.since_restart += 1;
+            S.W = W1;
+            S.avg_w = avg_w;
+        } else {
+            S.rejections += 1;
+        }
+        S.eta = eta;
+    }
+};
+
 constexpr int kEvalQ = 18;  // reductions of an evaluation: 8 of the rows, 10 of the columns
 
 // Sums of a side's segments with the first candidate point, to s and e by local segment.
@@ -271,9 +382,9 @@ __device__ __forceinline__ void eval_sums(bool comp, const int4* pass, int passe
         const Pass t(pass[p], rows);
         float s, e;
         if (comp)
-            pass_sums<true>(t.rows, t.width, t.lg, vec, s, e);
+            pass_sums<true, 2>(t.rows, t.width, t.lg, FromShared{vec}, s, e);
         else
-            pass_sums<false>(t.rows, t.width, t.lg, vec, s, e);
+            pass_sums<false, 2>(t.rows, t.width, t.lg, FromShared{vec}, s, e);
         if (t.on && t.sub == 0) {
             s_out[t.local] = s;
             e_out[t.local] = e;
@@ -291,9 +402,9 @@ __device__ __forceinline__ void eval_apply(bool comp, const int4* pass, int pass
         const Pass t(pass[p], rows);
         SegDot<2> d;
         if (comp)
-            pass_sums<true>(t.rows, t.width, t.lg, vec, d.s[1], d.e[1]);
+            pass_sums<true, 2>(t.rows, t.width, t.lg, FromShared{vec}, d.s[1], d.e[1]);
         else
-            pass_sums<false>(t.rows, t.width, t.lg, vec, d.s[1], d.e[1]);
+            pass_sums<false, 2>(t.rows, t.width, t.lg, FromShared{vec}, d.s[1], d.e[1]);
         if (t.on && t.sub == 0) {
             d.s[0] = s_in[t.local];
             d.e[0] = e_in[t.local];
@@ -430,13 +541,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
         }
         cluster_arrive();
         cluster_wait();
-        // Everything of the controller that does not need this phase's sums
-        // runs beside it, and what is left after it is one chain of FP64
-        // operations, which are slow here (65 cycles an addition or
-        // multiplication, 550 a division): a lane each for eta_bar, the next
-        // eta and its tau and sigma, one division for all of them.
-        double coef = 1.0, grow = 0.0, om = 0.0, inv_om = 0.0, eta = 0.0, W1 = 0.0, avg_w = 0.0, total_dy2 = 0.0;
-        bool nan = false, accept = false;
+        StepCtrl ctl;
         if (!ctrl) {
             Acc inter, dx2;
             if (comp)
@@ -450,15 +555,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
             }
             if (lane == 16) wsum[warp].dx2 = make_float2(inter.s, inter.c);
         } else {
-            om = S.omega;
-            eta = S.eta;
-            W1 = S.W + eta;
-            const double quot = (lane == 1 ? eta : 1.0) / (lane == 1 ? W1 : om);
-            inv_om = __shfl_sync(FULL_MASK, quot, 0);
-            avg_w = __shfl_sync(FULL_MASK, quot, 1);
-            const double per = lane == 2 ? inv_om : (lane == 3 ? om : 1.0);
-            grow = (1.0 + S.pow06) * eta * per;
-            coef = lane == 0 ? 1.0 : (1.0 - S.pow03) * per;
+            ctl.prepare(S);
         }
         __syncthreads();
         if (ctrl) {  // the block's sums to every block: lane r (inter, |dy|^2) and 16 + r (|dx|^2) to block r
@@ -471,59 +568,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
         }
         cluster_arrive();
         cluster_wait();
-        if (ctrl) {
-            Acc two, d[1];
-            reduce_sums(bsum, cluster, two, d[0]);
-            const double mine = (double)two.s + (double)two.c, dy2 = (double)d[0].s + (double)d[0].c;
-            const double inter = __shfl_sync(FULL_MASK, mine, 0), dx2 = __shfl_sync(FULL_MASK, mine, 16);
-            // step_controller: lane 0 eta_bar, lane 1 (1 - k^-0.3) eta_bar, lanes
-            // 2 and 3 the same / and * omega.  Non-negative FP64 numbers compare
-            // as integers (FP64 compares have the latency of FP64 sums); a NaN
-            // compares above infinity.
-            const double movement = om * dx2 + dy2 * inv_om;
-            const double ai = fabs(inter);
-            const double quot = __double_as_longlong(ai) != 0 ? coef * movement / (2.0 * ai) : INFINITY;
-            const long long qb = __double_as_longlong(quot), inf = 0x7ff0000000000000ll;
-            const bool less = __shfl_sync(FULL_MASK, (int)(qb < __double_as_longlong(grow)), 1) != 0;
-            const double next = less ? quot : grow;
-            nan = __double_as_longlong(fabs(movement)) > inf || __double_as_longlong(ai) > inf;
-            accept = !nan && __double_as_longlong(eta) <= qb && qb <= inf;  // lane 0
-            if (nan) {
-                if (lane == 0) pub.done = 3;
-            } else {
-                if (lane == 2) pub.tau = (float)next;
-                if (lane == 3) pub.sigma = (float)next;
-                if (lane == 0) {
-                    pub.avg = accept;
-                    if (accept) {
-                        pub.cur = cur ^ 1;
-                        pub.w = (float)avg_w;
-                    }
-                }
-                eta = __shfl_sync(FULL_MASK, next, 1);
-            }
-            total_dy2 = dy2;
-        }
+        if (ctrl) ctl.decide(bsum, cluster, pub);
         __syncthreads();
-        if (ctrl && lane == 0) {  // the instance's counters, beside the next phase
-            S.attempts += 1;
-            if (nan) {
-                S.done = 3;
-            } else {
-                S.dy2 = total_dy2;
-                S.eta = eta;
-                S.avg_pending = accept;
-                if (accept) {
-                    S.cur ^= 1;
-                    S.steps += 1;
-                    S.since_restart += 1;
-                    S.W = W1;
-                    S.avg_w = avg_w;
-                } else {
-                    S.rejections += 1;
-                }
-            }
-        }
+        if (ctrl && lane == 0) ctl.record(S);
     }
     // The evaluation (as k_flush_avg, k_eval_rows, k_eval_cols and k_restart):
     // the copies hold the current point, then the average one; the epilogues
@@ -682,6 +729,421 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
     if (rank == 0 && ctrl && lane == 0) st[inst] = S;
 }
 
+// ---------------------------------------------------------------- grid form
+// One LP over every SM: the same layout with a block per SM instead of a block
+// of a cluster.  The matrix and the owners' data stay in shared memory; x' and
+// y' are gathered from L2 (x' computed by the gathering lane from its column's
+// record, so that a step needs two grid barriers), and the barrier after
+// A^T y' carries the blocks' sums.
+//
+// What bounds it (cycle counters, refinery LP with 24 / 168 periods, 18,000 /
+// 28,800 cycles a step): A x' 2,300 / 6,400, its barrier 4,400 / 4,900, A^T y' 2,900 /
+// 8,200, the block's sums 700, the second barrier 3,300, the grid's sums 1,300,
+// the controller 2,300.  The small LP is barriers (a release, an L2 round trip and
+// an acquire each) and the controller's FP64 chain; the large one as much the
+// instructions of its 50 passes a side and block (about 300 each, compensated
+// sums near the tolerance).  Measured per step, whole solves: 14.6 -> 9.0 us and
+// 26 -> 14.4 us against k_solo_steps, which reads the matrix from L2 and remains
+// for LPs that do not fit.
+// Grid-wide barrier.  Every block adds one to its counter of kArrive (fewer
+// additions queue up at one address) with release semantics; one warp of each
+// block polls all of them with relaxed loads, then acquires once (an acquire
+// per poll, or a flag per block polled by a thread each, took 5,600 - 7,300
+// cycles a barrier).  Waits are bounded as in gridsync.cuh; false: give up.
+constexpr int kArrive = 8;
+struct GridSync {
+    unsigned* count;  // [kArrive] counters, 32 words apart, then `turn`; zeroed before a run
+    int* status;
+    unsigned long long limit_ns;
+    unsigned turn;    // barriers passed
+
+    __device__ __forceinline__ bool operator()(bool* ok) {
+        ++turn;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const int lane = threadIdx.x;
+            if (lane == 0)
+                asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count + 32 * (blockIdx.x % kArrive))
+                             : "memory");
+            // blocks that share counter `lane`, times the barriers so far
+            const unsigned mine = lane < kArrive ? (gridDim.x - lane + kArrive - 1) / kArrive * turn : 0u;
+            const unsigned long long t0 = global_ns();
+            unsigned spins = 0;
+            bool good = true;
+            for (;;) {
+                unsigned v = mine;
+                if (lane < kArrive)
+                    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count + 32 * lane) : "memory");
+                if (__all_sync(FULL_MASK, (int)(v - mine) >= 0)) break;
+                if ((++spins & 31u) == 0u) {
+                    const bool late = global_ns() - t0 > limit_ns;
+                    if (lane == 0 && late) atomicExch(status, 1);
+                    if (__any_sync(FULL_MASK, late || ld_status(status) != 0)) {
+                        good = false;
+                        break;
+                    }
+                }
+            }
+            asm volatile("fence.acq_rel.gpu;" ::: "memory");
+            if (lane == 0) *ok = good;
+        }
+        __syncthreads();
+        return *ok;
+    }
+};
+
+// Columns of the grid form: K^T y' from L2, x' from the owner's record, the
+// next record, and the average update (the operations of KtyStepEpiPacked).
+template <bool COMP>
+__device__ __forceinline__ void grid_cols(const int4* pass, int passes, const int2* rows, float* C, int nl, int cur,
+                                          const float* y, float4* next, float tau, bool avg, float w, Acc& inter,
+                                          Acc& dx2) {
+    const int nw = (blockDim.x >> 5) - 1;
+    for (int p = threadIdx.x >> 5; p < passes; p += nw) {
+        const Pass t(pass[p], rows);
+        const float k = pass_dot<COMP, 2>(t.rows, t.width, t.lg, FromGlobal{y});
+        if (t.on && t.sub == 0) {
+            float* c = C + t.local;
+            const float x = c[cur * nl], kty = c[(2 + cur) * nl], cc = c[4 * nl], l = c[5 * nl], u = c[6 * nl];
+            const float xp = x_from_record(make_float4(x, cc + kty, l, u), tau);
+            if (avg) {
+                const float2 a = ff_axpy(make_float2(c[7 * nl], c[8 * nl]), w, x);
+                c[7 * nl] = a.x;
+                c[8 * nl] = a.y;
+            }
+            c[(cur ^ 1) * nl] = xp;
+            c[(2 + (cur ^ 1)) * nl] = k;
+            next[t.seg] = make_float4(xp, cc + k, l, u);
+            const float dx = xp - x;
+            inter.add(dx * (k - kty));
+            dx2.add(dx * dx);
+        }
+    }
+}
+
+// Rows: K x' gathered through the records, dual update, average update.
+template <bool COMP>
+__device__ __forceinline__ void grid_rows(const int4* pass, int passes, const int2* rows, float* R, int nl, int cur,
+                                          const float4* records, float tau, float sigma, float* y_next, bool avg,
+                                          float w, Acc& dy2) {
+    const int nw = (blockDim.x >> 5) - 1;
+    for (int p = threadIdx.x >> 5; p < passes; p += nw) {
+        const Pass t(pass[p], rows);
+        const float kxp = pass_dot<COMP, 2>(t.rows, t.width, t.lg, FromRecords{records, tau});
+        if (t.on && t.sub == 0) {
+            float* r = R + t.local;
+            const float yo = r[cur * nl], kx = r[(2 + cur) * nl], rl = r[4 * nl], ru = r[5 * nl];
+            if (avg) {
+                const float2 a = ff_axpy(make_float2(r[6 * nl], r[7 * nl]), w, yo);
+                r[6 * nl] = a.x;
+                r[7 * nl] = a.y;
+            }
+            const float wv = (2.0f * kxp - kx) + yo / sigma;
+            const float yv = sigma * (wv - fminf(fmaxf(wv, rl), ru));
+            r[(2 + (cur ^ 1)) * nl] = kxp;
+            r[(cur ^ 1) * nl] = yv;
+            y_next[t.seg] = yv;
+            const float dy = yv - yo;
+            dy2.add(dy * dy);
+        }
+    }
+}
+
+// The evaluation epilogue over a side, both candidates gathered from L2.
+template <bool COMP, class Epi>
+__device__ __forceinline__ void grid_eval(const int4* pass, int passes, const int2* rows, const float* v0,
+                                          const float* v1, Epi& epi) {
+    const int nw = (blockDim.x >> 5) - 1;
+    for (int p = threadIdx.x >> 5; p < passes; p += nw) {
+        const Pass t(pass[p], rows);
+        SegDot<2> d;
+        pass_sums<COMP, 1>(t.rows, t.width, t.lg, FromGlobal{v0}, d.s[0], d.e[0]);
+        pass_sums<COMP, 1>(t.rows, t.width, t.lg, FromGlobal{v1}, d.s[1], d.e[1]);
+        if (t.on && t.sub == 0) epi.apply(t.seg, d, epi.pre(t.seg));
+    }
+}
+
+__global__ void __launch_bounds__(kGridThreads, 1)
+    k_resident_grid(ResArgs A, int nsteps, int periods, Vecs V, Inst* st, unsigned* done_count, float4* records, int N,
+                    unsigned* count, Sums* bsum, float2* esums, GridBar gb) {
+    extern __shared__ char sm[];
+    __shared__ Inst S;
+    __shared__ StepPub pub;
+    __shared__ int flag;
+    __shared__ unsigned ignored;
+    __shared__ bool ok;
+    if (st->done || ld_status(gb.status) != 0) return;
+    const ResBlock& blk = A.blocks[blockIdx.x];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x >> 5) - 1, P = gridDim.x;
+    const bool ctrl = warp == nw;
+    int4* rpass = reinterpret_cast<int4*>(sm + A.sm.pass[0]);
+    int4* cpass = reinterpret_cast<int4*>(sm + A.sm.pass[1]);
+    int2* rrows = reinterpret_cast<int2*>(sm + A.sm.rows[0]);
+    int2* crows = reinterpret_cast<int2*>(sm + A.sm.rows[1]);
+    float* C = reinterpret_cast<float*>(sm + A.sm.col);  // x x' | K^T y K^T y' | c l u | average hi lo
+    float* R = reinterpret_cast<float*>(sm + A.sm.row);  // y y' | K x K x' | rl ru | average hi lo
+    Sums* wsum = reinterpret_cast<Sums*>(sm + A.sm.red);
+    float2* ewarp = reinterpret_cast<float2*>(sm + A.sm.eval);
+    double* etot = reinterpret_cast<double*>(ewarp + kEvalQ * 32);
+    const int ncl = A.sm.locals[1], nrl = A.sm.locals[0];
+    const int rp = blk.side[0].passes, cp = blk.side[1].passes;
+    GridSync sync{count, gb.status, gb.limit_ns, count[32 * kArrive]};  // barriers of this run's earlier launches
+    load_block(A, blk, sm);
+    if (threadIdx.x == 0) {
+        S = *st;
+        const StepScalars sc = step_scalars(S);
+        pub = StepPub{sc.cur, sc.avg, 0, sc.w, sc.tau, (float)(S.eta * S.omega)};
+    }
+    __syncthreads();
+    if (!ctrl) {  // owners' data and the records of the current point
+        const int cur = pub.cur;
+        for (int p = warp; p < cp; p += nw) {
+            const Pass t(cpass[p], crows);
+            if (t.on && t.sub == 0) {
+                const int j = t.seg;
+                float* c = C + t.local;
+                c[cur * ncl] = pick(V.x0, V.x1, cur)[j];
+                c[(2 + cur) * ncl] = pick(V.kty0, V.kty1, cur)[j];
+                c[4 * ncl] = V.c[j];
+                c[5 * ncl] = V.l[j];
+                c[6 * ncl] = V.u[j];
+                const float2 a = V.x_acc[j];
+                c[7 * ncl] = a.x;
+                c[8 * ncl] = a.y;
+                records[(size_t)cur * N + j] =
+                    make_float4(c[cur * ncl], c[4 * ncl] + c[(2 + cur) * ncl], c[5 * ncl], c[6 * ncl]);
+            }
+        }
+        for (int p = warp; p < rp; p += nw) {
+            const Pass t(rpass[p], rrows);
+            if (t.on && t.sub == 0) {
+                const int j = t.seg;
+                float* r = R + t.local;
+                r[cur * nrl] = pick(V.y0, V.y1, cur)[j];
+                r[(2 + cur) * nrl] = pick(V.kx0, V.kx1, cur)[j];
+                r[4 * nrl] = V.rl[j];
+                r[5 * nrl] = V.ru[j];
+                const float2 a = V.y_acc[j];
+                r[6 * nrl] = a.x;
+                r[7 * nrl] = a.y;
+            }
+        }
+    }
+    if (!sync(&ok)) return;
+    for (int period = 0; period < periods && !pub.done; ++period) {
+        const bool comp = S.refine != 0;
+        for (int k = 0; k < nsteps && !pub.done; ++k) {
+            const int cur = pub.cur;
+            const bool avg = pub.avg != 0;
+            const float w = pub.w, tau = pub.tau, sg = pub.sigma;
+            const float4* rec = records + (size_t)cur * N;
+            float* yn = pick(V.y0, V.y1, cur ^ 1);
+            Acc inter, dx2, dy2;
+            StepCtrl ctl;
+            if (!ctrl) {
+                if (comp)
+                    grid_rows<true>(rpass, rp, rrows, R, nrl, cur, rec, tau, sg, yn, avg, w, dy2);
+                else
+                    grid_rows<false>(rpass, rp, rrows, R, nrl, cur, rec, tau, sg, yn, avg, w, dy2);
+            } else if (lane == 0) {
+                schedule_pows(S, V);
+            }
+            if (!sync(&ok)) return;
+            if (!ctrl) {
+                float4* next = records + (size_t)(cur ^ 1) * N;
+                if (comp)
+                    grid_cols<true>(cpass, cp, crows, C, ncl, cur, yn, next, tau, avg, w, inter, dx2);
+                else
+                    grid_cols<false>(cpass, cp, crows, C, ncl, cur, yn, next, tau, avg, w, inter, dx2);
+                warp_reduce_three(inter, dx2, dy2);
+                if (lane == 0) {
+                    wsum[warp].inter = make_float2(inter.s, inter.c);
+                    wsum[warp].dy2 = make_float2(dy2.s, dy2.c);
+                }
+                if (lane == 16) wsum[warp].dx2 = make_float2(inter.s, inter.c);
+            } else {
+                ctl.prepare(S);
+            }
+            __syncthreads();
+            if (warp == 0) {
+                Acc a, c;
+                reduce_sums(wsum, nw, a, c);
+                if (lane == 0) {
+                    bsum[blockIdx.x].inter = make_float2(a.s, a.c);
+                    bsum[blockIdx.x].dy2 = make_float2(c.s, c.c);
+                }
+                if (lane == 16) bsum[blockIdx.x].dx2 = make_float2(a.s, a.c);
+                __syncwarp();
+            }
+            if (!sync(&ok)) return;
+            // the blocks' sums: one per thread, five warps, then the controller
+            // (overwritten only after the next barrier)
+            const int sw = (P + 31) / 32;
+            if (warp < sw) {
+                Acc i1, i2, i3;
+                if (threadIdx.x < P) {
+                    const float2* f = &bsum[threadIdx.x].inter;
+                    const float2 f1 = __ldcg(f), f2 = __ldcg(f + 1), f3 = __ldcg(f + 2);
+                    i1.s = f1.x;
+                    i1.c = f1.y;
+                    i2.s = f2.x;
+                    i2.c = f2.y;
+                    i3.s = f3.x;
+                    i3.c = f3.y;
+                }
+                warp_reduce_three(i1, i2, i3);
+                if (lane == 0) {
+                    wsum[warp].inter = make_float2(i1.s, i1.c);
+                    wsum[warp].dy2 = make_float2(i3.s, i3.c);
+                }
+                if (lane == 16) wsum[warp].dx2 = make_float2(i1.s, i1.c);
+            }
+            __syncthreads();
+            if (ctrl) ctl.decide(wsum, sw, pub);
+            __syncthreads();
+            if (ctrl && lane == 0) ctl.record(S);
+        }
+        // The evaluation (as k_flush_avg, k_eval_rows, k_eval_cols and k_restart).
+        const int cur = pub.cur;
+        const bool avg = pub.avg != 0;
+        const float w = pub.w;
+        if (!ctrl) {
+            for (int p = warp; p < cp; p += nw) {
+                const Pass t(cpass[p], crows);
+                if (t.on && t.sub == 0) {
+                    const int j = t.seg;
+                    float* c = C + t.local;
+                    const float x = c[cur * ncl];
+                    float2 a = make_float2(c[7 * ncl], c[8 * ncl]);
+                    if (avg) a = ff_axpy(a, w, x);
+                    c[7 * ncl] = a.x;
+                    c[8 * ncl] = a.y;
+                    pick(V.x0, V.x1, cur)[j] = x;
+                    pick(V.kty0, V.kty1, cur)[j] = c[(2 + cur) * ncl];
+                    V.x_acc[j] = a;
+                    V.x_avg[j] = __fadd_rn(a.x, a.y);
+                }
+            }
+            for (int p = warp; p < rp; p += nw) {
+                const Pass t(rpass[p], rrows);
+                if (t.on && t.sub == 0) {
+                    const int j = t.seg;
+                    float* r = R + t.local;
+                    const float y = r[cur * nrl];
+                    float2 a = make_float2(r[6 * nrl], r[7 * nrl]);
+                    if (avg) a = ff_axpy(a, w, y);
+                    r[6 * nrl] = a.x;
+                    r[7 * nrl] = a.y;
+                    pick(V.y0, V.y1, cur)[j] = y;
+                    pick(V.kx0, V.kx1, cur)[j] = r[(2 + cur) * nrl];
+                    V.y_acc[j] = a;
+                    V.y_avg[j] = __fadd_rn(a.x, a.y);
+                }
+            }
+        }
+        if (pub.done) break;  // a step failed: nothing to evaluate
+        if (!sync(&ok)) return;
+        if (!ctrl) {
+            EvalRowsEpi er{V};
+            er.begin(S);
+            Acc q[8];
+            if (comp)
+                grid_eval<true>(rpass, rp, rrows, er.xg[0], er.xg[1], er);
+            else
+                grid_eval<false>(rpass, rp, rrows, er.xg[0], er.xg[1], er);
+            er.values(q);
+            warp_reduce_acc<8>(q, 0x0Cu);
+            if (lane == 0)
+                for (int i = 0; i < 8; ++i) ewarp[i * 32 + warp] = make_float2(q[i].s, q[i].c);
+        }
+        if (!ctrl) {
+            EvalColsEpi ec{V, nullptr};
+            ec.begin(S);
+            Acc q[10];
+            if (comp)
+                grid_eval<true>(cpass, cp, crows, ec.yg[0], ec.yg[1], ec);
+            else
+                grid_eval<false>(cpass, cp, crows, ec.yg[0], ec.yg[1], ec);
+            ec.values(q);
+            warp_reduce_acc<10>(q, 0x0Cu);
+            if (lane == 0)
+                for (int i = 0; i < 10; ++i) ewarp[(8 + i) * 32 + warp] = make_float2(q[i].s, q[i].c);
+        }
+        __syncthreads();
+        for (int i = warp; i < kEvalQ; i += nw + 1) {
+            const Acc v = eval_total(ewarp + i * 32, nw, i);
+            if (lane == 0) esums[(size_t)i * P + blockIdx.x] = make_float2(v.s, v.c);
+        }
+        if (!sync(&ok)) return;
+        for (int i = warp; i < kEvalQ; i += nw + 1) {
+            const bool is_max = i == 2 || i == 3 || i == 10 || i == 11;
+            Acc v[1];
+            for (int k = lane; k < P; k += 32) {
+                const float2 f = __ldcg(esums + (size_t)i * P + k);
+                Acc b;
+                b.s = f.x;
+                b.c = f.y;
+                v[0] = acc_join(v[0], b, is_max);
+            }
+            warp_reduce_acc<1>(v, is_max ? 1u : 0u);
+            if (lane == 0) etot[i] = (double)v[0].s + (double)v[0].c;
+        }
+        __syncthreads();
+        if (ctrl && lane == 0) {
+            for (int i = 0; i < 8; ++i) S.row_eval[i] = etot[i];
+            S.col_eval_dist[0] = etot[16];
+            S.col_eval_dist[1] = etot[17];
+            eval_controller(S, etot + 8, blockIdx.x == 0 ? done_count : &ignored);
+            const StepScalars sc = step_scalars(S);
+            pub = StepPub{sc.cur, 0, S.done, sc.w, sc.tau, (float)(S.eta * S.omega)};
+            flag = S.restart_flag;
+        }
+        __syncthreads();
+        if (!ctrl && flag != 0) {  // restart at the current (1) or the average point (2)
+            for (int p = warp; p < cp; p += nw) {
+                const Pass t(cpass[p], crows);
+                if (t.on && t.sub == 0) {
+                    const int j = t.seg;
+                    float* c = C + t.local;
+                    if (flag == 2) {
+                        pick(V.x0, V.x1, cur)[j] = c[cur * ncl] = V.x_avg[j];
+                        pick(V.kty0, V.kty1, cur)[j] = c[(2 + cur) * ncl] = V.kty_eval[j];
+                        records[(size_t)cur * N + j] =
+                            make_float4(c[cur * ncl], c[4 * ncl] + c[(2 + cur) * ncl], c[5 * ncl], c[6 * ncl]);
+                    }
+                    const float x = c[cur * ncl];
+                    V.x_last[j] = x;
+                    V.x_acc[j] = make_float2(x, 0.f);
+                    c[7 * ncl] = x;
+                    c[8 * ncl] = 0.f;
+                }
+            }
+            for (int p = warp; p < rp; p += nw) {
+                const Pass t(rpass[p], rrows);
+                if (t.on && t.sub == 0) {
+                    const int j = t.seg;
+                    float* r = R + t.local;
+                    if (flag == 2) {
+                        pick(V.y0, V.y1, cur)[j] = r[cur * nrl] = V.y_avg[j];
+                        pick(V.kx0, V.kx1, cur)[j] = r[(2 + cur) * nrl] = V.kx_eval[j];
+                    }
+                    const float y = r[cur * nrl];
+                    V.y_last[j] = y;
+                    V.y_acc[j] = make_float2(y, 0.f);
+                    r[6 * nrl] = y;
+                    r[7 * nrl] = 0.f;
+                }
+            }
+        }
+        // (the next step gathers the records that a restart to the average rewrote)
+        if (period + 1 < periods && !pub.done && !sync(&ok)) return;
+    }
+    if (blockIdx.x == 0 && ctrl && lane == 0) {
+        *st = S;
+        count[32 * kArrive] = sync.turn;  // for the next launch
+    }
+}
+
 // Plain algorithm (the reference's FP32 PDHG): `checks` times `iterations`
 // iterations and the reference's convergence check, on one cluster.  Two
 // phases an iteration, no reduction and no controller between checks.  The
@@ -740,7 +1202,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, in
         for (int it = 0; it < iterations; ++it) {
             for (int p = warp; p < cp; p += nw) {
                 const Pass t(cpass[p], crows);
-                const float aty = pass_dot<false>(t.rows, t.width, t.lg, ys);
+                const float aty = pass_dot<false, 2>(t.rows, t.width, t.lg, FromShared{ys});
                 float x_new = 0.f;
                 if (t.on) {
                     const float* c = C + t.local;
@@ -757,7 +1219,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, in
             cluster_wait();
             for (int p = warp; p < rp; p += nw) {
                 const Pass t(rpass[p], rrows);
-                const float axbar = pass_dot<false>(t.rows, t.width, t.lg, xs);
+                const float axbar = pass_dot<false, 2>(t.rows, t.width, t.lg, FromShared{xs});
                 float y = 0.f;
                 if (t.on) {
                     const float* r = R + t.local;
@@ -784,7 +1246,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, in
         float most[2] = {0.f, 0.f};
         for (int p = warp; p < cp; p += nw) {
             const Pass t(cpass[p], crows);
-            const float aty = pass_dot<false>(t.rows, t.width, t.lg, ys);
+            const float aty = pass_dot<false, 2>(t.rows, t.width, t.lg, FromShared{ys});
             if (t.on) {
                 const float* c = C + t.local;
                 const float x = c[0], tau = c[4 * ncl];
@@ -797,7 +1259,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, in
         cluster_wait();
         for (int p = warp; p < rp; p += nw) {
             const Pass t(rpass[p], rrows);
-            const float ax = pass_dot<false>(t.rows, t.width, t.lg, xs);
+            const float ax = pass_dot<false, 2>(t.rows, t.width, t.lg, FromShared{xs});
             if (t.on) {
                 const float rl = R[nrl + t.local], ru = R[2 * nrl + t.local];
                 float viol = 0.0f;
@@ -879,13 +1341,19 @@ void ResidentPlan::release() {
     ready_ = false;
     tab_.release();
     rows_.release();
+    slots_.release();
+    esums_.release();
 }
 
 int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>& csc_ptr, const std::vector<int>& roff,
                         const std::vector<int>& coff, const std::vector<uint8_t>& row_lanes,
-                        const std::vector<uint8_t>& col_lanes, int sm_count, cudaStream_t s, bool plain) {
+                        const std::vector<uint8_t>& col_lanes, int sm_count, cudaStream_t s, Kind kind) {
     release();
-    const void* kernel = plain ? (const void*)k_resident_plain : (const void*)k_resident_steps;
+    kind_ = kind;
+    const bool plain = kind == kPlain, grid = kind == kGrid;
+    const void* kernel = plain  ? (const void*)k_resident_plain
+                         : grid ? (const void*)k_resident_grid
+                                : (const void*)k_resident_steps;
     const int col_words = plain ? kPlainColWords : kColWords, row_words = plain ? kPlainRowWords : kRowWords;
     const int B = (int)roff.size() - 1;
     instances_ = B;
@@ -902,7 +1370,9 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
     // over 16 blocks must fit; most batches end here
     for (int b = 0; b < B; ++b) {
         const double nnz = csr_ptr[roff[b + 1]] - csr_ptr[roff[b]], m = roff[b + 1] - roff[b], n = coff[b + 1] - coff[b];
-        if (4.0 * (m + n) + (16.0 * nnz + 4.0 * (col_words * n + row_words * m)) / 16.0 > budget) return SIH_PDHG_OK;
+        if (grid) {
+            if ((16.0 * nnz + 4.0 * (col_words * n + row_words * m)) / sm_count > budget) return SIH_PDHG_OK;
+        } else if (4.0 * (m + n) + (16.0 * nnz + 4.0 * (col_words * n + row_words * m)) / 16.0 > budget) return SIH_PDHG_OK;
     }
     std::vector<ResBlock> blocks;
     std::vector<int4> passes, place, inst(B);
@@ -923,8 +1393,9 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
                 const int other = (*offs[1 - h])[b];
                 std::vector<std::vector<int4>> mine(C), where(C);
                 std::vector<int> nrow(C, 0), nloc(C, 0);
-                int turn = 0;
-                for (int seg = s0; seg < s1; ++turn) {
+                // passes of equal lanes and width: runs [first pass, last)
+                std::vector<int4> all;  // {first segment, segments, width, log2 L}
+                for (int seg = s0; seg < s1;) {
                     const int L = (*lanes[h])[seg];
                     int e = seg, width = 0, lg = 0;
                     while ((1 << lg) < L) ++lg;
@@ -932,14 +1403,32 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
                         width = std::max(width, (ptr[e + 1] - ptr[e] + L - 1) / L);
                         ++e;
                     }
-                    // the passes run by descending length: dealt out back and forth
-                    const int q = turn % (2 * C), r = q < C ? q : 2 * C - 1 - q;
-                    mine[r].push_back(make_int4(nrow[r], width | (lg << 24), seg - s0, nloc[r] | ((e - seg) << 24)));
-                    where[r].push_back(make_int4(nrow[r], width, seg, e - seg));
-                    where[r].push_back(make_int4(other, h, L, 0));
-                    nrow[r] += width;
-                    nloc[r] += e - seg;
+                    all.push_back(make_int4(seg, e - seg, width, lg));
                     seg = e;
+                }
+                for (size_t q0 = 0; q0 < all.size();) {
+                    size_t q1 = q0;
+                    while (q1 < all.size() && all[q1].z == all[q0].z && all[q1].w == all[q0].w) ++q1;
+                    for (size_t q = q0; q < q1; ++q) {
+                        int r;
+                        if (grid) {
+                            // each run spread evenly in its order: segments of one length keep the caller's
+                            // order, so that a block gets the same part of the LP from every run and side,
+                            // and its gathers, where the LP has a block structure, meet in its L1
+                            r = (int)((long long)(q - q0) * C / (long long)(q1 - q0));
+                            if (q1 - q0 < (size_t)C) r = (int)((r + C / (2 * (long long)(q1 - q0))) % C);
+                        } else {  // the passes run by descending length: dealt out back and forth
+                            const int t = (int)(q % (2 * (size_t)C));
+                            r = t < C ? t : 2 * C - 1 - t;
+                        }
+                        const int4 a = all[q];
+                        mine[r].push_back(make_int4(nrow[r], a.z | (a.w << 24), a.x - s0, nloc[r] | (a.y << 24)));
+                        where[r].push_back(make_int4(nrow[r], a.z, a.x, a.y));
+                        where[r].push_back(make_int4(other, h, 1 << a.w, 0));
+                        nrow[r] += a.z;
+                        nloc[r] += a.y;
+                    }
+                    q0 = q1;
                 }
                 for (int r = 0; r < C; ++r) {
                     ResSide& sd = blocks[(size_t)b * C + r].side[h];
@@ -963,8 +1452,8 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
         };
         for (int h = 0; h < 2; ++h) sm.rows[h] = put(256ll * mrows[h]);
         for (int h = 0; h < 2; ++h) sm.pass[h] = put(16ll * mpass[h]);
-        sm.xs = put(4ll * mn);
-        sm.ys = put(4ll * mm);
+        sm.xs = put(grid ? 0 : 4ll * mn);
+        sm.ys = put(grid ? 0 : 4ll * mm);
         sm.locals[0] = mloc[0];
         sm.locals[1] = mloc[1];
         sm.col = put(4ll * col_words * mloc[1]);
@@ -979,18 +1468,29 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
     // scheduler): beyond that the barriers and pushes of more blocks cost what
     // the shorter phases save (317 x 803: 4 blocks of 9 passes and 8 of 5 are
     // equal).
-    int C = 1, most = 0;
+    int C = grid ? sm_count : 1, most = 0;
     long long rows = plan(C, most);
-    while (C < 16 && sm.total > budget) rows = plan(C *= 2, most);
+    while (!grid && C < 16 && sm.total > budget) rows = plan(C *= 2, most);
     if (sm.total > budget) return SIH_PDHG_OK;
-    while (C < 16 && (long long)B * 2 * C <= sm_count && most > 8) rows = plan(C *= 2, most);
+    while (!grid && C < 16 && (long long)B * 2 * C <= sm_count && most > 8) rows = plan(C *= 2, most);
     // 20 warps with passes at most (31: 3 % slower on the batch of 64, whose blocks have 39 passes)
-    const int nw = std::max(1, std::min(20, most));
+    // (grid form: a thread per block sums)
+    const int nw = grid ? kGridThreads / 32 - 1 : std::max(1, std::min(kResThreads / 32 - 1, most));
     threads_ = 32 * (nw + 1);
+    if (grid && sm_count > threads_) return SIH_PDHG_OK;
     npass_ = (int)passes.size();
     SIHG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
-    SIHG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    if (C > 1) {
+    if (grid) {
+        int occ = 0, coop = 0;
+        SIHG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+        SIHG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads_, sm.total));
+        if (!coop || occ < 1) return SIH_PDHG_OK;
+        SIHG_TRY(slots_.alloc(sizeof(unsigned) * 32 * (kArrive + 1) + sizeof(Sums) * (size_t)C));
+        SIHG_TRY(esums_.alloc(sizeof(float2) * kEvalQ * (size_t)C));
+    } else {
+        SIHG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    }
+    if (!grid && C > 1) {
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim = {(unsigned)C, 1, 1};
@@ -1050,6 +1550,27 @@ int ResidentPlan::launch(int nsteps, int periods, const Vecs& V, Inst* st, unsig
     cudaLaunchAttribute at[1];
     const cudaLaunchConfig_t cfg = config(at, s);
     SIHG_CUDA(cudaLaunchKernelEx(&cfg, k_resident_steps, args_, nsteps, periods, V, st, done_count));
+    return SIH_PDHG_OK;
+}
+
+int ResidentPlan::reset(cudaStream_t s) {
+    if (kind_ == kGrid) SIHG_CUDA(cudaMemsetAsync(slots_.as<void>(), 0, slots_.bytes(), s));
+    return SIH_PDHG_OK;
+}
+
+int ResidentPlan::launch_grid(int nsteps, int periods, const Vecs& V, Inst* st, unsigned* done_count, float4* records,
+                              int N, const GridBar& gb, cudaStream_t s) const {
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg = config(at, s);
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_resident_grid, args_, nsteps, periods, V, st, done_count, records,
+                                             N, slots_.as<unsigned>(), reinterpret_cast<Sums*>(slots_.as<unsigned>() + 32 * (kArrive + 1)), esums_.as<float2>(), gb);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {  // the device cannot hold the whole grid now; the caller falls back
+        (void)cudaGetLastError();
+        return SIH_PDHG_ERR_UNSUPPORTED;
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "resident grid kernel launch", __FILE__, __LINE__);
     return SIH_PDHG_OK;
 }
 

@@ -1,9 +1,10 @@
-// Resident step form: LPs whose matrix fits in the shared memory of one
-// thread-block cluster (see resident.cu).
+// Resident step forms: LPs whose matrix fits in the shared memory of one
+// thread-block cluster, or of all SMs (see resident.cu).
 #pragma once
 
 #include <vector>
 
+#include "gridsync.cuh"
 #include "mixed.h"
 
 namespace sihg {
@@ -42,28 +43,39 @@ struct PlainState;
 
 class ResidentPlan {
   public:
+    // kCluster: a cluster per instance; kGrid: one LP over every SM; kPlain: the
+    // plain algorithm of one LP on a cluster.
+    enum Kind { kCluster, kGrid, kPlain };
     // Plans the form for these instances (segment pointers of the batch, lanes
-    // per segment of both sides), of the mixed or the plain algorithm (one
-    // instance); ready() says whether they fit.
+    // per segment of both sides); ready() says whether they fit.
     int build(const std::vector<int>& csr_ptr, const std::vector<int>& csc_ptr, const std::vector<int>& roff,
               const std::vector<int>& coff, const std::vector<uint8_t>& row_lanes,
-              const std::vector<uint8_t>& col_lanes, int sm_count, cudaStream_t s, bool plain = false);
+              const std::vector<uint8_t>& col_lanes, int sm_count, cudaStream_t s, Kind kind);
     // Copies the scaled entries into the layout.
     int fill(const SegMatrix& rows_A, const SegMatrix& cols_A, cudaStream_t s);
     // `periods` times nsteps steps and an evaluation of every running instance.
     int launch(int nsteps, int periods, const Vecs& V, Inst* st, unsigned* done_count, cudaStream_t s) const;
+    // Start of a run: the grid form's barriers count from zero.
+    int reset(cudaStream_t s);
+    // The same for kGrid (cooperative launch; `records`: 2 N column records; gb:
+    // status word and limit of the barrier waits).  SIH_PDHG_ERR_UNSUPPORTED:
+    // the grid does not fit on the device now, nothing was launched.
+    int launch_grid(int nsteps, int periods, const Vecs& V, Inst* st, unsigned* done_count, float4* records, int N,
+                    const GridBar& gb, cudaStream_t s) const;
     // `checks` times `iterations` iterations and a check of the plain algorithm.
     int launch_plain(int iterations, int checks, const PlainVecs& v, PlainState* st, cudaStream_t s) const;
     bool ready() const { return ready_; }
+    Kind kind() const { return kind_; }
     int grid() const { return args_.cluster * instances_; }
     void release();
 
   private:
     cudaLaunchConfig_t config(cudaLaunchAttribute* at, cudaStream_t s) const;
     bool ready_ = false;
+    Kind kind_ = kCluster;
     int instances_ = 0, threads_ = 0, npass_ = 0;
     ResArgs args_{};
-    DevMem tab_, rows_;
+    DevMem tab_, rows_, slots_, esums_;
 };
 
 }  // namespace sihg

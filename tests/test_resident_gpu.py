@@ -66,6 +66,30 @@ def test_steps_equal_the_kernel_per_phase_form(sih, kind):
     assert b.kernel_launches < a.kernel_launches / 10  # the whole period is one launch
 
 
+# too large for a cluster: over every SM, from barely (30k entries a side more
+# than a cluster holds) to half of the SMs' shared memory, and one that does not fit (the older kernels)
+GRID = [("uniform", 9000, 20000, 5), ("uniform", 4001, 30011, 7), ("zipf", 30000, 60000, 400000), ("refinery", 12),
+        ("uniform", 90000, 150000, 10)]
+
+
+@pytest.mark.parametrize("kind", GRID, ids=str)
+def test_grid_form_steps_equal_the_kernel_per_phase_form(sih, kind):
+    from sih_pdhg.generators import refinery_lp, small_random_lp, zipf_lp
+
+    if kind[0] == "uniform":
+        p = small_random_lp(*kind[1:], 2)
+    else:
+        p = refinery_lp(kind[1], 1) if kind[0] == "refinery" else zipf_lp(*kind[1:], 2)
+    cfg = sih.GpuPdhgConfig(max_iterations=128, tol_primal=1e-12, tol_dual=1e-12, tol_gap=1e-12)
+    for compensated in (0, 2):
+        a = sih.solve_gpu_mixed(p, cfg, persistent=0, staged_kib=-1, compensated=compensated)
+        b = sih.solve_gpu_mixed(p, cfg, compensated=compensated)
+        assert a.simplex_iterations == b.simplex_iterations and a.restarts == b.restarts
+        assert a.step_rejections == b.step_rejections
+        for u, v in ((a.x, b.x), (a.row_duals, b.row_duals)):
+            assert np.max(np.abs(u - v)) <= 1e-5 * max(1.0, np.max(np.abs(u)))
+
+
 @pytest.mark.parametrize("compensated", [0, 2])
 def test_solves_to_the_same_optimum(sih, compensated):
     p = _problem(sih, (300, 700, 6))
