@@ -191,4 +191,47 @@ __device__ __forceinline__ float2 ff_axpy(float2 acc, float w, float x) {
     return make_float2(hi2, lo2);
 }
 
+// ---------------------------------------------------------------- chained launches
+// Programmatic dependent launch.  The kernels that call this first are
+// launched with programmatic stream serialization (launch_chained): their blocks may be
+// scheduled while the previous kernel in the stream finishes, and wait here,
+// before their first memory access, until it has completed and its writes are
+// visible; then they let the next kernel be scheduled.  Without the launch
+// attribute both instructions do nothing.
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// chain_wait for a kernel whose pointers are __restrict__: the compiler may
+// take loads through them as invariant and move them; passing the pointers
+// through here keeps every access behind the wait.
+template <class P>
+__device__ __forceinline__ void behind_wait(P& p) {
+    asm volatile("" : "+l"(p)::"memory");
+}
+template <class... P>
+__device__ __forceinline__ void chain_wait_for(P&... p) {
+    chain_wait();
+    (behind_wait(p), ...);
+}
+
+// Launches a kernel that starts with chain_wait with programmatic stream
+// serialization.
+template <class... P, class... A>
+static cudaError_t launch_chained(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s,
+                                  A... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 }  // namespace sihg

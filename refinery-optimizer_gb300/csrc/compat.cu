@@ -1,14 +1,12 @@
 // The reference's kernel launchers (core/src/gpu/cuda_pdhg.cu:155-203) with
 // their exact argument lists: separate int32 index and float value arrays,
 // device pointers, a caller stream.  The reference's host driver binds them at
-// core/src/gpu/gpu_solver.cpp:18-40.  The SpMVs use warp-cooperative segment
-// groups (lanes chosen from the mean segment length); updates are the
-// reference's element formulas with unfused float operations.
+// core/src/gpu/gpu_solver.cpp:18-40.  Updates are the reference's element
+// formulas with unfused float operations.
 #include <algorithm>
-#include <map>
-#include <mutex>
 
 #include "common.cuh"
+#include "compat.cuh"
 
 namespace sihg {
 
@@ -24,26 +22,128 @@ __device__ __forceinline__ float split_dot(const int* __restrict__ idx, const fl
     return s0 + s1;
 }
 
-__global__ void __launch_bounds__(256) split_spmv_kernel(int nseg, const int* __restrict__ ptr,
-                                                         const int* __restrict__ idx,
-                                                         const float* __restrict__ val,
-                                                         const float* __restrict__ vec, float* __restrict__ out,
-                                                         int L) {
+// Segments summed in place by groups of L lanes (few or long segments).
+__device__ __forceinline__ void spmv_by_groups(int nseg, const int* __restrict__ ptr, const int* __restrict__ idx,
+                                               const float* __restrict__ val, const float* __restrict__ vec,
+                                               float* __restrict__ out, int L) {
     const int lane = threadIdx.x & 31, sub = lane & (L - 1), gpw = 32 / L;
     const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-    for (int base = wid * gpw; base < nseg; base += nw * gpw) {
-        const int r = base + lane / L;
+    for (unsigned base = wid * gpw; base < (unsigned)nseg; base += nw * gpw) {  // unsigned: nseg + a turn may pass 2^31
+        const unsigned r = base + lane / L;
         float s = 0.f;
-        if (r < nseg) s = split_dot(idx, val, ptr[r], ptr[r + 1], sub, L, vec);
+        if (r < (unsigned)nseg) s = split_dot(idx, val, ptr[r], ptr[r + 1], sub, L, vec);
         for (int o = L >> 1; o > 0; o >>= 1) s += __shfl_down_sync(FULL_MASK, s, o, L);
-        if (r < nseg && sub == 0) out[r] = s;
+        if (r < (unsigned)nseg && sub == 0) out[r] = s;
     }
+}
+
+__device__ __forceinline__ int ld_stream(const int* p) {
+    int v;
+    asm("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ld_stream(const float* p) {
+    float v;
+    asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
+// Many short segments: a warp takes 32 consecutive segments and reads their
+// entries as one stream, eight per lane in flight, whatever the segments'
+// lengths (products go to shared memory; Greathouse and Daga's CSR-stream,
+// SC14); then each lane sums its own segment, and the warp together the ones
+// longer than kLong.  Groups of lanes leave the lanes of short segments idle
+// while the group of a long one works.  What bounds it is the gathers: one
+// cache line each, which the L1 takes one at a time per SM (12M of them: 46 us).
+// 500k x 1M LP, 12M entries: columns (Zipf lengths, 2 to 350, mean 12) 147 us by
+// groups, 62.8 by stream; rows (mean 24) 57.9 and 54.8.  64 warps per SM (32
+// registers) matter most: 48 warps 65.6 / 61.3 us; windows of 256 / 640 products
+// 76 / 69 us, 16 entries a lane in flight 83 us; kLong 24 / 32 / 64: 70.3 / 58.8 / 54.8 us
+// on the rows.
+constexpr int kWindow = 512;  // products of a warp at a time
+constexpr int kLong = 48;
+__device__ __forceinline__ void spmv_by_stream(int nseg, const int* __restrict__ ptr, const int* __restrict__ idx,
+                                               const float* __restrict__ val, const float* __restrict__ vec,
+                                               float* __restrict__ out, float* prod) {
+    constexpr int kU = 8;
+    const int lane = threadIdx.x & 31;
+    const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    const unsigned last = nseg;
+    for (unsigned base = wid * 32u; base < last; base += nw * 32u) {
+        const unsigned r = base + lane;
+        const int b = ptr[min(r, last)], e = ptr[min(r + 1, last)];
+        const int end = __shfl_sync(FULL_MASK, e, 31);
+        const unsigned longs = __ballot_sync(FULL_MASK, e - b > kLong);
+        float s = 0.f;
+        for (int w = __shfl_sync(FULL_MASK, b, 0); w < end; w += kWindow) {
+            const int n = min(kWindow, end - w);
+            for (int k0 = lane; k0 < n; k0 += 32 * kU) {
+                int i[kU];
+                float a[kU], g[kU];
+#pragma unroll
+                for (int u = 0; u < kU; ++u) {
+                    const bool on = k0 + 32 * u < n;
+                    i[u] = on ? ld_stream(idx + w + k0 + 32 * u) : -1;
+                    a[u] = on ? ld_stream(val + w + k0 + 32 * u) : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < kU; ++u) g[u] = i[u] >= 0 ? __ldg(vec + i[u]) : 0.f;
+#pragma unroll
+                for (int u = 0; u < kU; ++u)
+                    if (i[u] >= 0) prod[k0 + 32 * u] = a[u] * g[u];
+            }
+            __syncwarp();
+            const int lo = max(b - w, 0), hi = min(e - w, n);  // this lane's part of the window
+            if (e - b <= kLong) {
+                float t = 0.f;
+                int k = lo;
+                for (; k + 1 < hi; k += 2) {
+                    s += prod[k];
+                    t += prod[k + 1];
+                }
+                if (k < hi) s += prod[k];
+                s += t;
+            }
+            for (unsigned m = longs; m; m &= m - 1) {
+                const int from = __ffs(m) - 1;
+                const int lo1 = __shfl_sync(FULL_MASK, lo, from), hi1 = __shfl_sync(FULL_MASK, hi, from);
+                float t = 0.f;
+                for (int k = lo1 + lane; k < hi1; k += 32) t += prod[k];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(FULL_MASK, t, o);
+                if (lane == from) s += t;
+            }
+            __syncwarp();
+        }
+        if (r < last) out[r] = s;
+    }
+}
+
+// Lanes per segment from the mean segment length, from the last pointer: read
+// on the device, so that no launch has to ask the host for it.  By stream from
+// kStreamSegs segments on, where every SM has several warps of 32, and below a
+// mean of 64, where a segment keeps a half-warp busy by itself.
+__global__ void __launch_bounds__(kSplitThreads, 16) split_spmv_kernel(int nseg, const int* __restrict__ ptr,
+                                                                   const int* __restrict__ idx,
+                                                                   const float* __restrict__ val,
+                                                                   const float* __restrict__ vec,
+                                                                   float* __restrict__ out) {
+    __shared__ float prod[kSplitThreads / 32][kWindow];
+    chain_wait_for(ptr, idx, val, vec, out);
+    const long long nnz = ptr[nseg];
+    int L = 1;
+    while (L < 32 && 4ll * L * nseg <= nnz) L *= 2;
+    if (nseg >= kStreamSegs && L < 16)
+        spmv_by_stream(nseg, ptr, idx, val, vec, out, prod[threadIdx.x >> 5]);
+    else
+        spmv_by_groups(nseg, ptr, idx, val, vec, out, L);
 }
 
 __global__ void compat_primal_kernel(int n, const float* __restrict__ tau, const float* __restrict__ c,
                                      const float* __restrict__ aty, const float* __restrict__ l,
                                      const float* __restrict__ u, float* __restrict__ x,
                                      float* __restrict__ xbar) {
+    chain_wait_for(tau, c, aty, l, u, x, xbar);
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         const float x_old = x[j];
         float x_new = __fsub_rn(x_old, __fmul_rn(tau[j], __fadd_rn(c[j], aty[j])));
@@ -57,6 +157,7 @@ __global__ void compat_primal_kernel(int n, const float* __restrict__ tau, const
 __global__ void compat_dual_kernel(int m, const float* __restrict__ sigma, const float* __restrict__ axbar,
                                    const float* __restrict__ rl, const float* __restrict__ ru,
                                    float* __restrict__ y) {
+    chain_wait_for(sigma, axbar, rl, ru, y);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
         const float sig = sigma[i];
         const float w = __fadd_rn(axbar[i], y[i] / sig);
@@ -68,73 +169,51 @@ __global__ void compat_dual_kernel(int m, const float* __restrict__ sigma, const
 }
 
 __global__ void compat_copy_kernel(int n, const float* __restrict__ x, float* __restrict__ xbar) {
+    chain_wait_for(x, xbar);
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) xbar[j] = x[j];
 }
 
-__global__ void compat_row_viol_kernel(int m, const float* __restrict__ ax, const float* __restrict__ rl,
-                                       const float* __restrict__ ru, float* __restrict__ out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-        const float a = ax[i];
-        float viol = 0.0f;
-        if (rl[i] > -1e15f && a < rl[i]) viol = fmaxf(viol, __fsub_rn(rl[i], a));
-        if (ru[i] < 1e15f && a > ru[i]) viol = fmaxf(viol, __fsub_rn(a, ru[i]));
-        out[i] = viol;
-    }
-}
-
-__global__ void compat_col_viol_kernel(int n, const float* __restrict__ x, const float* __restrict__ c,
-                                       const float* __restrict__ aty, const float* __restrict__ l,
-                                       const float* __restrict__ u, const float* __restrict__ tau,
-                                       float* __restrict__ out) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+__global__ void compat_residuals_kernel(int m, int n, const float* __restrict__ ax, const float* __restrict__ rl,
+                                        const float* __restrict__ ru, float* __restrict__ row_out,
+                                        const float* __restrict__ x, const float* __restrict__ c,
+                                        const float* __restrict__ aty, const float* __restrict__ l,
+                                        const float* __restrict__ u, const float* __restrict__ tau,
+                                        float* __restrict__ col_out) {
+    chain_wait_for(ax, rl, ru, row_out, x, c, aty, l, u, tau, col_out);
+    const int stride = gridDim.x * blockDim.x;
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
         const float xj = x[j], step = tau[j];
         float proj = __fsub_rn(xj, __fmul_rn(step, __fadd_rn(c[j], aty[j])));
         if (proj < l[j]) proj = l[j];
         if (proj > u[j]) proj = u[j];
-        out[j] = fabsf(__fsub_rn(xj, proj)) / fmaxf(1e-4f, step);
+        col_out[j] = fabsf(__fsub_rn(xj, proj)) / fmaxf(1e-4f, step);
+    }
+    // rows from the other end of the grid, whose blocks have fewer columns
+    for (int i = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride) {
+        const float a = ax[i];
+        float viol = 0.0f;
+        if (rl[i] > -1e15f && a < rl[i]) viol = fmaxf(viol, __fsub_rn(rl[i], a));
+        if (ru[i] < 1e15f && a > ru[i]) viol = fmaxf(viol, __fsub_rn(a, ru[i]));
+        row_out[i] = viol;
     }
 }
 
-static int grid_for(int n, int per_block) {
+static int sm_count() {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return std::max(1, std::min((n + per_block - 1) / per_block, sms * 8));
+    return sms;
 }
 
-// Lanes per segment from the mean segment length.  The last pointer is read
-// once per (pointer, size) and cached, so only the first launch on a matrix
-// synchronizes its stream.
-static int lanes_for(int nseg, const int* d_ptr, cudaStream_t s) {
-    static std::mutex mu;
-    static std::map<std::pair<const int*, int>, int> cache;
-    {
-        std::lock_guard<std::mutex> g(mu);
-        auto it = cache.find({d_ptr, nseg});
-        if (it != cache.end()) return it->second;
-    }
-    int nnz = 0;
-    if (nseg > 0) {
-        cudaMemcpyAsync(&nnz, d_ptr + nseg, sizeof(int), cudaMemcpyDeviceToHost, s);
-        cudaStreamSynchronize(s);
-    }
-    const double mean = nseg > 0 ? (double)nnz / nseg : 1.0;
-    int L = 1;
-    while (L < 32 && 4.0 * L <= mean) L *= 2;
-    std::lock_guard<std::mutex> g(mu);
-    cache[{d_ptr, nseg}] = L;
-    return L;
-}
+static int grid_for(int n) { return std::max(1, std::min((n + 255) / 256, sm_count() * 8)); }
 
 static int split_spmv(int nseg, const int* ptr, const int* idx, const float* val, const float* vec, float* out,
                       void* stream) {
     if (nseg < 0) return fail(SIH_PDHG_ERR_INVALID_ARGUMENT, "negative dimension");
     if (nseg == 0) return SIH_PDHG_OK;
     if (!ptr || !out || !vec) return fail(SIH_PDHG_ERR_INVALID_ARGUMENT, "NULL device pointer");
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int L = lanes_for(nseg, ptr, s);
-    split_spmv_kernel<<<grid_for(nseg, 256 / L), 256, 0, s>>>(nseg, ptr, idx, val, vec, out, L);
-    SIHG_LAUNCH_CHECK();
+    SIHG_CUDA(launch_chained(split_spmv_kernel, split_grid(nseg, sm_count()), kSplitThreads, 0,
+                             static_cast<cudaStream_t>(stream), nseg, ptr, idx, val, vec, out));
     return SIH_PDHG_OK;
 }
 
@@ -142,8 +221,10 @@ static int split_spmv(int nseg, const int* ptr, const int* idx, const float* val
 
 using namespace sihg;
 
-// Every launcher runs inside guarded(): the lane cache (std::map, std::mutex)
-// and the error messages can throw, and no exception may cross the C ABI.
+// Every launcher runs inside guarded(): the error messages can throw, and no
+// exception may cross the C ABI.  The kernels are chained (launch_chained): a
+// launcher's kernel is scheduled while the one before it in the stream ends, and
+// waits for it on the device.
 extern "C" int sih_pdhg_launch_csr_spmv(int m, const int* d_row_ptr, const int* d_col_ind, const float* d_values,
                                         const float* d_x, float* d_y, void* stream) {
     return guarded([&] { return split_spmv(m, d_row_ptr, d_col_ind, d_values, d_x, d_y, stream); });
@@ -160,9 +241,8 @@ extern "C" int sih_pdhg_launch_primal_update(int n, const float* d_tau, const fl
     return guarded([&]() -> int {
         if (n < 0) return fail(SIH_PDHG_ERR_INVALID_ARGUMENT, "negative dimension");
         if (n == 0) return SIH_PDHG_OK;
-        compat_primal_kernel<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(n, d_tau, d_c, d_AT_y, d_l, d_u, d_x,
-                                                                                 d_x_bar);
-        SIHG_LAUNCH_CHECK();
+        SIHG_CUDA(launch_chained(compat_primal_kernel, grid_for(n), 256, 0, (cudaStream_t)stream, n, d_tau, d_c, d_AT_y,
+                                 d_l, d_u, d_x, d_x_bar));
         return SIH_PDHG_OK;
     });
 }
@@ -172,9 +252,8 @@ extern "C" int sih_pdhg_launch_dual_update(int m, const float* d_sigma, const fl
     return guarded([&]() -> int {
         if (m < 0) return fail(SIH_PDHG_ERR_INVALID_ARGUMENT, "negative dimension");
         if (m == 0) return SIH_PDHG_OK;
-        compat_dual_kernel<<<grid_for(m, 256), 256, 0, (cudaStream_t)stream>>>(m, d_sigma, d_A_xbar, d_row_l, d_row_u,
-                                                                               d_y);
-        SIHG_LAUNCH_CHECK();
+        SIHG_CUDA(launch_chained(compat_dual_kernel, grid_for(m), 256, 0, (cudaStream_t)stream, m, d_sigma, d_A_xbar,
+                                 d_row_l, d_row_u, d_y));
         return SIH_PDHG_OK;
     });
 }
@@ -183,8 +262,7 @@ extern "C" int sih_pdhg_launch_restart(int n, const float* d_x, float* d_x_bar, 
     return guarded([&]() -> int {
         if (n < 0) return fail(SIH_PDHG_ERR_INVALID_ARGUMENT, "negative dimension");
         if (n == 0) return SIH_PDHG_OK;
-        compat_copy_kernel<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(n, d_x, d_x_bar);
-        SIHG_LAUNCH_CHECK();
+        SIHG_CUDA(launch_chained(compat_copy_kernel, grid_for(n), 256, 0, (cudaStream_t)stream, n, d_x, d_x_bar));
         return SIH_PDHG_OK;
     });
 }
@@ -195,11 +273,9 @@ extern "C" int sih_pdhg_launch_residuals(int m, int n, const float* d_Ax, const 
                                          void* stream) {
     return guarded([&]() -> int {
         if (m < 0 || n < 0) return fail(SIH_PDHG_ERR_INVALID_ARGUMENT, "negative dimension");
-        cudaStream_t s = (cudaStream_t)stream;
-        if (m > 0) compat_row_viol_kernel<<<grid_for(m, 256), 256, 0, s>>>(m, d_Ax, d_row_l, d_row_u, d_row_viols);
-        if (n > 0)
-            compat_col_viol_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, d_x, d_c, d_AT_y, d_l, d_u, d_tau, d_col_viols);
-        SIHG_LAUNCH_CHECK();
+        if (m == 0 && n == 0) return SIH_PDHG_OK;
+        SIHG_CUDA(launch_chained(compat_residuals_kernel, grid_for(std::max(m, n)), 256, 0, (cudaStream_t)stream, m, n,
+                                 d_Ax, d_row_l, d_row_u, d_row_viols, d_x, d_c, d_AT_y, d_l, d_u, d_tau, d_col_viols));
         return SIH_PDHG_OK;
     });
 }

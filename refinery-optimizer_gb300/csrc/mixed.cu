@@ -46,17 +46,6 @@
 
 namespace sihg {
 
-// Programmatic dependent launch.  The step kernels are launched with
-// programmatic stream serialization (launch_chained): their blocks may be
-// scheduled while the previous kernel in the stream finishes, and wait here,
-// before their first memory access, until it has completed and its writes are
-// visible; then they let the next kernel be scheduled.  Without the launch
-// attribute both instructions do nothing.
-__device__ __forceinline__ void chain_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // ---------------------------------------------------------------- step kernels
 // Elementwise part of a step.  Columns: pending float-float average update of
 // x, then x' = clip(x - tau (c + K^T y), l, u).  Rows: pending average update of y.
@@ -1595,24 +1584,6 @@ int check_grid_barrier(int blocks, int missing, int rounds, double limit_sec, in
     if (timed_out) *timed_out = (int)h[2];
     if (passed) *passed = (int)(h[6] / (unsigned)blocks);
     return SIH_PDHG_OK;
-}
-
-// Launches a step kernel (which starts with chain_wait) with programmatic
-// stream serialization.
-template <class... P, class... A>
-static cudaError_t launch_chained(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s,
-                                  A... args) {
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 int MixedSolver::launch_step(cudaStream_t s) {

@@ -50,12 +50,6 @@ __global__ void noalloc_finish_kernel(const unsigned* words, float max_abs_b, fl
     }
 }
 
-static int lanes_for_mean(double mean) {  // the launchers' choice (compat.cu)
-    int L = 1;
-    while (L < 32 && 4.0 * L <= mean) L *= 2;
-    return L;
-}
-
 static int grid_for(int n, int per_block, int sms) {
     return std::max(1, std::min((n + per_block - 1) / per_block, sms * 8));
 }
@@ -152,11 +146,10 @@ static int check_norms_noalloc_impl(int m, int n, int nnz, const int* d_row_ptr,
     unsigned* words = reinterpret_cast<unsigned*>(scratch + 2 * kNoAllocMaxRowsCols);  // 2 max words
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     noalloc_clear_kernel<<<1, 32, 0, s>>>(words);
-    const int Lr = lanes_for_mean((double)nnz / m), Lc = lanes_for_mean((double)nnz / n);
-    split_spmv_kernel<<<grid_for(m, 256 / Lr, sms), 256, 0, s>>>(m, d_row_ptr, d_col_ind, d_csr_values, d_x, ax, Lr);
-    split_spmv_kernel<<<grid_for(n, 256 / Lc, sms), 256, 0, s>>>(n, d_col_ptr, d_row_ind, d_csc_values, d_y, aty, Lc);
-    compat_row_viol_kernel<<<grid_for(m, 256, sms), 256, 0, s>>>(m, ax, d_row_l, d_row_u, row_map);
-    compat_col_viol_kernel<<<grid_for(n, 256, sms), 256, 0, s>>>(n, d_x, d_c, aty, d_l, d_u, d_tau, col_map);
+    split_spmv_kernel<<<split_grid(m, sms), kSplitThreads, 0, s>>>(m, d_row_ptr, d_col_ind, d_csr_values, d_x, ax);
+    split_spmv_kernel<<<split_grid(n, sms), kSplitThreads, 0, s>>>(n, d_col_ptr, d_row_ind, d_csc_values, d_y, aty);
+    compat_residuals_kernel<<<grid_for(std::max(m, n), 256, sms), 256, 0, s>>>(
+        m, n, ax, d_row_l, d_row_u, row_map, d_x, d_c, aty, d_l, d_u, d_tau, col_map);
     noalloc_max_kernel<<<grid_for(m, 256, sms), 256, 0, s>>>(m, row_map, words, 0);
     noalloc_max_kernel<<<grid_for(n, 256, sms), 256, 0, s>>>(n, col_map, words, 1);
     noalloc_finish_kernel<<<1, 32, 0, s>>>(words, max_abs_b, max_abs_c, d_out);

@@ -108,3 +108,52 @@ def test_update_launchers_bit_exact(env):
     proj = np.minimum(np.maximum(proj, l), u)
     meas = (np.abs(xn - proj) / np.maximum(np.float32(1e-4), tau)).astype(np.float32)
     np.testing.assert_array_equal(cvl.cpu().numpy(), meas)
+
+
+@pytest.mark.parametrize("nseg", [1, 31, 32767, 32768, 32769, 40001])
+@pytest.mark.parametrize("kind", ["mixed", "short", "long"])
+def test_spmv_launcher_by_segment_count_and_lengths(env, nseg, kind):
+    """Both ways of the SpMV kernel (groups of lanes; from 32,768 segments and
+    below a mean of 64 entries, 32 segments a warp by stream) on empty
+    segments and lengths around a lane's, a warp's and a window's share.  FP32
+    products and sums of k terms: |error| <= (k + 1) eps sum |a x|."""
+    torch, lib, _ = env
+    rng = np.random.default_rng(nseg)
+    lens = {"mixed": rng.choice([0, 1, 2, 7, 31, 32, 33, 48, 49, 255], nseg),
+            "short": rng.integers(0, 4, nseg), "long": np.full(nseg, 70)}[kind]
+    for k, v in ((3, 513), (nseg // 2, 2047), (nseg - 1, 512)):  # windows end inside and at segments
+        if k < nseg and kind != "long":
+            lens[k] = v
+    ptr = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    nnz, nvec = int(ptr[-1]), 5000
+    idx = rng.integers(0, nvec, nnz).astype(np.int32)
+    val = rng.standard_normal(nnz).astype(np.float32)
+    vec = rng.standard_normal(nvec).astype(np.float32)
+    d = [_dev(torch, a) for a in (ptr, idx, val, vec)]
+    out = torch.full((nseg,), 7.0, dtype=torch.float32, device="cuda")
+    for fn in (lib.sih_pdhg_launch_csr_spmv, lib.sih_pdhg_launch_csc_spmv):
+        out.fill_(7.0)
+        assert fn(nseg, *[a.data_ptr() for a in d], out.data_ptr(), None) == 0
+        torch.cuda.synchronize()
+        seg = np.repeat(np.arange(nseg), lens)
+        prod = val.astype(np.float64) * vec[idx]
+        ref = np.bincount(seg, weights=prod, minlength=nseg)
+        tol = (lens + 1) * 1.2e-7 * np.bincount(seg, weights=np.abs(prod), minlength=nseg)
+        assert np.all(np.abs(out.cpu().numpy() - ref) <= tol + 1e-30)
+
+
+def test_chained_launchers_see_each_other(env):
+    """Launchers wait on the device for the kernel before them: a chain in one
+    stream, each reading what the one before wrote, and a copy behind it."""
+    torch, lib, _ = env
+    n = 200_000
+    s = torch.cuda.Stream()
+    a = torch.zeros(n, device="cuda")
+    b = torch.zeros(n, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        for k in range(1, 21):
+            a.add_(1.0)  # not a chained kernel
+            assert lib.sih_pdhg_launch_restart(n, a.data_ptr(), b.data_ptr(), s.cuda_stream) == 0
+            assert lib.sih_pdhg_launch_restart(n, b.data_ptr(), a.data_ptr(), s.cuda_stream) == 0
+            assert float(b.min()) == k and float(a.max()) == k
