@@ -126,18 +126,21 @@ struct CgSEpi {
 };
 
 __global__ void __launch_bounds__(kThreads) k_cg_q(Side res_side, CgVecs V, CgInst* __restrict__ st) {
+    chain_wait();
     CgQEpi epi{V};
     spmv_engine<1, false, 1>(res_side, st, epi, 0u);
 }
 
 __global__ void __launch_bounds__(kThreads) k_cg_s(Side unk_side, CgVecs V, CgInst* __restrict__ st,
                                                    unsigned* done_count, double tol) {
+    chain_wait();
     CgSEpi epi{V, done_count, tol};
     spmv_engine<1, false, 1>(unk_side, st, epi, 0u);
 }
 
 // r -= alpha q (residual side), z += alpha p (unknown side)
 __global__ void __launch_bounds__(kThreads) k_cg_step(Chunks ch, CgVecs V, CgInst* __restrict__ st, int unk_col) {
+    chain_wait();
     for_each_element(ch, st, [](const CgInst& S) { return (float)S.alpha; }, [&](bool is_col, float a, int k) {
         if (is_col == (unk_col != 0))
             V.z[k] = fmaf(a, V.p[k], V.z[k]);
@@ -148,6 +151,7 @@ __global__ void __launch_bounds__(kThreads) k_cg_step(Chunks ch, CgVecs V, CgIns
 
 // p = s + beta p (unknown side)
 __global__ void __launch_bounds__(kThreads) k_cg_dir(Chunks ch, CgVecs V, CgInst* __restrict__ st, int unk_col) {
+    chain_wait();
     for_each_element(ch, st, [](const CgInst& S) { return (float)S.beta; }, [&](bool is_col, float b, int k) {
         if (is_col == (unk_col != 0)) V.p[k] = fmaf(b, V.p[k], V.s[k]);
     });
@@ -218,8 +222,6 @@ class CglsBatch {
     CglsBatch(const CglsBatch&) = delete;
     CglsBatch& operator=(const CglsBatch&) = delete;
     ~CglsBatch() {
-        for (auto& g : graph_)
-            if (g) cudaGraphExecDestroy(g);
         if (s_) cudaStreamDestroy(s_);
     }
 
@@ -229,6 +231,7 @@ class CglsBatch {
     // R-masked] for every instance; z in FP64 on the unknown side (global
     // order).  iters and status accumulate over calls.
     int solve(bool primal, const std::vector<double>& rhs, std::vector<double>& z);
+    long long nnz() const { return nnz_; }
 
     std::vector<int> roff, coff;
     std::vector<long long> iters;
@@ -242,10 +245,10 @@ class CglsBatch {
     const sih_pdhg_problem* probs_ = nullptr;
     const std::vector<Basis>* basis_ = nullptr;
     int B_ = 0, M_ = 0, N_ = 0, grid_ = 1, egrid_ = 1;
+    long long nnz_ = 0;
     long long max_iters_opt_ = 0;
     double tol_ = 1e-6;
     cudaStream_t s_ = nullptr;
-    cudaGraphExec_t graph_[2] = {nullptr, nullptr};
     DevMem csr_ptr_, csc_ptr_, csr_, csc_, vec_, state_, done_;
     TaskLayout layout_;
     Side rows_{}, cols_{};
@@ -275,6 +278,7 @@ int CglsBatch::setup(const sih_pdhg_problem* problems, int count, const std::vec
     }
     M_ = roff[count];
     N_ = coff[count];
+    nnz_ = nnz;
     if ((long long)M_ >= INT32_MAX - 64 || (long long)N_ >= INT32_MAX - 64 || nnz >= INT32_MAX - 64)
         return fail(SIH_PDHG_ERR_UNSUPPORTED, "batch exceeds the 32-bit index layout");
     std::vector<int> csr_ptr((size_t)M_ + 1), csc_ptr((size_t)N_ + 1);
@@ -283,7 +287,7 @@ int CglsBatch::setup(const sih_pdhg_problem* problems, int count, const std::vec
     R_.assign(M_, 0.f);
     std::vector<long long> koff(count + 1, 0);
     for (int b = 0; b < count; ++b) koff[b + 1] = koff[b] + hps[b].nnz;
-    parallel_for_min(count, 1, [&](int64_t b0, int64_t b1) {
+    parallel_for_min(count, work_chunk(count, 2.0 * (double)nnz), [&](int64_t b0, int64_t b1) {
         for (int64_t b = b0; b < b1; ++b) {
             const HostProblem& hp = hps[b];
             const int ro = roff[b], co = coff[b];
@@ -345,7 +349,7 @@ int CglsBatch::setup(const sih_pdhg_problem* problems, int count, const std::vec
 // dual out[cols] = F .* A^T (R .* z).
 void CglsBatch::product(bool primal, const std::vector<double>& z, std::vector<double>& out) const {
     out.assign(primal ? M_ : N_, 0.0);
-    parallel_for_min(B_, 1, [&](int64_t b0, int64_t b1) {
+    parallel_for_min(B_, work_chunk(B_, 2.0 * (double)nnz_), [&](int64_t b0, int64_t b1) {
         for (int64_t b = b0; b < b1; ++b) {
             const sih_pdhg_problem* p = &probs_[b];
             const Basis& bs = (*basis_)[b];
@@ -386,27 +390,21 @@ int CglsBatch::run_cgls(bool primal, const std::vector<float>& rhs, std::vector<
     CgInst* st = state_.as<CgInst>();
     unsigned* done = done_.as<unsigned>();
     constexpr int kBlock = 32;
-    cudaGraphExec_t& ge = graph_[primal ? 1 : 0];
-    if (!ge) {  // CGLS iterations in blocks of 32, one CUDA graph per orientation
-        cudaGraph_t g = nullptr;
-        SIHG_CUDA(cudaStreamBeginCapture(s_, cudaStreamCaptureModeThreadLocal));
+    // CGLS iterations in blocks of 32, chained launches (a graph of a block cost
+    // more to instantiate per call, 0.3 ms, than its launches)
+    auto block = [&]() -> int {
         // the task counters restart with every block (a launch takes a fixed
         // number of counter values, see task_loop)
-        cudaError_t e = cudaMemsetAsync(rows_.counters, 0, sizeof(unsigned), s_);
-        if (e == cudaSuccess) e = cudaMemsetAsync(cols_.counters, 0, sizeof(unsigned), s_);
-        for (int k = 0; k < kBlock && e == cudaSuccess; ++k) {
-            k_cg_q<<<grid_, kThreads, 0, s_>>>(res_side, V, st);
-            k_cg_step<<<egrid_, kThreads, 0, s_>>>(ch_, V, st, unk_col);
-            k_cg_s<<<grid_, kThreads, 0, s_>>>(unk_side, V, st, done, tol_);
-            k_cg_dir<<<egrid_, kThreads, 0, s_>>>(ch_, V, st, unk_col);
+        SIHG_CUDA(cudaMemsetAsync(rows_.counters, 0, sizeof(unsigned), s_));
+        SIHG_CUDA(cudaMemsetAsync(cols_.counters, 0, sizeof(unsigned), s_));
+        for (int k = 0; k < kBlock; ++k) {
+            SIHG_CUDA(launch_chained(k_cg_q, grid_, kThreads, 0, s_, res_side, V, st));
+            SIHG_CUDA(launch_chained(k_cg_step, egrid_, kThreads, 0, s_, ch_, V, st, unk_col));
+            SIHG_CUDA(launch_chained(k_cg_s, grid_, kThreads, 0, s_, unk_side, V, st, done, tol_));
+            SIHG_CUDA(launch_chained(k_cg_dir, egrid_, kThreads, 0, s_, ch_, V, st, unk_col));
         }
-        const cudaError_t e2 = cudaStreamEndCapture(s_, &g);
-        if (e != cudaSuccess) return cuda_fail(e, "graph capture", __FILE__, __LINE__);
-        if (e2 != cudaSuccess) return cuda_fail(e2, "cudaStreamEndCapture", __FILE__, __LINE__);
-        e = cudaGraphInstantiate(&ge, g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate", __FILE__, __LINE__);
-    }
+        return SIH_PDHG_OK;
+    };
     const int nres = primal ? M_ : N_, nunk = primal ? N_ : M_;
     SIHG_CUDA(cudaMemcpyAsync(V.r, rhs.data(), sizeof(float) * nres, cudaMemcpyHostToDevice, s_));
     SIHG_CUDA(cudaMemsetAsync(V.q, 0, sizeof(float) * nres, s_));
@@ -431,7 +429,7 @@ int CglsBatch::run_cgls(bool primal, const std::vector<float>& rhs, std::vector<
         SIHG_CUDA(cudaMemcpyAsync(&h_done, done, sizeof(unsigned), cudaMemcpyDeviceToHost, s_));
         SIHG_CUDA(cudaStreamSynchronize(s_));
         if ((int)h_done >= B_) break;
-        SIHG_CUDA(cudaGraphLaunch(ge, s_));
+        SIHG_TRY(block());
     }
     z.resize(nunk);
     SIHG_CUDA(cudaMemcpyAsync(z.data(), V.z, sizeof(float) * nunk, cudaMemcpyDeviceToHost, s_));
@@ -486,7 +484,9 @@ int prepare(const sih_pdhg_problem* problems, int count, const double* const* xs
         SIHG_TRY(build_host_problem(&problems[b], hps[b]));
         if (!xs[b] || !ys[b]) return fail(SIH_PDHG_ERR_INVALID_ARGUMENT, "NULL x or row_duals");
     }
-    parallel_for_min(count, 1, [&](int64_t b0, int64_t b1) {
+    double work = 0.0;  // products, norms, logarithms and a sort
+    for (const HostProblem& hp : hps) work += 4.0 * hp.nnz + 64.0 * ((double)hp.m + hp.n);
+    parallel_for_min(count, work_chunk(count, work), [&](int64_t b0, int64_t b1) {
         for (int64_t b = b0; b < b1; ++b) choose_basis(&problems[b], xs[b], ys[b], basis[b]);
     });
     return SIH_PDHG_OK;
@@ -543,7 +543,7 @@ static int adjoint_batch_impl(const sih_pdhg_problem* problems, int32_t count, c
     for (int b = 0; b < count; ++b)
         for (int64_t j = 0; j < problems[b].num_cols; ++j) rhs[cg.coff[b] + j] = grad_x[b][j];
     SIHG_TRY(cg.solve(false, rhs, lam));
-    parallel_for_min(count, 1, [&](int64_t b0, int64_t b1) {
+    parallel_for_min(count, work_chunk(count, 2.0 * (double)cg.nnz()), [&](int64_t b0, int64_t b1) {
         for (int64_t b = b0; b < b1; ++b) {
             const sih_pdhg_problem* p = &problems[b];
             const Basis& bs = basis[b];
@@ -613,7 +613,7 @@ static int polish_batch_impl(const sih_pdhg_problem* problems, int32_t count, co
     const int M = cg.roff[count], N = cg.coff[count];
     // primal: B x_F = b_act - A[act, N] x_N, the non-free columns at their bounds
     std::vector<double> xn((size_t)N, 0.0), rhs((size_t)M, 0.0), xf, cf((size_t)N, 0.0), lam;
-    parallel_for_min(count, 1, [&](int64_t b0, int64_t b1) {
+    parallel_for_min(count, work_chunk(count, 2.0 * (double)cg.nnz()), [&](int64_t b0, int64_t b1) {
         for (int64_t b = b0; b < b1; ++b) {
             const sih_pdhg_problem* p = &problems[b];
             const Basis& bs = basis[b];
@@ -641,7 +641,7 @@ static int polish_batch_impl(const sih_pdhg_problem* problems, int32_t count, co
     const std::vector<double> res_p(cg.residual);
     // dual: B^T lambda = c_F (simplex duals of the internal minimisation)
     SIHG_TRY(cg.solve(false, cf, lam));
-    parallel_for_min(count, 1, [&](int64_t b0, int64_t b1) {
+    parallel_for_min(count, work_chunk(count, 2.0 * (double)cg.nnz()), [&](int64_t b0, int64_t b1) {
         for (int64_t b = b0; b < b1; ++b) {
             const sih_pdhg_problem* p = &problems[b];
             const Basis& bs = basis[b];

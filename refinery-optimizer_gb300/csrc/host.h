@@ -84,6 +84,13 @@ void parallel_for(int64_t count, F&& f) {
     parallel_for_min(count, (int64_t)1 << 16, static_cast<F&&>(f));
 }
 
+// Least items per thread for `count` items of `work` operations in all, so that
+// a thread (about 20 us to start and join) has at least 65,536 of them.
+inline int64_t work_chunk(int64_t count, double work) {
+    const double items = work > 0.0 ? 65536.0 * (double)count / work : (double)count;
+    return items >= (double)count ? (count > 0 ? count : 1) : (int64_t)items + 1;
+}
+
 // Splits [0, count) into `parts` contiguous ranges (range t to part t) and runs
 // f(begin, end, t) on them in parallel; below 2 x 65,536 items everything runs
 // as part 0 on the calling thread.

@@ -80,7 +80,7 @@ int TaskLayout::build(const std::vector<int>& csr_ptr, const std::vector<int>& c
                       const std::vector<int>& coff, const SegMatrix& rows_A, const SegMatrix& cols_A, int task_nnz,
                       bool all_active, cudaStream_t s, int row_lanes, int col_lanes, int max_segs) {
     const int B = (int)roff.size() - 1;
-    SideSchedule rs, cs;
+    SideSchedule &rs = row_schedule, &cs = col_schedule;
     make_schedule(csr_ptr, roff, task_nnz, rs, row_lanes, max_segs);
     make_schedule(csc_ptr, coff, task_nnz, cs, col_lanes, max_segs);
     // per side: tickets [B] + counters [2] + group tickets [ngroups], zeroed once;

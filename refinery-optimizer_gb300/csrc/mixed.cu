@@ -29,6 +29,7 @@
 // the reference's y <- sigma (w - clip(w, rl, ru)), w = K xbar + y / sigma
 // (core/src/gpu/cuda_pdhg.cu:82-103), with K xbar = 2 K x' - K x by linearity.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -1195,7 +1196,8 @@ int MixedSolver::setup(const std::vector<const HostProblem*>& probs, const sih_p
     std::vector<long long> k_off(B_ + 1, 0);
     for (int b = 0; b < B_; ++b) k_off[b + 1] = k_off[b] + probs[b]->nnz;
     const bool reorder = opts.reorder != 0;
-    parallel_for_min(2 * (int64_t)B_, 1, [&](int64_t w0, int64_t w1) {
+    const double vec_work = 8.0 * ((double)N_ + M_);
+    parallel_for_min(2 * (int64_t)B_, work_chunk(2 * (int64_t)B_, vec_work), [&](int64_t w0, int64_t w1) {
         for (int64_t w = w0; w < w1; ++w) {
             const int b = (int)(w >> 1);
             const HostProblem& p = *probs[b];
@@ -1237,7 +1239,7 @@ int MixedSolver::setup(const std::vector<const HostProblem*>& probs, const sih_p
         if (std::isinf(v) || std::fabs(v) >= 1e20) return v > 0 ? INFINITY : -INFINITY;
         return (float)v;
     };
-    parallel_for_min((int64_t)pieces.size(), 1, [&](int64_t q0, int64_t q1) {
+    parallel_for_min((int64_t)pieces.size(), work_chunk((int64_t)pieces.size(), vec_work), [&](int64_t q0, int64_t q1) {
         for (int64_t q = q0; q < q1; ++q) {
             const Piece& pc = pieces[q];
             const HostProblem& p = *probs[pc.b];
@@ -1419,11 +1421,7 @@ int MixedSolver::setup_resident() {
     if (B_ == 1 && persistent_ != 2) return SIH_PDHG_OK;
     // (a batch: no cluster holds the mean instance)
     if (B_ > 1 && 16.0 * (double)nnz_ > 220.0 * 1024.0 * 16.0 * B_) return SIH_PDHG_OK;
-    SideSchedule rs, cs;
-    const int segs = latency_bound() ? kSoloTaskSegs : kTaskSegs;
-    make_schedule(h_csr_ptr_, row_off_, task_nnz_, rs, lanes_r_, segs);
-    make_schedule(h_csc_ptr_, col_off_, task_nnz_, cs, lanes_c_, segs);
-    const std::vector<uint8_t> rl = segment_lanes(rs, M_), cl = segment_lanes(cs, N_);
+    const std::vector<uint8_t> rl = segment_lanes(layout_.row_schedule, M_), cl = segment_lanes(layout_.col_schedule, N_);
     SIHG_TRY(resident_->build(h_csr_ptr_, h_csc_ptr_, row_off_, col_off_, rl, cl, sm_count_, stream_,
                               ResidentPlan::kCluster));
     if (!resident_->ready() && B_ == 1)
@@ -1702,6 +1700,7 @@ int MixedSolver::launch_compact(cudaStream_t s) {
 
 int MixedSolver::reset_state() {
     cudaStream_t s = stream_;
+    pulled_ = false;
     const int g = sm_count_ * 4;
     for (int b = 0; b < B_; ++b) {
         Inst& S = host_inst_[b];
@@ -1805,6 +1804,7 @@ int MixedSolver::run() {
     // stopped (a window of kWindow blocks in flight; the done count of the
     // oldest is read back before the next is queued).
     auto run_blocks = [&]() -> int {
+        pulled_ = false;
         for (long long k = 0; blk < blk_end; blk += periods, ++k) {
             const int slot = (int)(k % kWindow);
             if (k >= kWindow) {
@@ -1859,16 +1859,33 @@ int MixedSolver::run() {
     constexpr int kVerifyRounds = 4;
     for (int round = 0; rc == SIH_PDHG_OK && round <= kVerifyRounds && !timed_out_; ++round) {
         std::vector<int> redo;
-        std::vector<double> x, y;
-        for (int b = 0; b < B_ && rc == SIH_PDHG_OK; ++b) {
-            const Inst& S = host_inst_[b];
-            if (S.done != 1) continue;
-            rc = fetch(b, x, y);
-            if (rc != SIH_PDHG_OK) break;
-            const KktReport k = host_kkt(probs_[b]->src, x.data(), y.data(), nullptr, nullptr);
-            if (!(k.rel_primal <= cfg_.tol_primal && k.rel_dual <= cfg_.tol_dual && k.rel_gap <= cfg_.tol_gap))
-                redo.push_back(b);
+        std::vector<char> fails(B_, 0);
+        std::atomic<bool> no_memory{false};
+        bool any = false;
+        for (int b = 0; b < B_; ++b) any = any || host_inst_[b].done == 1;
+        if (any) rc = pull_points();
+        if (rc != SIH_PDHG_OK) break;
+        // instances side by side; one large instance splits its own rows and columns
+        parallel_for_min(any ? B_ : 0, work_chunk(B_, 2.0 * (double)nnz_), [&](int64_t b0, int64_t b1) {
+            try {  // (an exception must not leave a thread)
+                std::vector<double> x, y;
+                for (int64_t b = b0; b < b1; ++b) {
+                    if (host_inst_[b].done != 1) continue;
+                    unscale((int)b, x, y);
+                    const KktReport k = host_kkt(probs_[b]->src, x.data(), y.data(), nullptr, nullptr);
+                    fails[b] =
+                        !(k.rel_primal <= cfg_.tol_primal && k.rel_dual <= cfg_.tol_dual && k.rel_gap <= cfg_.tol_gap);
+                }
+            } catch (const std::exception&) {
+                no_memory.store(true);
+            }
+        });
+        if (no_memory.load()) {
+            rc = fail(SIH_PDHG_ERR_OUT_OF_MEMORY, "out of host memory");
+            break;
         }
+        for (int b = 0; b < B_; ++b)
+            if (fails[b]) redo.push_back(b);
         if (rc != SIH_PDHG_OK || redo.empty()) break;
         if (round == kVerifyRounds) {  // still above the tolerance in FP64: not reported as optimal
             for (int b : redo) host_inst_[b].done = 4;
@@ -1908,20 +1925,58 @@ int MixedSolver::run() {
     return SIH_PDHG_OK;
 }
 
-int MixedSolver::fetch(int b, std::vector<double>& x, std::vector<double>& y) {
-    const Inst& S = host_inst_[b];
+// Host copies of every instance's returned point (device order, scaled) and
+// of the scales, after a run: a copy per array that some instance returns from,
+// not several small ones per instance.
+int MixedSolver::pull_points() {
+    if (pulled_) return SIH_PDHG_OK;
+    if (h_scale_.empty()) {
+        h_scale_.resize((size_t)N_ + M_);
+        SIHG_CUDA(cudaMemcpy(h_scale_.data(), V_.dcol, sizeof(float) * N_, cudaMemcpyDeviceToHost));
+        SIHG_CUDA(cudaMemcpy(h_scale_.data() + N_, V_.drow, sizeof(float) * M_, cudaMemcpyDeviceToHost));
+    }
+    bool used[3] = {false, false, false};
+    auto which = [&](int b) { return host_inst_[b].out_sel == 1 ? 2 : (host_inst_[b].cur ? 1 : 0); };
+    for (int b = 0; b < B_; ++b) used[which(b)] = true;
+    const float* xs[3] = {V_.x0, V_.x1, V_.x_avg};
+    const float* ys[3] = {V_.y0, V_.y1, V_.y_avg};
+    std::vector<float> part;  // more than one source: the instances' parts are picked out
+    h_point_.resize((size_t)N_ + M_);
+    const bool one = (int)used[0] + used[1] + used[2] == 1;
+    if (!one) part.resize((size_t)N_ + M_);
+    for (int k = 0; k < 3; ++k) {
+        if (!used[k]) continue;
+        float* to = one ? h_point_.data() : part.data();
+        SIHG_CUDA(cudaMemcpy(to, xs[k], sizeof(float) * N_, cudaMemcpyDeviceToHost));
+        SIHG_CUDA(cudaMemcpy(to + N_, ys[k], sizeof(float) * M_, cudaMemcpyDeviceToHost));
+        for (int b = 0; b < B_ && !one; ++b) {
+            if (which(b) != k) continue;
+            std::copy(to + col_off_[b], to + col_off_[b + 1], h_point_.data() + col_off_[b]);
+            std::copy(to + N_ + row_off_[b], to + N_ + row_off_[b + 1], h_point_.data() + N_ + row_off_[b]);
+        }
+    }
+    pulled_ = true;
+    return SIH_PDHG_OK;
+}
+
+// Instance b's point from the host copies, unscaled and in the caller's order.
+void MixedSolver::unscale(int b, std::vector<double>& x, std::vector<double>& y) const {
     const int n = probs_[b]->n, m = probs_[b]->m, co = col_off_[b], ro = row_off_[b];
-    std::vector<float> xs(n), ys(m), dc(n), dr(m);
-    const float* xsrc = S.out_sel == 1 ? V_.x_avg : (S.cur ? V_.x1 : V_.x0);
-    const float* ysrc = S.out_sel == 1 ? V_.y_avg : (S.cur ? V_.y1 : V_.y0);
-    SIHG_CUDA(cudaMemcpy(xs.data(), xsrc + co, sizeof(float) * n, cudaMemcpyDeviceToHost));
-    SIHG_CUDA(cudaMemcpy(ys.data(), ysrc + ro, sizeof(float) * m, cudaMemcpyDeviceToHost));
-    SIHG_CUDA(cudaMemcpy(dc.data(), V_.dcol + co, sizeof(float) * n, cudaMemcpyDeviceToHost));
-    SIHG_CUDA(cudaMemcpy(dr.data(), V_.drow + ro, sizeof(float) * m, cudaMemcpyDeviceToHost));
+    const float *xs = h_point_.data() + co, *ys = h_point_.data() + N_ + ro;
+    const float *dc = h_scale_.data() + co, *dr = h_scale_.data() + N_ + ro;
     x.resize(n);
     y.resize(m);
-    for (int j = 0; j < n; ++j) x[col_perm_[co + j]] = (double)xs[j] * (double)dc[j];
-    for (int i = 0; i < m; ++i) y[row_perm_[ro + i]] = (double)ys[i] * (double)dr[i];
+    parallel_for(n, [&](int64_t j0, int64_t j1) {
+        for (int64_t j = j0; j < j1; ++j) x[col_perm_[co + j]] = (double)xs[j] * (double)dc[j];
+    });
+    parallel_for(m, [&](int64_t i0, int64_t i1) {
+        for (int64_t i = i0; i < i1; ++i) y[row_perm_[ro + i]] = (double)ys[i] * (double)dr[i];
+    });
+}
+
+int MixedSolver::fetch(int b, std::vector<double>& x, std::vector<double>& y) {
+    SIHG_TRY(pull_points());
+    unscale(b, x, y);
     return SIH_PDHG_OK;
 }
 

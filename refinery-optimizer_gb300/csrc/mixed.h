@@ -126,6 +126,7 @@ class TaskLayout {
 
     Side rows{}, cols{};
     Chunks chunks{};
+    SideSchedule row_schedule, col_schedule;  // as built
     // 3 x B ints after the three active counts (scratch of the compaction)
     int* compaction_offsets() const { return rows.nactive + 3; }
 
@@ -184,6 +185,8 @@ class MixedSolver {
 
   private:
     int reset_state();
+    int pull_points();
+    void unscale(int b, std::vector<double>& x, std::vector<double>& y) const;
     int build_schedules(int task_nnz);
     bool latency_bound() const;  // one LP small enough that its steps are latency-bound
     int autotune();
@@ -240,6 +243,9 @@ class MixedSolver {
     int packed_ = 0;  // options.packed: two kernels per step on packed column records
     Vecs V_{};
     std::vector<Inst> host_inst_;
+    // host copies of the last run's points (columns, then rows), and the scales (constant after set-up)
+    std::vector<float> h_point_, h_scale_;
+    bool pulled_ = false;
     std::vector<std::vector<float>> start_x_, start_y_;  // warm starts (device order, unscaled)
 };
 

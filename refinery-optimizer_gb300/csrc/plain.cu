@@ -248,19 +248,17 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
         SIHG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, plain_primal_tasks, kThreads, 0));
         task_grid_ = sm_count_ * std::max(1, occ);
         const long long warps = (long long)task_grid_ * (kThreads / 32);
-        task_nnz_ = opts.tile_nnz > 0
-                        ? opts.tile_nnz
-                        : (int)std::max(128LL, std::min(2048LL, (long long)nnz / std::max(1LL, 3 * warps)));
+        const int task_nnz = opts.tile_nnz > 0
+                                 ? opts.tile_nnz
+                                 : (int)std::max(128LL, std::min(2048LL, (long long)nnz / std::max(1LL, 3 * warps)));
         SIHG_TRY(layout_.build(hp.csr_ptr, hp.csc_ptr, std::vector<int>{0, m}, std::vector<int>{0, n}, A_, At_,
-                               task_nnz_, true, s));
+                               task_nnz, true, s));
     }
 
     if (layout_.rows.ntasks > 0 && opts.use_graph) {  // LPs that fit: every iteration in one cluster
-        SideSchedule rs, cs;
-        make_schedule(hp.csr_ptr, std::vector<int>{0, m}, task_nnz_, rs);
-        make_schedule(hp.csc_ptr, std::vector<int>{0, n}, task_nnz_, cs);
         SIHG_TRY(resident_->build(hp.csr_ptr, hp.csc_ptr, std::vector<int>{0, m}, std::vector<int>{0, n},
-                                  segment_lanes(rs, m), segment_lanes(cs, n), sm_count_, s, ResidentPlan::kPlain));
+                                  segment_lanes(layout_.row_schedule, m), segment_lanes(layout_.col_schedule, n),
+                                  sm_count_, s, ResidentPlan::kPlain));
         if (resident_->ready()) SIHG_TRY(resident_->fill(A_, At_, s));
     }
 

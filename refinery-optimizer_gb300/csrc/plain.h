@@ -102,7 +102,7 @@ class PlainSolver {
     cudaGraphExec_t block_exec_ = nullptr, tail_exec_ = nullptr;
     DevMem csc_ptr_, csr_ptr_, csc_pairs_, csr_pairs_, colvec_, rowvec_, state_, heavy_;
     TaskLayout layout_;   // task engine of the fast (non-exact) iteration kernels
-    int task_grid_ = 1, task_nnz_ = 0;
+    int task_grid_ = 1;
     std::unique_ptr<ResidentPlan> resident_;  // LPs that fit in a cluster: iterations and checks there
     SegMatrix A_{}, At_{};
     SpmvPlan plan_csr_{}, plan_csc_{};

@@ -1333,7 +1333,6 @@ __global__ void k_resident_fill(int npass, const int4* __restrict__ place, SegMa
     }
 }
 
-int align16(int v) { return (v + 15) & ~15; }
 
 }  // namespace
 
@@ -1374,76 +1373,76 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
             if ((16.0 * nnz + 4.0 * (col_words * n + row_words * m)) / sm_count > budget) return SIH_PDHG_OK;
         } else if (4.0 * (m + n) + (16.0 * nnz + 4.0 * (col_words * n + row_words * m)) / 16.0 > budget) return SIH_PDHG_OK;
     }
-    std::vector<ResBlock> blocks;
-    std::vector<int4> passes, place, inst(B);
-    for (int b = 0; b < B; ++b) inst[b] = make_int4(coff[b], coff[b + 1] - coff[b], roff[b], roff[b + 1] - roff[b]);
+    // every instance's passes: {first segment, segments, width, log2 L}, rows of A then columns
+    std::vector<int4> inst(B), all;
+    std::vector<size_t> first(2 * (size_t)B + 1, 0);
+    for (int b = 0; b < B; ++b) {
+        inst[b] = make_int4(coff[b], coff[b + 1] - coff[b], roff[b], roff[b + 1] - roff[b]);
+        for (int h = 0; h < 2; ++h) {
+            const std::vector<int>& ptr = *ptrs[h];
+            const uint8_t* ln = lanes[h]->data();
+            const int s1 = (*offs[h])[b + 1];
+            for (int seg = (*offs[h])[b]; seg < s1;) {
+                const int L = ln[seg];
+                int e = seg, width = 0, lg = 0;
+                while ((1 << lg) < L) ++lg;
+                while (e < s1 && e - seg < 32 / L && ln[e] == L) {
+                    width = std::max(width, (ptr[e + 1] - ptr[e] + L - 1) / L);
+                    ++e;
+                }
+                all.push_back(make_int4(seg, e - seg, width, lg));
+                seg = e;
+            }
+            first[2 * b + h + 1] = all.size();
+        }
+    }
+    // calls f(pass, block of C) for the passes of an instance's side
+    auto deal = [&](int b, int h, int C, auto&& f) {
+        const size_t a0 = first[2 * b + h], a1 = first[2 * b + h + 1];
+        for (size_t q0 = a0; q0 < a1;) {
+            size_t q1 = q0;  // runs of equal lanes and width
+            while (q1 < a1 && all[q1].z == all[q0].z && all[q1].w == all[q0].w) ++q1;
+            const long long len = (long long)(q1 - q0);
+            for (size_t q = q0; q < q1; ++q) {
+                int r;
+                if (grid) {
+                    // each run spread evenly in its order: segments of one length keep the caller's
+                    // order, so that a block gets the same part of the LP from every run and side,
+                    // and its gathers, where the LP has a block structure, meet in its L1
+                    r = (int)((long long)(q - q0) * C / len);
+                    if (len < C) r = (int)((r + C / (2 * len)) % C);
+                } else {  // the passes run by descending length: dealt out back and forth
+                    const int t = (int)((q - a0) % (2 * (size_t)C));
+                    r = t < C ? t : 2 * C - 1 - t;
+                }
+                f(all[q], r);
+            }
+            q0 = q1;
+        }
+    };
     ResSmem sm{};
-    auto plan = [&](int C, int& most) -> long long {  // rows of entries; `most`: passes of a block
-        blocks.assign((size_t)B * C, ResBlock{});
-        passes.clear();
-        place.clear();
-        long long row = 0;
-        int mrows[2] = {0, 0}, mpass[2] = {0, 0}, mloc[2] = {0, 0}, mn = 0, mm = 0;
+    auto measure = [&](int C) -> int {  // the shared memory layout for clusters of C; most passes of a block
+        long long mrows[2] = {0, 0};
+        int mpass[2] = {0, 0}, mloc[2] = {0, 0}, mn = 0, mm = 0;
+        std::vector<int> npass(C), nloc(C);
+        std::vector<long long> nrow(C);
         for (int b = 0; b < B; ++b) {
             mn = std::max(mn, inst[b].y);
             mm = std::max(mm, inst[b].w);
             for (int h = 0; h < 2; ++h) {
-                const std::vector<int>& ptr = *ptrs[h];
-                const int s0 = (*offs[h])[b], s1 = (*offs[h])[b + 1];
-                const int other = (*offs[1 - h])[b];
-                std::vector<std::vector<int4>> mine(C), where(C);
-                std::vector<int> nrow(C, 0), nloc(C, 0);
-                // passes of equal lanes and width: runs [first pass, last)
-                std::vector<int4> all;  // {first segment, segments, width, log2 L}
-                for (int seg = s0; seg < s1;) {
-                    const int L = (*lanes[h])[seg];
-                    int e = seg, width = 0, lg = 0;
-                    while ((1 << lg) < L) ++lg;
-                    while (e < s1 && e - seg < 32 / L && (*lanes[h])[e] == L) {
-                        width = std::max(width, (ptr[e + 1] - ptr[e] + L - 1) / L);
-                        ++e;
-                    }
-                    all.push_back(make_int4(seg, e - seg, width, lg));
-                    seg = e;
-                }
-                for (size_t q0 = 0; q0 < all.size();) {
-                    size_t q1 = q0;
-                    while (q1 < all.size() && all[q1].z == all[q0].z && all[q1].w == all[q0].w) ++q1;
-                    for (size_t q = q0; q < q1; ++q) {
-                        int r;
-                        if (grid) {
-                            // each run spread evenly in its order: segments of one length keep the caller's
-                            // order, so that a block gets the same part of the LP from every run and side,
-                            // and its gathers, where the LP has a block structure, meet in its L1
-                            r = (int)((long long)(q - q0) * C / (long long)(q1 - q0));
-                            if (q1 - q0 < (size_t)C) r = (int)((r + C / (2 * (long long)(q1 - q0))) % C);
-                        } else {  // the passes run by descending length: dealt out back and forth
-                            const int t = (int)(q % (2 * (size_t)C));
-                            r = t < C ? t : 2 * C - 1 - t;
-                        }
-                        const int4 a = all[q];
-                        mine[r].push_back(make_int4(nrow[r], a.z | (a.w << 24), a.x - s0, nloc[r] | (a.y << 24)));
-                        where[r].push_back(make_int4(nrow[r], a.z, a.x, a.y));
-                        where[r].push_back(make_int4(other, h, 1 << a.w, 0));
-                        nrow[r] += a.z;
-                        nloc[r] += a.y;
-                    }
-                    q0 = q1;
-                }
-                for (int r = 0; r < C; ++r) {
-                    ResSide& sd = blocks[(size_t)b * C + r].side[h];
-                    sd = ResSide{(int)passes.size(), (int)mine[r].size(), (int)row, nrow[r], nloc[r]};
-                    for (size_t k = 0; k < where[r].size(); k += 2) where[r][k].x += (int)row;
-                    passes.insert(passes.end(), mine[r].begin(), mine[r].end());
-                    place.insert(place.end(), where[r].begin(), where[r].end());
-                    row += nrow[r];
-                    mrows[h] = std::max(mrows[h], nrow[r]);
-                    mpass[h] = std::max(mpass[h], sd.passes);
-                    mloc[h] = std::max(mloc[h], nloc[r]);
-                }
+                std::fill(npass.begin(), npass.end(), 0);
+                std::fill(nloc.begin(), nloc.end(), 0);
+                std::fill(nrow.begin(), nrow.end(), 0);
+                deal(b, h, C, [&](const int4& p, int r) {
+                    npass[r] += 1;
+                    nloc[r] += p.y;
+                    nrow[r] += p.z;
+                });
+                mpass[h] = std::max(mpass[h], *std::max_element(npass.begin(), npass.end()));
+                mloc[h] = std::max(mloc[h], *std::max_element(nloc.begin(), nloc.end()));
+                mrows[h] = std::max(mrows[h], *std::max_element(nrow.begin(), nrow.end()));
             }
         }
-        most = std::max(mpass[0], mpass[1]);
         long long at = 0;
         auto put = [&](long long bytes) {
             const long long a = at;
@@ -1461,24 +1460,23 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
         sm.red = put((long long)sizeof(Sums) * (32 + 16));
         sm.eval = put(kEvalQ * (8ll * 32 + 8ll * 16 + 8));
         sm.total = (int)std::min<long long>(at, INT32_MAX);
-        return row;
+        return std::max(mpass[0], mpass[1]);
     };
     // The smallest cluster that holds an instance; a larger one while SMs are
     // left over and a block has more than 8 passes a side (two warps per
     // scheduler): beyond that the barriers and pushes of more blocks cost what
     // the shorter phases save (317 x 803: 4 blocks of 9 passes and 8 of 5 are
     // equal).
-    int C = grid ? sm_count : 1, most = 0;
-    long long rows = plan(C, most);
-    while (!grid && C < 16 && sm.total > budget) rows = plan(C *= 2, most);
+    int C = grid ? sm_count : 1, most = measure(C);
+    while (!grid && C < 16 && sm.total > budget) most = measure(C *= 2);
     if (sm.total > budget) return SIH_PDHG_OK;
-    while (!grid && C < 16 && (long long)B * 2 * C <= sm_count && most > 8) rows = plan(C *= 2, most);
+    while (!grid && C < 16 && (long long)B * 2 * C <= sm_count && most > 8) most = measure(C *= 2);
     // 20 warps with passes at most (31: 3 % slower on the batch of 64, whose blocks have 39 passes)
     // (grid form: a thread per block sums)
     const int nw = grid ? kGridThreads / 32 - 1 : std::max(1, std::min(kResThreads / 32 - 1, most));
     threads_ = 32 * (nw + 1);
     if (grid && sm_count > threads_) return SIH_PDHG_OK;
-    npass_ = (int)passes.size();
+    npass_ = (int)all.size();
     SIHG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
     if (grid) {
         int occ = 0, coop = 0;
@@ -1506,14 +1504,45 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
             return SIH_PDHG_OK;
         }
     }
-    const size_t nb = sizeof(ResBlock) * blocks.size(), ni = sizeof(int4) * inst.size(),
-                 np = sizeof(int4) * passes.size(), nl = sizeof(int4) * place.size();
-    const size_t o_i = align16((int)nb), o_p = o_i + ni, o_l = o_p + np;
-    std::vector<char> buf(o_l + nl);
-    std::memcpy(buf.data(), blocks.data(), nb);
+    // the tables: blocks, instances, passes by block, and each pass's place in the matrix for the fill
+    const size_t nb = sizeof(ResBlock) * (size_t)B * C, ni = sizeof(int4) * (size_t)B, np = sizeof(int4) * all.size();
+    const size_t o_i = (nb + 15) & ~(size_t)15, o_p = o_i + ni, o_l = o_p + np;
+    std::vector<char> buf(o_l + 2 * np);
+    ResBlock* blocks = reinterpret_cast<ResBlock*>(buf.data());
     std::memcpy(buf.data() + o_i, inst.data(), ni);
-    std::memcpy(buf.data() + o_p, passes.data(), np);
-    std::memcpy(buf.data() + o_l, place.data(), nl);
+    int4* passes = reinterpret_cast<int4*>(buf.data() + o_p);
+    int4* place = reinterpret_cast<int4*>(buf.data() + o_l);
+    long long rows = 0;
+    {
+        std::vector<int> next(C);
+        int at = 0;
+        for (int b = 0; b < B; ++b)
+            for (int h = 0; h < 2; ++h) {
+                ResBlock* blk = blocks + (size_t)b * C;
+                for (int r = 0; r < C; ++r) blk[r].side[h] = ResSide{};
+                deal(b, h, C, [&](const int4& p, int r) {
+                    blk[r].side[h].passes += 1;
+                    blk[r].side[h].rows += p.z;
+                });
+                for (int r = 0; r < C; ++r) {
+                    ResSide& sd = blk[r].side[h];
+                    next[r] = sd.pass_begin = at;
+                    at += sd.passes;
+                    sd.row_begin = (int)rows;
+                    rows += sd.rows;
+                    sd.rows = 0;  // counted again below
+                }
+                deal(b, h, C, [&](const int4& p, int r) {
+                    ResSide& sd = blk[r].side[h];
+                    const int k = next[r]++;
+                    passes[k] = make_int4(sd.rows, p.z | (p.w << 24), p.x - (*offs[h])[b], sd.locals | (p.y << 24));
+                    place[2 * (size_t)k] = make_int4(sd.row_begin + sd.rows, p.z, p.x, p.y);
+                    place[2 * (size_t)k + 1] = make_int4((*offs[1 - h])[b], h, 1 << p.w, 0);
+                    sd.rows += p.z;
+                    sd.locals += p.y;
+                });
+            }
+    }
     SIHG_TRY(tab_.alloc(buf.size()));
     SIHG_CUDA(cudaMemcpyAsync(tab_.as<void>(), buf.data(), buf.size(), cudaMemcpyHostToDevice, s));
     SIHG_TRY(rows_.alloc(256 * (size_t)std::max<long long>(1, rows)));
