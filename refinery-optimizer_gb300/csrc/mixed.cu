@@ -1420,7 +1420,7 @@ int MixedSolver::setup_resident() {
         return SIH_PDHG_OK;
     if (B_ == 1 && persistent_ != 2) return SIH_PDHG_OK;
     // (a batch: no cluster holds the mean instance)
-    if (B_ > 1 && 16.0 * (double)nnz_ > 220.0 * 1024.0 * 16.0 * B_) return SIH_PDHG_OK;
+    if (B_ > 1 && 12.0 * (double)nnz_ > 220.0 * 1024.0 * 16.0 * B_) return SIH_PDHG_OK;
     const std::vector<uint8_t> rl = segment_lanes(layout_.row_schedule, M_), cl = segment_lanes(layout_.col_schedule, N_);
     SIHG_TRY(resident_->build(h_csr_ptr_, h_csc_ptr_, row_off_, col_off_, rl, cl, sm_count_, stream_,
                               ResidentPlan::kCluster));

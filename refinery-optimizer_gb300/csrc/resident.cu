@@ -42,8 +42,10 @@ namespace {
 
 constexpr int kResThreads = 672;   // most threads of a block of a cluster: 20 warps with passes, the controller
 constexpr int kGridThreads = 768;  // threads of a block of the grid form
-constexpr int kColWords = 9;       // per column: x (2), K^T y (2), c, l, u, average (2)
-constexpr int kRowWords = 8;       // per row: y (2), K x (2), rl, ru, average (2)
+constexpr int kColWords = 8;       // per column: x, K^T y (2), c, l, u, average (2); x' is in the copy
+constexpr int kRowWords = 7;       // per row: y, K x (2), rl, ru, average (2); y' is in the copy
+constexpr int kGridColWords = 5;   // over every SM: K^T y (2), c, average (2); the rest is in the column's record
+constexpr int kGridRowWords = 6;   // K x (2), rl, ru, average (2); y and y' are in global memory
 constexpr int kPlainColWords = 6;  // plain algorithm, per column: x, c, l, u, tau, best x
 constexpr int kPlainRowWords = 4;  // per row: y, rl, ru, sigma
 
@@ -87,6 +89,85 @@ __device__ __forceinline__ void push(float* p, float v, int sub, int L, int clus
     for (int r = sub; r < cluster; r += L) st_rank(map_rank(p, r), v);
 }
 
+// Entries of a side: a lane's entries of a pass two at a time, 32 lanes together.
+// In a cluster indices have 16 bits (its vectors fit in shared memory): 12
+// bytes a pair instead of 16, a quarter less of what decides how many blocks
+// an LP needs.  Empty places hold value 0 and the index of a zero behind the
+// gathered vector, so that no lane has to ask.
+struct Compact {
+    static constexpr int kPair = 32 * 12;
+    static __device__ __forceinline__ void load(const char* p, bool on, int none, int& i0, float& a0, int& i1,
+                                                float& a1) {
+        const int lane = threadIdx.x & 31;
+        const float2 a = on ? *reinterpret_cast<const float2*>(p + 8 * lane) : make_float2(0.f, 0.f);
+        const unsigned i = on ? *reinterpret_cast<const unsigned*>(p + 256 + 4 * lane) : none * 0x10001u;
+        i0 = i & 0xffffu;
+        i1 = i >> 16;
+        a0 = a.x;
+        a1 = a.y;
+    }
+    static __device__ __forceinline__ void store(char* p, int i0, float a0, int i1, float a1) {
+        const int lane = threadIdx.x & 31;
+        *reinterpret_cast<float2*>(p + 8 * lane) = make_float2(a0, a1);
+        *reinterpret_cast<unsigned*>(p + 256 + 4 * lane) = (unsigned)i0 | (unsigned)i1 << 16;
+    }
+};
+// Over every SM: 32-bit indices, empty places -1.
+struct Wide {
+    static constexpr int kPair = 32 * 16;
+    static __device__ __forceinline__ void load(const char* p, bool on, int none, int& i0, float& a0, int& i1,
+                                                float& a1) {
+        const int4 q = on ? *reinterpret_cast<const int4*>(p + 16 * (threadIdx.x & 31)) : make_int4(none, 0, none, 0);
+        i0 = q.x;
+        a0 = __int_as_float(q.y);
+        i1 = q.z;
+        a1 = __int_as_float(q.w);
+    }
+    static __device__ __forceinline__ void store(char* p, int i0, float a0, int i1, float a1) {
+        *reinterpret_cast<int4*>(p + 16 * (threadIdx.x & 31)) =
+            make_int4(i0, __float_as_int(a0), i1, __float_as_int(a1));
+    }
+};
+
+// Gathers from a copy in shared memory; `none`: the index of the zero behind it.
+struct FromShared {
+    using Entries = Compact;
+    const float* v;
+    int none;
+    __device__ __forceinline__ float operator()(int i) const { return v[i]; }
+};
+
+// Gathers of a vector written earlier in the same launch (coherent loads).
+struct FromGlobal {
+    using Entries = Wide;
+    const float* v;
+    static constexpr int none = -1;
+    __device__ __forceinline__ float operator()(int i) const {
+        float x = 0.f;
+        if (i >= 0) asm volatile("ld.global.f32 %0, [%1];" : "=f"(x) : "l"(v + i));
+        return x;
+    }
+};
+
+// The candidate x' of a column from its record {x, c + K^T y, l, u}.
+__device__ __forceinline__ float x_from_record(const float4& r, float tau) {
+    return fminf(fmaxf(fmaf(-tau, r.y, r.x), r.z), r.w);
+}
+__device__ __forceinline__ float4 ld_record(const float4* p) {
+    float4 r;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p));
+    return r;
+}
+struct FromRecords {
+    using Entries = Wide;
+    const float4* v;
+    float tau;
+    static constexpr int none = -1;
+    __device__ __forceinline__ float operator()(int i) const {
+        return i >= 0 ? x_from_record(ld_record(v + i), tau) : 0.f;
+    }
+};
+
 // Dot products of one pass: lane (group, sub) sums its entries with the values
 // gather(index); the sum s + e (e: the compensation) is valid in each group's
 // first lane.  The phases are bound by the latency and the number of these
@@ -94,29 +175,30 @@ __device__ __forceinline__ void push(float* p, float v, int sub, int L, int clus
 // read before the first is summed, and rows past the pass's width add 0 * 0 (a
 // branch over them costs more).
 template <bool COMP, int BATCHES, class Gather>
-__device__ __forceinline__ void pass_sums(const int2* __restrict__ rows, int width, int lg, Gather&& gather, float& s,
+__device__ __forceinline__ void pass_sums(const char* rows, int width, int lg, const Gather& gather, float& s,
                                           float& e) {
+    using Entries = typename Gather::Entries;
     constexpr int kU = BATCHES * kBatch;
     float acc[kBatch] = {0.f, 0.f, 0.f, 0.f};
     s = e = 0.f;
-    const int2* p = rows + (threadIdx.x & 31);
-    for (int k = 0; k < width; k += kU, p += 32 * kU) {
-        int2 w[kU];
-        float g[kU];
+    for (int k = 0; k < width; k += kU, rows += kU / 2 * Entries::kPair) {
+        int i[kU];
+        float a[kU], g[kU];
 #pragma unroll
-        for (int u = 0; u < kU; ++u) w[u] = k + u < width ? p[32 * u] : make_int2(-1, 0);
+        for (int u = 0; u < kU; u += 2)
+            Entries::load(rows + u / 2 * Entries::kPair, k + u < width, gather.none, i[u], a[u], i[u + 1], a[u + 1]);
 #pragma unroll
-        for (int u = 0; u < kU; ++u) g[u] = w[u].x >= 0 ? gather(w[u].x) : 0.f;
+        for (int u = 0; u < kU; ++u) g[u] = gather(i[u]);
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
             if (COMP) {
                 float pr, pe, ss, se;
-                two_prod(__int_as_float(w[u].y), g[u], pr, pe);
+                two_prod(a[u], g[u], pr, pe);
                 two_sum(s, pr, ss, se);
                 s = ss;
                 e = __fadd_rn(e, __fadd_rn(pe, se));
             } else {
-                acc[u % kBatch] = fmaf(__int_as_float(w[u].y), g[u], acc[u % kBatch]);
+                acc[u % kBatch] = fmaf(a[u], g[u], acc[u % kBatch]);
             }
         }
     }
@@ -138,44 +220,12 @@ __device__ __forceinline__ void pass_sums(const int2* __restrict__ rows, int wid
 
 // The same rounded to float, in every lane of the group.
 template <bool COMP, int BATCHES, class Gather>
-__device__ __forceinline__ float pass_dot(const int2* __restrict__ rows, int width, int lg, Gather&& gather) {
+__device__ __forceinline__ float pass_dot(const char* rows, int width, int lg, const Gather& gather) {
     float s, e;
     pass_sums<COMP, BATCHES>(rows, width, lg, gather, s, e);
     if (!COMP) return s;
     return __shfl_sync(FULL_MASK, __fadd_rn(s, e), (threadIdx.x & 31) >> lg << lg);
 }
-
-// Gathers from a copy in shared memory.
-struct FromShared {
-    const float* v;
-    __device__ __forceinline__ float operator()(int i) const { return v[i]; }
-};
-
-// Gathers of a vector written earlier in the same launch (coherent loads).
-struct FromGlobal {
-    const float* v;
-    __device__ __forceinline__ float operator()(int i) const {
-        float x;
-        asm volatile("ld.global.f32 %0, [%1];" : "=f"(x) : "l"(v + i));
-        return x;
-    }
-};
-
-// The candidate x' of a column from its record {x, c + K^T y, l, u}.
-__device__ __forceinline__ float x_from_record(const float4& r, float tau) {
-    return fminf(fmaxf(fmaf(-tau, r.y, r.x), r.z), r.w);
-}
-struct FromRecords {
-    const float4* v;
-    float tau;
-    __device__ __forceinline__ float operator()(int i) const {
-        float4 r;
-        asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
-                     : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
-                     : "l"(v + i));
-        return x_from_record(r, tau);
-    }
-};
 
 // What a step needs of the controller's state (FP32), published to the block.
 struct StepPub {
@@ -184,13 +234,14 @@ struct StepPub {
 };
 
 // One pass as a warp sees it: the segment of this lane's group.
-struct Pass {
-    const int2* rows;
+template <class Entries>
+struct PassOf {
+    const char* rows;
     int width, lg, sub, seg, local;  // seg: in the instance, local: in the block
     bool on;                         // the group has a segment
-    __device__ __forceinline__ Pass(const int4& t, const int2* side_rows) {
+    __device__ __forceinline__ PassOf(const int4& t, const char* side_rows) {
         const int lane = threadIdx.x & 31;
-        rows = side_rows + (size_t)t.x * 32;
+        rows = side_rows + t.x * Entries::kPair;
         width = t.y & 0xffffff;
         lg = t.y >> 24;
         const int g = lane >> lg;
@@ -201,35 +252,38 @@ struct Pass {
     }
 };
 
+using Pass = PassOf<Compact>;
+using GridPass = PassOf<Wide>;
+
 // Copies this block's passes and entries of both sides to shared memory.
+template <class Entries>
 __device__ __forceinline__ void load_block(const ResArgs& A, const ResBlock& blk, char* sm) {
     for (int h = 0; h < 2; ++h) {
         const ResSide& sd = blk.side[h];
         int4* pass = reinterpret_cast<int4*>(sm + A.sm.pass[h]);
         for (int k = threadIdx.x; k < sd.passes; k += blockDim.x) pass[k] = A.passes[sd.pass_begin + k];
-        const int4* src = reinterpret_cast<const int4*>(A.rows + (size_t)sd.row_begin * 32);
+        const int4* src = reinterpret_cast<const int4*>(A.rows + (size_t)sd.row_begin * Entries::kPair);
         int4* dst = reinterpret_cast<int4*>(sm + A.sm.rows[h]);
-        for (int k = threadIdx.x; k < sd.rows * 16; k += blockDim.x) dst[k] = __ldg(src + k);
+        for (int k = threadIdx.x; k < sd.rows * (Entries::kPair / 16); k += blockDim.x) dst[k] = __ldg(src + k);
     }
 }
 
 // Rows: K x' and the dual update (the operations of DualStepEpi::apply).
 template <bool COMP>
-__device__ __forceinline__ void dual_phase(const int4* pass, int passes, const int2* rows, float* R, int nl, int cur,
-                                           const float* xs, float* ys, float sigma, int cluster, Acc& dy2) {
+__device__ __forceinline__ void dual_phase(const int4* pass, int passes, const char* rows, float* R, int nl, int cur,
+                                           const FromShared& xs, float* ys, float sigma, int cluster, Acc& dy2) {
     const int nw = (blockDim.x >> 5) - 1;
     for (int p = threadIdx.x >> 5; p < passes; p += nw) {
         const Pass t(pass[p], rows);
-        const float kxp = pass_dot<COMP, 2>(t.rows, t.width, t.lg, FromShared{xs});
+        const float kxp = pass_dot<COMP, 2>(t.rows, t.width, t.lg, xs);
         if (t.on) {
             const float* r = R + t.local;
-            const float yo = r[cur * nl], kx = r[(2 + cur) * nl], rl = r[4 * nl], ru = r[5 * nl];
+            const float yo = r[0], kx = r[(1 + cur) * nl], rl = r[3 * nl], ru = r[4 * nl];
             const float wv = (2.0f * kxp - kx) + yo / sigma;
             const float yv = sigma * (wv - fminf(fmaxf(wv, rl), ru));
             push(ys + t.seg, yv, t.sub, 1 << t.lg, cluster);
             if (t.sub == 0) {
-                R[(2 + (cur ^ 1)) * nl + t.local] = kxp;
-                R[(cur ^ 1) * nl + t.local] = yv;
+                R[(1 + (cur ^ 1)) * nl + t.local] = kxp;
                 const float dy = yv - yo;
                 dy2.add(dy * dy);
             }
@@ -239,17 +293,17 @@ __device__ __forceinline__ void dual_phase(const int4* pass, int passes, const i
 
 // Columns: K^T y', interaction and movement (the operations of KtyStepEpi::apply).
 template <bool COMP>
-__device__ __forceinline__ void kty_phase(const int4* pass, int passes, const int2* rows, float* C, int nl, int cur,
-                                          const float* ys, Acc& inter, Acc& dx2) {
+__device__ __forceinline__ void kty_phase(const int4* pass, int passes, const char* rows, float* C, int nl, int cur,
+                                          const FromShared& ys, const float* xs, Acc& inter, Acc& dx2) {
     const int nw = (blockDim.x >> 5) - 1;
     for (int p = threadIdx.x >> 5; p < passes; p += nw) {
         const Pass t(pass[p], rows);
-        const float k = pass_dot<COMP, 2>(t.rows, t.width, t.lg, FromShared{ys});
+        const float k = pass_dot<COMP, 2>(t.rows, t.width, t.lg, ys);
         if (t.on && t.sub == 0) {
-            const float* c = C + t.local;
-            const float dx = c[(cur ^ 1) * nl] - c[cur * nl];
-            C[(2 + (cur ^ 1)) * nl + t.local] = k;
-            inter.add(dx * (k - c[(2 + cur) * nl]));
+            float* c = C + t.local;
+            const float dx = xs[t.seg] - c[0];
+            c[(1 + (cur ^ 1)) * nl] = k;
+            inter.add(dx * (k - c[(1 + cur) * nl]));
             dx2.add(dx * dx);
         }
     }
@@ -375,16 +429,16 @@ struct StepCtrl {
 constexpr int kEvalQ = 18;  // reductions of an evaluation: 8 of the rows, 10 of the columns
 
 // Sums of a side's segments with the first candidate point, to s and e by local segment.
-__device__ __forceinline__ void eval_sums(bool comp, const int4* pass, int passes, const int2* rows, const float* vec,
+__device__ __forceinline__ void eval_sums(bool comp, const int4* pass, int passes, const char* rows, const FromShared& vec,
                                           float* s_out, float* e_out) {
     const int nw = (blockDim.x >> 5) - 1;
     for (int p = threadIdx.x >> 5; p < passes; p += nw) {
         const Pass t(pass[p], rows);
         float s, e;
         if (comp)
-            pass_sums<true, 2>(t.rows, t.width, t.lg, FromShared{vec}, s, e);
+            pass_sums<true, 2>(t.rows, t.width, t.lg, vec, s, e);
         else
-            pass_sums<false, 2>(t.rows, t.width, t.lg, FromShared{vec}, s, e);
+            pass_sums<false, 2>(t.rows, t.width, t.lg, vec, s, e);
         if (t.on && t.sub == 0) {
             s_out[t.local] = s;
             e_out[t.local] = e;
@@ -395,16 +449,16 @@ __device__ __forceinline__ void eval_sums(bool comp, const int4* pass, int passe
 // The evaluation epilogue of a side's segments: first candidate's sums from s
 // and e, the second's from `vec`; `first` is the instance's first segment.
 template <class Epi>
-__device__ __forceinline__ void eval_apply(bool comp, const int4* pass, int passes, const int2* rows, const float* vec,
+__device__ __forceinline__ void eval_apply(bool comp, const int4* pass, int passes, const char* rows, const FromShared& vec,
                                            const float* s_in, const float* e_in, int first, Epi& epi) {
     const int nw = (blockDim.x >> 5) - 1;
     for (int p = threadIdx.x >> 5; p < passes; p += nw) {
         const Pass t(pass[p], rows);
         SegDot<2> d;
         if (comp)
-            pass_sums<true, 2>(t.rows, t.width, t.lg, FromShared{vec}, d.s[1], d.e[1]);
+            pass_sums<true, 2>(t.rows, t.width, t.lg, vec, d.s[1], d.e[1]);
         else
-            pass_sums<false, 2>(t.rows, t.width, t.lg, FromShared{vec}, d.s[1], d.e[1]);
+            pass_sums<false, 2>(t.rows, t.width, t.lg, vec, d.s[1], d.e[1]);
         if (t.on && t.sub == 0) {
             d.s[0] = s_in[t.local];
             d.e[0] = e_in[t.local];
@@ -446,17 +500,19 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
     const bool ctrl = warp == nw;
     int4* rpass = reinterpret_cast<int4*>(sm + A.sm.pass[0]);
     int4* cpass = reinterpret_cast<int4*>(sm + A.sm.pass[1]);
-    int2* rrows = reinterpret_cast<int2*>(sm + A.sm.rows[0]);
-    int2* crows = reinterpret_cast<int2*>(sm + A.sm.rows[1]);
+    const char* rrows = sm + A.sm.rows[0];
+    const char* crows = sm + A.sm.rows[1];
     float* xs = reinterpret_cast<float*>(sm + A.sm.xs);
     float* ys = reinterpret_cast<float*>(sm + A.sm.ys);
-    float* C = reinterpret_cast<float*>(sm + A.sm.col);  // x x' | K^T y K^T y' | c l u | average hi lo
-    float* R = reinterpret_cast<float*>(sm + A.sm.row);  // y y' | K x K x' | rl ru | average hi lo
+    float* C = reinterpret_cast<float*>(sm + A.sm.col);  // x | K^T y, K^T y' | c l u | average hi lo
+    float* R = reinterpret_cast<float*>(sm + A.sm.row);  // y | K x, K x' | rl ru | average hi lo
     Sums* wsum = reinterpret_cast<Sums*>(sm + A.sm.red);  // of every warp of this block
     Sums* bsum = wsum + 32;                               // of every block of the cluster
     const int ncl = A.sm.locals[1], nrl = A.sm.locals[0];
     const int rp = blk.side[0].passes, cp = blk.side[1].passes;
-    load_block(A, blk, sm);
+    const FromShared gx{xs, io.y}, gy{ys, io.w};
+    if (threadIdx.x == 0) xs[io.y] = ys[io.w] = 0.f;
+    load_block<Compact>(A, blk, sm);
     if (threadIdx.x == 0) {
         S = st[inst];
         const StepScalars sc = step_scalars(S);
@@ -470,14 +526,14 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
             if (t.on && t.sub == 0) {
                 const int j = io.x + t.seg;
                 float* c = C + t.local;
-                c[cur * ncl] = pick(V.x0, V.x1, cur)[j];
-                c[(2 + cur) * ncl] = pick(V.kty0, V.kty1, cur)[j];
-                c[4 * ncl] = V.c[j];
-                c[5 * ncl] = V.l[j];
-                c[6 * ncl] = V.u[j];
+                xs[t.seg] = c[0] = pick(V.x0, V.x1, cur)[j];
+                c[(1 + cur) * ncl] = pick(V.kty0, V.kty1, cur)[j];
+                c[3 * ncl] = V.c[j];
+                c[4 * ncl] = V.l[j];
+                c[5 * ncl] = V.u[j];
                 const float2 a = V.x_acc[j];
-                c[7 * ncl] = a.x;
-                c[8 * ncl] = a.y;
+                c[6 * ncl] = a.x;
+                c[7 * ncl] = a.y;
             }
         }
         for (int p = warp; p < rp; p += nw) {
@@ -485,13 +541,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
             if (t.on && t.sub == 0) {
                 const int j = io.z + t.seg;
                 float* r = R + t.local;
-                r[cur * nrl] = pick(V.y0, V.y1, cur)[j];
-                r[(2 + cur) * nrl] = pick(V.kx0, V.kx1, cur)[j];
-                r[4 * nrl] = V.rl[j];
-                r[5 * nrl] = V.ru[j];
+                ys[t.seg] = r[0] = pick(V.y0, V.y1, cur)[j];
+                r[(1 + cur) * nrl] = pick(V.kx0, V.kx1, cur)[j];
+                r[3 * nrl] = V.rl[j];
+                r[4 * nrl] = V.ru[j];
                 const float2 a = V.y_acc[j];
-                r[6 * nrl] = a.x;
-                r[7 * nrl] = a.y;
+                r[5 * nrl] = a.x;
+                r[6 * nrl] = a.y;
             }
         }
     }
@@ -503,16 +559,22 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
         const int cur = pub.cur;
         const bool avg = pub.avg != 0;
         const float w = pub.w, tau = pub.tau, sg = pub.sigma;
-        // x' = clip(x - tau (c + K^T y), l, u)
+        // x' = clip(x - tau (c + K^T y), l, u); after an accepted step x is the
+        // candidate of that step, still in the copy
         if (!ctrl) {
             for (int p = warp; p < cp; p += nw) {
                 const Pass t(cpass[p], crows);
+                float x = 0.f, xp = 0.f;
                 if (t.on) {
                     const float* c = C + t.local;
-                    const float v = fmaf(-tau, c[4 * ncl] + c[(2 + cur) * ncl], c[cur * ncl]);
-                    const float xp = fminf(fmaxf(v, c[5 * ncl]), c[6 * ncl]);
-                    if (t.sub == 0) C[(cur ^ 1) * ncl + t.local] = xp;
+                    x = avg ? xs[t.seg] : c[0];
+                    const float v = fmaf(-tau, c[3 * ncl] + c[(1 + cur) * ncl], x);
+                    xp = fminf(fmaxf(v, c[4 * ncl]), c[5 * ncl]);
+                }
+                __syncwarp();  // every lane of the group has read x
+                if (t.on) {
                     push(xs + t.seg, xp, t.sub, 1 << t.lg, cluster);
+                    if (t.sub == 0) C[t.local] = x;
                 }
             }
         }
@@ -520,24 +582,34 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
         if (ctrl) {
             if (lane == 0) schedule_pows(S, V);
         } else if (avg) {  // the pending average updates, while the other blocks arrive
-            for (int k2 = threadIdx.x; k2 < blk.side[1].locals; k2 += nw * 32) {
-                const float2 a = ff_axpy(make_float2(C[7 * ncl + k2], C[8 * ncl + k2]), w, C[cur * ncl + k2]);
-                C[7 * ncl + k2] = a.x;
-                C[8 * ncl + k2] = a.y;
+            for (int p = warp; p < cp; p += nw) {
+                const Pass t(cpass[p], crows);
+                if (t.on && t.sub == 0) {
+                    float* c = C + t.local;
+                    const float2 a = ff_axpy(make_float2(c[6 * ncl], c[7 * ncl]), w, c[0]);
+                    c[6 * ncl] = a.x;
+                    c[7 * ncl] = a.y;
+                }
             }
-            for (int k2 = threadIdx.x; k2 < blk.side[0].locals; k2 += nw * 32) {
-                const float2 a = ff_axpy(make_float2(R[6 * nrl + k2], R[7 * nrl + k2]), w, R[cur * nrl + k2]);
-                R[6 * nrl + k2] = a.x;
-                R[7 * nrl + k2] = a.y;
+            for (int p = warp; p < rp; p += nw) {
+                const Pass t(rpass[p], rrows);
+                if (t.on && t.sub == 0) {
+                    float* r = R + t.local;
+                    const float y = r[0] = ys[t.seg];
+                    const float2 a = ff_axpy(make_float2(r[5 * nrl], r[6 * nrl]), w, y);
+                    r[5 * nrl] = a.x;
+                    r[6 * nrl] = a.y;
+                }
             }
+            __syncwarp();  // the whole group reads y in the next phase
         }
         cluster_wait();
         Acc dy2;
         if (!ctrl) {
             if (comp)
-                dual_phase<true>(rpass, rp, rrows, R, nrl, cur, xs, ys, sg, cluster, dy2);
+                dual_phase<true>(rpass, rp, rrows, R, nrl, cur, gx, ys, sg, cluster, dy2);
             else
-                dual_phase<false>(rpass, rp, rrows, R, nrl, cur, xs, ys, sg, cluster, dy2);
+                dual_phase<false>(rpass, rp, rrows, R, nrl, cur, gx, ys, sg, cluster, dy2);
         }
         cluster_arrive();
         cluster_wait();
@@ -545,9 +617,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
         if (!ctrl) {
             Acc inter, dx2;
             if (comp)
-                kty_phase<true>(cpass, cp, crows, C, ncl, cur, ys, inter, dx2);
+                kty_phase<true>(cpass, cp, crows, C, ncl, cur, gy, xs, inter, dx2);
             else
-                kty_phase<false>(cpass, cp, crows, C, ncl, cur, ys, inter, dx2);
+                kty_phase<false>(cpass, cp, crows, C, ncl, cur, gy, xs, inter, dx2);
             warp_reduce_three(inter, dx2, dy2);  // inter: |dx|^2 in the upper lanes
             if (lane == 0) {
                 wsum[warp].inter = make_float2(inter.s, inter.c);
@@ -583,18 +655,20 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
     if (!ctrl) {
         for (int p = warp; p < cp; p += nw) {
             const Pass t(cpass[p], crows);
+            float x = 0.f;
+            if (t.on) x = avg ? xs[t.seg] : C[t.local];
+            __syncwarp();
             if (t.on) {
-                const int j = io.x + t.seg;
-                float* c = C + t.local;
-                const float x = c[cur * ncl];
                 if (!failed) push(xs + t.seg, x, t.sub, 1 << t.lg, cluster);
                 if (t.sub == 0) {
-                    float2 a = make_float2(c[7 * ncl], c[8 * ncl]);
+                    const int j = io.x + t.seg;
+                    float* c = C + t.local;
+                    float2 a = make_float2(c[6 * ncl], c[7 * ncl]);
                     if (avg) a = ff_axpy(a, w, x);
-                    c[7 * ncl] = a.x;
-                    c[8 * ncl] = a.y;
+                    c[6 * ncl] = a.x;
+                    c[7 * ncl] = a.y;
                     pick(V.x0, V.x1, cur)[j] = x;
-                    pick(V.kty0, V.kty1, cur)[j] = c[(2 + cur) * ncl];
+                    pick(V.kty0, V.kty1, cur)[j] = c[(1 + cur) * ncl];
                     V.x_acc[j] = a;
                     V.x_avg[j] = __fadd_rn(a.x, a.y);
                 }
@@ -602,23 +676,26 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
         }
         for (int p = warp; p < rp; p += nw) {
             const Pass t(rpass[p], rrows);
+            float y = 0.f;
+            if (t.on) y = avg ? ys[t.seg] : R[t.local];
+            __syncwarp();
             if (t.on) {
-                const int j = io.z + t.seg;
-                float* r = R + t.local;
-                const float y = r[cur * nrl];
                 if (!failed) push(ys + t.seg, y, t.sub, 1 << t.lg, cluster);
                 if (t.sub == 0) {
-                    float2 a = make_float2(r[6 * nrl], r[7 * nrl]);
+                    const int j = io.z + t.seg;
+                    float* r = R + t.local;
+                    float2 a = make_float2(r[5 * nrl], r[6 * nrl]);
                     if (avg) a = ff_axpy(a, w, y);
-                    r[6 * nrl] = a.x;
-                    r[7 * nrl] = a.y;
+                    r[5 * nrl] = a.x;
+                    r[6 * nrl] = a.y;
                     pick(V.y0, V.y1, cur)[j] = y;
-                    pick(V.kx0, V.kx1, cur)[j] = r[(2 + cur) * nrl];
+                    pick(V.kx0, V.kx1, cur)[j] = r[(1 + cur) * nrl];
                     V.y_acc[j] = a;
                     V.y_avg[j] = __fadd_rn(a.x, a.y);
                 }
             }
         }
+        __syncwarp();  // the groups read the averages below
     }
     if (failed) {
         if (rank == 0 && ctrl && lane == 0) st[inst] = S;
@@ -626,9 +703,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
     }
     cluster_arrive();
     cluster_wait();
-    if (!ctrl) {  // the current point's sums, kept where the candidate point was
-        eval_sums(comp, rpass, rp, rrows, xs, R + (cur ^ 1) * nrl, R + (2 + (cur ^ 1)) * nrl);
-        eval_sums(comp, cpass, cp, crows, ys, C + (cur ^ 1) * ncl, C + (2 + (cur ^ 1)) * ncl);
+    if (!ctrl) {  // the current point's sums, kept where the point (now in global memory) and the candidate's product were
+        eval_sums(comp, rpass, rp, rrows, gx, R, R + (1 + (cur ^ 1)) * nrl);
+        eval_sums(comp, cpass, cp, crows, gy, C, C + (1 + (cur ^ 1)) * ncl);
     }
     cluster_arrive();
     cluster_wait();
@@ -636,12 +713,12 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
         for (int p = warp; p < cp; p += nw) {
             const Pass t(cpass[p], crows);
             if (t.on)
-                push(xs + t.seg, __fadd_rn(C[7 * ncl + t.local], C[8 * ncl + t.local]), t.sub, 1 << t.lg, cluster);
+                push(xs + t.seg, __fadd_rn(C[6 * ncl + t.local], C[7 * ncl + t.local]), t.sub, 1 << t.lg, cluster);
         }
         for (int p = warp; p < rp; p += nw) {
             const Pass t(rpass[p], rrows);
             if (t.on)
-                push(ys + t.seg, __fadd_rn(R[6 * nrl + t.local], R[7 * nrl + t.local]), t.sub, 1 << t.lg, cluster);
+                push(ys + t.seg, __fadd_rn(R[5 * nrl + t.local], R[6 * nrl + t.local]), t.sub, 1 << t.lg, cluster);
         }
     }
     cluster_arrive();
@@ -653,7 +730,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
         EvalRowsEpi er{V};
         er.begin(S);
         Acc q[8];
-        eval_apply(comp, rpass, rp, rrows, xs, R + (cur ^ 1) * nrl, R + (2 + (cur ^ 1)) * nrl, io.z, er);
+        eval_apply(comp, rpass, rp, rrows, gx, R, R + (1 + (cur ^ 1)) * nrl, io.z, er);
         er.values(q);
         warp_reduce_acc<8>(q, 0x0Cu);
         if (lane == 0)
@@ -663,7 +740,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
         EvalColsEpi ec{V, nullptr};
         ec.begin(S);
         Acc q[10];
-        eval_apply(comp, cpass, cp, crows, ys, C + (cur ^ 1) * ncl, C + (2 + (cur ^ 1)) * ncl, io.x, ec);
+        eval_apply(comp, cpass, cp, crows, gy, C, C + (1 + (cur ^ 1)) * ncl, io.x, ec);
         ec.values(q);
         warp_reduce_acc<10>(q, 0x0Cu);
         if (lane == 0)
@@ -691,21 +768,24 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
         flag = S.restart_flag;
     }
     __syncthreads();
-    if (!ctrl && flag != 0) {  // restart at the current (1) or the average point (2)
+    if (!ctrl) {  // the point back, after a restart at the current (1) or the average point (2) with its average
         for (int p = warp; p < cp; p += nw) {
             const Pass t(cpass[p], crows);
             if (t.on && t.sub == 0) {
                 const int j = io.x + t.seg;
                 float* c = C + t.local;
+                float* gx0 = pick(V.x0, V.x1, cur) + j;
                 if (flag == 2) {
-                    pick(V.x0, V.x1, cur)[j] = c[cur * ncl] = V.x_avg[j];
-                    pick(V.kty0, V.kty1, cur)[j] = c[(2 + cur) * ncl] = V.kty_eval[j];
+                    *gx0 = V.x_avg[j];
+                    pick(V.kty0, V.kty1, cur)[j] = c[(1 + cur) * ncl] = V.kty_eval[j];
                 }
-                const float x = c[cur * ncl];
-                V.x_last[j] = x;
-                V.x_acc[j] = make_float2(x, 0.f);
-                c[7 * ncl] = x;
-                c[8 * ncl] = 0.f;
+                const float x = c[0] = *gx0;
+                if (flag != 0) {
+                    V.x_last[j] = x;
+                    V.x_acc[j] = make_float2(x, 0.f);
+                    c[6 * ncl] = x;
+                    c[7 * ncl] = 0.f;
+                }
             }
         }
         for (int p = warp; p < rp; p += nw) {
@@ -713,17 +793,21 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
             if (t.on && t.sub == 0) {
                 const int j = io.z + t.seg;
                 float* r = R + t.local;
+                float* gy0 = pick(V.y0, V.y1, cur) + j;
                 if (flag == 2) {
-                    pick(V.y0, V.y1, cur)[j] = r[cur * nrl] = V.y_avg[j];
-                    pick(V.kx0, V.kx1, cur)[j] = r[(2 + cur) * nrl] = V.kx_eval[j];
+                    *gy0 = V.y_avg[j];
+                    pick(V.kx0, V.kx1, cur)[j] = r[(1 + cur) * nrl] = V.kx_eval[j];
                 }
-                const float y = r[cur * nrl];
-                V.y_last[j] = y;
-                V.y_acc[j] = make_float2(y, 0.f);
-                r[6 * nrl] = y;
-                r[7 * nrl] = 0.f;
+                const float y = r[0] = *gy0;
+                if (flag != 0) {
+                    V.y_last[j] = y;
+                    V.y_acc[j] = make_float2(y, 0.f);
+                    r[5 * nrl] = y;
+                    r[6 * nrl] = 0.f;
+                }
             }
         }
+        __syncwarp();  // the groups read x and y in the next step
     }
     }
     if (rank == 0 && ctrl && lane == 0) st[inst] = S;
@@ -795,25 +879,26 @@ struct GridSync {
 // Columns of the grid form: K^T y' from L2, x' from the owner's record, the
 // next record, and the average update (the operations of KtyStepEpiPacked).
 template <bool COMP>
-__device__ __forceinline__ void grid_cols(const int4* pass, int passes, const int2* rows, float* C, int nl, int cur,
-                                          const float* y, float4* next, float tau, bool avg, float w, Acc& inter,
-                                          Acc& dx2) {
+__device__ __forceinline__ void grid_cols(const int4* pass, int passes, const char* rows, float* C, int nl, int cur,
+                                          const float* y, const float4* records, float4* next, float tau, bool avg,
+                                          float w, Acc& inter, Acc& dx2) {
     const int nw = (blockDim.x >> 5) - 1;
     for (int p = threadIdx.x >> 5; p < passes; p += nw) {
-        const Pass t(pass[p], rows);
+        const GridPass t(pass[p], rows);
+        float4 rec = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t.on && t.sub == 0) rec = ld_record(records + t.seg);
         const float k = pass_dot<COMP, 2>(t.rows, t.width, t.lg, FromGlobal{y});
         if (t.on && t.sub == 0) {
             float* c = C + t.local;
-            const float x = c[cur * nl], kty = c[(2 + cur) * nl], cc = c[4 * nl], l = c[5 * nl], u = c[6 * nl];
-            const float xp = x_from_record(make_float4(x, cc + kty, l, u), tau);
+            const float x = rec.x, kty = c[cur * nl], cc = c[2 * nl];
+            const float xp = x_from_record(rec, tau);
             if (avg) {
-                const float2 a = ff_axpy(make_float2(c[7 * nl], c[8 * nl]), w, x);
-                c[7 * nl] = a.x;
-                c[8 * nl] = a.y;
+                const float2 a = ff_axpy(make_float2(c[3 * nl], c[4 * nl]), w, x);
+                c[3 * nl] = a.x;
+                c[4 * nl] = a.y;
             }
-            c[(cur ^ 1) * nl] = xp;
-            c[(2 + (cur ^ 1)) * nl] = k;
-            next[t.seg] = make_float4(xp, cc + k, l, u);
+            c[(cur ^ 1) * nl] = k;
+            next[t.seg] = make_float4(xp, cc + k, rec.z, rec.w);
             const float dx = xp - x;
             inter.add(dx * (k - kty));
             dx2.add(dx * dx);
@@ -823,25 +908,26 @@ __device__ __forceinline__ void grid_cols(const int4* pass, int passes, const in
 
 // Rows: K x' gathered through the records, dual update, average update.
 template <bool COMP>
-__device__ __forceinline__ void grid_rows(const int4* pass, int passes, const int2* rows, float* R, int nl, int cur,
-                                          const float4* records, float tau, float sigma, float* y_next, bool avg,
-                                          float w, Acc& dy2) {
+__device__ __forceinline__ void grid_rows(const int4* pass, int passes, const char* rows, float* R, int nl, int cur,
+                                          const float4* records, float tau, float sigma, const float* y, float* y_next,
+                                          bool avg, float w, Acc& dy2) {
     const int nw = (blockDim.x >> 5) - 1;
     for (int p = threadIdx.x >> 5; p < passes; p += nw) {
-        const Pass t(pass[p], rows);
+        const GridPass t(pass[p], rows);
+        float yo = 0.f;
+        if (t.on && t.sub == 0) yo = FromGlobal{y}(t.seg);
         const float kxp = pass_dot<COMP, 2>(t.rows, t.width, t.lg, FromRecords{records, tau});
         if (t.on && t.sub == 0) {
             float* r = R + t.local;
-            const float yo = r[cur * nl], kx = r[(2 + cur) * nl], rl = r[4 * nl], ru = r[5 * nl];
+            const float kx = r[cur * nl], rl = r[2 * nl], ru = r[3 * nl];
             if (avg) {
-                const float2 a = ff_axpy(make_float2(r[6 * nl], r[7 * nl]), w, yo);
-                r[6 * nl] = a.x;
-                r[7 * nl] = a.y;
+                const float2 a = ff_axpy(make_float2(r[4 * nl], r[5 * nl]), w, yo);
+                r[4 * nl] = a.x;
+                r[5 * nl] = a.y;
             }
             const float wv = (2.0f * kxp - kx) + yo / sigma;
             const float yv = sigma * (wv - fminf(fmaxf(wv, rl), ru));
-            r[(2 + (cur ^ 1)) * nl] = kxp;
-            r[(cur ^ 1) * nl] = yv;
+            r[(cur ^ 1) * nl] = kxp;
             y_next[t.seg] = yv;
             const float dy = yv - yo;
             dy2.add(dy * dy);
@@ -851,11 +937,11 @@ __device__ __forceinline__ void grid_rows(const int4* pass, int passes, const in
 
 // The evaluation epilogue over a side, both candidates gathered from L2.
 template <bool COMP, class Epi>
-__device__ __forceinline__ void grid_eval(const int4* pass, int passes, const int2* rows, const float* v0,
+__device__ __forceinline__ void grid_eval(const int4* pass, int passes, const char* rows, const float* v0,
                                           const float* v1, Epi& epi) {
     const int nw = (blockDim.x >> 5) - 1;
     for (int p = threadIdx.x >> 5; p < passes; p += nw) {
-        const Pass t(pass[p], rows);
+        const GridPass t(pass[p], rows);
         SegDot<2> d;
         pass_sums<COMP, 1>(t.rows, t.width, t.lg, FromGlobal{v0}, d.s[0], d.e[0]);
         pass_sums<COMP, 1>(t.rows, t.width, t.lg, FromGlobal{v1}, d.s[1], d.e[1]);
@@ -878,17 +964,17 @@ __global__ void __launch_bounds__(kGridThreads, 1)
     const bool ctrl = warp == nw;
     int4* rpass = reinterpret_cast<int4*>(sm + A.sm.pass[0]);
     int4* cpass = reinterpret_cast<int4*>(sm + A.sm.pass[1]);
-    int2* rrows = reinterpret_cast<int2*>(sm + A.sm.rows[0]);
-    int2* crows = reinterpret_cast<int2*>(sm + A.sm.rows[1]);
-    float* C = reinterpret_cast<float*>(sm + A.sm.col);  // x x' | K^T y K^T y' | c l u | average hi lo
-    float* R = reinterpret_cast<float*>(sm + A.sm.row);  // y y' | K x K x' | rl ru | average hi lo
+    const char* rrows = sm + A.sm.rows[0];
+    const char* crows = sm + A.sm.rows[1];
+    float* C = reinterpret_cast<float*>(sm + A.sm.col);  // K^T y, K^T y' | c | average hi lo
+    float* R = reinterpret_cast<float*>(sm + A.sm.row);  // K x, K x' | rl ru | average hi lo
     Sums* wsum = reinterpret_cast<Sums*>(sm + A.sm.red);
     float2* ewarp = reinterpret_cast<float2*>(sm + A.sm.eval);
     double* etot = reinterpret_cast<double*>(ewarp + kEvalQ * 32);
     const int ncl = A.sm.locals[1], nrl = A.sm.locals[0];
     const int rp = blk.side[0].passes, cp = blk.side[1].passes;
     GridSync sync{count, gb.status, gb.limit_ns, count[32 * kArrive]};  // barriers of this run's earlier launches
-    load_block(A, blk, sm);
+    load_block<Wide>(A, blk, sm);
     if (threadIdx.x == 0) {
         S = *st;
         const StepScalars sc = step_scalars(S);
@@ -898,34 +984,29 @@ __global__ void __launch_bounds__(kGridThreads, 1)
     if (!ctrl) {  // owners' data and the records of the current point
         const int cur = pub.cur;
         for (int p = warp; p < cp; p += nw) {
-            const Pass t(cpass[p], crows);
+            const GridPass t(cpass[p], crows);
             if (t.on && t.sub == 0) {
                 const int j = t.seg;
                 float* c = C + t.local;
-                c[cur * ncl] = pick(V.x0, V.x1, cur)[j];
-                c[(2 + cur) * ncl] = pick(V.kty0, V.kty1, cur)[j];
-                c[4 * ncl] = V.c[j];
-                c[5 * ncl] = V.l[j];
-                c[6 * ncl] = V.u[j];
+                const float kty = c[cur * ncl] = pick(V.kty0, V.kty1, cur)[j];
+                const float cc = c[2 * ncl] = V.c[j];
                 const float2 a = V.x_acc[j];
-                c[7 * ncl] = a.x;
-                c[8 * ncl] = a.y;
-                records[(size_t)cur * N + j] =
-                    make_float4(c[cur * ncl], c[4 * ncl] + c[(2 + cur) * ncl], c[5 * ncl], c[6 * ncl]);
+                c[3 * ncl] = a.x;
+                c[4 * ncl] = a.y;
+                records[(size_t)cur * N + j] = make_float4(pick(V.x0, V.x1, cur)[j], cc + kty, V.l[j], V.u[j]);
             }
         }
         for (int p = warp; p < rp; p += nw) {
-            const Pass t(rpass[p], rrows);
+            const GridPass t(rpass[p], rrows);
             if (t.on && t.sub == 0) {
                 const int j = t.seg;
                 float* r = R + t.local;
-                r[cur * nrl] = pick(V.y0, V.y1, cur)[j];
-                r[(2 + cur) * nrl] = pick(V.kx0, V.kx1, cur)[j];
-                r[4 * nrl] = V.rl[j];
-                r[5 * nrl] = V.ru[j];
+                r[cur * nrl] = pick(V.kx0, V.kx1, cur)[j];
+                r[2 * nrl] = V.rl[j];
+                r[3 * nrl] = V.ru[j];
                 const float2 a = V.y_acc[j];
-                r[6 * nrl] = a.x;
-                r[7 * nrl] = a.y;
+                r[4 * nrl] = a.x;
+                r[5 * nrl] = a.y;
             }
         }
     }
@@ -937,14 +1018,15 @@ __global__ void __launch_bounds__(kGridThreads, 1)
             const bool avg = pub.avg != 0;
             const float w = pub.w, tau = pub.tau, sg = pub.sigma;
             const float4* rec = records + (size_t)cur * N;
+            const float* yc = pick(V.y0, V.y1, cur);
             float* yn = pick(V.y0, V.y1, cur ^ 1);
             Acc inter, dx2, dy2;
             StepCtrl ctl;
             if (!ctrl) {
                 if (comp)
-                    grid_rows<true>(rpass, rp, rrows, R, nrl, cur, rec, tau, sg, yn, avg, w, dy2);
+                    grid_rows<true>(rpass, rp, rrows, R, nrl, cur, rec, tau, sg, yc, yn, avg, w, dy2);
                 else
-                    grid_rows<false>(rpass, rp, rrows, R, nrl, cur, rec, tau, sg, yn, avg, w, dy2);
+                    grid_rows<false>(rpass, rp, rrows, R, nrl, cur, rec, tau, sg, yc, yn, avg, w, dy2);
             } else if (lane == 0) {
                 schedule_pows(S, V);
             }
@@ -952,9 +1034,9 @@ __global__ void __launch_bounds__(kGridThreads, 1)
             if (!ctrl) {
                 float4* next = records + (size_t)(cur ^ 1) * N;
                 if (comp)
-                    grid_cols<true>(cpass, cp, crows, C, ncl, cur, yn, next, tau, avg, w, inter, dx2);
+                    grid_cols<true>(cpass, cp, crows, C, ncl, cur, yn, rec, next, tau, avg, w, inter, dx2);
                 else
-                    grid_cols<false>(cpass, cp, crows, C, ncl, cur, yn, next, tau, avg, w, inter, dx2);
+                    grid_cols<false>(cpass, cp, crows, C, ncl, cur, yn, rec, next, tau, avg, w, inter, dx2);
                 warp_reduce_three(inter, dx2, dy2);
                 if (lane == 0) {
                     wsum[warp].inter = make_float2(inter.s, inter.c);
@@ -1009,33 +1091,31 @@ __global__ void __launch_bounds__(kGridThreads, 1)
         const float w = pub.w;
         if (!ctrl) {
             for (int p = warp; p < cp; p += nw) {
-                const Pass t(cpass[p], crows);
+                const GridPass t(cpass[p], crows);
                 if (t.on && t.sub == 0) {
                     const int j = t.seg;
                     float* c = C + t.local;
-                    const float x = c[cur * ncl];
-                    float2 a = make_float2(c[7 * ncl], c[8 * ncl]);
+                    const float x = ld_record(records + (size_t)cur * N + j).x;
+                    float2 a = make_float2(c[3 * ncl], c[4 * ncl]);
                     if (avg) a = ff_axpy(a, w, x);
-                    c[7 * ncl] = a.x;
-                    c[8 * ncl] = a.y;
+                    c[3 * ncl] = a.x;
+                    c[4 * ncl] = a.y;
                     pick(V.x0, V.x1, cur)[j] = x;
-                    pick(V.kty0, V.kty1, cur)[j] = c[(2 + cur) * ncl];
+                    pick(V.kty0, V.kty1, cur)[j] = c[cur * ncl];
                     V.x_acc[j] = a;
                     V.x_avg[j] = __fadd_rn(a.x, a.y);
                 }
             }
             for (int p = warp; p < rp; p += nw) {
-                const Pass t(rpass[p], rrows);
+                const GridPass t(rpass[p], rrows);
                 if (t.on && t.sub == 0) {
                     const int j = t.seg;
                     float* r = R + t.local;
-                    const float y = r[cur * nrl];
-                    float2 a = make_float2(r[6 * nrl], r[7 * nrl]);
-                    if (avg) a = ff_axpy(a, w, y);
-                    r[6 * nrl] = a.x;
-                    r[7 * nrl] = a.y;
-                    pick(V.y0, V.y1, cur)[j] = y;
-                    pick(V.kx0, V.kx1, cur)[j] = r[(2 + cur) * nrl];
+                    float2 a = make_float2(r[4 * nrl], r[5 * nrl]);
+                    if (avg) a = ff_axpy(a, w, FromGlobal{pick(V.y0, V.y1, cur)}(j));
+                    r[4 * nrl] = a.x;
+                    r[5 * nrl] = a.y;
+                    pick(V.kx0, V.kx1, cur)[j] = r[cur * nrl];
                     V.y_acc[j] = a;
                     V.y_avg[j] = __fadd_rn(a.x, a.y);
                 }
@@ -1101,37 +1181,37 @@ __global__ void __launch_bounds__(kGridThreads, 1)
         __syncthreads();
         if (!ctrl && flag != 0) {  // restart at the current (1) or the average point (2)
             for (int p = warp; p < cp; p += nw) {
-                const Pass t(cpass[p], crows);
+                const GridPass t(cpass[p], crows);
                 if (t.on && t.sub == 0) {
                     const int j = t.seg;
                     float* c = C + t.local;
+                    float* x = pick(V.x0, V.x1, cur) + j;
                     if (flag == 2) {
-                        pick(V.x0, V.x1, cur)[j] = c[cur * ncl] = V.x_avg[j];
-                        pick(V.kty0, V.kty1, cur)[j] = c[(2 + cur) * ncl] = V.kty_eval[j];
-                        records[(size_t)cur * N + j] =
-                            make_float4(c[cur * ncl], c[4 * ncl] + c[(2 + cur) * ncl], c[5 * ncl], c[6 * ncl]);
+                        *x = V.x_avg[j];
+                        const float kty = c[cur * ncl] = pick(V.kty0, V.kty1, cur)[j] = V.kty_eval[j];
+                        float4* rec = records + (size_t)cur * N + j;
+                        *rec = make_float4(*x, c[2 * ncl] + kty, rec->z, rec->w);
                     }
-                    const float x = c[cur * ncl];
-                    V.x_last[j] = x;
-                    V.x_acc[j] = make_float2(x, 0.f);
-                    c[7 * ncl] = x;
-                    c[8 * ncl] = 0.f;
+                    V.x_last[j] = *x;
+                    V.x_acc[j] = make_float2(*x, 0.f);
+                    c[3 * ncl] = *x;
+                    c[4 * ncl] = 0.f;
                 }
             }
             for (int p = warp; p < rp; p += nw) {
-                const Pass t(rpass[p], rrows);
+                const GridPass t(rpass[p], rrows);
                 if (t.on && t.sub == 0) {
                     const int j = t.seg;
                     float* r = R + t.local;
+                    float* y = pick(V.y0, V.y1, cur) + j;
                     if (flag == 2) {
-                        pick(V.y0, V.y1, cur)[j] = r[cur * nrl] = V.y_avg[j];
-                        pick(V.kx0, V.kx1, cur)[j] = r[(2 + cur) * nrl] = V.kx_eval[j];
+                        *y = V.y_avg[j];
+                        pick(V.kx0, V.kx1, cur)[j] = r[cur * nrl] = V.kx_eval[j];
                     }
-                    const float y = r[cur * nrl];
-                    V.y_last[j] = y;
-                    V.y_acc[j] = make_float2(y, 0.f);
-                    r[6 * nrl] = y;
-                    r[7 * nrl] = 0.f;
+                    V.y_last[j] = *y;
+                    V.y_acc[j] = make_float2(*y, 0.f);
+                    r[4 * nrl] = *y;
+                    r[5 * nrl] = 0.f;
                 }
             }
         }
@@ -1162,17 +1242,20 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, in
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     int4* rpass = reinterpret_cast<int4*>(sm + A.sm.pass[0]);
     int4* cpass = reinterpret_cast<int4*>(sm + A.sm.pass[1]);
-    int2* rrows = reinterpret_cast<int2*>(sm + A.sm.rows[0]);
-    int2* crows = reinterpret_cast<int2*>(sm + A.sm.rows[1]);
+    const char* rrows = sm + A.sm.rows[0];
+    const char* crows = sm + A.sm.rows[1];
     float* xs = reinterpret_cast<float*>(sm + A.sm.xs);  // x_bar; x in a check
     float* ys = reinterpret_cast<float*>(sm + A.sm.ys);
     float* C = reinterpret_cast<float*>(sm + A.sm.col);  // x | c | l | u | tau | best x
     float* R = reinterpret_cast<float*>(sm + A.sm.row);  // y | rl | ru | sigma
     const int ncl = A.sm.locals[1], nrl = A.sm.locals[0];
     const int rp = blk.side[0].passes, cp = blk.side[1].passes;
-    load_block(A, blk, sm);
+    const int n = A.inst[0].y, m = A.inst[0].w;
+    const FromShared gx{xs, n}, gy{ys, m};
+    if (threadIdx.x == 0) xs[n] = ys[m] = 0.f;
+    load_block<Compact>(A, blk, sm);
     if (threadIdx.x == 0) S = *st;
-    for (int k = threadIdx.x; k < A.inst[0].w; k += blockDim.x) ys[k] = v.y[k];
+    for (int k = threadIdx.x; k < m; k += blockDim.x) ys[k] = v.y[k];
     __syncthreads();
     for (int p = warp; p < cp; p += nw) {
         const Pass t(cpass[p], crows);
@@ -1202,7 +1285,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, in
         for (int it = 0; it < iterations; ++it) {
             for (int p = warp; p < cp; p += nw) {
                 const Pass t(cpass[p], crows);
-                const float aty = pass_dot<false, 2>(t.rows, t.width, t.lg, FromShared{ys});
+                const float aty = pass_dot<false, 2>(t.rows, t.width, t.lg, gy);
                 float x_new = 0.f;
                 if (t.on) {
                     const float* c = C + t.local;
@@ -1219,7 +1302,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, in
             cluster_wait();
             for (int p = warp; p < rp; p += nw) {
                 const Pass t(rpass[p], rrows);
-                const float axbar = pass_dot<false, 2>(t.rows, t.width, t.lg, FromShared{xs});
+                const float axbar = pass_dot<false, 2>(t.rows, t.width, t.lg, gx);
                 float y = 0.f;
                 if (t.on) {
                     const float* r = R + t.local;
@@ -1246,7 +1329,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, in
         float most[2] = {0.f, 0.f};
         for (int p = warp; p < cp; p += nw) {
             const Pass t(cpass[p], crows);
-            const float aty = pass_dot<false, 2>(t.rows, t.width, t.lg, FromShared{ys});
+            const float aty = pass_dot<false, 2>(t.rows, t.width, t.lg, gy);
             if (t.on) {
                 const float* c = C + t.local;
                 const float x = c[0], tau = c[4 * ncl];
@@ -1259,7 +1342,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, in
         cluster_wait();
         for (int p = warp; p < rp; p += nw) {
             const Pass t(rpass[p], rrows);
-            const float ax = pass_dot<false, 2>(t.rows, t.width, t.lg, FromShared{xs});
+            const float ax = pass_dot<false, 2>(t.rows, t.width, t.lg, gx);
             if (t.on) {
                 const float rl = R[nrl + t.local], ru = R[2 * nrl + t.local];
                 float viol = 0.0f;
@@ -1306,10 +1389,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, in
 namespace {
 
 // Entries of every pass from the (renumbered, scaled) matrix: a warp per pass.
+// place: {first pair, width, first segment in the batch, segments}, then
+// {the other side's first index, side, lanes, the other side's length}.
+template <class Entries>
 __global__ void k_resident_fill(int npass, const int4* __restrict__ place, SegMatrix R, SegMatrix C,
-                                int2* __restrict__ rows) {
-    // place: {first row of entries, width | log2 L << 24 | side << 30, first segment in the batch | -, segments | -},
-    // followed by the other side's first index in the next int4
+                                char* __restrict__ rows) {
     const int lane = threadIdx.x & 31;
     const int nw = gridDim.x * (blockDim.x >> 5);
     for (int p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); p < npass; p += nw) {
@@ -1317,22 +1401,20 @@ __global__ void k_resident_fill(int npass, const int4* __restrict__ place, SegMa
         const int4 o = place[2 * p + 1];
         const SegMatrix& A = o.y ? C : R;
         const int L = o.z, sub = lane & (L - 1), g = lane / L;
+        const int none = Entries::kPair == Compact::kPair ? o.w : -1;
         int k = 0, e = 0;
         if (g < t.w) {
             k = A.ptr[t.z + g] + sub;
             e = A.ptr[t.z + g + 1];
         }
-        for (int r = 0; r < t.y; ++r, k += L) {
-            int2 v = make_int2(-1, 0);
-            if (k < e) {
-                v = A.pairs[k];
-                v.x -= o.x;
-            }
-            rows[((size_t)t.x + r) * 32 + lane] = v;
+        char* out = rows + (size_t)t.x * Entries::kPair;
+        for (int r = 0; r < t.y; r += 2, k += 2 * L, out += Entries::kPair) {
+            const int2 v = k < e ? A.pairs[k] : make_int2(none + o.x, 0);
+            const int2 w = k + L < e ? A.pairs[k + L] : make_int2(none + o.x, 0);
+            Entries::store(out, v.x - o.x, __int_as_float(v.y), w.x - o.x, __int_as_float(w.y));
         }
     }
 }
-
 
 }  // namespace
 
@@ -1353,7 +1435,9 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
     const void* kernel = plain  ? (const void*)k_resident_plain
                          : grid ? (const void*)k_resident_grid
                                 : (const void*)k_resident_steps;
-    const int col_words = plain ? kPlainColWords : kColWords, row_words = plain ? kPlainRowWords : kRowWords;
+    const long long pair_bytes = grid ? Wide::kPair : Compact::kPair;
+    const int col_words = plain ? kPlainColWords : grid ? kGridColWords : kColWords;
+    const int row_words = plain ? kPlainRowWords : grid ? kGridRowWords : kRowWords;
     const int B = (int)roff.size() - 1;
     instances_ = B;
     int dev = 0, optin = 0;
@@ -1369,9 +1453,10 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
     // over 16 blocks must fit; most batches end here
     for (int b = 0; b < B; ++b) {
         const double nnz = csr_ptr[roff[b + 1]] - csr_ptr[roff[b]], m = roff[b + 1] - roff[b], n = coff[b + 1] - coff[b];
+        if (!grid && (m > 0xfffe || n > 0xfffe)) return SIH_PDHG_OK;  // 16-bit indices
         if (grid) {
             if ((16.0 * nnz + 4.0 * (col_words * n + row_words * m)) / sm_count > budget) return SIH_PDHG_OK;
-        } else if (4.0 * (m + n) + (16.0 * nnz + 4.0 * (col_words * n + row_words * m)) / 16.0 > budget) return SIH_PDHG_OK;
+        } else if (4.0 * (m + n) + (12.0 * nnz + 4.0 * (col_words * n + row_words * m)) / 16.0 > budget) return SIH_PDHG_OK;
     }
     // every instance's passes: {first segment, segments, width, log2 L}, rows of A then columns
     std::vector<int4> inst(B), all;
@@ -1436,7 +1521,7 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
                 deal(b, h, C, [&](const int4& p, int r) {
                     npass[r] += 1;
                     nloc[r] += p.y;
-                    nrow[r] += p.z;
+                    nrow[r] += (p.z + 1) / 2;
                 });
                 mpass[h] = std::max(mpass[h], *std::max_element(npass.begin(), npass.end()));
                 mloc[h] = std::max(mloc[h], *std::max_element(nloc.begin(), nloc.end()));
@@ -1449,10 +1534,10 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
             at = (at + bytes + 15) & ~15ll;
             return (int)std::min<long long>(a, INT32_MAX);
         };
-        for (int h = 0; h < 2; ++h) sm.rows[h] = put(256ll * mrows[h]);
+        for (int h = 0; h < 2; ++h) sm.rows[h] = put(pair_bytes * mrows[h]);
         for (int h = 0; h < 2; ++h) sm.pass[h] = put(16ll * mpass[h]);
-        sm.xs = put(grid ? 0 : 4ll * mn);
-        sm.ys = put(grid ? 0 : 4ll * mm);
+        sm.xs = put(grid ? 0 : 4ll * (mn + 1));
+        sm.ys = put(grid ? 0 : 4ll * (mm + 1));
         sm.locals[0] = mloc[0];
         sm.locals[1] = mloc[1];
         sm.col = put(4ll * col_words * mloc[1]);
@@ -1522,7 +1607,7 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
                 for (int r = 0; r < C; ++r) blk[r].side[h] = ResSide{};
                 deal(b, h, C, [&](const int4& p, int r) {
                     blk[r].side[h].passes += 1;
-                    blk[r].side[h].rows += p.z;
+                    blk[r].side[h].rows += (p.z + 1) / 2;
                 });
                 for (int r = 0; r < C; ++r) {
                     ResSide& sd = blk[r].side[h];
@@ -1537,25 +1622,28 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
                     const int k = next[r]++;
                     passes[k] = make_int4(sd.rows, p.z | (p.w << 24), p.x - (*offs[h])[b], sd.locals | (p.y << 24));
                     place[2 * (size_t)k] = make_int4(sd.row_begin + sd.rows, p.z, p.x, p.y);
-                    place[2 * (size_t)k + 1] = make_int4((*offs[1 - h])[b], h, 1 << p.w, 0);
-                    sd.rows += p.z;
+                    place[2 * (size_t)k + 1] = make_int4((*offs[1 - h])[b], h, 1 << p.w, (*offs[1 - h])[b + 1] - (*offs[1 - h])[b]);
+                    sd.rows += (p.z + 1) / 2;
                     sd.locals += p.y;
                 });
             }
     }
     SIHG_TRY(tab_.alloc(buf.size()));
     SIHG_CUDA(cudaMemcpyAsync(tab_.as<void>(), buf.data(), buf.size(), cudaMemcpyHostToDevice, s));
-    SIHG_TRY(rows_.alloc(256 * (size_t)std::max<long long>(1, rows)));
+    SIHG_TRY(rows_.alloc((size_t)pair_bytes * (size_t)std::max<long long>(1, rows)));
     char* d = tab_.as<char>();
-    args_ = ResArgs{(const ResBlock*)d, (const int4*)(d + o_i), (const int4*)(d + o_p), rows_.as<int2>(), sm, C};
+    args_ = ResArgs{(const ResBlock*)d, (const int4*)(d + o_i), (const int4*)(d + o_p), rows_.as<char>(), sm, C};
     ready_ = true;
     return SIH_PDHG_OK;
 }
 
 int ResidentPlan::fill(const SegMatrix& rows_A, const SegMatrix& cols_A, cudaStream_t s) {
     const int4* place = args_.passes + npass_;
-    k_resident_fill<<<std::max(1, std::min(1216, (npass_ + 7) / 8)), 256, 0, s>>>(npass_, place, rows_A, cols_A,
-                                                                                rows_.as<int2>());
+    const int g = std::max(1, std::min(1216, (npass_ + 7) / 8));
+    if (kind_ == kGrid)
+        k_resident_fill<Wide><<<g, 256, 0, s>>>(npass_, place, rows_A, cols_A, rows_.as<char>());
+    else
+        k_resident_fill<Compact><<<g, 256, 0, s>>>(npass_, place, rows_A, cols_A, rows_.as<char>());
     SIHG_LAUNCH_CHECK();
     return SIH_PDHG_OK;
 }

@@ -13,7 +13,7 @@ namespace sihg {
 // where its share of the layout lies.
 struct ResSide {
     int pass_begin, passes;  // in the pass table
-    int row_begin, rows;     // rows of 32 entries
+    int row_begin, rows;     // pairs of entries of 32 lanes
     int locals;              // segments of the side this block owns
 };
 
@@ -30,10 +30,11 @@ struct ResSmem {
 struct ResArgs {
     const ResBlock* blocks;  // [instances x cluster]
     const int4* inst;        // {first column, columns, first row, rows} of each instance
-    // pass: {first row of entries in its block, width | log2 L << 24, first
-    // segment in the instance, first local segment | segments << 24}
+    // pass: {first pair in its block, width | log2 L << 24, first segment in the
+    // instance, first local segment | segments << 24}; a pass of width w holds
+    // (w + 1) / 2 pairs per lane
     const int4* passes;
-    const int2* rows;        // entries {index in the instance, value}; empty {-1, 0}
+    const char* rows;        // the pairs (Compact or Wide, see resident.cu), indices in the instance
     ResSmem sm;
     int cluster;
 };
