@@ -76,6 +76,43 @@ std::vector<uint8_t> segment_lanes(const SideSchedule& sc, int nseg) {
     return lanes;
 }
 
+std::vector<int> order_by_lanes(const int* ptr, const uint8_t* lanes, int cnt) {
+    // counting sort on (lanes descending, length descending)
+    int longest = 0;
+    for (int k = 0; k < cnt; ++k) longest = std::max(longest, ptr[k + 1] - ptr[k]);
+    int group[33] = {};
+    for (int lg = 0; lg <= 5; ++lg) group[1 << lg] = 5 - lg;
+    const size_t span = (size_t)longest + 1;
+    auto key = [&](int k) { return group[lanes[k]] * span + (size_t)(longest - (ptr[k + 1] - ptr[k])); };
+    std::vector<int> start(6 * span + 1, 0), order(cnt);
+    for (int k = 0; k < cnt; ++k) start[key(k) + 1]++;
+    for (size_t v = 0; v < 6 * span; ++v) start[v + 1] += start[v];
+    for (int k = 0; k < cnt; ++k) order[start[key(k)]++] = k;
+    return order;
+}
+
+void make_packs(const std::vector<int>& ptr, const std::vector<uint8_t>& lanes, int warps, std::vector<int4>& packs,
+                std::vector<int>& warp_begin) {
+    const int nseg = (int)ptr.size() - 1;
+    packs.clear();
+    std::vector<long long> cost(1, 0);  // running; an entry and a constant part per pack and segment
+    for (int s = 0; s < nseg;) {
+        int e = s + 1, lg = 0;
+        while ((1 << lg) < lanes[s]) ++lg;
+        while (e < nseg && e - s < 32 && lanes[e] == lanes[s] && ptr[e + 1] - ptr[s] <= kPackEntries) ++e;
+        const int n = ptr[e] - ptr[s];
+        packs.push_back(make_int4(s, ptr[s], (e - s) | (lg << 8), n));
+        cost.push_back(cost.back() + n + 128);
+        s = e;
+    }
+    warp_begin.assign((size_t)warps + 1, (int)packs.size());
+    int p = 0;
+    for (int w = 0; w < warps; ++w) {  // a share ends where its part of the cost does
+        while (p < (int)packs.size() && cost[p] * warps < cost.back() * w) ++p;
+        warp_begin[w] = p;
+    }
+}
+
 int TaskLayout::build(const std::vector<int>& csr_ptr, const std::vector<int>& csc_ptr, const std::vector<int>& roff,
                       const std::vector<int>& coff, const SegMatrix& rows_A, const SegMatrix& cols_A, int task_nnz,
                       bool all_active, cudaStream_t s, int row_lanes, int col_lanes, int max_segs) {

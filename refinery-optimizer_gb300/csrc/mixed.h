@@ -110,6 +110,33 @@ void make_schedule(const std::vector<int>& ptr, const std::vector<int>& inst_off
 // Lanes per segment that a schedule gives to each of nseg segments.
 std::vector<uint8_t> segment_lanes(const SideSchedule& sc, int nseg);
 
+// Packs of one side for kernels whose segments lie by lanes, then by descending
+// length (see spmv_packs): a pack is up to 32 consecutive segments of equal
+// lanes with at most kPackEntries entries, or one longer segment.
+// {first segment, first entry, segments | log2 lanes << 8, entries}
+// 384 entries (12 per lane) at four blocks of 256 threads per SM, measured on
+// the 100k x 200k LP of 2.4M entries (us per iteration of two kernels; 43.5
+// with tasks handed out by a counter, 35.5 with the same tasks on fixed
+// shares): 29.8; 256 / 320 / 512 entries 34.0 / 30.2 / 39.8; eight per lane at a
+// time 32.4 (512 entries); 3 / 5 / 6 blocks 32.8 / 39.7 / 42.6 and up.
+constexpr int kPackEntries = 384;
+struct PackSide {
+    const int4* packs;
+    const int* warp_begin;
+    const int* ptr;
+    const int2* pairs;
+};
+// Host: the packs of a side and one share of them per warp: warp w works packs
+// [warp_begin[w], warp_begin[w + 1]).
+void make_packs(const std::vector<int>& ptr, const std::vector<uint8_t>& lanes, int warps, std::vector<int4>& packs,
+                std::vector<int>& warp_begin);
+// Order of `cnt` segments by lanes, then by descending length (stable).
+std::vector<int> order_by_lanes(const int* ptr, const uint8_t* lanes, int cnt);
+// Renumbered pairs of one side on the device (mixed.cu): segment s takes the
+// entries from src[s].x on, indices mapped through inv[src[s].y + index].
+__global__ void k_renumber_pairs(int nseg, const int* __restrict__ ptr, const int2* __restrict__ src,
+                                 const int2* __restrict__ in, const int* __restrict__ inv, int2* __restrict__ out);
+
 // Device task layout of a block-diagonal (batched) matrix for the task engine
 // (warp.cuh): per side (rows = CSR for A x, columns = CSC for A^T y) the SpMV
 // tasks, their reduction groups, partial slots, tickets and active list; the

@@ -3,8 +3,8 @@
 // Per iteration (core/src/gpu/gpu_solver.cpp:227-239) the reference launches
 // four kernels: CSC SpMV A^T y, the primal update, CSR SpMV A x_bar and the dual
 // update.  Here the SpMVs and their updates are fused:
-//   plain_primal_kernel : z_j = (A^T y)_j (CSC)  ->  x, x_bar update   (cuda_pdhg.cu:33-77)
-//   plain_dual_kernel   : w_i = (A x_bar)_i (CSR) ->  y update         (cuda_pdhg.cu:14-30, 82-103)
+//   plain_primal_packs, _kernel (exact) : z_j = (A^T y)_j (CSC)  ->  x, x_bar update   (cuda_pdhg.cu:33-77)
+//   plain_dual_packs, _kernel (exact)   : w_i = (A x_bar)_i (CSR) ->  y update         (cuda_pdhg.cu:14-30, 82-103)
 // so A^T y and A x_bar never reach HBM.  The reference's restart kernel
 // (x_bar <- x every 250 iterations, cuda_pdhg.cu:106-111) has no effect on the
 // iterates because the next primal update overwrites x_bar before it is read,
@@ -102,29 +102,32 @@ __global__ void __launch_bounds__(256, 8) plain_dual_kernel(SegMatrix A, SpmvPla
     spmv_run<EXACT>(A, P, v.xbar, epi);
 }
 
-// Fast path of the iteration (exact_arithmetic = 0): the same epilogues on
-// the task engine (warp.cuh: dynamic warp tasks, software-pipelined loads).
-template <class E>
-struct PlainTaskEpi {
-    E e;
-    const float* vec;
-    using Pre = typename E::Pre;
-    __device__ __forceinline__ Pre pre(int k) const { return e.pre(k); }
-    __device__ __forceinline__ void begin(const PlainState&) {}
-    __device__ __forceinline__ const float* gather(int) const { return vec; }
-    __device__ __forceinline__ void apply(int k, const SegDot<1>& d, const Pre& p) { e.apply(k, d.s[0], p); }
+// Fast path of the iteration (exact_arithmetic = 0): the same epilogues over
+// packs (warp.cuh).
+struct PackPrimal : PrimalEpi {
+    __device__ __forceinline__ const float* gather(int) const { return v.y; }
 };
+struct PackDual : DualEpi {
+    __device__ __forceinline__ const float* gather(int) const { return v.xbar; }
+};
+constexpr int kPackBlocks = 4;  // blocks per SM (packs of 384 entries, see kPackEntries)
 
-__global__ void __launch_bounds__(kThreads, 4) plain_primal_tasks(Side cols, PlainVecs v, PlainState* st) {
+__global__ void __launch_bounds__(kThreads, kPackBlocks) plain_primal_packs(PackSide cols, PlainVecs v,
+                                                                            const PlainState* st) {
+    __shared__ float2 window[kThreads / 32][kPackEntries];
+    chain_wait();
     if (st->done) return;
-    PlainTaskEpi<PrimalEpi> epi{PrimalEpi{v}, v.y};
-    spmv_engine<1, false, 0>(cols, st, epi, 0u);
+    PackPrimal epi{{v}};
+    spmv_packs(cols, epi, window[threadIdx.x >> 5]);
 }
 
-__global__ void __launch_bounds__(kThreads, 4) plain_dual_tasks(Side rows, PlainVecs v, PlainState* st) {
+__global__ void __launch_bounds__(kThreads, kPackBlocks) plain_dual_packs(PackSide rows, PlainVecs v,
+                                                                          const PlainState* st) {
+    __shared__ float2 window[kThreads / 32][kPackEntries];
+    chain_wait();
     if (st->done) return;
-    PlainTaskEpi<DualEpi> epi{DualEpi{v}, v.xbar};
-    spmv_engine<1, false, 0>(rows, st, epi, 0u);
+    PackDual epi{{v}};
+    spmv_packs(rows, epi, window[threadIdx.x >> 5]);
 }
 
 template <bool EXACT>
@@ -194,6 +197,48 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
     SIHG_CUDA(cudaEventCreate(&ev_start_));
     SIHG_CUDA(cudaEventCreate(&ev_stop_));
 
+    cudaStream_t s = stream_;
+    // Lanes per segment of the fast iteration (they fix the order of its sums):
+    // make_schedule's for tasks of a third of a warp's share at four blocks per
+    // SM.  LPs that fit run in one cluster in the caller's order; the others are
+    // renumbered by lanes and length, so that packs of segments are uniform.
+    bool packs = false;
+    std::vector<uint8_t> row_lanes, col_lanes;
+    if (!exact_ && m > 0 && n > 0) {
+        const long long warps = (long long)sm_count_ * 4 * (kThreads / 32);
+        const int task_nnz = opts.tile_nnz > 0
+                                 ? opts.tile_nnz
+                                 : (int)std::max(128LL, std::min(2048LL, (long long)nnz / std::max(1LL, 3 * warps)));
+        SideSchedule rs, cs;
+        make_schedule(hp.csr_ptr, std::vector<int>{0, m}, task_nnz, rs);
+        make_schedule(hp.csc_ptr, std::vector<int>{0, n}, task_nnz, cs);
+        row_lanes = segment_lanes(rs, m);
+        col_lanes = segment_lanes(cs, n);
+        if (opts.use_graph)
+            SIHG_TRY(resident_->build(hp.csr_ptr, hp.csc_ptr, std::vector<int>{0, m}, std::vector<int>{0, n}, row_lanes,
+                                      col_lanes, sm_count_, s, ResidentPlan::kPlain));
+        packs = !resident_->ready();
+    }
+    std::vector<int> csc_ptr, csr_ptr;
+    if (packs) {
+        auto renumber = [](const std::vector<int>& ptr, std::vector<uint8_t>& lanes, std::vector<int>& order,
+                           std::vector<int>& new_ptr) {
+            const int cnt = (int)ptr.size() - 1;
+            order = order_by_lanes(ptr.data(), lanes.data(), cnt);
+            new_ptr.assign((size_t)cnt + 1, 0);
+            std::vector<uint8_t> l(cnt);
+            for (int k = 0; k < cnt; ++k) {
+                new_ptr[k + 1] = new_ptr[k] + ptr[order[k] + 1] - ptr[order[k]];
+                l[k] = lanes[order[k]];
+            }
+            lanes.swap(l);
+        };
+        renumber(hp.csc_ptr, col_lanes, col_order_, csc_ptr);
+        renumber(hp.csr_ptr, row_lanes, row_order_, csr_ptr);
+    }
+    const std::vector<int>& cptr = packs ? csc_ptr : hp.csc_ptr;
+    const std::vector<int>& rptr = packs ? csr_ptr : hp.csr_ptr;
+
     SIHG_TRY(csc_ptr_.alloc(sizeof(int) * (n + 1)));
     SIHG_TRY(csr_ptr_.alloc(sizeof(int) * (m + 1)));
     SIHG_TRY(csc_pairs_.alloc(sizeof(Pair) * nnz));
@@ -202,12 +247,40 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
     SIHG_TRY(rowvec_.alloc(sizeof(float) * (size_t)m * 4));
     SIHG_TRY(state_.alloc(sizeof(PlainState)));
 
-    cudaStream_t s = stream_;
-    SIHG_CUDA(cudaMemcpyAsync(csc_ptr_.as<int>(), hp.csc_ptr.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s));
-    SIHG_CUDA(cudaMemcpyAsync(csr_ptr_.as<int>(), hp.csr_ptr.data(), sizeof(int) * (m + 1), cudaMemcpyHostToDevice, s));
-    if (nnz > 0) {
+    SIHG_CUDA(cudaMemcpyAsync(csc_ptr_.as<int>(), cptr.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s));
+    SIHG_CUDA(cudaMemcpyAsync(csr_ptr_.as<int>(), rptr.data(), sizeof(int) * (m + 1), cudaMemcpyHostToDevice, s));
+    if (nnz > 0 && !packs) {
         SIHG_CUDA(cudaMemcpyAsync(csc_pairs_.as<Pair>(), hp.csc.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
         SIHG_CUDA(cudaMemcpyAsync(csr_pairs_.as<Pair>(), hp.csr.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
+    } else if (nnz > 0) {  // the pairs as they are, renumbered on the device
+        std::vector<int2> src((size_t)n + m);
+        std::vector<int> inv((size_t)n + m);  // rows' new numbers, then columns'
+        parallel_for(n, [&](int64_t k0, int64_t k1) {
+            for (int64_t k = k0; k < k1; ++k) {
+                src[k] = make_int2(hp.csc_ptr[col_order_[k]], 0);
+                inv[(size_t)m + col_order_[k]] = (int)k;
+            }
+        });
+        parallel_for(m, [&](int64_t k0, int64_t k1) {
+            for (int64_t k = k0; k < k1; ++k) {
+                src[(size_t)n + k] = make_int2(hp.csr_ptr[row_order_[k]], m);
+                inv[row_order_[k]] = (int)k;
+            }
+        });
+        DevMem raw, seg, map;
+        SIHG_TRY(raw.alloc(sizeof(Pair) * 2 * (size_t)nnz));
+        SIHG_TRY(seg.alloc(sizeof(int2) * src.size()));
+        SIHG_TRY(map.alloc(sizeof(int) * inv.size()));
+        SIHG_CUDA(cudaMemcpyAsync(raw.as<Pair>(), hp.csc.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
+        SIHG_CUDA(cudaMemcpyAsync(raw.as<Pair>() + nnz, hp.csr.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
+        SIHG_CUDA(cudaMemcpyAsync(seg.as<int2>(), src.data(), sizeof(int2) * src.size(), cudaMemcpyHostToDevice, s));
+        SIHG_CUDA(cudaMemcpyAsync(map.as<int>(), inv.data(), sizeof(int) * inv.size(), cudaMemcpyHostToDevice, s));
+        k_renumber_pairs<<<sm_count_ * 8, 256, 0, s>>>(n, csc_ptr_.as<int>(), seg.as<int2>(), raw.as<int2>(),
+                                                       map.as<int>(), csc_pairs_.as<int2>());
+        k_renumber_pairs<<<sm_count_ * 8, 256, 0, s>>>(m, csr_ptr_.as<int>(), seg.as<int2>() + n, raw.as<int2>() + nnz,
+                                                       map.as<int>(), csr_pairs_.as<int2>());
+        SIHG_LAUNCH_CHECK();
+        SIHG_CUDA(cudaStreamSynchronize(s));  // the staging buffers are released at scope end
     }
     float* cv = colvec_.as<float>();
     float* rv = rowvec_.as<float>();
@@ -223,16 +296,29 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
     vec_.ru = rv + 1 * (size_t)m;
     vec_.sigma = rv + 2 * (size_t)m;
     vec_.y = rv + 3 * (size_t)m;
-    SIHG_CUDA(cudaMemcpyAsync(cv + 0 * (size_t)n, hp.c.data(), sizeof(float) * n, cudaMemcpyHostToDevice, s));
-    SIHG_CUDA(cudaMemcpyAsync(cv + 1 * (size_t)n, hp.l.data(), sizeof(float) * n, cudaMemcpyHostToDevice, s));
-    SIHG_CUDA(cudaMemcpyAsync(cv + 2 * (size_t)n, hp.u.data(), sizeof(float) * n, cudaMemcpyHostToDevice, s));
-    SIHG_CUDA(cudaMemcpyAsync(rv + 0 * (size_t)m, hp.rl.data(), sizeof(float) * m, cudaMemcpyHostToDevice, s));
-    SIHG_CUDA(cudaMemcpyAsync(rv + 1 * (size_t)m, hp.ru.data(), sizeof(float) * m, cudaMemcpyHostToDevice, s));
+    std::vector<float> host((size_t)3 * n + 2 * (size_t)m);  // c l u | rl ru in device order
+    parallel_for(n, [&](int64_t k0, int64_t k1) {
+        for (int64_t k = k0; k < k1; ++k) {
+            const int64_t j = packs ? col_order_[k] : k;
+            host[k] = hp.c[j];
+            host[(size_t)n + k] = hp.l[j];
+            host[2 * (size_t)n + k] = hp.u[j];
+        }
+    });
+    parallel_for(m, [&](int64_t k0, int64_t k1) {
+        for (int64_t k = k0; k < k1; ++k) {
+            const int64_t i = packs ? row_order_[k] : k;
+            host[3 * (size_t)n + k] = hp.rl[i];
+            host[3 * (size_t)n + m + k] = hp.ru[i];
+        }
+    });
+    SIHG_CUDA(cudaMemcpyAsync(cv, host.data(), sizeof(float) * 3 * (size_t)n, cudaMemcpyHostToDevice, s));
+    SIHG_CUDA(cudaMemcpyAsync(rv, host.data() + 3 * (size_t)n, sizeof(float) * 2 * (size_t)m, cudaMemcpyHostToDevice, s));
 
     // plans and heavy lists
     std::vector<int> heavy_c, heavy_r;
-    plan_csc_ = make_plan(hp.csc_ptr, opts.lanes_csc, opts.heavy_factor, exact_, sm_count_, heavy_c);
-    plan_csr_ = make_plan(hp.csr_ptr, opts.lanes_csr, opts.heavy_factor, exact_, sm_count_, heavy_r);
+    plan_csc_ = make_plan(cptr, opts.lanes_csc, opts.heavy_factor, exact_, sm_count_, heavy_c);
+    plan_csr_ = make_plan(rptr, opts.lanes_csr, opts.heavy_factor, exact_, sm_count_, heavy_r);
     SIHG_TRY(heavy_.alloc(sizeof(int) * (heavy_c.size() + heavy_r.size() + 1)));
     if (!heavy_c.empty())
         SIHG_CUDA(cudaMemcpyAsync(heavy_.as<int>(), heavy_c.data(), sizeof(int) * heavy_c.size(), cudaMemcpyHostToDevice, s));
@@ -243,23 +329,23 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
     plan_csr_.heavy_idx = heavy_.as<int>() + heavy_c.size();
     At_ = SegMatrix{n, csc_ptr_.as<int>(), csc_pairs_.as<int2>()};
     A_ = SegMatrix{m, csr_ptr_.as<int>(), csr_pairs_.as<int2>()};
-    if (!exact_ && m > 0 && n > 0) {  // task engine of the fast iteration kernels
-        int occ = 0;
-        SIHG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, plain_primal_tasks, kThreads, 0));
-        task_grid_ = sm_count_ * std::max(1, occ);
-        const long long warps = (long long)task_grid_ * (kThreads / 32);
-        const int task_nnz = opts.tile_nnz > 0
-                                 ? opts.tile_nnz
-                                 : (int)std::max(128LL, std::min(2048LL, (long long)nnz / std::max(1LL, 3 * warps)));
-        SIHG_TRY(layout_.build(hp.csr_ptr, hp.csc_ptr, std::vector<int>{0, m}, std::vector<int>{0, n}, A_, At_,
-                               task_nnz, true, s));
-    }
-
-    if (layout_.rows.ntasks > 0 && opts.use_graph) {  // LPs that fit: every iteration in one cluster
-        SIHG_TRY(resident_->build(hp.csr_ptr, hp.csc_ptr, std::vector<int>{0, m}, std::vector<int>{0, n},
-                                  segment_lanes(layout_.row_schedule, m), segment_lanes(layout_.col_schedule, n),
-                                  sm_count_, s, ResidentPlan::kPlain));
-        if (resident_->ready()) SIHG_TRY(resident_->fill(A_, At_, s));
+    if (resident_->ready()) SIHG_TRY(resident_->fill(A_, At_, s));
+    if (packs) {
+        pack_grid_ = sm_count_ * kPackBlocks;
+        const int warps = pack_grid_ * (kThreads / 32);
+        std::vector<int4> pc, pr;
+        std::vector<int> bc, br;
+        make_packs(cptr, col_lanes, warps, pc, bc);
+        make_packs(rptr, row_lanes, warps, pr, br);
+        const size_t nc = sizeof(int4) * pc.size(), nr = sizeof(int4) * pr.size(), nb = sizeof(int) * bc.size();
+        SIHG_TRY(packs_.alloc(nc + nr + 2 * nb));
+        char* d = packs_.as<char>();
+        SIHG_CUDA(cudaMemcpyAsync(d, pc.data(), nc, cudaMemcpyHostToDevice, s));
+        SIHG_CUDA(cudaMemcpyAsync(d + nc, pr.data(), nr, cudaMemcpyHostToDevice, s));
+        SIHG_CUDA(cudaMemcpyAsync(d + nc + nr, bc.data(), nb, cudaMemcpyHostToDevice, s));
+        SIHG_CUDA(cudaMemcpyAsync(d + nc + nr + nb, br.data(), nb, cudaMemcpyHostToDevice, s));
+        cols_ = PackSide{(const int4*)d, (const int*)(d + nc + nr), At_.ptr, At_.pairs};
+        rows_ = PackSide{(const int4*)(d + nc), (const int*)(d + nc + nr + nb), A_.ptr, A_.pairs};
     }
 
     // step sizes on the device, in the reference's summation order
@@ -275,9 +361,10 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
     }
     // initial point x = clip(0, l, u) (gpu_solver.cpp:192-196), x_bar = x, y = 0
     x0_.resize(n);
-    for (int j = 0; j < n; ++j) {
+    for (int k = 0; k < n; ++k) {
+        const int j = packs ? col_order_[k] : k;
         const float up0 = (0.0f < hp.u[j]) ? 0.0f : hp.u[j];   // std::min(u, 0)
-        x0_[j] = (hp.l[j] < up0) ? up0 : hp.l[j];              // std::max(l, .)
+        x0_[k] = (hp.l[j] < up0) ? up0 : hp.l[j];              // std::max(l, .)
     }
     // max |c| and max |b| over finite bounds (gpu_solver.cpp:112-126)
     max_abs_c_ = 1.0f;
@@ -297,9 +384,8 @@ int PlainSolver::launch_iteration(cudaStream_t s) {
         plain_primal_kernel<true><<<plan_csc_.grid(), plan_csc_.threads, 0, s>>>(At_, plan_csc_, vec_, st);
         plain_dual_kernel<true><<<plan_csr_.grid(), plan_csr_.threads, 0, s>>>(A_, plan_csr_, vec_, st);
     } else {
-        PlainState* sw = state_.as<PlainState>();
-        plain_primal_tasks<<<task_grid_, kThreads, 0, s>>>(layout_.cols, vec_, sw);
-        plain_dual_tasks<<<task_grid_, kThreads, 0, s>>>(layout_.rows, vec_, sw);
+        SIHG_CUDA(launch_chained(plain_primal_packs, pack_grid_, kThreads, 0, s, cols_, vec_, st));
+        SIHG_CUDA(launch_chained(plain_dual_packs, pack_grid_, kThreads, 0, s, rows_, vec_, st));
     }
     SIHG_LAUNCH_CHECK();
     return SIH_PDHG_OK;
@@ -325,11 +411,6 @@ int PlainSolver::record_block(int iters, cudaGraphExec_t* exec) {
     cudaGraph_t g = nullptr;
     SIHG_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     int rc = SIH_PDHG_OK;
-    if (!exact_ && layout_.rows.counters) {  // the task counters restart with every block
-        cudaError_t e = cudaMemsetAsync(layout_.rows.counters, 0, sizeof(unsigned), stream_);
-        if (e == cudaSuccess) e = cudaMemsetAsync(layout_.cols.counters, 0, sizeof(unsigned), stream_);
-        if (e != cudaSuccess) rc = cuda_fail(e, "cudaMemsetAsync", __FILE__, __LINE__);
-    }
     for (int k = 0; k < iters && rc == SIH_PDHG_OK; ++k) rc = launch_iteration(stream_);
     if (rc == SIH_PDHG_OK) rc = launch_check(stream_);
     cudaError_t e = cudaStreamEndCapture(stream_, &g);
@@ -371,10 +452,6 @@ int PlainSolver::reset_state() {
     st.max_iterations = cfg_.max_iterations;
     host_state_ = st;
     SIHG_CUDA(cudaMemcpyAsync(state_.as<PlainState>(), &host_state_, sizeof(PlainState), cudaMemcpyHostToDevice, s));
-    if (!exact_ && layout_.rows.counters) {
-        SIHG_CUDA(cudaMemsetAsync(layout_.rows.counters, 0, sizeof(unsigned), s));
-        SIHG_CUDA(cudaMemsetAsync(layout_.cols.counters, 0, sizeof(unsigned), s));
-    }
     return SIH_PDHG_OK;
 }
 
@@ -428,10 +505,6 @@ int PlainSolver::iterate() {
                 if (e != cudaSuccess) { rc = cuda_fail(e, "cudaGraphLaunch", __FILE__, __LINE__); break; }
             } else {
                 const int its = is_tail ? tail : cf;
-                if (!exact_ && layout_.rows.counters) {  // task counters restart with every block
-                    cudaMemsetAsync(layout_.rows.counters, 0, sizeof(unsigned), s);
-                    cudaMemsetAsync(layout_.cols.counters, 0, sizeof(unsigned), s);
-                }
                 for (int k = 0; k < its && rc == SIH_PDHG_OK; ++k) rc = launch_iteration(s);
                 if (rc == SIH_PDHG_OK) rc = launch_check(s);
             }
@@ -458,6 +531,14 @@ int PlainSolver::fetch(std::vector<float>& best_x, std::vector<float>& y) {
     y.resize(hp_->m);
     SIHG_CUDA(cudaMemcpy(best_x.data(), vec_.best_x, sizeof(float) * hp_->n, cudaMemcpyDeviceToHost));
     SIHG_CUDA(cudaMemcpy(y.data(), vec_.y, sizeof(float) * hp_->m, cudaMemcpyDeviceToHost));
+    auto back = [](std::vector<float>& v, const std::vector<int>& order) {  // to the caller's order
+        if (order.empty()) return;
+        std::vector<float> t(v.size());
+        for (size_t k = 0; k < v.size(); ++k) t[order[k]] = v[k];
+        v.swap(t);
+    };
+    back(best_x, col_order_);
+    back(y, row_order_);
     return SIH_PDHG_OK;
 }
 

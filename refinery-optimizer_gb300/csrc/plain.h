@@ -29,7 +29,7 @@ struct PlainState {
     float tol_d;
     int check_frequency;
     int max_iterations;
-    int refine;          // task-engine flag (compensated SpMVs): always 0 here
+    int reserved;
 };
 
 // The host part of the reference check (gpu_solver.cpp:252-268) for the largest
@@ -101,8 +101,10 @@ class PlainSolver {
     cudaEvent_t ev_start_ = nullptr, ev_stop_ = nullptr;
     cudaGraphExec_t block_exec_ = nullptr, tail_exec_ = nullptr;
     DevMem csc_ptr_, csr_ptr_, csc_pairs_, csr_pairs_, colvec_, rowvec_, state_, heavy_;
-    TaskLayout layout_;   // task engine of the fast (non-exact) iteration kernels
-    int task_grid_ = 1;
+    DevMem packs_;  // packs of the fast iteration (columns, rows), then each warp's first (columns, rows)
+    PackSide cols_{}, rows_{};
+    int pack_grid_ = 1;
+    std::vector<int> col_order_, row_order_;  // device order -> caller's (empty: the same)
     std::unique_ptr<ResidentPlan> resident_;  // LPs that fit in a cluster: iterations and checks there
     SegMatrix A_{}, At_{};
     SpmvPlan plan_csr_{}, plan_csc_{};

@@ -1227,7 +1227,7 @@ __global__ void __launch_bounds__(kGridThreads, 1)
 // Plain algorithm (the reference's FP32 PDHG): `checks` times `iterations`
 // iterations and the reference's convergence check, on one cluster.  Two
 // phases an iteration, no reduction and no controller between checks.  The
-// element updates are those of plain_primal_tasks / plain_dual_tasks; the
+// element updates are those of plain_primal_packs / plain_dual_packs; the
 // check takes its maxima over the same sums.
 __global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, int iterations, int checks, PlainVecs v,
                                                                    PlainState* st) {

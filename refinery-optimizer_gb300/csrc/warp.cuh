@@ -455,6 +455,84 @@ __device__ __forceinline__ void spmv_engine(const Side& side, State* st, Epi& ep
     });
 }
 
+// SpMV without reductions over packs (make_packs), every warp on its fixed
+// share.  A warp reads a pack's entries at once, all of them in flight, into its
+// window of shared memory ({value, gathered}), then the lane groups sum their
+// segments from there, in the order in which seg_dots does.  What counts is
+// the number of gathers in flight per SM: a whole pack per warp, loads that do
+// not wait for a segment's pointers, a counter or a task record, and an L1
+// that holds a line for every miss (shared memory takes its space).
+template <class Epi>
+__device__ __forceinline__ void spmv_packs(const PackSide& P, Epi& epi, float2* __restrict__ window) {
+    constexpr int kU = kPackEntries / 32;
+    static_assert(kPackEntries % (32 * kBatch) == 0, "a long segment continues on the same chains");
+    const int lane = threadIdx.x & 31;
+    const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int p0 = P.warp_begin[w], p1 = P.warp_begin[w + 1];
+    if (p0 >= p1) return;
+    const float* __restrict__ vec = epi.gather(0);
+    int4 rec = P.packs[p0];
+    for (int p = p0; p < p1; ++p) {
+        const int4 next = P.packs[min(p + 1, p1 - 1)];
+        const int nseg = rec.z & 0xff, lg = rec.z >> 8, n = rec.w;
+        const int L = 1 << lg, gpw = 32 >> lg, sub = lane & (L - 1);
+        const bool mine = lane < nseg;
+        int beg = 0, end = 0;  // this lane's segment in the pack
+        typename Epi::Pre pre{};
+        if (mine) {
+            beg = P.ptr[rec.x + lane] - rec.y;
+            end = P.ptr[rec.x + lane + 1] - rec.y;
+            pre = epi.pre(rec.x + lane);
+        }
+        float acc[kBatch] = {0.f, 0.f, 0.f, 0.f}, res = 0.f;
+        for (int w0 = 0; w0 < n; w0 += kPackEntries) {
+            const int cnt = min(kPackEntries, n - w0);
+            const int2* __restrict__ pairs = P.pairs + rec.y + w0;
+            for (int k0 = lane; k0 < cnt; k0 += 32 * kU) {
+                int2 q[kU];
+                float g[kU];
+#pragma unroll
+                for (int u = 0; u < kU; ++u) q[u] = k0 + 32 * u < cnt ? ld_pair(pairs + k0 + 32 * u) : make_int2(-1, 0);
+#pragma unroll
+                for (int u = 0; u < kU; ++u) g[u] = q[u].x >= 0 ? ld_vec(vec + q[u].x) : 0.f;
+#pragma unroll
+                for (int u = 0; u < kU; ++u)
+                    if (q[u].x >= 0) window[k0 + 32 * u] = make_float2(__int_as_float(q[u].y), g[u]);
+            }
+            __syncwarp();
+            // entries lo + sub, + L, ... on chain 0, 1, 2, 3, 0, ...
+            auto chains = [&](int lo, int hi) {
+                for (int k = lo + sub; k < hi; k += kBatch * L) {
+#pragma unroll
+                    for (int u = 0; u < kBatch; ++u) {
+                        const float2 v = k + u * L < hi ? window[k + u * L] : make_float2(0.f, 0.f);
+                        acc[u] = fmaf(v.x, v.y, acc[u]);
+                    }
+                }
+            };
+            if (n <= kPackEntries) {
+                for (int s0 = 0; s0 < nseg; s0 += gpw) {
+                    const int from = s0 + (lane >> lg);
+                    const int lo = __shfl_sync(FULL_MASK, beg, from & 31), hi = __shfl_sync(FULL_MASK, end, from & 31);
+#pragma unroll
+                    for (int u = 0; u < kBatch; ++u) acc[u] = 0.f;
+                    if (from < nseg) chains(lo, hi);
+                    __syncwarp();
+                    const float s = group_sum((acc[0] + acc[1]) + (acc[2] + acc[3]), L);
+                    const float v = __shfl_sync(FULL_MASK, s, (lane & (gpw - 1)) << lg);
+                    if ((lane & ~(gpw - 1)) == s0) res = v;
+                }
+            } else if (lane < L) {  // one long segment, kPackEntries (a multiple of 4 L) at a time
+                chains(0, cnt);
+            }
+            __syncwarp();
+        }
+        if (n > kPackEntries) res = group_sum((acc[0] + acc[1]) + (acc[2] + acc[3]), L);
+        if (mine) epi.apply(rec.x + lane, res, pre);
+        rec = next;
+    }
+}
+
 // Elementwise pass over every column (is_col) and row of the running
 // instances: blocks take chunks of kChunk consecutive elements of one
 // instance, threads stride through a chunk (coalesced).  `prep(S)` turns the
