@@ -91,26 +91,17 @@ std::vector<int> order_by_lanes(const int* ptr, const uint8_t* lanes, int cnt) {
     return order;
 }
 
-void make_packs(const std::vector<int>& ptr, const std::vector<uint8_t>& lanes, int warps, std::vector<int4>& packs,
-                std::vector<int>& warp_begin) {
+std::vector<int4> make_packs(const std::vector<int>& ptr, const std::vector<uint8_t>& lanes) {
     const int nseg = (int)ptr.size() - 1;
-    packs.clear();
-    std::vector<long long> cost(1, 0);  // running; an entry and a constant part per pack and segment
+    std::vector<int4> packs;
     for (int s = 0; s < nseg;) {
         int e = s + 1, lg = 0;
         while ((1 << lg) < lanes[s]) ++lg;
         while (e < nseg && e - s < 32 && lanes[e] == lanes[s] && ptr[e + 1] - ptr[s] <= kPackEntries) ++e;
-        const int n = ptr[e] - ptr[s];
-        packs.push_back(make_int4(s, ptr[s], (e - s) | (lg << 8), n));
-        cost.push_back(cost.back() + n + 128);
+        packs.push_back(make_int4(s, ptr[s], (e - s) | (lg << 8), ptr[e] - ptr[s]));
         s = e;
     }
-    warp_begin.assign((size_t)warps + 1, (int)packs.size());
-    int p = 0;
-    for (int w = 0; w < warps; ++w) {  // a share ends where its part of the cost does
-        while (p < (int)packs.size() && cost[p] * warps < cost.back() * w) ++p;
-        warp_begin[w] = p;
-    }
+    return packs;
 }
 
 int TaskLayout::build(const std::vector<int>& csr_ptr, const std::vector<int>& csc_ptr, const std::vector<int>& roff,

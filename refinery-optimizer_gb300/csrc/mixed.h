@@ -115,21 +115,20 @@ std::vector<uint8_t> segment_lanes(const SideSchedule& sc, int nseg);
 // lanes with at most kPackEntries entries, or one longer segment.
 // {first segment, first entry, segments | log2 lanes << 8, entries}
 // 384 entries (12 per lane) at four blocks of 256 threads per SM, measured on
-// the 100k x 200k LP of 2.4M entries (us per iteration of two kernels; 43.5
-// with tasks handed out by a counter, 35.5 with the same tasks on fixed
-// shares): 29.8; 256 / 320 / 512 entries 34.0 / 30.2 / 39.8; eight per lane at a
-// time 32.4 (512 entries); 3 / 5 / 6 blocks 32.8 / 39.7 / 42.6 and up.
+// the 100k x 200k LP of 2.4M entries (us per iteration of two kernels, with one
+// run of packs per warp; 43.5 with tasks handed out by a counter, 35.5 with the
+// same tasks on fixed shares): 29.8; 256 / 320 / 512 entries 34.0 / 30.2 / 39.8;
+// eight per lane at a time 32.4 (512 entries); 3 / 5 / 6 blocks 32.8 / 39.7 /
+// 42.6 and up.
 constexpr int kPackEntries = 384;
 struct PackSide {
     const int4* packs;
-    const int* warp_begin;
+    int count;
     const int* ptr;
     const int2* pairs;
 };
-// Host: the packs of a side and one share of them per warp: warp w works packs
-// [warp_begin[w], warp_begin[w + 1]).
-void make_packs(const std::vector<int>& ptr, const std::vector<uint8_t>& lanes, int warps, std::vector<int4>& packs,
-                std::vector<int>& warp_begin);
+// Host: the packs of a side.
+std::vector<int4> make_packs(const std::vector<int>& ptr, const std::vector<uint8_t>& lanes);
 // Order of `cnt` segments by lanes, then by descending length (stable).
 std::vector<int> order_by_lanes(const int* ptr, const uint8_t* lanes, int cnt);
 // Renumbered pairs of one side on the device (mixed.cu): segment s takes the

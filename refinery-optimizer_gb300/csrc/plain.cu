@@ -332,20 +332,13 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
     if (resident_->ready()) SIHG_TRY(resident_->fill(A_, At_, s));
     if (packs) {
         pack_grid_ = sm_count_ * kPackBlocks;
-        const int warps = pack_grid_ * (kThreads / 32);
-        std::vector<int4> pc, pr;
-        std::vector<int> bc, br;
-        make_packs(cptr, col_lanes, warps, pc, bc);
-        make_packs(rptr, row_lanes, warps, pr, br);
-        const size_t nc = sizeof(int4) * pc.size(), nr = sizeof(int4) * pr.size(), nb = sizeof(int) * bc.size();
-        SIHG_TRY(packs_.alloc(nc + nr + 2 * nb));
-        char* d = packs_.as<char>();
-        SIHG_CUDA(cudaMemcpyAsync(d, pc.data(), nc, cudaMemcpyHostToDevice, s));
-        SIHG_CUDA(cudaMemcpyAsync(d + nc, pr.data(), nr, cudaMemcpyHostToDevice, s));
-        SIHG_CUDA(cudaMemcpyAsync(d + nc + nr, bc.data(), nb, cudaMemcpyHostToDevice, s));
-        SIHG_CUDA(cudaMemcpyAsync(d + nc + nr + nb, br.data(), nb, cudaMemcpyHostToDevice, s));
-        cols_ = PackSide{(const int4*)d, (const int*)(d + nc + nr), At_.ptr, At_.pairs};
-        rows_ = PackSide{(const int4*)(d + nc), (const int*)(d + nc + nr + nb), A_.ptr, A_.pairs};
+        const std::vector<int4> pc = make_packs(cptr, col_lanes), pr = make_packs(rptr, row_lanes);
+        SIHG_TRY(packs_.alloc(sizeof(int4) * (pc.size() + pr.size())));
+        int4* d = packs_.as<int4>();
+        SIHG_CUDA(cudaMemcpyAsync(d, pc.data(), sizeof(int4) * pc.size(), cudaMemcpyHostToDevice, s));
+        SIHG_CUDA(cudaMemcpyAsync(d + pc.size(), pr.data(), sizeof(int4) * pr.size(), cudaMemcpyHostToDevice, s));
+        cols_ = PackSide{d, (int)pc.size(), At_.ptr, At_.pairs};
+        rows_ = PackSide{d + pc.size(), (int)pr.size(), A_.ptr, A_.pairs};
     }
 
     // step sizes on the device, in the reference's summation order

@@ -101,7 +101,7 @@ class PlainSolver {
     cudaEvent_t ev_start_ = nullptr, ev_stop_ = nullptr;
     cudaGraphExec_t block_exec_ = nullptr, tail_exec_ = nullptr;
     DevMem csc_ptr_, csr_ptr_, csc_pairs_, csr_pairs_, colvec_, rowvec_, state_, heavy_;
-    DevMem packs_;  // packs of the fast iteration (columns, rows), then each warp's first (columns, rows)
+    DevMem packs_;  // packs of the fast iteration (columns, rows)
     PackSide cols_{}, rows_{};
     int pack_grid_ = 1;
     std::vector<int> col_order_, row_order_;  // device order -> caller's (empty: the same)

@@ -455,25 +455,33 @@ __device__ __forceinline__ void spmv_engine(const Side& side, State* st, Epi& ep
     });
 }
 
-// SpMV without reductions over packs (make_packs), every warp on its fixed
-// share.  A warp reads a pack's entries at once, all of them in flight, into its
+// SpMV without reductions over packs (make_packs), handed out in turn: first to
+// every block's first warp, then to its second, and so on.  Neighbours cost
+// about the same, so the warps and the SMs get even shares, also when there are
+// fewer packs than warps, and the grid sweeps the matrix from front to back.
+// A warp reads a pack's entries at once, all of them in flight, into its
 // window of shared memory ({value, gathered}), then the lane groups sum their
 // segments from there, in the order in which seg_dots does.  What counts is
 // the number of gathers in flight per SM: a whole pack per warp, loads that do
 // not wait for a segment's pointers, a counter or a task record, and an L1
 // that holds a line for every miss (shared memory takes its space).
+// Microseconds per iteration (two kernels) with tasks from a counter, with one
+// run of neighbouring packs per warp and with packs in turn: 20k x 50k, 0.5M
+// entries 15.7 / 10.7 / 9.6; 60k x 130k, 1M entries 24.1 / 15.8 / 15.1; 250k x
+// 500k, 3M, lengths by a power law 60.8 / 49.2 / 41.8; 500k x 1M, 12M, likewise
+// 139.9 / 145.8 / 133.8.
 template <class Epi>
 __device__ __forceinline__ void spmv_packs(const PackSide& P, Epi& epi, float2* __restrict__ window) {
     constexpr int kU = kPackEntries / 32;
     static_assert(kPackEntries % (32 * kBatch) == 0, "a long segment continues on the same chains");
     const int lane = threadIdx.x & 31;
-    const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int p0 = P.warp_begin[w], p1 = P.warp_begin[w + 1];
-    if (p0 >= p1) return;
+    const int w = blockIdx.x + gridDim.x * (threadIdx.x >> 5);
+    const int nw = gridDim.x * (blockDim.x >> 5);
+    if (w >= P.count) return;
     const float* __restrict__ vec = epi.gather(0);
-    int4 rec = P.packs[p0];
-    for (int p = p0; p < p1; ++p) {
-        const int4 next = P.packs[min(p + 1, p1 - 1)];
+    int4 rec = P.packs[w];
+    for (int p = w; p < P.count; p += nw) {
+        const int4 next = P.packs[min(p + nw, P.count - 1)];
         const int nseg = rec.z & 0xff, lg = rec.z >> 8, n = rec.w;
         const int L = 1 << lg, gpw = 32 >> lg, sub = lane & (L - 1);
         const bool mine = lane < nseg;
