@@ -380,6 +380,115 @@ __device__ __forceinline__ void solo_grid_total(const float2* __restrict__ part,
     }
 }
 
+// ---------------------------------------------------------------- steps of one LP over packs
+// The two step SpMVs of one LP by kernels: packs of uniform segments dealt to
+// the warps in turn (spmv_packs), the same per-segment sums as the task
+// engine's.  Each block leaves one partial of the step's sums; the block that
+// arrives last adds them in block order and runs the instance's part (finish),
+// where the task engine has a slot and a ticket per task.  Gathers bound both
+// kernels (a sector of L2 each).  Microseconds of K x' / K^T y', tasks -> packs:
+// 200k x 400k, 4.8M nonzeros 44.0 / 41.4 -> 27.1 / 26.5; 500k x 1M, 12M nonzeros,
+// lengths by a power law 69.9 (staged) / 77.5 -> 61.9 / 70.0.  There a prefix of
+// the gathered vector in shared memory no longer pays: the windows and the prefix
+// leave L1 too few lines for the gathers that miss it (one block of 512 threads:
+// 68.9 to 71.5 / 101; of 1024: 85 and up / 112 and up).
+//
+// The epilogues over packs pick their vectors where they use them: a pack's
+// loads in flight leave no registers for a dozen pointers.
+struct DualPackEpi {
+    Vecs V;
+    int cur;
+    float sigma;
+    Acc dy2;
+    struct Pre { float kx = 0.f, y = 0.f, rl = 0.f, ru = 0.f; };
+    __device__ void begin(const Inst& S) {
+        cur = S.cur;
+        sigma = (float)(S.eta * S.omega);
+    }
+    __device__ const float* gather(int) const { return pick(V.x0, V.x1, cur ^ 1); }
+    __device__ Pre pre(int i) const {
+        return Pre{pick(V.kx0, V.kx1, cur)[i], pick(V.y0, V.y1, cur)[i], V.rl[i], V.ru[i]};
+    }
+    __device__ void apply(int i, const SegDot<1>& d, const Pre& p) {
+        const float kxp = d.f(0);  // hi + lo when compensated
+        const float wv = (2.0f * kxp - p.kx) + p.y / sigma;
+        const float yv = sigma * (wv - fminf(fmaxf(wv, p.rl), p.ru));
+        pick(V.kx0, V.kx1, cur ^ 1)[i] = kxp;
+        pick(V.y0, V.y1, cur ^ 1)[i] = yv;
+        const float dy = yv - p.y;
+        dy2.add(dy * dy);
+    }
+    __device__ void values(Acc (&q)[1]) const { q[0] = dy2; }
+    __device__ void finish(Inst& S, const double* tot) const { S.dy2 = tot[0]; }
+};
+
+struct KtyPackEpi {
+    Vecs V;
+    int cur;
+    Acc inter, dx2;
+    struct Pre { float x = 0.f, xn = 0.f, kty = 0.f; };
+    __device__ void begin(const Inst& S) { cur = S.cur; }
+    __device__ const float* gather(int) const { return pick(V.y0, V.y1, cur ^ 1); }
+    __device__ Pre pre(int j) const {
+        return Pre{pick(V.x0, V.x1, cur)[j], pick(V.x0, V.x1, cur ^ 1)[j], pick(V.kty0, V.kty1, cur)[j]};
+    }
+    __device__ void apply(int j, const SegDot<1>& d, const Pre& p) {
+        const float k = d.f(0);
+        pick(V.kty0, V.kty1, cur ^ 1)[j] = k;
+        const float dx = p.xn - p.x;
+        inter.add(dx * (k - p.kty));
+        dx2.add(dx * dx);
+    }
+    __device__ void values(Acc (&q)[2]) const {
+        q[0] = inter;
+        q[1] = dx2;
+    }
+    __device__ void finish(Inst& S, const double* tot) const { step_controller(S, tot[1], tot[0]); }
+};
+
+template <int Q, class Epi>
+__device__ __forceinline__ void step_packs(const PackSide& side, Inst* st, Epi& epi, float2* window,
+                                           const PackTotals& T) {
+    __shared__ Acc sh[32 * Q];
+    __shared__ unsigned last;
+    Inst& S = st[0];
+    if (S.done) return;  // it changes between steps only
+    epi.begin(S);
+    if (S.refine)
+        spmv_packs<true>(side, epi, window);
+    else
+        spmv_packs<false>(side, epi, window);
+    Acc q[Q];
+    epi.values(q);
+    solo_block_partial<Q>(q, T.part + Q * blockIdx.x, sh);
+    if (threadIdx.x == 0) last = ticket_add(T.ticket) + 1u == gridDim.x;
+    __syncthreads();
+    if (!last) return;
+    double tot[Q];
+    solo_grid_total<Q>(T.part, gridDim.x, tot, sh);
+    if (threadIdx.x == 0) {
+        *T.ticket = 0u;
+        epi.finish(S, tot);
+    }
+}
+
+__global__ void __launch_bounds__(kThreads, kStepPackBlocks)
+    k_step_dual_packs(PackSide rows, Vecs V, Inst* __restrict__ st, PackTotals T) {
+    __shared__ float2 window[kThreads / 32][kPackEntries];
+    chain_wait();
+    step_schedule_pows(1, st, V);
+    DualPackEpi epi{V};
+    step_packs<1>(rows, st, epi, window[threadIdx.x >> 5], T);
+}
+
+__global__ void __launch_bounds__(kThreads, kStepPackBlocks)
+    k_step_kty_packs(PackSide cols, Vecs V, Inst* __restrict__ st, PackTotals T) {
+    __shared__ float2 window[kThreads / 32][kPackEntries];
+    chain_wait();
+    KtyPackEpi epi{V};
+    step_packs<2>(cols, st, epi, window[threadIdx.x >> 5], T);
+}
+
 // This warp's static share of a side's tasks with epilogue `epi`; the lanes'
 // partials (over all the warp's tasks) end in q.
 template <int Q, class Epi>
@@ -1130,6 +1239,10 @@ static int upload(DevMem& d, const void* h, size_t bytes, cudaStream_t s) {
 // One LP whose matrix (both sides, 16 bytes per nonzero) fits in half of L2.
 bool MixedSolver::latency_bound() const { return B_ == 1 && 16.0 * (double)nnz_ <= kSoloMaxBytes; }
 
+bool MixedSolver::use_packs() const {
+    return B_ == 1 && opts_.packed <= 0 && opts_.staged_kib <= 0 && M_ > 0 && N_ > 0 && (double)nnz_ >= kPackMinNnz;
+}
+
 // Tasks, reduction groups, tickets, element chunks and active lists for SpMV
 // tasks of about `task_nnz` nonzeros (rebuilt by the autotuner).
 int MixedSolver::build_schedules(int task_nnz) {
@@ -1145,6 +1258,25 @@ int MixedSolver::build_schedules(int task_nnz) {
     rows_ = layout_.rows;
     cols_ = layout_.cols;
     chunks_all_ = layout_.chunks;
+    return build_packs();
+}
+
+// Packs of the steps by kernels (one LP beyond the latency-bound range).
+int MixedSolver::build_packs() {
+    pack_cols_.count = pack_rows_.count = 0;
+    if (!use_packs()) return SIH_PDHG_OK;
+    const std::vector<int4> pc = make_packs(h_csc_ptr_, segment_lanes(layout_.col_schedule, N_));
+    const std::vector<int4> pr = make_packs(h_csr_ptr_, segment_lanes(layout_.row_schedule, M_));
+    const size_t bc = sizeof(int4) * pc.size(), br = sizeof(int4) * pr.size();
+    const size_t bt = sizeof(float2) * 2 * (size_t)sm_count_ * kStepPackBlocks;
+    SIHG_TRY(packs_.alloc(bc + br + bt + sizeof(unsigned)));
+    char* d = packs_.as<char>();
+    SIHG_CUDA(cudaMemcpyAsync(d, pc.data(), bc, cudaMemcpyHostToDevice, stream_));
+    SIHG_CUDA(cudaMemcpyAsync(d + bc, pr.data(), br, cudaMemcpyHostToDevice, stream_));
+    pack_totals_ = PackTotals{(float2*)(d + bc + br), (unsigned*)(d + bc + br + bt)};
+    SIHG_CUDA(cudaMemsetAsync(pack_totals_.ticket, 0, sizeof(unsigned), stream_));
+    pack_cols_ = PackSide{(const int4*)d, (int)pc.size(), csc_ptr_.as<int>(), csc_pairs_.as<int2>()};
+    pack_rows_ = PackSide{(const int4*)(d + bc), (int)pr.size(), csr_ptr_.as<int>(), csr_pairs_.as<int2>()};
     return SIH_PDHG_OK;
 }
 
@@ -1427,7 +1559,10 @@ int MixedSolver::setup_resident() {
     if (!resident_->ready() && B_ == 1)
         SIHG_TRY(resident_->build(h_csr_ptr_, h_csc_ptr_, row_off_, col_off_, rl, cl, sm_count_, stream_,
                                   ResidentPlan::kGrid));
-    if (!resident_->ready()) return SIH_PDHG_OK;
+    if (!resident_->ready()) {
+        // one LP beyond the resident forms: steps over packs (see kPackMinNnz)
+        return B_ == 1 && opts_.persistent < 0 && opts_.use_graph && use_packs() ? set_form(0) : SIH_PDHG_OK;
+    }
     SIHG_TRY(resident_->fill(SegMatrix{M_, csr_ptr_.as<int>(), csr_pairs_.as<int2>()},
                              SegMatrix{N_, csc_ptr_.as<int>(), csc_pairs_.as<int2>()}, stream_));
     persistent_ = B_ == 1 ? 2 : 1;
@@ -1609,6 +1744,14 @@ int MixedSolver::launch_step_spmvs(cudaStream_t s, int which) {
             SIHG_CUDA(launch_chained(k_step_kty_packed, grid_, kThreads, 0, s, cols_, V_, st, pack_.as<float4>(), N_));
         return SIH_PDHG_OK;
     }
+    if (pack_rows_.count > 0) {
+        const int grid = sm_count_ * kStepPackBlocks;
+        if (which == 1)
+            SIHG_CUDA(launch_chained(k_step_dual_packs, grid, kThreads, 0, s, pack_rows_, V_, st, pack_totals_));
+        else
+            SIHG_CUDA(launch_chained(k_step_kty_packs, grid, kThreads, 0, s, pack_cols_, V_, st, pack_totals_));
+        return SIH_PDHG_OK;
+    }
     if (which == 1) {
         if (stage_x_ > 0)
             SIHG_CUDA(launch_chained(k_step_dual_staged, sm_count_, kStagedThreads, sizeof(float) * stage_x_, s, B_,
@@ -1633,7 +1776,7 @@ int MixedSolver::launch_step_spmvs(cudaStream_t s, int which) {
 int MixedSolver::choose_staging() {
     constexpr double kStagedShare = 0.5;
     stage_x_ = stage_y_ = 0;
-    if (B_ != 1 || opts_.staged_kib < 0 || nnz_ == 0) return SIH_PDHG_OK;
+    if (B_ != 1 || opts_.staged_kib < 0 || nnz_ == 0 || use_packs()) return SIH_PDHG_OK;
     int dev = 0, optin = 0;
     SIHG_CUDA(cudaGetDevice(&dev));
     SIHG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));

@@ -177,6 +177,22 @@ struct Vecs {
 
 class ResidentPlan;  // resident.h
 
+// Steps over packs of one LP (mixed.cu): blocks per SM, and the nonzeros from
+// which one LP takes them instead of the task engine and, where it does not fit
+// a resident form, instead of k_solo_steps.  Microseconds per step, tasks /
+// k_solo_steps / packs: 60k x 120k, 1.4M nonzeros, lengths by a power law 54.7 /
+// 36.2 / 32.9; 100k x 200k, 1.6M, equal lengths 56.5 / 36.3 / 32.6; refinery
+// planning over 336 periods 58.6 / 41.7 / 32.1; 200k x 400k, 4.8M 93.8 / - / 64.1;
+// 500k x 1M, 12M, power law 163.8 (longest columns staged) / - / 149.1.  Below
+// the line (20k x 50k, 0.4M: 30.7 / - / 22.5) the resident forms hold the LP, and
+// the forms that a caller asks for by number keep their common order of sums.
+constexpr int kStepPackBlocks = 4;
+constexpr double kPackMinNnz = 0.25e6;
+struct PackTotals {
+    float2* part;      // a partial per block and sum
+    unsigned* ticket;  // 0 between launches
+};
+
 class MixedSolver {
   public:
     MixedSolver();
@@ -214,6 +230,8 @@ class MixedSolver {
     int pull_points();
     void unscale(int b, std::vector<double>& x, std::vector<double>& y) const;
     int build_schedules(int task_nnz);
+    bool use_packs() const;
+    int build_packs();
     bool latency_bound() const;  // one LP small enough that its steps are latency-bound
     int autotune();
     int launch_compact(cudaStream_t s);
@@ -253,6 +271,10 @@ class MixedSolver {
     Side rows_{}, cols_{};
     Chunks chunks_all_{};
     int elem_grid_ = 1;
+    // packs of the steps by kernels (one LP; count 0: none), their block partials
+    PackSide pack_cols_{}, pack_rows_{};
+    PackTotals pack_totals_{};
+    DevMem packs_;
     // staged gathers (single LP): entries of x (for K x) and of y (for K^T y)
     // copied to shared memory by every block of the step kernels; 0 = off
     int stage_x_ = 0, stage_y_ = 0;

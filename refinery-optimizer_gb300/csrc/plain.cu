@@ -106,9 +106,11 @@ __global__ void __launch_bounds__(256, 8) plain_dual_kernel(SegMatrix A, SpmvPla
 // packs (warp.cuh).
 struct PackPrimal : PrimalEpi {
     __device__ __forceinline__ const float* gather(int) const { return v.y; }
+    __device__ __forceinline__ void apply(int j, const SegDot<1>& d, const Pre& p) { PrimalEpi::apply(j, d.s[0], p); }
 };
 struct PackDual : DualEpi {
     __device__ __forceinline__ const float* gather(int) const { return v.xbar; }
+    __device__ __forceinline__ void apply(int i, const SegDot<1>& d, const Pre& p) { DualEpi::apply(i, d.s[0], p); }
 };
 constexpr int kPackBlocks = 4;  // blocks per SM (packs of 384 entries, see kPackEntries)
 
@@ -118,7 +120,7 @@ __global__ void __launch_bounds__(kThreads, kPackBlocks) plain_primal_packs(Pack
     chain_wait();
     if (st->done) return;
     PackPrimal epi{{v}};
-    spmv_packs(cols, epi, window[threadIdx.x >> 5]);
+    spmv_packs<false>(cols, epi, window[threadIdx.x >> 5]);
 }
 
 __global__ void __launch_bounds__(kThreads, kPackBlocks) plain_dual_packs(PackSide rows, PlainVecs v,
@@ -127,7 +129,7 @@ __global__ void __launch_bounds__(kThreads, kPackBlocks) plain_dual_packs(PackSi
     chain_wait();
     if (st->done) return;
     PackDual epi{{v}};
-    spmv_packs(rows, epi, window[threadIdx.x >> 5]);
+    spmv_packs<false>(rows, epi, window[threadIdx.x >> 5]);
 }
 
 template <bool EXACT>

@@ -455,7 +455,7 @@ __device__ __forceinline__ void spmv_engine(const Side& side, State* st, Epi& ep
     });
 }
 
-// SpMV without reductions over packs (make_packs), handed out in turn: first to
+// SpMV over packs (make_packs), handed out in turn: first to
 // every block's first warp, then to its second, and so on.  Neighbours cost
 // about the same, so the warps and the SMs get even shares, also when there are
 // fewer packs than warps, and the grid sweeps the matrix from front to back.
@@ -465,12 +465,15 @@ __device__ __forceinline__ void spmv_engine(const Side& side, State* st, Epi& ep
 // the number of gathers in flight per SM: a whole pack per warp, loads that do
 // not wait for a segment's pointers, a counter or a task record, and an L1
 // that holds a line for every miss (shared memory takes its space).
-// Microseconds per iteration (two kernels) with tasks from a counter, with one
-// run of neighbouring packs per warp and with packs in turn: 20k x 50k, 0.5M
-// entries 15.7 / 10.7 / 9.6; 60k x 130k, 1M entries 24.1 / 15.8 / 15.1; 250k x
-// 500k, 3M, lengths by a power law 60.8 / 49.2 / 41.8; 500k x 1M, 12M, likewise
-// 139.9 / 145.8 / 133.8.
-template <class Epi>
+// The epilogue's operands load behind the gathers, when the pairs' registers
+// are free (before them: 64 registers spill, 2 % slower); packs of up to 128
+// short segments, four per lane, spill as well (6 to 15 % slower).
+// Microseconds per iteration of the plain algorithm (two kernels) with tasks from
+// a counter, with one run of neighbouring packs per warp and with packs in turn:
+// 20k x 50k, 0.5M entries 15.7 / 10.7 / 9.6; 60k x 130k, 1M entries 24.1 / 15.8 /
+// 14.9; 250k x 500k, 3M, lengths by a power law 60.8 / 49.2 / 41.0; 500k x 1M, 12M,
+// likewise 139.9 / 145.8 / 137.5 (gathers through L1 and L2: 175 G a second).
+template <bool COMP, class Epi>
 __device__ __forceinline__ void spmv_packs(const PackSide& P, Epi& epi, float2* __restrict__ window) {
     constexpr int kU = kPackEntries / 32;
     static_assert(kPackEntries % (32 * kBatch) == 0, "a long segment continues on the same chains");
@@ -484,59 +487,98 @@ __device__ __forceinline__ void spmv_packs(const PackSide& P, Epi& epi, float2* 
         const int4 next = P.packs[min(p + nw, P.count - 1)];
         const int nseg = rec.z & 0xff, lg = rec.z >> 8, n = rec.w;
         const int L = 1 << lg, gpw = 32 >> lg, sub = lane & (L - 1);
-        const bool mine = lane < nseg;
-        int beg = 0, end = 0;  // this lane's segment in the pack
-        typename Epi::Pre pre{};
-        if (mine) {
-            beg = P.ptr[rec.x + lane] - rec.y;
-            end = P.ptr[rec.x + lane + 1] - rec.y;
-            pre = epi.pre(rec.x + lane);
-        }
-        float acc[kBatch] = {0.f, 0.f, 0.f, 0.f}, res = 0.f;
-        for (int w0 = 0; w0 < n; w0 += kPackEntries) {
-            const int cnt = min(kPackEntries, n - w0);
+        // entries [w0, w0 + cnt) of the pack to the window
+        auto fill = [&](int w0, int cnt) {
             const int2* __restrict__ pairs = P.pairs + rec.y + w0;
-            for (int k0 = lane; k0 < cnt; k0 += 32 * kU) {
-                int2 q[kU];
-                float g[kU];
+            int2 q[kU];
+            float g[kU];
 #pragma unroll
-                for (int u = 0; u < kU; ++u) q[u] = k0 + 32 * u < cnt ? ld_pair(pairs + k0 + 32 * u) : make_int2(-1, 0);
+            for (int u = 0; u < kU; ++u)
+                q[u] = lane + 32 * u < cnt ? ld_pair(pairs + lane + 32 * u) : make_int2(-1, 0);
 #pragma unroll
-                for (int u = 0; u < kU; ++u) g[u] = q[u].x >= 0 ? ld_vec(vec + q[u].x) : 0.f;
+            for (int u = 0; u < kU; ++u) g[u] = q[u].x >= 0 ? ld_vec(vec + q[u].x) : 0.f;
 #pragma unroll
-                for (int u = 0; u < kU; ++u)
-                    if (q[u].x >= 0) window[k0 + 32 * u] = make_float2(__int_as_float(q[u].y), g[u]);
-            }
-            __syncwarp();
-            // entries lo + sub, + L, ... on chain 0, 1, 2, 3, 0, ...
-            auto chains = [&](int lo, int hi) {
-                for (int k = lo + sub; k < hi; k += kBatch * L) {
+            for (int u = 0; u < kU; ++u)
+                if (q[u].x >= 0) window[lane + 32 * u] = make_float2(__int_as_float(q[u].y), g[u]);
+        };
+        float acc[kBatch], err;  // COMP: sum acc[0], its error err
+        auto clear = [&]() {
 #pragma unroll
-                    for (int u = 0; u < kBatch; ++u) {
-                        const float2 v = k + u * L < hi ? window[k + u * L] : make_float2(0.f, 0.f);
+            for (int u = 0; u < kBatch; ++u) acc[u] = 0.f;
+            err = 0.f;
+        };
+        // entries lo + sub, + L, ... of the window on chain 0, 1, 2, 3, 0, ...
+        auto chains = [&](int lo, int hi) {
+            for (int k = lo + sub; k < hi; k += kBatch * L) {
+#pragma unroll
+                for (int u = 0; u < kBatch; ++u) {
+                    const float2 v = k + u * L < hi ? window[k + u * L] : make_float2(0.f, 0.f);
+                    if (COMP) {
+                        float pr, pe, ss, se;
+                        two_prod(v.x, v.y, pr, pe);
+                        two_sum(acc[0], pr, ss, se);
+                        acc[0] = ss;
+                        err = __fadd_rn(err, __fadd_rn(pe, se));
+                    } else {
                         acc[u] = fmaf(v.x, v.y, acc[u]);
                     }
                 }
-            };
-            if (n <= kPackEntries) {
-                for (int s0 = 0; s0 < nseg; s0 += gpw) {
-                    const int from = s0 + (lane >> lg);
-                    const int lo = __shfl_sync(FULL_MASK, beg, from & 31), hi = __shfl_sync(FULL_MASK, end, from & 31);
-#pragma unroll
-                    for (int u = 0; u < kBatch; ++u) acc[u] = 0.f;
-                    if (from < nseg) chains(lo, hi);
-                    __syncwarp();
-                    const float s = group_sum((acc[0] + acc[1]) + (acc[2] + acc[3]), L);
-                    const float v = __shfl_sync(FULL_MASK, s, (lane & (gpw - 1)) << lg);
-                    if ((lane & ~(gpw - 1)) == s0) res = v;
-                }
-            } else if (lane < L) {  // one long segment, kPackEntries (a multiple of 4 L) at a time
-                chains(0, cnt);
             }
+        };
+        // the lane group's sum (in its first lane)
+        auto total = [&](float& e) {
+            float s = COMP ? acc[0] : (acc[0] + acc[1]) + (acc[2] + acc[3]);
+            e = err;
+            if (COMP)
+                group_sum2(s, e, L);
+            else
+                s = group_sum(s, L);
+            return s;
+        };
+        if (n <= kPackEntries) {
+            int beg = 0, end = 0;  // this lane's segment in the pack
+            typename Epi::Pre pre;
+            if (lane < nseg) {
+                beg = P.ptr[rec.x + lane] - rec.y;
+                end = P.ptr[rec.x + lane + 1] - rec.y;
+            }
+            fill(0, n);
+            if (lane < nseg) pre = epi.pre(rec.x + lane);
             __syncwarp();
+            SegDot<1> d{};
+            for (int s0 = 0; s0 < nseg; s0 += gpw) {
+                const int from = s0 + (lane >> lg);
+                const int lo = __shfl_sync(FULL_MASK, beg, from & 31), hi = __shfl_sync(FULL_MASK, end, from & 31);
+                clear();
+                if (from < nseg) chains(lo, hi);
+                __syncwarp();
+                float e;
+                const float s = total(e);
+                const int owner = (lane & (gpw - 1)) << lg;
+                const float v = __shfl_sync(FULL_MASK, s, owner);
+                const float ve = COMP ? __shfl_sync(FULL_MASK, e, owner) : 0.f;
+                if ((lane & ~(gpw - 1)) == s0) {
+                    d.s[0] = v;
+                    d.e[0] = ve;
+                }
+            }
+            if (lane < nseg) epi.apply(rec.x + lane, d, pre);
+            __syncwarp();
+        } else {  // one long segment, kPackEntries (a multiple of 4 L) at a time
+            typename Epi::Pre pre{};
+            if (lane == 0) pre = epi.pre(rec.x);
+            clear();
+            for (int w0 = 0; w0 < n; w0 += kPackEntries) {
+                const int cnt = min(kPackEntries, n - w0);
+                fill(w0, cnt);
+                __syncwarp();
+                if (lane < L) chains(0, cnt);
+                __syncwarp();
+            }
+            SegDot<1> d;
+            d.s[0] = total(d.e[0]);
+            if (lane == 0) epi.apply(rec.x, d, pre);
         }
-        if (n > kPackEntries) res = group_sum((acc[0] + acc[1]) + (acc[2] + acc[3]), L);
-        if (mine) epi.apply(rec.x + lane, res, pre);
         rec = next;
     }
 }
