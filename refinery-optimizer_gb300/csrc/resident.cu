@@ -19,15 +19,22 @@
 // other forms up to the order of the compensated norms, whose FP64 totals
 // differ in the last bits at most.
 //
-// What bounds it (cycle counters around each phase, 2,000 x 5,000 LP on 16
-// blocks, 14,100 cycles = 6.8 us per step): the x' phase 1,050, its barrier with
-// the average updates 2,100, A x' 2,200, barrier 1,150, A^T y' 3,250, barrier
-// 1,400, the controller 2,550 (of which one FP64 division 550 and a dozen
-// dependent FP64 operations of 65 each).  The phases are chains of dependent
-// instructions on one or two passes per warp; the entries themselves are a
-// small part.  Measured per step, whole solves: 317 x 803 13.7 -> 5.2 us (1, 2, 4, 8
-// blocks: 8.7, 6.6, 5.2, 5.2), 2,000 x 5,000 13.7 -> 7.4 us (8 blocks: 9.9), 64 of
-// the latter as a batch 84 -> 43 us.
+// What bounds it: with one or two passes per warp the chains of dependent
+// instructions (cycle counters around each phase, 2,000 x 5,000 LP on 16 blocks,
+// 14,100 cycles a step before the last line of the measurements below: the x'
+// phase 1,050, its barrier with the average updates 2,100, A x' 2,200, barrier
+// 1,150, A^T y' 3,250, barrier 1,400, the controller 2,550, of which one FP64
+// division 550 and a dozen dependent FP64 operations of 65 each); with four and
+// more the number of instructions as well.  Measured per step, whole solves:
+// 317 x 803 13.7 -> 5.2 us (1, 2, 4, 8 blocks: 8.7, 6.6, 5.2, 5.2), 2,000 x 5,000
+// 13.7 -> 7.4 us (8 blocks: 9.9), 64 of the latter as a batch 84 -> 43 us, with
+// 12 bytes a pair of entries (four blocks an instance, two rounds of clusters) ->
+// 20.8 us.  Fewer instructions from there, steps alone: 16 warps with passes
+// instead of 20 and as few as do the passes in the same rounds, x' by a thread per
+// column instead of the lanes of its passes, the rest of a pass by code of its
+// length: the batch 20.8 -> 18.7 us, 64 of 1,000 x 2,500 by a power law 16.0 ->
+// 13.5, 2,000 x 5,000 6.9 -> 6.4, 317 x 803 4.5 -> 4.3 (26 and 30 warps: 23.0 and
+// 22.5 on the batch, 13: 23.2).
 #include <algorithm>
 #include <cstring>
 
@@ -40,7 +47,8 @@ namespace sihg {
 
 namespace {
 
-constexpr int kResThreads = 672;   // most threads of a block of a cluster: 20 warps with passes, the controller
+constexpr int kResThreads = 544;   // most threads of a block of a cluster: 16 warps with passes, the controller
+constexpr int kResWarps = kResThreads / 32;
 constexpr int kGridThreads = 768;  // threads of a block of the grid form
 constexpr int kColWords = 8;       // per column: x, K^T y (2), c, l, u, average (2); x' is in the copy
 constexpr int kRowWords = 7;       // per row: y, K x (2), rl, ru, average (2); y' is in the copy
@@ -96,11 +104,10 @@ __device__ __forceinline__ void push(float* p, float v, int sub, int L, int clus
 // gathered vector, so that no lane has to ask.
 struct Compact {
     static constexpr int kPair = 32 * 12;
-    static __device__ __forceinline__ void load(const char* p, bool on, int none, int& i0, float& a0, int& i1,
-                                                float& a1) {
+    static __device__ __forceinline__ void load(const char* p, int& i0, float& a0, int& i1, float& a1) {
         const int lane = threadIdx.x & 31;
-        const float2 a = on ? *reinterpret_cast<const float2*>(p + 8 * lane) : make_float2(0.f, 0.f);
-        const unsigned i = on ? *reinterpret_cast<const unsigned*>(p + 256 + 4 * lane) : none * 0x10001u;
+        const float2 a = *reinterpret_cast<const float2*>(p + 8 * lane);
+        const unsigned i = *reinterpret_cast<const unsigned*>(p + 256 + 4 * lane);
         i0 = i & 0xffffu;
         i1 = i >> 16;
         a0 = a.x;
@@ -115,9 +122,8 @@ struct Compact {
 // Over every SM: 32-bit indices, empty places -1.
 struct Wide {
     static constexpr int kPair = 32 * 16;
-    static __device__ __forceinline__ void load(const char* p, bool on, int none, int& i0, float& a0, int& i1,
-                                                float& a1) {
-        const int4 q = on ? *reinterpret_cast<const int4*>(p + 16 * (threadIdx.x & 31)) : make_int4(none, 0, none, 0);
+    static __device__ __forceinline__ void load(const char* p, int& i0, float& a0, int& i1, float& a1) {
+        const int4 q = *reinterpret_cast<const int4*>(p + 16 * (threadIdx.x & 31));
         i0 = q.x;
         a0 = __int_as_float(q.y);
         i1 = q.z;
@@ -171,36 +177,49 @@ struct FromRecords {
 // Dot products of one pass: lane (group, sub) sums its entries with the values
 // gather(index); the sum s + e (e: the compensation) is valid in each group's
 // first lane.  The phases are bound by the latency and the number of these
-// instructions, not by shared-memory bandwidth: BATCHES batches of entries are
-// read before the first is summed, and rows past the pass's width add 0 * 0 (a
-// branch over them costs more).
-template <bool COMP, int BATCHES, class Gather>
-__device__ __forceinline__ void pass_sums(const char* rows, int width, int lg, const Gather& gather, float& s,
+// instructions, not by shared-memory bandwidth: four pairs of entries are read
+// before the first is summed, and the rest of a pass by code of its length.
+template <bool COMP, int PAIRS, class Gather>
+__device__ __forceinline__ void sum_pairs(const char* rows, const Gather& gather, float (&acc)[kBatch], float& s,
                                           float& e) {
     using Entries = typename Gather::Entries;
-    constexpr int kU = BATCHES * kBatch;
+    int i[2 * PAIRS];
+    float a[2 * PAIRS], g[2 * PAIRS];
+#pragma unroll
+    for (int u = 0; u < PAIRS; ++u)
+        Entries::load(rows + u * Entries::kPair, i[2 * u], a[2 * u], i[2 * u + 1], a[2 * u + 1]);
+#pragma unroll
+    for (int u = 0; u < 2 * PAIRS; ++u) g[u] = gather(i[u]);
+#pragma unroll
+    for (int u = 0; u < 2 * PAIRS; ++u) {
+        if (COMP) {
+            float pr, pe, ss, se;
+            two_prod(a[u], g[u], pr, pe);
+            two_sum(s, pr, ss, se);
+            s = ss;
+            e = __fadd_rn(e, __fadd_rn(pe, se));
+        } else {
+            acc[u % kBatch] = fmaf(a[u], g[u], acc[u % kBatch]);
+        }
+    }
+}
+
+template <bool COMP, class Gather>
+__device__ __forceinline__ void pass_sums(const char* rows, int width, int lg, const Gather& gather, float& s,
+                                          float& e) {
     float acc[kBatch] = {0.f, 0.f, 0.f, 0.f};
     s = e = 0.f;
-    for (int k = 0; k < width; k += kU, rows += kU / 2 * Entries::kPair) {
-        int i[kU];
-        float a[kU], g[kU];
-#pragma unroll
-        for (int u = 0; u < kU; u += 2)
-            Entries::load(rows + u / 2 * Entries::kPair, k + u < width, gather.none, i[u], a[u], i[u + 1], a[u + 1]);
-#pragma unroll
-        for (int u = 0; u < kU; ++u) g[u] = gather(i[u]);
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            if (COMP) {
-                float pr, pe, ss, se;
-                two_prod(a[u], g[u], pr, pe);
-                two_sum(s, pr, ss, se);
-                s = ss;
-                e = __fadd_rn(e, __fadd_rn(pe, se));
-            } else {
-                acc[u % kBatch] = fmaf(a[u], g[u], acc[u % kBatch]);
-            }
-        }
+    int pairs = (width + 1) >> 1;
+    for (; pairs > 4; pairs -= 4, rows += 4 * Gather::Entries::kPair) sum_pairs<COMP, 4>(rows, gather, acc, s, e);
+    if (pairs > 2) {
+        if (pairs == 4)
+            sum_pairs<COMP, 4>(rows, gather, acc, s, e);
+        else
+            sum_pairs<COMP, 3>(rows, gather, acc, s, e);
+    } else if (pairs == 2) {
+        sum_pairs<COMP, 2>(rows, gather, acc, s, e);
+    } else if (pairs == 1) {
+        sum_pairs<COMP, 1>(rows, gather, acc, s, e);
     }
     if (!COMP) s = (acc[0] + acc[1]) + (acc[2] + acc[3]);
     // the group's tree (the group's first lane adds as group_sum / group_sum2 do)
@@ -219,10 +238,10 @@ __device__ __forceinline__ void pass_sums(const char* rows, int width, int lg, c
 }
 
 // The same rounded to float, in every lane of the group.
-template <bool COMP, int BATCHES, class Gather>
+template <bool COMP, class Gather>
 __device__ __forceinline__ float pass_dot(const char* rows, int width, int lg, const Gather& gather) {
     float s, e;
-    pass_sums<COMP, BATCHES>(rows, width, lg, gather, s, e);
+    pass_sums<COMP>(rows, width, lg, gather, s, e);
     if (!COMP) return s;
     return __shfl_sync(FULL_MASK, __fadd_rn(s, e), (threadIdx.x & 31) >> lg << lg);
 }
@@ -275,7 +294,7 @@ __device__ __forceinline__ void dual_phase(const int4* pass, int passes, const c
     const int nw = (blockDim.x >> 5) - 1;
     for (int p = threadIdx.x >> 5; p < passes; p += nw) {
         const Pass t(pass[p], rows);
-        const float kxp = pass_dot<COMP, 2>(t.rows, t.width, t.lg, xs);
+        const float kxp = pass_dot<COMP>(t.rows, t.width, t.lg, xs);
         if (t.on) {
             const float* r = R + t.local;
             const float yo = r[0], kx = r[(1 + cur) * nl], rl = r[3 * nl], ru = r[4 * nl];
@@ -298,7 +317,7 @@ __device__ __forceinline__ void kty_phase(const int4* pass, int passes, const ch
     const int nw = (blockDim.x >> 5) - 1;
     for (int p = threadIdx.x >> 5; p < passes; p += nw) {
         const Pass t(pass[p], rows);
-        const float k = pass_dot<COMP, 2>(t.rows, t.width, t.lg, ys);
+        const float k = pass_dot<COMP>(t.rows, t.width, t.lg, ys);
         if (t.on && t.sub == 0) {
             float* c = C + t.local;
             const float dx = xs[t.seg] - c[0];
@@ -436,9 +455,9 @@ __device__ __forceinline__ void eval_sums(bool comp, const int4* pass, int passe
         const Pass t(pass[p], rows);
         float s, e;
         if (comp)
-            pass_sums<true, 2>(t.rows, t.width, t.lg, vec, s, e);
+            pass_sums<true>(t.rows, t.width, t.lg, vec, s, e);
         else
-            pass_sums<false, 2>(t.rows, t.width, t.lg, vec, s, e);
+            pass_sums<false>(t.rows, t.width, t.lg, vec, s, e);
         if (t.on && t.sub == 0) {
             s_out[t.local] = s;
             e_out[t.local] = e;
@@ -456,9 +475,9 @@ __device__ __forceinline__ void eval_apply(bool comp, const int4* pass, int pass
         const Pass t(pass[p], rows);
         SegDot<2> d;
         if (comp)
-            pass_sums<true, 2>(t.rows, t.width, t.lg, vec, d.s[1], d.e[1]);
+            pass_sums<true>(t.rows, t.width, t.lg, vec, d.s[1], d.e[1]);
         else
-            pass_sums<false, 2>(t.rows, t.width, t.lg, vec, d.s[1], d.e[1]);
+            pass_sums<false>(t.rows, t.width, t.lg, vec, d.s[1], d.e[1]);
         if (t.on && t.sub == 0) {
             d.s[0] = s_in[t.local];
             d.e[0] = e_in[t.local];
@@ -507,9 +526,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
     float* C = reinterpret_cast<float*>(sm + A.sm.col);  // x | K^T y, K^T y' | c l u | average hi lo
     float* R = reinterpret_cast<float*>(sm + A.sm.row);  // y | K x, K x' | rl ru | average hi lo
     Sums* wsum = reinterpret_cast<Sums*>(sm + A.sm.red);  // of every warp of this block
-    Sums* bsum = wsum + 32;                               // of every block of the cluster
+    Sums* bsum = wsum + kResWarps;                        // of every block of the cluster
+    unsigned short* cseg = reinterpret_cast<unsigned short*>(sm + A.sm.seg);  // segment of each local column
     const int ncl = A.sm.locals[1], nrl = A.sm.locals[0];
-    const int rp = blk.side[0].passes, cp = blk.side[1].passes;
+    const int rp = blk.side[0].passes, cp = blk.side[1].passes, nc = blk.side[1].locals;
     const FromShared gx{xs, io.y}, gy{ys, io.w};
     if (threadIdx.x == 0) xs[io.y] = ys[io.w] = 0.f;
     load_block<Compact>(A, blk, sm);
@@ -526,6 +546,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
             if (t.on && t.sub == 0) {
                 const int j = io.x + t.seg;
                 float* c = C + t.local;
+                cseg[t.local] = (unsigned short)t.seg;
                 xs[t.seg] = c[0] = pick(V.x0, V.x1, cur)[j];
                 c[(1 + cur) * ncl] = pick(V.kty0, V.kty1, cur)[j];
                 c[3 * ncl] = V.c[j];
@@ -562,34 +583,24 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
         // x' = clip(x - tau (c + K^T y), l, u); after an accepted step x is the
         // candidate of that step, still in the copy
         if (!ctrl) {
-            for (int p = warp; p < cp; p += nw) {
-                const Pass t(cpass[p], crows);
-                float x = 0.f, xp = 0.f;
-                if (t.on) {
-                    const float* c = C + t.local;
-                    x = avg ? xs[t.seg] : c[0];
-                    const float v = fmaf(-tau, c[3 * ncl] + c[(1 + cur) * ncl], x);
-                    xp = fminf(fmaxf(v, c[4 * ncl]), c[5 * ncl]);
-                }
-                __syncwarp();  // every lane of the group has read x
-                if (t.on) {
-                    push(xs + t.seg, xp, t.sub, 1 << t.lg, cluster);
-                    if (t.sub == 0) C[t.local] = x;
-                }
+            for (int l = threadIdx.x; l < nc; l += 32 * nw) {
+                float* c = C + l;
+                const int seg = cseg[l];
+                const float x = avg ? xs[seg] : c[0];
+                const float v = fmaf(-tau, c[3 * ncl] + c[(1 + cur) * ncl], x);
+                push(xs + seg, fminf(fmaxf(v, c[4 * ncl]), c[5 * ncl]), 0, 1, cluster);
+                c[0] = x;
             }
         }
         cluster_arrive();
         if (ctrl) {
             if (lane == 0) schedule_pows(S, V);
         } else if (avg) {  // the pending average updates, while the other blocks arrive
-            for (int p = warp; p < cp; p += nw) {
-                const Pass t(cpass[p], crows);
-                if (t.on && t.sub == 0) {
-                    float* c = C + t.local;
-                    const float2 a = ff_axpy(make_float2(c[6 * ncl], c[7 * ncl]), w, c[0]);
-                    c[6 * ncl] = a.x;
-                    c[7 * ncl] = a.y;
-                }
+            for (int l = threadIdx.x; l < nc; l += 32 * nw) {
+                float* c = C + l;
+                const float2 a = ff_axpy(make_float2(c[6 * ncl], c[7 * ncl]), w, c[0]);
+                c[6 * ncl] = a.x;
+                c[7 * ncl] = a.y;
             }
             for (int p = warp; p < rp; p += nw) {
                 const Pass t(rpass[p], rrows);
@@ -723,8 +734,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
     }
     cluster_arrive();
     cluster_wait();
-    float2* ewarp = reinterpret_cast<float2*>(sm + A.sm.eval);  // [kEvalQ][32] of the block's warps
-    float2* eblock = ewarp + kEvalQ * 32;                       // [kEvalQ][16] of the cluster's blocks
+    float2* ewarp = reinterpret_cast<float2*>(sm + A.sm.eval);  // [kEvalQ][kResWarps] of the block's warps
+    float2* eblock = ewarp + kEvalQ * kResWarps;                // [kEvalQ][16] of the cluster's blocks
     double* etot = reinterpret_cast<double*>(eblock + kEvalQ * 16);
     if (!ctrl) {
         EvalRowsEpi er{V};
@@ -734,7 +745,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
         er.values(q);
         warp_reduce_acc<8>(q, 0x0Cu);
         if (lane == 0)
-            for (int i = 0; i < 8; ++i) ewarp[i * 32 + warp] = make_float2(q[i].s, q[i].c);
+            for (int i = 0; i < 8; ++i) ewarp[i * kResWarps + warp] = make_float2(q[i].s, q[i].c);
     }
     if (!ctrl) {
         EvalColsEpi ec{V, nullptr};
@@ -744,11 +755,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
         ec.values(q);
         warp_reduce_acc<10>(q, 0x0Cu);
         if (lane == 0)
-            for (int i = 0; i < 10; ++i) ewarp[(8 + i) * 32 + warp] = make_float2(q[i].s, q[i].c);
+            for (int i = 0; i < 10; ++i) ewarp[(8 + i) * kResWarps + warp] = make_float2(q[i].s, q[i].c);
     }
     __syncthreads();
     for (int i = warp; i < kEvalQ; i += nw + 1) {
-        const Acc v = eval_total(ewarp + i * 32, nw, i);
+        const Acc v = eval_total(ewarp + i * kResWarps, nw, i);
         if (lane < cluster) st_rank2(map_rank(eblock + i * 16 + rank, lane), v.s, v.c);
     }
     cluster_arrive();
@@ -807,8 +818,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
                 }
             }
         }
-        __syncwarp();  // the groups read x and y in the next step
     }
+    __syncthreads();  // other threads read x and y in the next step
     }
     if (rank == 0 && ctrl && lane == 0) st[inst] = S;
 }
@@ -827,8 +838,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_steps(ResArgs A, in
 // an acquire each) and the controller's FP64 chain; the large one as much the
 // instructions of its 50 passes a side and block (about 300 each, compensated
 // sums near the tolerance).  Measured per step, whole solves: 14.6 -> 9.0 us and
-// 26 -> 14.4 us against k_solo_steps, which reads the matrix from L2 and remains
-// for LPs that do not fit.
+// 26 -> 14.4 us against k_solo_steps, which reads the matrix from L2 (LPs that do
+// not fit step over packs, see kPackMinNnz); with the rest of a pass by code of
+// its length, steps alone, 8.75 -> 8.6 and 13.8 -> 12.9 us.
+//
 // Grid-wide barrier.  Every block adds one to its counter of kArrive (fewer
 // additions queue up at one address) with release semantics; one warp of each
 // block polls all of them with relaxed loads, then acquires once (an acquire
@@ -887,7 +900,7 @@ __device__ __forceinline__ void grid_cols(const int4* pass, int passes, const ch
         const GridPass t(pass[p], rows);
         float4 rec = make_float4(0.f, 0.f, 0.f, 0.f);
         if (t.on && t.sub == 0) rec = ld_record(records + t.seg);
-        const float k = pass_dot<COMP, 2>(t.rows, t.width, t.lg, FromGlobal{y});
+        const float k = pass_dot<COMP>(t.rows, t.width, t.lg, FromGlobal{y});
         if (t.on && t.sub == 0) {
             float* c = C + t.local;
             const float x = rec.x, kty = c[cur * nl], cc = c[2 * nl];
@@ -916,7 +929,7 @@ __device__ __forceinline__ void grid_rows(const int4* pass, int passes, const ch
         const GridPass t(pass[p], rows);
         float yo = 0.f;
         if (t.on && t.sub == 0) yo = FromGlobal{y}(t.seg);
-        const float kxp = pass_dot<COMP, 2>(t.rows, t.width, t.lg, FromRecords{records, tau});
+        const float kxp = pass_dot<COMP>(t.rows, t.width, t.lg, FromRecords{records, tau});
         if (t.on && t.sub == 0) {
             float* r = R + t.local;
             const float kx = r[cur * nl], rl = r[2 * nl], ru = r[3 * nl];
@@ -943,8 +956,8 @@ __device__ __forceinline__ void grid_eval(const int4* pass, int passes, const ch
     for (int p = threadIdx.x >> 5; p < passes; p += nw) {
         const GridPass t(pass[p], rows);
         SegDot<2> d;
-        pass_sums<COMP, 1>(t.rows, t.width, t.lg, FromGlobal{v0}, d.s[0], d.e[0]);
-        pass_sums<COMP, 1>(t.rows, t.width, t.lg, FromGlobal{v1}, d.s[1], d.e[1]);
+        pass_sums<COMP>(t.rows, t.width, t.lg, FromGlobal{v0}, d.s[0], d.e[0]);
+        pass_sums<COMP>(t.rows, t.width, t.lg, FromGlobal{v1}, d.s[1], d.e[1]);
         if (t.on && t.sub == 0) epi.apply(t.seg, d, epi.pre(t.seg));
     }
 }
@@ -1285,7 +1298,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, in
         for (int it = 0; it < iterations; ++it) {
             for (int p = warp; p < cp; p += nw) {
                 const Pass t(cpass[p], crows);
-                const float aty = pass_dot<false, 2>(t.rows, t.width, t.lg, gy);
+                const float aty = pass_dot<false>(t.rows, t.width, t.lg, gy);
                 float x_new = 0.f;
                 if (t.on) {
                     const float* c = C + t.local;
@@ -1302,7 +1315,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, in
             cluster_wait();
             for (int p = warp; p < rp; p += nw) {
                 const Pass t(rpass[p], rrows);
-                const float axbar = pass_dot<false, 2>(t.rows, t.width, t.lg, gx);
+                const float axbar = pass_dot<false>(t.rows, t.width, t.lg, gx);
                 float y = 0.f;
                 if (t.on) {
                     const float* r = R + t.local;
@@ -1329,7 +1342,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, in
         float most[2] = {0.f, 0.f};
         for (int p = warp; p < cp; p += nw) {
             const Pass t(cpass[p], crows);
-            const float aty = pass_dot<false, 2>(t.rows, t.width, t.lg, gy);
+            const float aty = pass_dot<false>(t.rows, t.width, t.lg, gy);
             if (t.on) {
                 const float* c = C + t.local;
                 const float x = c[0], tau = c[4 * ncl];
@@ -1342,7 +1355,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident_plain(ResArgs A, in
         cluster_wait();
         for (int p = warp; p < rp; p += nw) {
             const Pass t(rpass[p], rrows);
-            const float ax = pass_dot<false, 2>(t.rows, t.width, t.lg, gx);
+            const float ax = pass_dot<false>(t.rows, t.width, t.lg, gx);
             if (t.on) {
                 const float rl = R[nrl + t.local], ru = R[2 * nrl + t.local];
                 float viol = 0.0f;
@@ -1506,6 +1519,7 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
         }
     };
     ResSmem sm{};
+    int sides[2] = {0, 0};  // most passes of a block, by side
     auto measure = [&](int C) -> int {  // the shared memory layout for clusters of C; most passes of a block
         long long mrows[2] = {0, 0};
         int mpass[2] = {0, 0}, mloc[2] = {0, 0}, mn = 0, mm = 0;
@@ -1542,9 +1556,13 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
         sm.locals[1] = mloc[1];
         sm.col = put(4ll * col_words * mloc[1]);
         sm.row = put(4ll * row_words * mloc[0]);
-        sm.red = put((long long)sizeof(Sums) * (32 + 16));
-        sm.eval = put(kEvalQ * (8ll * 32 + 8ll * 16 + 8));
+        const int warps = grid ? 32 : kResWarps;
+        sm.seg = put(kind == kCluster ? 2ll * mloc[1] : 0);
+        sm.red = put((long long)sizeof(Sums) * (warps + 16));
+        sm.eval = put(plain ? 0 : kEvalQ * (8ll * warps + 8ll * 16 + 8));
         sm.total = (int)std::min<long long>(at, INT32_MAX);
+        sides[0] = mpass[0];
+        sides[1] = mpass[1];
         return std::max(mpass[0], mpass[1]);
     };
     // The smallest cluster that holds an instance; a larger one while SMs are
@@ -1556,9 +1574,10 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
     while (!grid && C < 16 && sm.total > budget) most = measure(C *= 2);
     if (sm.total > budget) return SIH_PDHG_OK;
     while (!grid && C < 16 && (long long)B * 2 * C <= sm_count && most > 8) most = measure(C *= 2);
-    // 20 warps with passes at most (31: 3 % slower on the batch of 64, whose blocks have 39 passes)
-    // (grid form: a thread per block sums)
-    const int nw = grid ? kGridThreads / 32 - 1 : std::max(1, std::min(kResThreads / 32 - 1, most));
+    // as few warps as do both sides in the same rounds (grid form: a thread per block sums)
+    int nw = grid ? kGridThreads / 32 - 1 : std::max(1, std::min(kResThreads / 32 - 1, most));
+    auto rounds = [&](int w) { return (sides[0] + w - 1) / w + (sides[1] + w - 1) / w; };
+    while (!grid && nw > 1 && rounds(nw - 1) == rounds(nw)) --nw;
     threads_ = 32 * (nw + 1);
     if (grid && sm_count > threads_) return SIH_PDHG_OK;
     npass_ = (int)all.size();

@@ -24,7 +24,7 @@ struct ResBlock {
 // Where a block keeps what, in bytes of dynamic shared memory; the same in
 // every block of a launch.
 struct ResSmem {
-    int pass[2], rows[2], xs, ys, col, row, red, eval, locals[2], total;
+    int pass[2], rows[2], xs, ys, col, row, seg, red, eval, locals[2], total;
 };
 
 struct ResArgs {
