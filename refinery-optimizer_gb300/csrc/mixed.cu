@@ -396,6 +396,7 @@ __device__ __forceinline__ void solo_grid_total(const float2* __restrict__ part,
 // The epilogues over packs pick their vectors where they use them: a pack's
 // loads in flight leave no registers for a dozen pointers.
 struct DualPackEpi {
+    static constexpr bool kPreFirst = false;
     Vecs V;
     int cur;
     float sigma;
@@ -423,6 +424,7 @@ struct DualPackEpi {
 };
 
 struct KtyPackEpi {
+    static constexpr bool kPreFirst = false;
     Vecs V;
     int cur;
     Acc inter, dx2;

@@ -105,10 +105,12 @@ __global__ void __launch_bounds__(256, 8) plain_dual_kernel(SegMatrix A, SpmvPla
 // Fast path of the iteration (exact_arithmetic = 0): the same epilogues over
 // packs (warp.cuh).
 struct PackPrimal : PrimalEpi {
+    static constexpr bool kPreFirst = true;
     __device__ __forceinline__ const float* gather(int) const { return v.y; }
     __device__ __forceinline__ void apply(int j, const SegDot<1>& d, const Pre& p) { PrimalEpi::apply(j, d.s[0], p); }
 };
 struct PackDual : DualEpi {
+    static constexpr bool kPreFirst = true;
     __device__ __forceinline__ const float* gather(int) const { return v.xbar; }
     __device__ __forceinline__ void apply(int i, const SegDot<1>& d, const Pre& p) { DualEpi::apply(i, d.s[0], p); }
 };

@@ -467,12 +467,18 @@ __device__ __forceinline__ void spmv_engine(const Side& side, State* st, Epi& ep
 // that holds a line for every miss (shared memory takes its space).
 // The epilogue's operands load behind the gathers, when the pairs' registers
 // are free (before them: 64 registers spill, 2 % slower); packs of up to 128
-// short segments, four per lane, spill as well (6 to 15 % slower).
+// short segments, four per lane, spill as well (6 to 15 % slower).  The entries
+// of one segment of 32 lanes are on their chains' lanes as they load and need no
+// window (500k x 1M, 12M entries below: 137.5 -> 129.0, the mixed step 150.2 ->
+// 147.9); there Epi::kPreFirst says whether the operands load first (plain
+// algorithm 142.7 -> 129.0) or, where that spills, last (the mixed step 152.9 ->
+// 147.9).
 // Microseconds per iteration of the plain algorithm (two kernels) with tasks from
 // a counter, with one run of neighbouring packs per warp and with packs in turn:
 // 20k x 50k, 0.5M entries 15.7 / 10.7 / 9.6; 60k x 130k, 1M entries 24.1 / 15.8 /
 // 14.9; 250k x 500k, 3M, lengths by a power law 60.8 / 49.2 / 41.0; 500k x 1M, 12M,
-// likewise 139.9 / 145.8 / 137.5 (gathers through L1 and L2: 175 G a second).
+// likewise 139.9 / 145.8 / 129.0.  The gathers' way through L1 (a line a cycle and
+// SM) is 70 % busy there, 80 % while the SM has work.
 template <bool COMP, class Epi>
 __device__ __forceinline__ void spmv_packs(const PackSide& P, Epi& epi, float2* __restrict__ window) {
     constexpr int kU = kPackEntries / 32;
@@ -487,8 +493,25 @@ __device__ __forceinline__ void spmv_packs(const PackSide& P, Epi& epi, float2* 
         const int4 next = P.packs[min(p + nw, P.count - 1)];
         const int nseg = rec.z & 0xff, lg = rec.z >> 8, n = rec.w;
         const int L = 1 << lg, gpw = 32 >> lg, sub = lane & (L - 1);
-        // entries [w0, w0 + cnt) of the pack to the window
-        auto fill = [&](int w0, int cnt) {
+        float acc[kBatch], err;  // COMP: sum acc[0], its error err
+        auto clear = [&]() {
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) acc[u] = 0.f;
+            err = 0.f;
+        };
+        auto add = [&](int u, float a, float g) {
+            if (COMP) {
+                float pr, pe, ss, se;
+                two_prod(a, g, pr, pe);
+                two_sum(acc[0], pr, ss, se);
+                acc[0] = ss;
+                err = __fadd_rn(err, __fadd_rn(pe, se));
+            } else {
+                acc[u % kBatch] = fmaf(a, g, acc[u % kBatch]);
+            }
+        };
+        // entries [w0, w0 + cnt) of the pack to the window, or on their chains
+        auto fill = [&](int w0, int cnt, bool direct) {
             const int2* __restrict__ pairs = P.pairs + rec.y + w0;
             int2 q[kU];
             float g[kU];
@@ -498,14 +521,12 @@ __device__ __forceinline__ void spmv_packs(const PackSide& P, Epi& epi, float2* 
 #pragma unroll
             for (int u = 0; u < kU; ++u) g[u] = q[u].x >= 0 ? ld_vec(vec + q[u].x) : 0.f;
 #pragma unroll
-            for (int u = 0; u < kU; ++u)
-                if (q[u].x >= 0) window[lane + 32 * u] = make_float2(__int_as_float(q[u].y), g[u]);
-        };
-        float acc[kBatch], err;  // COMP: sum acc[0], its error err
-        auto clear = [&]() {
-#pragma unroll
-            for (int u = 0; u < kBatch; ++u) acc[u] = 0.f;
-            err = 0.f;
+            for (int u = 0; u < kU; ++u) {
+                if (direct)
+                    add(u, __int_as_float(q[u].y), g[u]);
+                else if (q[u].x >= 0)
+                    window[lane + 32 * u] = make_float2(__int_as_float(q[u].y), g[u]);
+            }
         };
         // entries lo + sub, + L, ... of the window on chain 0, 1, 2, 3, 0, ...
         auto chains = [&](int lo, int hi) {
@@ -513,15 +534,7 @@ __device__ __forceinline__ void spmv_packs(const PackSide& P, Epi& epi, float2* 
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u) {
                     const float2 v = k + u * L < hi ? window[k + u * L] : make_float2(0.f, 0.f);
-                    if (COMP) {
-                        float pr, pe, ss, se;
-                        two_prod(v.x, v.y, pr, pe);
-                        two_sum(acc[0], pr, ss, se);
-                        acc[0] = ss;
-                        err = __fadd_rn(err, __fadd_rn(pe, se));
-                    } else {
-                        acc[u] = fmaf(v.x, v.y, acc[u]);
-                    }
+                    add(u, v.x, v.y);
                 }
             }
         };
@@ -535,14 +548,22 @@ __device__ __forceinline__ void spmv_packs(const PackSide& P, Epi& epi, float2* 
                 s = group_sum(s, L);
             return s;
         };
-        if (n <= kPackEntries) {
+        if (!COMP && L == 32 && nseg == 1) {  // the loads are on their chains' lanes already
+            typename Epi::Pre pre{};
+            if (Epi::kPreFirst && lane == 0) pre = epi.pre(rec.x);
+            clear();
+            for (int w0 = 0; w0 < n; w0 += kPackEntries) fill(w0, min(kPackEntries, n - w0), true);
+            SegDot<1> d;
+            d.s[0] = total(d.e[0]);
+            if (lane == 0) epi.apply(rec.x, d, Epi::kPreFirst ? pre : epi.pre(rec.x));
+        } else if (n <= kPackEntries) {
             int beg = 0, end = 0;  // this lane's segment in the pack
             typename Epi::Pre pre;
             if (lane < nseg) {
                 beg = P.ptr[rec.x + lane] - rec.y;
                 end = P.ptr[rec.x + lane + 1] - rec.y;
             }
-            fill(0, n);
+            fill(0, n, false);
             if (lane < nseg) pre = epi.pre(rec.x + lane);
             __syncwarp();
             SegDot<1> d{};
@@ -570,7 +591,7 @@ __device__ __forceinline__ void spmv_packs(const PackSide& P, Epi& epi, float2* 
             clear();
             for (int w0 = 0; w0 < n; w0 += kPackEntries) {
                 const int cnt = min(kPackEntries, n - w0);
-                fill(w0, cnt);
+                fill(w0, cnt, false);
                 __syncwarp();
                 if (lane < L) chains(0, cnt);
                 __syncwarp();
