@@ -311,9 +311,11 @@ __global__ void __launch_bounds__(kThreads, 4)
 // Deterministic; the sums are grouped differently from the task engine's, so
 // the iterates agree with the other forms to rounding, not bit for bit.
 constexpr int kSoloThreads = 640;  // 20 warps per SM at 96 registers (measured best of 640 / 768 / 1024)
-// Automatic step form: the single-LP form when the matrix (both sides) takes
-// at most this many bytes, half of the 129 MB L2 (measured per step: 80k
-// nonzeros 30.9 -> 20.8 us, 1.1M nonzeros 46.1 -> 38.8 us).
+// One LP whose matrix (both sides) takes at most this many bytes, half of the
+// 129 MB L2, counts as latency-bound: it tries the resident forms, then steps over
+// packs (see setup_resident); its light tasks are shorter (kSoloTaskSegs).  This
+// form runs where it is asked for and the resident forms don't hold the LP, or
+// where the LP is too small for packs.
 constexpr double kSoloMaxBytes = 64.0 * 1024.0 * 1024.0;
 // Segments per light task on such an LP (the others keep kTaskSegs): a task's
 // lane groups walk its segments one pointer round trip per pass, so on an
@@ -383,12 +385,14 @@ __device__ __forceinline__ void solo_grid_total(const float2* __restrict__ part,
 // ---------------------------------------------------------------- steps of one LP over packs
 // The two step SpMVs of one LP by kernels: packs of uniform segments dealt to
 // the warps in turn (spmv_packs), the same per-segment sums as the task
-// engine's.  Each block leaves one partial of the step's sums; the block that
-// arrives last adds them in block order and runs the instance's part (finish),
-// where the task engine has a slot and a ticket per task.  Gathers bound both
+// engine's.  Each block leaves one partial of each of the step's sums; the block
+// of K^T y' that arrives last adds them in block order and runs the controller,
+// where the task engine has a slot and a ticket per task (with a total in K x' as
+// well: 63.2 instead of 61.6 us per step of the 200k x 400k LP below, 39.8 instead
+// of 38.4 on 100k x 200k, 2.6M nonzeros by a power law).  Gathers bound both
 // kernels (a sector of L2 each).  Microseconds of K x' / K^T y', tasks -> packs:
-// 200k x 400k, 4.8M nonzeros 44.0 / 41.4 -> 27.1 / 26.5; 500k x 1M, 12M nonzeros,
-// lengths by a power law 69.9 (staged) / 77.5 -> 61.9 / 70.0.  There a prefix of
+// 200k x 400k, 4.8M nonzeros 44.0 / 41.4 -> 23.8 / 27.1; 500k x 1M, 12M nonzeros,
+// lengths by a power law 69.9 (staged) / 77.5 -> 60.5 / 70.2.  There a prefix of
 // the gathered vector in shared memory no longer pays: the windows and the prefix
 // leave L1 too few lines for the gathers that miss it (one block of 512 threads:
 // 68.9 to 71.5 / 101; of 1024: 85 and up / 112 and up).
@@ -419,8 +423,6 @@ struct DualPackEpi {
         const float dy = yv - p.y;
         dy2.add(dy * dy);
     }
-    __device__ void values(Acc (&q)[1]) const { q[0] = dy2; }
-    __device__ void finish(Inst& S, const double* tot) const { S.dy2 = tot[0]; }
 };
 
 struct KtyPackEpi {
@@ -441,54 +443,52 @@ struct KtyPackEpi {
         inter.add(dx * (k - p.kty));
         dx2.add(dx * dx);
     }
-    __device__ void values(Acc (&q)[2]) const {
-        q[0] = inter;
-        q[1] = dx2;
-    }
-    __device__ void finish(Inst& S, const double* tot) const { step_controller(S, tot[1], tot[0]); }
 };
 
-template <int Q, class Epi>
-__device__ __forceinline__ void step_packs(const PackSide& side, Inst* st, Epi& epi, float2* window,
-                                           const PackTotals& T) {
-    __shared__ Acc sh[32 * Q];
-    __shared__ unsigned last;
-    Inst& S = st[0];
-    if (S.done) return;  // it changes between steps only
+template <class Epi>
+__device__ __forceinline__ void step_packs(const PackSide& side, const Inst& S, Epi& epi, float2* window) {
     epi.begin(S);
     if (S.refine)
         spmv_packs<true>(side, epi, window);
     else
         spmv_packs<false>(side, epi, window);
-    Acc q[Q];
-    epi.values(q);
-    solo_block_partial<Q>(q, T.part + Q * blockIdx.x, sh);
-    if (threadIdx.x == 0) last = ticket_add(T.ticket) + 1u == gridDim.x;
-    __syncthreads();
-    if (!last) return;
-    double tot[Q];
-    solo_grid_total<Q>(T.part, gridDim.x, tot, sh);
-    if (threadIdx.x == 0) {
-        *T.ticket = 0u;
-        epi.finish(S, tot);
-    }
 }
 
 __global__ void __launch_bounds__(kThreads, kStepPackBlocks)
     k_step_dual_packs(PackSide rows, Vecs V, Inst* __restrict__ st, PackTotals T) {
     __shared__ float2 window[kThreads / 32][kPackEntries];
+    __shared__ Acc sh[kThreads / 32];
     chain_wait();
+    if (st[0].done) return;  // it changes between steps only
     step_schedule_pows(1, st, V);
     DualPackEpi epi{V};
-    step_packs<1>(rows, st, epi, window[threadIdx.x >> 5], T);
+    step_packs(rows, st[0], epi, window[threadIdx.x >> 5]);
+    Acc q[1] = {epi.dy2};
+    solo_block_partial<1>(q, T.part + 3 * blockIdx.x, sh);
 }
 
 __global__ void __launch_bounds__(kThreads, kStepPackBlocks)
     k_step_kty_packs(PackSide cols, Vecs V, Inst* __restrict__ st, PackTotals T) {
     __shared__ float2 window[kThreads / 32][kPackEntries];
+    __shared__ Acc sh[3 * (kThreads / 32)];
+    __shared__ unsigned last;
     chain_wait();
+    Inst& S = st[0];
+    if (S.done) return;
     KtyPackEpi epi{V};
-    step_packs<2>(cols, st, epi, window[threadIdx.x >> 5], T);
+    step_packs(cols, S, epi, window[threadIdx.x >> 5]);
+    Acc q[2] = {epi.inter, epi.dx2};
+    solo_block_partial<2>(q, T.part + 3 * blockIdx.x + 1, sh);
+    if (threadIdx.x == 0) last = ticket_add(T.ticket) + 1u == gridDim.x;
+    __syncthreads();
+    if (!last) return;
+    double tot[3];
+    solo_grid_total<3>(T.part, gridDim.x, tot, sh);
+    if (threadIdx.x == 0) {
+        *T.ticket = 0u;
+        S.dy2 = tot[0];
+        step_controller(S, tot[2], tot[1]);
+    }
 }
 
 // This warp's static share of a side's tasks with epilogue `epi`; the lanes'
@@ -1270,13 +1270,13 @@ int MixedSolver::build_packs() {
     const std::vector<int4> pc = make_packs(h_csc_ptr_, segment_lanes(layout_.col_schedule, N_));
     const std::vector<int4> pr = make_packs(h_csr_ptr_, segment_lanes(layout_.row_schedule, M_));
     const size_t bc = sizeof(int4) * pc.size(), br = sizeof(int4) * pr.size();
-    const size_t bt = sizeof(float2) * 2 * (size_t)sm_count_ * kStepPackBlocks;
+    const size_t bt = sizeof(float2) * 3 * (size_t)sm_count_ * kStepPackBlocks;
     SIHG_TRY(packs_.alloc(bc + br + bt + sizeof(unsigned)));
     char* d = packs_.as<char>();
     SIHG_CUDA(cudaMemcpyAsync(d, pc.data(), bc, cudaMemcpyHostToDevice, stream_));
     SIHG_CUDA(cudaMemcpyAsync(d + bc, pr.data(), br, cudaMemcpyHostToDevice, stream_));
     pack_totals_ = PackTotals{(float2*)(d + bc + br), (unsigned*)(d + bc + br + bt)};
-    SIHG_CUDA(cudaMemsetAsync(pack_totals_.ticket, 0, sizeof(unsigned), stream_));
+    SIHG_CUDA(cudaMemsetAsync(pack_totals_.part, 0, bt + sizeof(unsigned), stream_));
     pack_cols_ = PackSide{(const int4*)d, (int)pc.size(), csc_ptr_.as<int>(), csc_pairs_.as<int2>()};
     pack_rows_ = PackSide{(const int4*)(d + bc), (int)pr.size(), csr_ptr_.as<int>(), csr_pairs_.as<int2>()};
     return SIH_PDHG_OK;
@@ -1563,7 +1563,7 @@ int MixedSolver::setup_resident() {
                                   ResidentPlan::kGrid));
     if (!resident_->ready()) {
         // one LP beyond the resident forms: steps over packs (see kPackMinNnz)
-        return B_ == 1 && opts_.persistent < 0 && opts_.use_graph && use_packs() ? set_form(0) : SIH_PDHG_OK;
+        return B_ == 1 && opts_.persistent < 0 && opts_.use_graph && !tuned_ && use_packs() ? set_form(0) : SIH_PDHG_OK;
     }
     SIHG_TRY(resident_->fill(SegMatrix{M_, csr_ptr_.as<int>(), csr_pairs_.as<int2>()},
                              SegMatrix{N_, csc_ptr_.as<int>(), csc_pairs_.as<int2>()}, stream_));
@@ -1602,8 +1602,8 @@ int MixedSolver::setup_persistent() {
     }
     int form = opts_.persistent;
     if (form < 0) {
-        // automatic: the single-LP form for one LP whose matrix (both sides,
-        // 16 bytes per nonzero) fits in half of L2: its steps are latency-bound
+        // automatic: form 2 for one LP whose matrix (both sides, 16 bytes per
+        // nonzero) fits in half of L2; setup_resident then looks further
         form = latency_bound() ? 2 : 0;
     }
     if (form == 2 && B_ != 1) form = 1;  // the single-LP form needs one LP
@@ -1774,7 +1774,8 @@ int MixedSolver::launch_step_spmvs(cudaStream_t s, int which) {
 // fit in options.staged_kib of shared memory (automatic: the block opt-in
 // limit, at most 128 KiB) are staged on a side when, after the renumbering by
 // length, their segments on the other side hold at least kStagedShare of the
-// nonzeros; the staged kernels run one block per SM.
+// nonzeros; the staged kernels run one block per SM.  Not for an LP that steps
+// over packs (see the figures there).
 int MixedSolver::choose_staging() {
     constexpr double kStagedShare = 0.5;
     stage_x_ = stage_y_ = 0;

@@ -181,15 +181,15 @@ class ResidentPlan;  // resident.h
 // which one LP takes them instead of the task engine and, where it does not fit
 // a resident form, instead of k_solo_steps.  Microseconds per step, tasks /
 // k_solo_steps / packs: 60k x 120k, 1.4M nonzeros, lengths by a power law 54.7 /
-// 36.2 / 32.9; 100k x 200k, 1.6M, equal lengths 56.5 / 36.3 / 32.6; refinery
-// planning over 336 periods 58.6 / 41.7 / 32.1; 200k x 400k, 4.8M 93.8 / - / 64.1;
-// 500k x 1M, 12M, power law 163.8 (longest columns staged) / - / 149.1.  Below
+// 36.2 / 31.3; 100k x 200k, 1.6M, equal lengths 56.5 / 36.3 / 32.6; refinery
+// planning over 336 periods 58.6 / 41.7 / 32.1; 200k x 400k, 4.8M 93.8 / - / 61.6;
+// 500k x 1M, 12M, power law 163.8 (longest columns staged) / - / 147.  Below
 // the line (20k x 50k, 0.4M: 30.7 / - / 22.5) the resident forms hold the LP, and
 // the forms that a caller asks for by number keep their common order of sums.
 constexpr int kStepPackBlocks = 4;
 constexpr double kPackMinNnz = 0.25e6;
 struct PackTotals {
-    float2* part;      // a partial per block and sum
+    float2* part;      // [grid][3]: |dy|^2, interaction, |dx|^2 of a block
     unsigned* ticket;  // 0 between launches
 };
 
