@@ -74,8 +74,8 @@ PLAIN_CAP = {
 # dram__bytes_write.sum,gpu__time_duration.sum --clock-control none -k
 # regex:k_step_ -c 6 python bench.py --profile-solve 64`; summaries in profiles/).
 NCU_TRAFFIC_PER_LAUNCH = {
-    ("zipf-500kx1m", "k_step_kty"): 117.22e6,
-    ("zipf-500kx1m", "k_step_dual"): 112.58e6,
+    ("zipf-500kx1m", "k_step_kty_packs"): 117.71e6,
+    ("zipf-500kx1m", "k_step_dual_packs"): 113.74e6,
 }
 
 
@@ -489,6 +489,8 @@ def run_gb300(args) -> None:
     secs, byts = handle.time_kernels(20)
     shape = handle.launch_shape()
     names = (["k_step_primal", "k_step_dual_packed", "k_step_kty_packed"] if shape["packed"]
+             else ["k_step_primal", "k_step_dual_packs", "k_step_kty_packs"]
+             if len(probs) == 1 and probs[0].num_nonzeros() >= 250_000  # one LP over packs of uniform segments
              else ["k_step_primal", "k_step_dual", "k_step_kty"])
     timed = [k for k in range(3) if secs[k] > 0]  # the packed step has no elementwise kernel
     dom = max(timed, key=lambda k: secs[k])

@@ -111,12 +111,13 @@ typedef struct sih_pdhg_options {
     int32_t eval_frequency;    /* mixed: iterations between restart/termination checks (64) */
     int32_t compensated;       /* mixed: 0 off, 1 on near tolerance (default), 2 always */
     int32_t dual_sign;         /* 0 = PDHG sign of the reference (row_duals = -simplex duals), 1 = simplex sign */
-    int32_t use_graph;         /* 1 = replay iteration blocks as CUDA graphs */
+    int32_t use_graph;         /* 1 = replay iteration blocks as CUDA graphs (plain: LPs that fit run resident in
+                                  one thread-block cluster instead); 0 = launch kernel by kernel */
     int32_t autotune;          /* mixed: 1 = at creation, time the step kernels' launch shapes (task size, lanes
                                   per segment of each side, staged gathers, and with persistent < 0 the step
                                   form) on this batch and keep the fastest, once per batch shape (instances,
                                   rows, columns, nonzeros; cached per process); 0 = off; -1 = on for batches
-                                  of two or more LPs (default) */
+                                  of two or more LPs that are not resident (see persistent; default) */
     int32_t verbose;           /* 0 */
     double time_limit_sec;     /* <= 0: none */
     double restart_sufficient; /* mixed: 0.2 */
@@ -136,8 +137,10 @@ typedef struct sih_pdhg_options {
                                   lines (default); 0 = keep the input order */
     int32_t staged_kib;        /* mixed, single LP: shared memory (KiB per block) that holds the first entries of
                                   a gathered vector, so that gathers of the longest segments of the other side
-                                  skip L2; the step SpMVs then run one 1024-thread block per SM.  0 = automatic
-                                  (on where the staged entries carry a large share of the nonzeros), -1 = off */
+                                  skip L2; the step SpMVs then run one 1024-thread block per SM.  > 0: that
+                                  many, with the task engine; -1: never; 0 = automatic: LPs of 250,000 nonzeros
+                                  and more step over packs instead, smaller ones stage where the staged
+                                  entries carry a large share of the nonzeros */
     int32_t persistent;        /* mixed: run the steps between two evaluations as ONE persistent cooperative
                                   kernel, phases separated by grid barriers with bounded waits (for LPs whose
                                   steps are latency-bound).  1 = the same tasks and reductions as the
@@ -145,8 +148,10 @@ typedef struct sih_pdhg_options {
                                   task shares with per-block partials reduced by every block (no ticket chain;
                                   deterministic, equal to the other forms up to rounding; a batch runs form 1).
                                   0 = one kernel per phase, replayed as CUDA graphs; -1 = automatic (default):
-                                  form 2 for one LP whose matrix fits in half of L2, the autotuner's choice
-                                  when it runs, else 0. */
+                                  the resident forms where they hold the LP (every instance of a batch in the
+                                  shared memory of a thread-block cluster, reported as 2 for one LP and 1 for
+                                  a batch; one LP over the shared memory of every SM, 2), else 0 for one LP
+                                  and the autotuner's choice for a batch.  2 takes the resident forms too. */
     int32_t packed;            /* mixed, kernels per phase: 1 = two kernels per step, the elementwise primal
                                   step folded into the SpMVs (the lanes that gather x' compute it from a packed
                                   16-byte record per column; the column owners store it); same iterates as the
@@ -185,7 +190,8 @@ typedef struct sih_pdhg_result {
     double final_primal_weight;
     uint64_t h2d_bytes;     /* host -> device bytes this solve moved (problem upload, start point) */
     uint64_t d2h_bytes;     /* device -> host bytes this solve moved (returned point, status) */
-    uint64_t kernel_launches; /* kernels this solve launched (graph nodes counted one by one) */
+    uint64_t kernel_launches; /* kernels this solve launched (graph nodes counted one by one; a resident form
+                                 runs several evaluation periods in one launch) */
 } sih_pdhg_result;
 
 /* Opaque solver handle: one LP or a batch of LPs resident on the device. */

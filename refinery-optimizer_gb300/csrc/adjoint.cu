@@ -15,9 +15,10 @@
 // slacks) with the largest primal-slack / dual-slack ratio are basic, so B is
 // square.  The systems are solved on the GPU by CGLS on the masked matrix, a
 // block per instance where it fits, else with the task engine's SpMVs (every
-// instance with its own scalars and stopping test; FP32 vectors, compensated reductions, FP64 scalars) inside FP64
-// iterative refinement: the residual is recomputed in FP64 on the host and a
-// correction solved again, up to four rounds.
+// instance with its own scalars and stopping test; FP32 vectors, compensated
+// reductions, FP64 scalars) inside FP64 iterative refinement: the residual is
+// recomputed in FP64 on the host and a correction solved again, up to four
+// rounds.
 //
 // The polish (sih_pdhg_polish_batch) returns the basis's vertex and duals:
 // from a PDHG point at 1e-6 it recovers the vertex x* whose neighbourhood the
