@@ -91,6 +91,11 @@ inline int64_t work_chunk(int64_t count, double work) {
     return items >= (double)count ? (count > 0 ? count : 1) : (int64_t)items + 1;
 }
 
+// f(0) and f(1), the second on a thread of its own when `apart`; what either
+// throws is thrown here.
+template <class F>
+void both_sides(bool apart, F&& f);
+
 // Splits [0, count) into `parts` contiguous ranges (range t to part t) and runs
 // f(begin, end, t) on them in parallel; below 2 x 65,536 items everything runs
 // as part 0 on the calling thread.
@@ -102,6 +107,7 @@ int hardware_threads();
 
 }  // namespace sihg
 
+#include <exception>
 #include <thread>
 
 namespace sihg {
@@ -122,6 +128,31 @@ void parallel_for_min(int64_t count, int64_t min_chunk, F&& f) {
         pool.emplace_back([&f, b, e] { f(b, e); });
     }
     for (auto& th : pool) th.join();
+}
+
+template <class F>
+void both_sides(bool apart, F&& f) {
+    if (!apart) {
+        f(0);
+        f(1);
+        return;
+    }
+    std::exception_ptr error;
+    std::thread other([&] {
+        try {
+            f(1);
+        } catch (...) {
+            error = std::current_exception();
+        }
+    });
+    try {
+        f(0);
+    } catch (...) {
+        other.join();
+        throw;
+    }
+    other.join();
+    if (error) std::rethrow_exception(error);
 }
 
 template <class F>

@@ -1315,8 +1315,13 @@ int MixedSolver::build_schedules(int task_nnz) {
 int MixedSolver::build_packs() {
     pack_cols_.count = pack_rows_.count = 0;
     if (!use_packs()) return SIH_PDHG_OK;
-    const std::vector<int4> pc = make_packs(h_csc_ptr_, segment_lanes(layout_.col_schedule, N_));
-    const std::vector<int4> pr = make_packs(h_csr_ptr_, segment_lanes(layout_.row_schedule, M_));
+    std::vector<int4> pc, pr;
+    both_sides(M_ + N_ >= 65536, [&](int h) {
+        if (h == 0)
+            pr = make_packs(h_csr_ptr_, segment_lanes(layout_.row_schedule, M_));
+        else
+            pc = make_packs(h_csc_ptr_, segment_lanes(layout_.col_schedule, N_));
+    });
     const size_t bc = sizeof(int4) * pc.size(), br = sizeof(int4) * pr.size();
     const size_t bt = sizeof(float2) * 3 * (size_t)sm_count_ * kStepPackBlocks;
     SIHG_TRY(packs_.alloc(bc + br + bt + sizeof(unsigned)));

@@ -213,11 +213,11 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
         const int task_nnz = opts.tile_nnz > 0
                                  ? opts.tile_nnz
                                  : (int)std::max(128LL, std::min(2048LL, (long long)nnz / std::max(1LL, 3 * warps)));
-        SideSchedule rs, cs;
-        make_schedule(hp.csr_ptr, std::vector<int>{0, m}, task_nnz, rs);
-        make_schedule(hp.csc_ptr, std::vector<int>{0, n}, task_nnz, cs);
-        row_lanes = segment_lanes(rs, m);
-        col_lanes = segment_lanes(cs, n);
+        both_sides(m + n >= 65536, [&](int h) {
+            SideSchedule sc;
+            make_schedule(h == 0 ? hp.csr_ptr : hp.csc_ptr, std::vector<int>{0, h == 0 ? m : n}, task_nnz, sc);
+            (h == 0 ? row_lanes : col_lanes) = segment_lanes(sc, h == 0 ? m : n);
+        });
         if (opts.use_graph)
             SIHG_TRY(resident_->build(hp.csr_ptr, hp.csc_ptr, std::vector<int>{0, m}, std::vector<int>{0, n}, row_lanes,
                                       col_lanes, sm_count_, s, ResidentPlan::kPlain));
@@ -237,8 +237,12 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
             }
             lanes.swap(l);
         };
-        renumber(hp.csc_ptr, col_lanes, col_order_, csc_ptr);
-        renumber(hp.csr_ptr, row_lanes, row_order_, csr_ptr);
+        both_sides(m + n >= 65536, [&](int h) {
+            if (h == 0)
+                renumber(hp.csr_ptr, row_lanes, row_order_, csr_ptr);
+            else
+                renumber(hp.csc_ptr, col_lanes, col_order_, csc_ptr);
+        });
     }
     const std::vector<int>& cptr = packs ? csc_ptr : hp.csc_ptr;
     const std::vector<int>& rptr = packs ? csr_ptr : hp.csr_ptr;
@@ -271,18 +275,18 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
                 inv[row_order_[k]] = (int)k;
             }
         });
-        DevMem raw, seg, map;
-        SIHG_TRY(raw.alloc(sizeof(Pair) * 2 * (size_t)nnz));
-        SIHG_TRY(seg.alloc(sizeof(int2) * src.size()));
-        SIHG_TRY(map.alloc(sizeof(int) * inv.size()));
-        SIHG_CUDA(cudaMemcpyAsync(raw.as<Pair>(), hp.csc.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
-        SIHG_CUDA(cudaMemcpyAsync(raw.as<Pair>() + nnz, hp.csr.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
-        SIHG_CUDA(cudaMemcpyAsync(seg.as<int2>(), src.data(), sizeof(int2) * src.size(), cudaMemcpyHostToDevice, s));
-        SIHG_CUDA(cudaMemcpyAsync(map.as<int>(), inv.data(), sizeof(int) * inv.size(), cudaMemcpyHostToDevice, s));
-        k_renumber_pairs<<<sm_count_ * 8, 256, 0, s>>>(n, csc_ptr_.as<int>(), seg.as<int2>(), raw.as<int2>(),
-                                                       map.as<int>(), csc_pairs_.as<int2>());
-        k_renumber_pairs<<<sm_count_ * 8, 256, 0, s>>>(m, csr_ptr_.as<int>(), seg.as<int2>() + n, raw.as<int2>() + nnz,
-                                                       map.as<int>(), csr_pairs_.as<int2>());
+        DevMem staging;  // the pairs of both sides, each segment's source, the new numbers
+        SIHG_TRY(staging.alloc(sizeof(Pair) * 2 * (size_t)nnz + sizeof(int2) * src.size() + sizeof(int) * inv.size()));
+        int2* raw = staging.as<int2>();
+        int2* seg = raw + 2 * (size_t)nnz;
+        int* map = reinterpret_cast<int*>(seg + src.size());
+        SIHG_CUDA(cudaMemcpyAsync(raw, hp.csc.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
+        SIHG_CUDA(cudaMemcpyAsync(raw + nnz, hp.csr.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
+        SIHG_CUDA(cudaMemcpyAsync(seg, src.data(), sizeof(int2) * src.size(), cudaMemcpyHostToDevice, s));
+        SIHG_CUDA(cudaMemcpyAsync(map, inv.data(), sizeof(int) * inv.size(), cudaMemcpyHostToDevice, s));
+        k_renumber_pairs<<<sm_count_ * 8, 256, 0, s>>>(n, csc_ptr_.as<int>(), seg, raw, map, csc_pairs_.as<int2>());
+        k_renumber_pairs<<<sm_count_ * 8, 256, 0, s>>>(m, csr_ptr_.as<int>(), seg + n, raw + nnz, map,
+                                                       csr_pairs_.as<int2>());
         SIHG_LAUNCH_CHECK();
         SIHG_CUDA(cudaStreamSynchronize(s));  // the staging buffers are released at scope end
     }
@@ -336,7 +340,13 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
     if (resident_->ready()) SIHG_TRY(resident_->fill(A_, At_, s));
     if (packs) {
         pack_grid_ = sm_count_ * kPackBlocks;
-        const std::vector<int4> pc = make_packs(cptr, col_lanes), pr = make_packs(rptr, row_lanes);
+        std::vector<int4> pc, pr;
+        both_sides(m + n >= 65536, [&](int h) {
+            if (h == 0)
+                pr = make_packs(rptr, row_lanes);
+            else
+                pc = make_packs(cptr, col_lanes);
+        });
         SIHG_TRY(packs_.alloc(sizeof(int4) * (pc.size() + pr.size())));
         int4* d = packs_.as<int4>();
         SIHG_CUDA(cudaMemcpyAsync(d, pc.data(), sizeof(int4) * pc.size(), cudaMemcpyHostToDevice, s));
