@@ -490,7 +490,7 @@ def run_gb300(args) -> None:
     shape = handle.launch_shape()
     names = (["k_step_primal", "k_step_dual_packed", "k_step_kty_packed"] if shape["packed"]
              else ["k_step_primal", "k_step_dual_packs", "k_step_kty_packs"]
-             if len(probs) == 1 and probs[0].num_nonzeros() >= 250_000  # one LP over packs of uniform segments
+             if shape["persistent"] == 0 and len(probs) == 1 and probs[0].num_nonzeros() >= 250_000  # over packs
              else ["k_step_primal", "k_step_dual", "k_step_kty"])
     timed = [k for k in range(3) if secs[k] > 0]  # the packed step has no elementwise kernel
     dom = max(timed, key=lambda k: secs[k])

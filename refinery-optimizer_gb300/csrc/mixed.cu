@@ -1308,13 +1308,15 @@ int MixedSolver::build_schedules(int task_nnz) {
     rows_ = layout_.rows;
     cols_ = layout_.cols;
     chunks_all_ = layout_.chunks;
-    return build_packs();
+    pack_cols_.count = pack_rows_.count = 0;
+    // packs where the steps surely run as kernels or these are to be timed (an
+    // LP that then does not fit a resident form gets them in setup_resident)
+    const bool kernels = opts_.autotune > 0 || opts_.persistent == 0 || (opts_.persistent < 0 && !latency_bound());
+    return kernels && use_packs() ? build_packs() : SIH_PDHG_OK;
 }
 
-// Packs of the steps by kernels (one LP beyond the latency-bound range).
+// Packs of the steps by kernels.
 int MixedSolver::build_packs() {
-    pack_cols_.count = pack_rows_.count = 0;
-    if (!use_packs()) return SIH_PDHG_OK;
     std::vector<int4> pc, pr;
     both_sides(M_ + N_ >= 65536, [&](int h) {
         if (h == 0)
@@ -1630,7 +1632,9 @@ int MixedSolver::setup_resident() {
                                   ResidentPlan::kGrid));
     if (!resident_->ready()) {
         // one LP beyond the resident forms: steps over packs (see kPackMinNnz)
-        return B_ == 1 && opts_.persistent < 0 && opts_.use_graph && !tuned_ && use_packs() ? set_form(0) : SIH_PDHG_OK;
+        if (!(B_ == 1 && opts_.persistent < 0 && opts_.use_graph && !tuned_ && use_packs())) return SIH_PDHG_OK;
+        if (pack_rows_.count == 0) SIHG_TRY(build_packs());
+        return set_form(0);
     }
     SIHG_TRY(resident_->fill(SegMatrix{M_, csr_ptr_.as<int>(), csr_pairs_.as<int2>()},
                              SegMatrix{N_, csc_ptr_.as<int>(), csc_pairs_.as<int2>()}, stream_));
