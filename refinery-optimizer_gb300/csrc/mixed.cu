@@ -2015,14 +2015,16 @@ int MixedSolver::run() {
     long long blk = 0, blk_end = max_blocks;
     timed_out_ = false;
     // a launch of the resident form runs several evaluation periods (an
-    // instance that stops leaves it); one when the host watches the time
-    const int periods = resident_->ready() && !(opts_.time_limit_sec > 0) ? 4 : 1;
+    // instance that stops leaves it); one when the host watches the time, and
+    // one again once the resident form was given up (launch_resident)
+    int periods = resident_->ready() && !(opts_.time_limit_sec > 0) ? 4 : 1;
     // Blocks of eval_freq steps and one evaluation until every instance
     // stopped (a window of kWindow blocks in flight; the done count of the
     // oldest is read back before the next is queued).
     auto run_blocks = [&]() -> int {
         pulled_ = false;
         for (long long k = 0; blk < blk_end; blk += periods, ++k) {
+            if (!resident_->ready()) periods = 1;
             const int slot = (int)(k % kWindow);
             if (k >= kWindow) {
                 cudaError_t e = cudaEventSynchronize(ev[slot]);
