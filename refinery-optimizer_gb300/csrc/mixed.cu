@@ -2146,8 +2146,10 @@ int MixedSolver::run() {
 
 // Host copies of every instance's returned point (device order, scaled) and
 // of the scales, after a run: a copy per array that some instance returns from,
-// not several small ones per instance.
+// not several small ones per instance.  Locked: threads may read the results of
+// different instances at the same time.
 int MixedSolver::pull_points() {
+    std::lock_guard<std::mutex> lock(points_mutex_);
     if (pulled_) return SIH_PDHG_OK;
     if (h_scale_.empty()) {
         h_scale_.resize((size_t)N_ + M_);

@@ -4,6 +4,7 @@
 #pragma once
 
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -294,6 +295,7 @@ class MixedSolver {
     // host copies of the last run's points (columns, then rows), and the scales (constant after set-up)
     std::vector<float> h_point_, h_scale_;
     bool pulled_ = false;
+    std::mutex points_mutex_;
     std::vector<std::vector<float>> start_x_, start_y_;  // warm starts (device order, unscaled)
 };
 
