@@ -510,7 +510,7 @@ int CglsBatch::setup_blocks(const std::vector<int>& csr_ptr, const std::vector<i
         entries = std::max<long long>(entries, csr_ptr[roff[b + 1]] - csr_ptr[roff[b]]);
     }
     if (16 * entries + 16 * (size[0] + size[1]) > budget) return SIH_PDHG_OK;
-    const std::vector<int>*ptrs[2] = {&csr_ptr, &csc_ptr}, *offs[2] = {&roff, &coff};
+    const std::vector<int>* offs[2] = {&roff, &coff};
     const std::vector<uint8_t> lanes[2] = {segment_lanes(layout_.row_schedule, M_),
                                            segment_lanes(layout_.col_schedule, N_)};
     std::vector<int4> passes[2];

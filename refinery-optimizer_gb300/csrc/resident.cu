@@ -147,7 +147,6 @@ struct FromShared {
 struct FromGlobal {
     using Entries = Wide;
     const float* v;
-    static constexpr int none = -1;
     __device__ __forceinline__ float operator()(int i) const {
         float x = 0.f;
         if (i >= 0) asm volatile("ld.global.f32 %0, [%1];" : "=f"(x) : "l"(v + i));
@@ -168,7 +167,6 @@ struct FromRecords {
     using Entries = Wide;
     const float4* v;
     float tau;
-    static constexpr int none = -1;
     __device__ __forceinline__ float operator()(int i) const {
         return i >= 0 ? x_from_record(ld_record(v + i), tau) : 0.f;
     }
