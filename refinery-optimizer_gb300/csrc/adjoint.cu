@@ -551,8 +551,8 @@ int CglsBatch::setup_blocks(const std::vector<int>& csr_ptr, const std::vector<i
         L.total = (int)at;
         if (at > budget) return SIH_PDHG_OK;
     }
-    SIHG_CUDA(cudaFuncSetAttribute(k_cgls_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   std::max(block_smem_[0].total, block_smem_[1].total)));
+    // the device's limit, not this batch's need: the attribute is the function's, for every thread of the process
+    SIHG_CUDA(cudaFuncSetAttribute(k_cgls_block, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
     // tables: passes, each instance's first pass and first segment
     std::vector<char> buf;
     size_t at[2][3];

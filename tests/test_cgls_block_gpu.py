@@ -61,3 +61,37 @@ def test_block_form_stops_at_the_iteration_limit(sih):
     _, info = sih.adjoint_batch([p, p], [x, x], [y, y], [np.ones(250)] * 2, max_iterations=3)
     for i in info:
         assert i["status"] == 1 and i["iterations"] == 12  # three in each of four rounds
+
+
+def test_threads_with_batches_of_different_sizes(sih):
+    """Entry points are re-entrant: calls on batches near a block's limit and on
+    small ones at the same time (every launch asks for its own amount of shared
+    memory) succeed and return what they return alone."""
+    import threading
+
+    from sih_pdhg.generators import small_random_lp
+
+    def call(p):
+        r = np.random.default_rng(3)
+        x, y = r.uniform(0, 1, p.num_cols()), r.standard_normal(p.num_rows())
+        g, info = sih.adjoint_batch([p, p], [x, x], [y, y], [np.ones(p.num_cols())] * 2, max_iterations=50)
+        return np.concatenate([np.concatenate([q[k] for k in sorted(q)]) for q in g])
+
+    ps = [small_random_lp(300, 1200, 9, 0), small_random_lp(50, 120, 4, 0)]
+    alone = [call(p) for p in ps]
+    wrong = []
+
+    def work(i):
+        for _ in range(40):
+            try:
+                if not np.array_equal(call(ps[i]), alone[i]):
+                    wrong.append("other results")
+            except sih._lib.SihPdhgError as e:
+                wrong.append(str(e))
+
+    threads = [threading.Thread(target=work, args=(i % 2,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong[:3]
