@@ -1873,7 +1873,12 @@ int MixedSolver::choose_staging() {
     auto enable = [&](const void* fn, int P, int& out) -> int {
         if (P == 0) return SIH_PDHG_OK;
         const int smem = (int)(sizeof(float) * P);
-        SIHG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        cudaFuncAttributes fa{};
+        SIHG_CUDA(cudaFuncGetAttributes(&fa, fn));
+        // the device's limit, not this LP's need (more is refused here): the attribute is the function's, for
+        // every handle and thread of the process
+        SIHG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       std::max(smem, optin - (int)fa.sharedSizeBytes)));
         int occ = 0;
         SIHG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kStagedThreads, smem));
         if (occ < 1) out = 0;

@@ -162,3 +162,18 @@ def test_lane_width_override_solves(sih, lanes):
     assert s.is_optimal()
     ref = entry["highs_objective"]
     assert abs(s.primal_objective - ref) <= 40 * 1e-6 * (1 + abs(ref))
+
+
+def test_handles_with_other_staged_prefixes_side_by_side(sih):
+    """A handle with a larger staged prefix still runs after one with a smaller
+    prefix was set up (both above the 48 KiB that need no permission)."""
+    from sih_pdhg.generators import small_random_lp
+
+    prob = small_random_lp(20000, 50000, 4, 0)
+    cfg = sih.GpuPdhgConfig(max_iterations=64, tol_primal=1e-12, tol_dual=1e-12, tol_gap=1e-12)
+    kw = dict(algorithm=sih.ALGO_MIXED, persistent=0, autotune=0)
+    with sih.PdhgHandle(prob, cfg, staged_kib=128, **kw) as a, sih.PdhgHandle(prob, cfg, staged_kib=60, **kw) as b:
+        assert a.launch_shape()["staged_x"] == 32768 and b.launch_shape()["staged_x"] == 15360
+        a.run()
+        b.run()
+        np.testing.assert_array_equal(a.result(0).x, b.result(0).x)
