@@ -7,6 +7,7 @@
 
 #include "common.cuh"
 #include "compat.cuh"
+#include "spmv.cuh"
 
 namespace sihg {
 
@@ -48,6 +49,14 @@ __device__ __forceinline__ float ld_stream(const float* p) {
     return v;
 }
 
+// s + c <- s + c + v, c the compensation
+__device__ __forceinline__ void comp_add(float& s, float& c, float v) {
+    float t, e;
+    two_sum(s, v, t, e);
+    s = t;
+    c = __fadd_rn(c, e);
+}
+
 // Many short segments: a warp takes 32 consecutive segments and reads their
 // entries as one stream, eight per lane in flight, whatever the segments'
 // lengths (products go to shared memory; Greathouse and Daga's CSR-stream,
@@ -55,11 +64,19 @@ __device__ __forceinline__ float ld_stream(const float* p) {
 // longer than kLong.  Groups of lanes leave the lanes of short segments idle
 // while the group of a long one works.  What bounds it is the gathers: one
 // cache line each, which the L1 takes one at a time per SM (12M of them: 46 us).
-// 500k x 1M LP, 12M entries: columns (Zipf lengths, 2 to 350, mean 12) 147 us by
-// groups, 62.8 by stream; rows (mean 24) 57.9 and 54.8.  64 warps per SM (32
-// registers) matter most: 48 warps 65.6 / 61.3 us; windows of 256 / 640 products
-// 76 / 69 us, 16 entries a lane in flight 83 us; kLong 24 / 32 / 64: 70.3 / 58.8 / 54.8 us
-// on the rows.
+//
+// The products are rounded on their way through shared memory, so the sums are
+// compensated: relative error 3.5e-8 at any length, against 3.9e-8 (3 entries) to
+// 6.2e-8 (31) of fused multiply-adds by groups of lanes and 4.2e-8 to 8.1e-8 of
+// plain sums of the products.  Values and gathered entries side by side in shared
+// memory, for fused multiply-adds here too, leave the gathers too little L1.
+//
+// 1M segments of 12 entries (12M) and 500k of 24, us by groups / plain sums / so: equal
+// lengths 53 / 48 / 48 and 54 / 49 / 49, lengths by a power law (2 to 2000) 147 / 58 / 62
+// and 130 / 66 / 72.  64 warps per SM (32 registers; the pointers are read again
+// after the gathers to stay within them) matter most: 48 warps 5 to 12 % more;
+// windows of 256 / 640 products 20 / 10 %, 16 entries a lane in flight 32 %; kLong 24 / 32:
+// 28 / 7 % more on rows of 24.
 constexpr int kWindow = 512;  // products of a warp at a time
 constexpr int kLong = 48;
 __device__ __forceinline__ void spmv_by_stream(int nseg, const int* __restrict__ ptr, const int* __restrict__ idx,
@@ -70,12 +87,9 @@ __device__ __forceinline__ void spmv_by_stream(int nseg, const int* __restrict__
     const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
     const unsigned last = nseg;
     for (unsigned base = wid * 32u; base < last; base += nw * 32u) {
-        const unsigned r = base + lane;
-        const int b = ptr[min(r, last)], e = ptr[min(r + 1, last)];
-        const int end = __shfl_sync(FULL_MASK, e, 31);
-        const unsigned longs = __ballot_sync(FULL_MASK, e - b > kLong);
-        float s = 0.f;
-        for (int w = __shfl_sync(FULL_MASK, b, 0); w < end; w += kWindow) {
+        const int end = ptr[min(base + 32u, last)];
+        float s = 0.f, c = 0.f;
+        for (int w = ptr[base]; w < end; w += kWindow) {
             const int n = min(kWindow, end - w);
             for (int k0 = lane; k0 < n; k0 += 32 * kU) {
                 int i[kU];
@@ -93,29 +107,30 @@ __device__ __forceinline__ void spmv_by_stream(int nseg, const int* __restrict__
                     if (i[u] >= 0) prod[k0 + 32 * u] = a[u] * g[u];
             }
             __syncwarp();
-            const int lo = max(b - w, 0), hi = min(e - w, n);  // this lane's part of the window
-            if (e - b <= kLong) {
-                float t = 0.f;
-                int k = lo;
-                for (; k + 1 < hi; k += 2) {
-                    s += prod[k];
-                    t += prod[k + 1];
-                }
-                if (k < hi) s += prod[k];
-                s += t;
-            }
-            for (unsigned m = longs; m; m &= m - 1) {
+            // this lane's segment and its part of the window
+            const unsigned r = base + lane;
+            const int b = ptr[min(r, last)] - w, e = ptr[min(r + 1, last)] - w;
+            const int lo = max(b, 0), hi = min(e, n);
+            if (e - b <= kLong)
+                for (int k = lo; k < hi; ++k) comp_add(s, c, prod[k]);
+            for (unsigned m = __ballot_sync(FULL_MASK, e - b > kLong); m; m &= m - 1) {
                 const int from = __ffs(m) - 1;
                 const int lo1 = __shfl_sync(FULL_MASK, lo, from), hi1 = __shfl_sync(FULL_MASK, hi, from);
-                float t = 0.f;
-                for (int k = lo1 + lane; k < hi1; k += 32) t += prod[k];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(FULL_MASK, t, o);
-                if (lane == from) s += t;
+                float p = 0.f, pc = 0.f;
+                for (int k = lo1 + lane; k < hi1; k += 32) comp_add(p, pc, prod[k]);
+                __syncwarp();
+                group_sum2(p, pc, 32);
+                p = __shfl_sync(FULL_MASK, p, 0);
+                pc = __shfl_sync(FULL_MASK, pc, 0);
+                if (lane == from) {
+                    comp_add(s, c, p);
+                    c += pc;
+                }
             }
             __syncwarp();
         }
-        if (r < last) out[r] = s;
+        // (an infinite sum has no compensation)
+        if (base + lane < last) out[base + lane] = isfinite(s) ? s + c : s;
     }
 }
 

@@ -157,3 +157,59 @@ def test_chained_launchers_see_each_other(env):
             assert lib.sih_pdhg_launch_restart(n, a.data_ptr(), b.data_ptr(), s.cuda_stream) == 0
             assert lib.sih_pdhg_launch_restart(n, b.data_ptr(), a.data_ptr(), s.cuda_stream) == 0
             assert float(b.min()) == k and float(a.max()) == k
+
+
+def _spmv(torch, lib, lens, idx, val, vec):
+    nseg = len(lens)
+    ptr = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    d = [_dev(torch, a) for a in (ptr, idx.astype(np.int32), val, vec)]
+    out = torch.full((nseg,), 7.0, dtype=torch.float32, device="cuda")
+    assert lib.sih_pdhg_launch_csr_spmv(nseg, *[a.data_ptr() for a in d], out.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+@pytest.mark.parametrize("length", [3, 20, 31, "uneven"])
+def test_spmv_by_stream_loses_only_the_products_roundings(env, length):
+    """40,000 short segments go by stream (a mean below 32, asserted): products
+    rounded to FP32, compensated sums.  Each of the two roundings left (product,
+    result) is uniform within 2^-24 of its value at most, sqrt(1/3) of that in the
+    mean square; terms of zero mean, so |error| <= sqrt(2/3) 2^-24 |result| over
+    all segments.  Plain sums of 20 and more terms are past that."""
+    torch, lib, _ = env
+    rng = np.random.default_rng(7)
+    nseg = 40000
+    # lanes' own segments up to 48 entries, the warp's from 49 on, several of each side by side, windows of 512
+    lens = np.full(nseg, length) if length != "uneven" else rng.choice(
+        [0, 1, 2, 5, 9, 16, 31, 33, 48, 49, 64, 130], nseg, p=[.1, .1, .1, .1, .2, .1, .1, .05, .05, .05, .04, .01])
+    nnz = int(lens.sum())
+    assert nnz < 32 * nseg
+    idx = rng.integers(0, 9000, nnz)
+    val, vec = rng.standard_normal(nnz).astype(np.float32), rng.standard_normal(9000).astype(np.float32)
+    out = _spmv(torch, lib, lens, idx, val, vec)
+    ref = np.bincount(np.repeat(np.arange(nseg), lens), weights=val.astype(np.float64) * vec[idx], minlength=nseg)
+    assert np.linalg.norm(out - ref) <= np.sqrt(2 / 3) * 2.0**-24 * np.linalg.norm(ref)
+
+
+def test_spmv_by_stream_keeps_infinities_and_nan(env):
+    """Infinite and NaN entries of the vector, in segments of a lane and of a
+    warp: the sums that plain additions give."""
+    torch, lib, _ = env
+    rng = np.random.default_rng(8)
+    nseg = 40000
+    lens = rng.choice([1, 2, 7, 30, 60, 700], nseg, p=[.3, .3, .2, .15, .045, .005])
+    nnz = int(lens.sum())
+    assert nnz < 32 * nseg
+    vec = rng.standard_normal(5000).astype(np.float32)
+    vec[:3] = np.inf, -np.inf, np.nan
+    idx = rng.integers(3, 5000, nnz)
+    odd = rng.choice(nnz, 9000, replace=False)
+    idx[odd] = rng.integers(0, 3, 9000)
+    val = rng.standard_normal(nnz).astype(np.float32)
+    out = _spmv(torch, lib, lens, idx, val, vec)
+    with np.errstate(invalid="ignore"):
+        prod = val.astype(np.float64) * vec[idx]
+        ref = np.bincount(np.repeat(np.arange(nseg), lens), weights=prod, minlength=nseg)
+    assert np.isposinf(ref).any() and np.isneginf(ref).any() and np.isnan(ref).any()
+    for f in (np.isposinf, np.isneginf, np.isnan):
+        np.testing.assert_array_equal(f(out), f(ref))
