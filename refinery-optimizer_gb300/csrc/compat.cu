@@ -77,14 +77,14 @@ __device__ __forceinline__ void comp_add(float& s, float& c, float v) {
 // after the gathers to stay within them) matter most: 48 warps 5 to 12 % more;
 // windows of 256 / 640 products 20 / 10 %, 16 entries a lane in flight 32 %; kLong 24 / 32:
 // 28 / 7 % more on rows of 24.
-constexpr int kWindow = 512;  // products of a warp at a time
 constexpr int kLong = 48;
 __device__ __forceinline__ void spmv_by_stream(int nseg, const int* __restrict__ ptr, const int* __restrict__ idx,
                                                const float* __restrict__ val, const float* __restrict__ vec,
                                                float* __restrict__ out, float* prod) {
     constexpr int kU = 8;
     const int lane = threadIdx.x & 31;
-    const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    // to every block's first warp first, so that the blocks have even shares
+    const int wid = blockIdx.x + gridDim.x * (threadIdx.x >> 5), nw = (gridDim.x * blockDim.x) >> 5;
     const unsigned last = nseg;
     for (unsigned base = wid * 32u; base < last; base += nw * 32u) {
         const int end = ptr[min(base + 32u, last)];
@@ -138,18 +138,18 @@ __device__ __forceinline__ void spmv_by_stream(int nseg, const int* __restrict__
 // on the device, so that no launch has to ask the host for it.  By stream from
 // kStreamSegs segments on, where every SM has several warps of 32, and below a
 // mean of 64, where a segment keeps a half-warp busy by itself.
-__global__ void __launch_bounds__(kSplitThreads, 16) split_spmv_kernel(int nseg, const int* __restrict__ ptr,
-                                                                   const int* __restrict__ idx,
-                                                                   const float* __restrict__ val,
-                                                                   const float* __restrict__ vec,
-                                                                   float* __restrict__ out) {
-    __shared__ float prod[kSplitThreads / 32][kWindow];
+__global__ void __launch_bounds__(kSplitThreads, 8) split_spmv_kernel(int nseg, const int* __restrict__ ptr,
+                                                                      const int* __restrict__ idx,
+                                                                      const float* __restrict__ val,
+                                                                      const float* __restrict__ vec,
+                                                                      float* __restrict__ out) {
+    extern __shared__ float prod[];  // [warps][kWindow]
     chain_wait_for(ptr, idx, val, vec, out);
     const long long nnz = ptr[nseg];
     int L = 1;
     while (L < 32 && 4ll * L * nseg <= nnz) L *= 2;
     if (nseg >= kStreamSegs && L < 16)
-        spmv_by_stream(nseg, ptr, idx, val, vec, out, prod[threadIdx.x >> 5]);
+        spmv_by_stream(nseg, ptr, idx, val, vec, out, prod + kWindow * (threadIdx.x >> 5));
     else
         spmv_by_groups(nseg, ptr, idx, val, vec, out, L);
 }
@@ -227,8 +227,9 @@ static int split_spmv(int nseg, const int* ptr, const int* idx, const float* val
     if (nseg < 0) return fail(SIH_PDHG_ERR_INVALID_ARGUMENT, "negative dimension");
     if (nseg == 0) return SIH_PDHG_OK;
     if (!ptr || !out || !vec) return fail(SIH_PDHG_ERR_INVALID_ARGUMENT, "NULL device pointer");
-    SIHG_CUDA(launch_chained(split_spmv_kernel, split_grid(nseg, sm_count()), kSplitThreads, 0,
-                             static_cast<cudaStream_t>(stream), nseg, ptr, idx, val, vec, out));
+    const SplitLaunch g = split_launch(nseg, sm_count());
+    SIHG_CUDA(launch_chained(split_spmv_kernel, g.blocks, g.threads, g.smem, static_cast<cudaStream_t>(stream), nseg, ptr,
+                             idx, val, vec, out));
     return SIH_PDHG_OK;
 }
 

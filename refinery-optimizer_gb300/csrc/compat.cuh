@@ -10,17 +10,30 @@ namespace sihg {
 __global__ void split_spmv_kernel(int nseg, const int* __restrict__ ptr, const int* __restrict__ idx,
                                   const float* __restrict__ val, const float* __restrict__ vec,
                                   float* __restrict__ out);
-constexpr int kSplitThreads = 128;
+constexpr int kSplitThreads = 256;  // most of a block
 // From this many segments on split_spmv_kernel may take 32 segments a warp.
 constexpr int kStreamSegs = 1 << 15;
-// Blocks of split_spmv_kernel.  Many segments: a warp per 32 of them, as many
-// blocks as that takes, so that the hardware hands out new blocks as old ones
-// end (columns of Zipf lengths).  Few: a warp per segment, what 32 lanes a segment would
-// need (the kernel takes fewer where the mean length says so), at most 16 a SM.
-inline int split_grid(int nseg, int sms) {
-    constexpr int kWarps = kSplitThreads / 32;
-    if (nseg >= kStreamSegs) return (nseg + 32 * kWarps - 1) / (32 * kWarps);
-    return std::max(1, std::min((nseg + kWarps - 1) / kWarps, sms * 16));
+constexpr int kWindow = 512;  // products of a warp at a time, there
+// Launch of split_spmv_kernel, which learns on the device whether it goes by
+// groups of lanes or by stream.  By groups it wants a warp per segment, what 32
+// lanes a segment would need (it takes fewer where the mean length says so), as
+// far as the SMs hold them: 64 warps each.  By stream a warp per 32 segments: with
+// more of those than the SMs hold, blocks of four warps, which the hardware hands
+// out as others end (columns of Zipf lengths); below, what the groups want, in
+// blocks of eight, of which the stream leaves some warps idle.  40,000 / 100,000
+// / 200,000 segments of 70 entries (groups) with a warp per 32 segments everywhere
+// 36.2 / 45.5 / 101, so 13.8 / 31.5 / 68 us; of 24 (stream) 8.0 / 13.5 / 28.5 and
+// 7.2 / 13.6 / 21.3 us (blocks of four warps: 7.3 / 15.4 / 21.3).
+struct SplitLaunch {
+    int blocks, threads, smem;
+};
+inline SplitLaunch split_launch(int nseg, int sms) {
+    const int units = (nseg - 1) / 32 + 1;
+    const bool many = nseg >= kStreamSegs && units > 64 * sms;
+    const int warps = many ? 4 : kSplitThreads / 32;
+    const int blocks = many ? (units - 1) / warps + 1 : std::min((nseg - 1) / warps + 1, 64 * sms / warps);
+    const int smem = nseg >= kStreamSegs ? (int)sizeof(float) * kWindow * warps : 0;
+    return SplitLaunch{std::max(1, blocks), 32 * warps, smem};
 }
 
 // Column measures (blocks first) and row violations of a point, one launch.
