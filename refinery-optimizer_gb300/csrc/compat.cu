@@ -14,12 +14,13 @@ namespace sihg {
 __device__ __forceinline__ float split_dot(const int* __restrict__ idx, const float* __restrict__ val, int beg,
                                            int end, int lane0, int L, const float* __restrict__ vec) {
     float s0 = 0.f, s1 = 0.f;
-    int k = beg + lane0;
-    for (; k + L < end; k += 2 * L) {
+    unsigned k = (unsigned)beg + lane0;  // (unsigned: a step may end past 2^31 - 1)
+    const unsigned last = end;
+    for (; (int)(last - k) > L; k += 2 * L) {
         s0 = fmaf(__ldg(val + k), __ldg(vec + __ldg(idx + k)), s0);
         s1 = fmaf(__ldg(val + k + L), __ldg(vec + __ldg(idx + k + L)), s1);
     }
-    if (k < end) s0 = fmaf(__ldg(val + k), __ldg(vec + __ldg(idx + k)), s0);
+    if ((int)(last - k) > 0) s0 = fmaf(__ldg(val + k), __ldg(vec + __ldg(idx + k)), s0);
     return s0 + s1;
 }
 
@@ -87,10 +88,11 @@ __device__ __forceinline__ void spmv_by_stream(int nseg, const int* __restrict__
     const int wid = blockIdx.x + gridDim.x * (threadIdx.x >> 5), nw = (gridDim.x * blockDim.x) >> 5;
     const unsigned last = nseg;
     for (unsigned base = wid * 32u; base < last; base += nw * 32u) {
-        const int end = ptr[min(base + 32u, last)];
+        const unsigned end = ptr[min(base + 32u, last)];
         float s = 0.f, c = 0.f;
-        for (int w = ptr[base]; w < end; w += kWindow) {
-            const int n = min(kWindow, end - w);
+        // (unsigned: the last window of 2^31 - 1 entries ends past them)
+        for (unsigned w = ptr[base]; (int)(end - w) > 0; w += kWindow) {
+            const int n = min(kWindow, (int)(end - w));
             for (int k0 = lane; k0 < n; k0 += 32 * kU) {
                 int i[kU];
                 float a[kU], g[kU];
@@ -109,7 +111,7 @@ __device__ __forceinline__ void spmv_by_stream(int nseg, const int* __restrict__
             __syncwarp();
             // this lane's segment and its part of the window
             const unsigned r = base + lane;
-            const int b = ptr[min(r, last)] - w, e = ptr[min(r + 1, last)] - w;
+            const int b = ptr[min(r, last)] - (int)w, e = ptr[min(r + 1, last)] - (int)w;
             const int lo = max(b, 0), hi = min(e, n);
             if (e - b <= kLong)
                 for (int k = lo; k < hi; ++k) comp_add(s, c, prod[k]);

@@ -213,3 +213,33 @@ def test_spmv_by_stream_keeps_infinities_and_nan(env):
     assert np.isposinf(ref).any() and np.isneginf(ref).any() and np.isnan(ref).any()
     for f in (np.isposinf, np.isneginf, np.isnan):
         np.testing.assert_array_equal(f(out), f(ref))
+
+
+@pytest.mark.parametrize("way", ["stream", "groups"])
+def test_spmv_of_the_most_entries_an_int_counts(env, way):
+    """2^31 - 1 entries: the last step of a lane group and the last window of the
+    stream end past the largest int, and read nothing there."""
+    torch, lib, _ = env
+    nnz = 2**31 - 1
+    if torch.cuda.mem_get_info()[0] < 24 * 2**30:
+        pytest.skip("needs 18 GB on the device")
+    nseg = nnz // 31 if way == "stream" else 20001
+    ptr = torch.arange(nseg + 1, dtype=torch.int64, device="cuda") * (nnz // nseg)
+    ptr[-1] = nnz  # the last segment takes the remainder
+    idx = torch.zeros(nnz, dtype=torch.int32, device="cuda")
+    val = torch.zeros(nnz, dtype=torch.float32, device="cuda")
+    if way == "stream":
+        val.fill_(1.0)  # sums: the lengths
+        ref = torch.diff(ptr).float()
+    else:  # the last 77 entries of every segment count
+        for k in range(1, 78):
+            val[ptr[1:] - k] = 1.0
+        ref = torch.full((nseg,), 77.0, device="cuda")
+    ptr = ptr.to(torch.int32)
+    vec, out = torch.ones(4, device="cuda"), torch.full((nseg,), 7.0, device="cuda")
+    assert lib.sih_pdhg_launch_csr_spmv(nseg, ptr.data_ptr(), idx.data_ptr(), val.data_ptr(), vec.data_ptr(),
+                                        out.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(out, ref)
+    del idx, val, ptr
+    torch.cuda.empty_cache()
