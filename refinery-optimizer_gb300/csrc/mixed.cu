@@ -1625,8 +1625,13 @@ int MixedSolver::setup_resident() {
     // (a batch: no cluster holds the mean instance)
     if (B_ > 1 && 12.0 * (double)nnz_ > 220.0 * 1024.0 * 16.0 * B_) return SIH_PDHG_OK;
     const std::vector<uint8_t> rl = segment_lanes(layout_.row_schedule, M_), cl = segment_lanes(layout_.col_schedule, N_);
+    // A batch's step over the task engine, in us by its millions of nonzeros: kernels
+    // per phase 46 (1.2), 55 (1.5), 68 (2.6), 84 (4.6), 98 (6.5), 125 (10.2), tuned 34, 35,
+    // 44, 55, 69, 114.  Where a step of the clusters takes longer, they lose.
+    const double millions = 1e-6 * (double)nnz_;
+    const double tasks_us = opts_.autotune != 0 ? 25.0 + 7.0 * millions : 40.0 + 9.5 * millions;
     SIHG_TRY(resident_->build(h_csr_ptr_, h_csc_ptr_, row_off_, col_off_, rl, cl, sm_count_, stream_,
-                              ResidentPlan::kCluster));
+                              ResidentPlan::kCluster, B_ > 1 ? tasks_us : 0.0));
     if (!resident_->ready() && B_ == 1)
         SIHG_TRY(resident_->build(h_csr_ptr_, h_csc_ptr_, row_off_, col_off_, rl, cl, sm_count_, stream_,
                                   ResidentPlan::kGrid));

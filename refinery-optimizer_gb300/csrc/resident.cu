@@ -36,6 +36,7 @@
 // 13.5, 2,000 x 5,000 6.9 -> 6.4, 317 x 803 4.5 -> 4.3 (26 and 30 warps: 23.0 and
 // 22.5 on the batch, 13: 23.2).
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "eval.cuh"
@@ -1439,7 +1440,7 @@ void ResidentPlan::release() {
 
 int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>& csc_ptr, const std::vector<int>& roff,
                         const std::vector<int>& coff, const std::vector<uint8_t>& row_lanes,
-                        const std::vector<uint8_t>& col_lanes, int sm_count, cudaStream_t s, Kind kind) {
+                        const std::vector<uint8_t>& col_lanes, int sm_count, cudaStream_t s, Kind kind, double most_us) {
     release();
     kind_ = kind;
     const bool plain = kind == kPlain, grid = kind == kGrid;
@@ -1590,6 +1591,7 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
     } else {
         SIHG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     }
+    int clusters = sm_count;  // at a time; blocks that share an SM gain nothing over taking turns
     if (!grid && C > 1) {
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1600,11 +1602,29 @@ int ResidentPlan::build(const std::vector<int>& csr_ptr, const std::vector<int>&
         cfg.dynamicSmemBytes = (size_t)sm.total;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        int clusters = 0;
         if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
             (void)cudaGetLastError();
             return SIH_PDHG_OK;
         }
+    }
+    if (kind == kCluster && B > clusters && most_us > 0.0) {
+        // Every instance takes the cluster that the largest one needs, and the
+        // clusters take turns (many of them overlap).  A turn's step takes 4.7 us for its
+        // barriers and controller alone, up to 9.3 us where an instance fills its
+        // cluster's memory.  Estimated / measured us per step: 64 of 2,000 x 5,000 (clusters
+        // of 4) 18.5 / 18.6, 512 of 1,000 x 2,500 (2) 62 / 63, 48 of 5,000 x 12,000 (16) 62 /
+        // 64, 64 of 200 to 3,000 rows (8) 32 / 30, 200 of 100 to 3,000 (8) 100 / 90, 300 of
+        // 200 x 500 with one of 5,000 x 12,000 (16) 215 / 207.
+        double sum = 0.0;
+        for (int b = 0; b < B; ++b) {
+            double bytes = 4.0 * (col_words + C) * inst[b].y + 4.0 * (row_words + C) * inst[b].w;
+            for (size_t q = first[2 * (size_t)b]; q < first[2 * (size_t)b + 2]; ++q) bytes += pair_bytes * ((all[q].z + 1) / 2);
+            const double full = std::min(1.0, bytes / ((double)C * budget));
+            sum += 4.7 + 4.6 * full * (2.0 - full);
+        }
+        double turns = (double)B / clusters;
+        if (turns < 4.0) turns = std::ceil(turns);
+        if (turns * sum / B > most_us) return SIH_PDHG_OK;
     }
     // the tables: blocks, instances, passes by block, and each pass's place in the matrix for the fill
     const size_t nb = sizeof(ResBlock) * (size_t)B * C, ni = sizeof(int4) * (size_t)B, np = sizeof(int4) * all.size();

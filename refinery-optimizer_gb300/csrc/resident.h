@@ -48,10 +48,12 @@ class ResidentPlan {
     // plain algorithm of one LP on a cluster.
     enum Kind { kCluster, kGrid, kPlain };
     // Plans the form for these instances (segment pointers of the batch, lanes
-    // per segment of both sides); ready() says whether they fit.
+    // per segment of both sides); ready() says whether they fit.  most_us > 0: a
+    // batch whose clusters take turns is left out where a step is estimated to
+    // take longer.
     int build(const std::vector<int>& csr_ptr, const std::vector<int>& csc_ptr, const std::vector<int>& roff,
               const std::vector<int>& coff, const std::vector<uint8_t>& row_lanes,
-              const std::vector<uint8_t>& col_lanes, int sm_count, cudaStream_t s, Kind kind);
+              const std::vector<uint8_t>& col_lanes, int sm_count, cudaStream_t s, Kind kind, double most_us = 0.0);
     // Copies the scaled entries into the layout.
     int fill(const SegMatrix& rows_A, const SegMatrix& cols_A, cudaStream_t s);
     // `periods` times nsteps steps and an evaluation of every running instance.

@@ -157,3 +157,20 @@ def test_plain_stops_at_the_same_check(sih):
     b = sih.solve_gpu_pdhg(p, cfg)
     assert a.is_optimal() and b.is_optimal()
     assert abs(a.simplex_iterations - b.simplex_iterations) <= cfg.check_frequency
+
+
+def test_batch_takes_the_clusters_only_where_their_turns_are_short(sih):
+    """One cluster size for the whole batch: a large LP among hundreds of small
+    ones would give each of them 16 blocks and a step some forty turns; that batch
+    steps over the task engine.  The small ones alone, and unequal ones in a few
+    turns, stay resident."""
+    from sih_pdhg.generators import small_random_lp
+
+    small = [small_random_lp(60, 150, 5, s) for s in range(300)]
+    mid = [small_random_lp(m, 5 * m // 2, 8, m) for m in range(200, 2000, 100)]
+    cfg = sih.GpuPdhgConfig(max_iterations=20000)
+    for ps, form in ((small + [small_random_lp(5000, 12000, 8, 7)], 0), (small, 1), (mid, 1)):
+        with sih.PdhgHandle(ps, cfg, algorithm=sih.ALGO_MIXED, autotune=0) as h:
+            assert h.launch_shape()["persistent"] == form
+            h.run()
+            assert all(h.result(b).is_optimal() for b in (0, len(ps) // 2, len(ps) - 1))
