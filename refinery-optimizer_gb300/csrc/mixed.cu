@@ -1603,15 +1603,10 @@ int MixedSolver::setup(const std::vector<const HostProblem*>& probs, const sih_p
     SIHG_TRY(setup_persistent());
     SIHG_TRY(setup_packed());
     // autotune: 1 on, 0 off, < 0 automatic (on for batches whose step form leaves something to tune)
-    if (opts.autotune < 0 && B_ > 1) {
-        SIHG_TRY(setup_resident());
-        if (resident_->ready()) {
-            tuned_ = 1;
-            return SIH_PDHG_OK;
-        }
-    }
-    if (opts.autotune > 0 || (opts.autotune < 0 && B_ > 1)) SIHG_TRY(autotune());
-    return setup_resident();
+    SIHG_TRY(setup_resident());
+    if (opts.autotune > 0 || (opts.autotune < 0 && B_ > 1 && !resident_->ready())) SIHG_TRY(autotune());
+    if (opts.autotune < 0 && B_ > 1) tuned_ = 1;
+    return SIH_PDHG_OK;
 }
 
 // The resident step forms where the step form is left to the engine (or form 2
@@ -1637,7 +1632,7 @@ int MixedSolver::setup_resident() {
                                   ResidentPlan::kGrid));
     if (!resident_->ready()) {
         // one LP beyond the resident forms: steps over packs (see kPackMinNnz)
-        if (!(B_ == 1 && opts_.persistent < 0 && opts_.use_graph && !tuned_ && use_packs())) return SIH_PDHG_OK;
+        if (!(B_ == 1 && opts_.persistent < 0 && opts_.use_graph && use_packs())) return SIH_PDHG_OK;
         if (pack_rows_.count == 0) SIHG_TRY(build_packs());
         return set_form(0);
     }
@@ -2314,18 +2309,27 @@ int MixedSolver::set_start(int b, const double* x, const double* y, double omega
 //     or 1, 2, 4, 8 forced),
 //   * the staged gathers of a single LP (on / off per side),
 // one coordinate after the other, keeping the fastest, then (options.persistent
-// < 0) the step form: kernels per phase replayed as a graph, or the persistent
-// kernel, by the device time of a block of steps and an evaluation.  The
+// < 0) the step form: kernels per phase replayed as a graph, the persistent
+// kernel, or the resident form where one holds the LPs (with the layout of the
+// rules), by the device time of a block of steps and an evaluation.  The
 // choice is cached per process for the shape (instances, rows, columns,
-// nonzeros), so repeated solves of one shape tune once.
+// nonzeros, and whether a resident form was there to choose), so repeated
+// solves of one shape tune once.
 namespace {
 struct TuneKey {
     int b, m, n;
     long long nnz;
-    bool operator<(const TuneKey& o) const { return std::tie(b, m, n, nnz) < std::tie(o.b, o.m, o.n, o.nnz); }
+    bool resident;
+    bool operator<(const TuneKey& o) const {
+        return std::tie(b, m, n, nnz, resident) < std::tie(o.b, o.m, o.n, o.nnz, o.resident);
+    }
+};
+struct TuneChoice {
+    bool resident;
+    sih_pdhg_launch_shape shape;  // of the kernels
 };
 std::mutex g_tune_mu;
-std::map<TuneKey, sih_pdhg_launch_shape> g_tune_cache;
+std::map<TuneKey, TuneChoice> g_tune_cache;
 }  // namespace
 
 void MixedSolver::launch_shape(sih_pdhg_launch_shape* out) const {
@@ -2358,9 +2362,11 @@ int MixedSolver::time_block(double* seconds) {
     const bool graph = opts_.use_graph && !persistent_;
     if (graph) SIHG_TRY(record_graph());
     if (persistent_) SIHG_CUDA(cudaMemsetAsync(bar_.as<void>(), 0, 4 * sizeof(unsigned), stream_));
+    if (resident_->ready()) SIHG_TRY(resident_->reset(stream_));
     SIHG_TRY(reset_state());
     cudaStream_t s = stream_;
     auto block = [&]() -> int {
+        if (resident_->ready()) return launch_resident(s, 1);
         if (persistent_) {
             SIHG_TRY(launch_persistent(s, eval_freq_));
             return launch_eval(s);
@@ -2385,15 +2391,28 @@ int MixedSolver::time_block(double* seconds) {
 }
 
 int MixedSolver::autotune() {
-    const TuneKey key{B_, M_, N_, nnz_};
+    const bool resident = resident_->ready() && opts_.persistent < 0;
+    const TuneKey key{B_, M_, N_, nnz_, resident};
     {
         std::lock_guard<std::mutex> g(g_tune_mu);
         auto it = g_tune_cache.find(key);
         if (it != g_tune_cache.end()) {
-            SIHG_TRY(apply_shape(it->second));
+            if (!it->second.resident) {
+                if (resident) resident_->release();
+                SIHG_TRY(apply_shape(it->second.shape));
+            }
             tuned_ = 1;
             return SIH_PDHG_OK;
         }
+    }
+    // the resident form first, then out of the way of the kernels
+    double resident_s = 0.0;
+    std::unique_ptr<ResidentPlan> held = std::make_unique<ResidentPlan>();
+    const int rule_nnz = task_nnz_, rule_r = lanes_r_, rule_c = lanes_c_, rule_form = persistent_, rule_grid = pgrid_;
+    if (resident) {
+        SIHG_TRY(time_block(&resident_s));
+        std::swap(held, resident_);
+        SIHG_TRY(set_form(B_ == 1 && latency_bound() ? 2 : 0));
     }
     const int reps = nnz_ > 64000000 ? 3 : (nnz_ > 4000000 ? 5 : 20);
     double sec[3];
@@ -2464,26 +2483,39 @@ int MixedSolver::autotune() {
         st = off < kTuneMargin * on ? 0 : rule;
     }
     // step form: graph of kernels per phase, or the persistent kernel
+    double kernels_s = INFINITY;
     if (opts_.persistent < 0) {
         const int alt = B_ == 1 ? 2 : 1;
+        SIHG_TRY(time_block(&kernels_s));
         if ((alt == 1 ? grid_form1_ : grid_form2_) > 0) {
             const int incumbent = persistent_;  // the automatic rule's form
             const int other = incumbent == 0 ? alt : 0;
-            double t0 = 0, t1 = 0;
-            SIHG_TRY(time_block(&t0));
+            double t1 = 0;
             SIHG_TRY(set_form(other));
             SIHG_TRY(time_block(&t1));
-            SIHG_TRY(set_form(t1 < kTuneMargin * t0 ? other : incumbent));
+            SIHG_TRY(set_form(t1 < kTuneMargin * kernels_s ? other : incumbent));
+            if (persistent_ == other) kernels_s = t1;
         }
     }
     tuned_ = 1;
     sih_pdhg_launch_shape sh{};
     launch_shape(&sh);
+    const bool keep = resident && !(kernels_s < kTuneMargin * resident_s);
+    if (keep) {  // as without the tuner
+        std::swap(held, resident_);
+        lanes_r_ = rule_r;
+        lanes_c_ = rule_c;
+        stage_x_ = stage_x_rule_;
+        stage_y_ = stage_y_rule_;
+        SIHG_TRY(build_schedules(rule_nnz));
+        persistent_ = rule_form;
+        pgrid_ = rule_grid;
+    }
     if (opts_.verbose)
         std::fprintf(stderr, "sih_pdhg autotune: task_nnz %d, lanes rows %d cols %d, staged %d/%d, form %d\n",
                      sh.task_nnz, sh.row_lanes, sh.col_lanes, sh.staged_x, sh.staged_y, sh.persistent);
     std::lock_guard<std::mutex> g(g_tune_mu);
-    g_tune_cache[key] = sh;
+    g_tune_cache[key] = TuneChoice{keep, sh};
     return SIH_PDHG_OK;
 }
 

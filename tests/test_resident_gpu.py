@@ -174,3 +174,19 @@ def test_batch_takes_the_clusters_only_where_their_turns_are_short(sih):
             assert h.launch_shape()["persistent"] == form
             h.run()
             assert all(h.result(b).is_optimal() for b in (0, len(ps) // 2, len(ps) - 1))
+
+
+def test_tuner_times_the_resident_form_too(sih):
+    """autotune = 1 on an LP that the SMs' shared memory holds: a step takes half
+    of what the fastest kernels take, so the tuner keeps the resident form (a few
+    launches, not three a step), the second time from its cache, with the same
+    point as without it."""
+    from sih_pdhg.generators import refinery_lp
+
+    p = refinery_lp(168, 0)
+    cfg = sih.GpuPdhgConfig(max_iterations=512, tol_primal=1e-12, tol_dual=1e-12, tol_gap=1e-12)
+    a = sih.solve_gpu_mixed(p, cfg, autotune=0)
+    for _ in range(2):
+        b = sih.solve_gpu_mixed(p, cfg, autotune=1)
+        assert b.kernel_launches == a.kernel_launches < 512
+        np.testing.assert_array_equal(a.x, b.x)
