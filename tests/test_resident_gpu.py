@@ -190,3 +190,70 @@ def test_tuner_times_the_resident_form_too(sih):
         b = sih.solve_gpu_mixed(p, cfg, autotune=1)
         assert b.kernel_launches == a.kernel_launches < 512
         np.testing.assert_array_equal(a.x, b.x)
+
+
+@pytest.mark.parametrize("kind", GRID, ids=str)
+def test_grid_form_runs_where_the_sms_hold_the_lp(sih, kind):
+    """The LPs above really take the grid form: thirteen launches to start and one for
+    up to four evaluation periods of 64 steps.  The last does not fit and takes three
+    launches a step; it steps over packs like its baseline above, so here against
+    the task engine (staged gathers ask for it)."""
+    from sih_pdhg.generators import refinery_lp, small_random_lp, zipf_lp
+
+    if kind[0] == "uniform":
+        p = small_random_lp(*kind[1:], 2)
+    else:
+        p = refinery_lp(kind[1], 1) if kind[0] == "refinery" else zipf_lp(*kind[1:], 2)
+    cfg = sih.GpuPdhgConfig(max_iterations=128, tol_primal=1e-12, tol_dual=1e-12, tol_gap=1e-12)
+    b = sih.solve_gpu_mixed(p, cfg)
+    if kind != GRID[-1]:
+        assert b.kernel_launches == 14
+        return
+    assert b.kernel_launches > 3 * 128
+    a = sih.solve_gpu_mixed(p, cfg, persistent=0, staged_kib=64)
+    assert a.simplex_iterations == b.simplex_iterations and a.restarts == b.restarts
+    for u, v in ((a.x, b.x), (a.row_duals, b.row_duals)):
+        assert np.max(np.abs(u - v)) <= 1e-5 * max(1.0, np.max(np.abs(u)))
+
+
+@pytest.mark.parametrize("compensated", [0, 2])
+def test_single_lp_kernel_beyond_the_sms_shared_memory(sih, compensated):
+    """persistent = 2 on an LP that no resident form holds (3.25M nonzeros, 39 MB
+    of entries): k_solo_steps, one launch a period beside the evaluation's,
+    against the kernels per phase."""
+    from sih_pdhg.generators import small_random_lp
+
+    p = small_random_lp(60000, 130000, 25, 3)
+    cfg = sih.GpuPdhgConfig(max_iterations=128, tol_primal=1e-12, tol_dual=1e-12, tol_gap=1e-12)
+    a = sih.solve_gpu_mixed(p, cfg, persistent=0, compensated=compensated)
+    with sih.PdhgHandle(p, cfg, algorithm=sih.ALGO_MIXED, persistent=2, compensated=compensated) as h:
+        assert h.launch_shape()["persistent"] == 2
+        h.run()
+        b = h.result(0)
+    # thirteen launches to start, two periods of a launch and an evaluation of six
+    assert b.kernel_launches == 27 and a.kernel_launches > 3 * 128
+    assert a.simplex_iterations == b.simplex_iterations and a.restarts == b.restarts
+    assert a.step_rejections == b.step_rejections
+    for u, v in ((a.x, b.x), (a.row_duals, b.row_duals)):
+        assert np.max(np.abs(u - v)) <= 1e-5 * max(1.0, np.max(np.abs(u)))
+
+
+def test_batch_beyond_the_clusters_is_tuned(sih):
+    """autotune = -1 on a batch with an instance that no cluster holds: the tuner
+    times the kernels' shapes, and a second handle of the same shape reuses what
+    it chose; the resident batches have nothing to tune."""
+    from sih_pdhg.generators import small_random_lp
+
+    ps = [small_random_lp(300, 700, 6, 0), small_random_lp(9000, 20000, 5, 1)]
+    cfg = sih.GpuPdhgConfig(max_iterations=20000)
+    shapes = []
+    for _ in range(2):
+        with sih.PdhgHandle(ps, cfg, algorithm=sih.ALGO_MIXED) as h:
+            shapes.append(h.launch_shape())
+            h.run()
+            res = [h.result(b) for b in range(2)]
+            assert all(r.is_optimal() for r in res)
+            # not the resident form: seven launches a period at least
+            assert res[0].kernel_launches >= 7 * (max(r.simplex_iterations for r in res) // 64)
+    assert shapes[0]["tuned"] == 1 and shapes[0] == shapes[1]
+    assert shapes[0]["row_lanes"] in (0, 1, 2, 4, 8) and shapes[0]["col_lanes"] in (0, 1, 2, 4, 8)
