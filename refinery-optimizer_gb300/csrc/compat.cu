@@ -139,7 +139,11 @@ __device__ __forceinline__ void spmv_by_stream(int nseg, const int* __restrict__
 // Lanes per segment from the mean segment length, from the last pointer: read
 // on the device, so that no launch has to ask the host for it.  By stream from
 // kStreamSegs segments on, where every SM has several warps of 32, and below a
-// mean of 64, where a segment keeps a half-warp busy by itself.
+// mean of 32 (L < 16), where equal lengths are no slower by it at any count.  us by
+// groups / by stream for segments of 20, 28, 36 and 56 entries (L2 flushed): 60,000
+// equal ones 15 / 15, 17 / 17, 19 / 21, 23 / 54; 400,000 equal ones 64 / 42, 76 / 52,
+// 108 / 66, 134 / 191 (past kLong the warp sums each alone); 400,000 by a power law
+// 112 / 55, 146 / 74, 146 / 95, 216 / 160.
 __global__ void __launch_bounds__(kSplitThreads, 8) split_spmv_kernel(int nseg, const int* __restrict__ ptr,
                                                                       const int* __restrict__ idx,
                                                                       const float* __restrict__ val,
