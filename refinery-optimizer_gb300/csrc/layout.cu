@@ -76,19 +76,54 @@ std::vector<uint8_t> segment_lanes(const SideSchedule& sc, int nseg) {
     return lanes;
 }
 
-std::vector<int> order_by_lanes(const int* ptr, const uint8_t* lanes, int cnt) {
-    // counting sort on (lanes descending, length descending)
-    int longest = 0;
-    for (int k = 0; k < cnt; ++k) longest = std::max(longest, ptr[k + 1] - ptr[k]);
+void order_by_lanes(const std::vector<int>& ptr, std::vector<uint8_t>& lanes, std::vector<int>& order,
+                    std::vector<int>& new_ptr) {
+    // counting sort on (lanes descending, length descending), a part of the
+    // segments per thread; lengths from kMost on share a bucket and are few (a
+    // bucket per length up to the longest is as many as the other side has
+    // segments).  With pointers and vectors brought into the order on the device,
+    // the plain set-up of 500k x 1M takes 24.1 ms instead of 32, of 100k x 200k 6.5
+    // instead of 8.2 (by one thread a side, and gathers on the host).
+    constexpr int kMost = 2047, kSpan = kMost + 1, kKeys = 6 * kSpan;
+    const int cnt = (int)ptr.size() - 1;
+    const int parts = std::max(1, std::min(hardware_threads(), cnt >> 16));
     int group[33] = {};
     for (int lg = 0; lg <= 5; ++lg) group[1 << lg] = 5 - lg;
-    const size_t span = (size_t)longest + 1;
-    auto key = [&](int k) { return group[lanes[k]] * span + (size_t)(longest - (ptr[k + 1] - ptr[k])); };
-    std::vector<int> start(6 * span + 1, 0), order(cnt);
-    for (int k = 0; k < cnt; ++k) start[key(k) + 1]++;
-    for (size_t v = 0; v < 6 * span; ++v) start[v + 1] += start[v];
-    for (int k = 0; k < cnt; ++k) order[start[key(k)]++] = k;
-    return order;
+    auto key = [&](int64_t k) { return group[lanes[k]] * kSpan + kMost - std::min(kMost, ptr[k + 1] - ptr[k]); };
+    std::vector<int> start((size_t)parts * kKeys, 0), begin(kKeys + 1);
+    parallel_parts(cnt, parts, [&](int64_t k0, int64_t k1, int t) {
+        for (int64_t k = k0; k < k1; ++k) start[(size_t)t * kKeys + key(k)]++;
+    });
+    int at = 0;
+    for (int v = 0; v < kKeys; ++v) {
+        begin[v] = at;
+        for (int t = 0; t < parts; ++t) {
+            int& c = start[(size_t)t * kKeys + v];
+            const int n = c;
+            c = at;
+            at += n;
+        }
+    }
+    begin[kKeys] = at;
+    order.resize(cnt);
+    parallel_parts(cnt, parts, [&](int64_t k0, int64_t k1, int t) {
+        for (int64_t k = k0; k < k1; ++k) order[start[(size_t)t * kKeys + key(k)]++] = (int)k;
+    });
+    // in the new order a bucket has one length and one number of lanes
+    new_ptr.resize((size_t)cnt + 1);
+    new_ptr[0] = 0;
+    for (int v = 0; v < kKeys; ++v) {
+        const int k0 = begin[v], k1 = begin[v + 1], len = kMost - v % kSpan;
+        if (len < kMost) {
+            for (int k = k0; k < k1; ++k) new_ptr[k + 1] = new_ptr[k] + len;
+        } else {
+            std::stable_sort(order.begin() + k0, order.begin() + k1,
+                             [&](int p, int q) { return ptr[p + 1] - ptr[p] > ptr[q + 1] - ptr[q]; });
+            for (int k = k0; k < k1; ++k) new_ptr[k + 1] = new_ptr[k] + ptr[order[k] + 1] - ptr[order[k]];
+        }
+    }
+    for (int g = 0; g < 6; ++g)
+        std::fill(lanes.begin() + begin[g * kSpan], lanes.begin() + begin[(g + 1) * kSpan], (uint8_t)(32 >> g));
 }
 
 std::vector<int4> make_packs(const std::vector<int>& ptr, const std::vector<uint8_t>& lanes) {

@@ -130,8 +130,10 @@ struct PackSide {
 };
 // Host: the packs of a side.
 std::vector<int4> make_packs(const std::vector<int>& ptr, const std::vector<uint8_t>& lanes);
-// Order of `cnt` segments by lanes, then by descending length (stable).
-std::vector<int> order_by_lanes(const int* ptr, const uint8_t* lanes, int cnt);
+// Order of segments by lanes, then by descending length (stable), with their
+// pointers and lanes in that order.
+void order_by_lanes(const std::vector<int>& ptr, std::vector<uint8_t>& lanes, std::vector<int>& order,
+                    std::vector<int>& new_ptr);
 // Renumbered pairs of one side on the device (mixed.cu): segment s takes the
 // entries from src[s].x on, indices mapped through inv[src[s].y + index].
 __global__ void k_renumber_pairs(int nseg, const int* __restrict__ ptr, const int2* __restrict__ src,

@@ -185,6 +185,19 @@ __global__ void abs_sum_step_kernel(int nseg, const int* __restrict__ ptr, const
     }
 }
 
+// A side in device order: `nvec` vectors, where each segment's entries begin (in
+// the matrix with map offset `base`), and the new number of every segment.
+__global__ void plain_order_kernel(int count, const int* __restrict__ order, const int* __restrict__ ptr, int base,
+                                   const float* __restrict__ vec, int nvec, float* __restrict__ out,
+                                   int2* __restrict__ src, int* __restrict__ inv) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
+        const int j = order[k];
+        src[k] = make_int2(ptr[j], base);
+        inv[j] = k;
+        for (int v = 0; v < nvec; ++v) out[(size_t)v * count + k] = vec[(size_t)v * count + j];
+    }
+}
+
 // ---------------------------------------------------------------- host driver
 PlainSolver::PlainSolver() : resident_(std::make_unique<ResidentPlan>()) {}
 
@@ -225,23 +238,11 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
     }
     std::vector<int> csc_ptr, csr_ptr;
     if (packs) {
-        auto renumber = [](const std::vector<int>& ptr, std::vector<uint8_t>& lanes, std::vector<int>& order,
-                           std::vector<int>& new_ptr) {
-            const int cnt = (int)ptr.size() - 1;
-            order = order_by_lanes(ptr.data(), lanes.data(), cnt);
-            new_ptr.assign((size_t)cnt + 1, 0);
-            std::vector<uint8_t> l(cnt);
-            for (int k = 0; k < cnt; ++k) {
-                new_ptr[k + 1] = new_ptr[k] + ptr[order[k] + 1] - ptr[order[k]];
-                l[k] = lanes[order[k]];
-            }
-            lanes.swap(l);
-        };
         both_sides(m + n >= 65536, [&](int h) {
             if (h == 0)
-                renumber(hp.csr_ptr, row_lanes, row_order_, csr_ptr);
+                order_by_lanes(hp.csr_ptr, row_lanes, row_order_, csr_ptr);
             else
-                renumber(hp.csc_ptr, col_lanes, col_order_, csc_ptr);
+                order_by_lanes(hp.csc_ptr, col_lanes, col_order_, csc_ptr);
         });
     }
     const std::vector<int>& cptr = packs ? csc_ptr : hp.csc_ptr;
@@ -257,39 +258,6 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
 
     SIHG_CUDA(cudaMemcpyAsync(csc_ptr_.as<int>(), cptr.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s));
     SIHG_CUDA(cudaMemcpyAsync(csr_ptr_.as<int>(), rptr.data(), sizeof(int) * (m + 1), cudaMemcpyHostToDevice, s));
-    if (nnz > 0 && !packs) {
-        SIHG_CUDA(cudaMemcpyAsync(csc_pairs_.as<Pair>(), hp.csc.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
-        SIHG_CUDA(cudaMemcpyAsync(csr_pairs_.as<Pair>(), hp.csr.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
-    } else if (nnz > 0) {  // the pairs as they are, renumbered on the device
-        std::vector<int2> src((size_t)n + m);
-        std::vector<int> inv((size_t)n + m);  // rows' new numbers, then columns'
-        parallel_for(n, [&](int64_t k0, int64_t k1) {
-            for (int64_t k = k0; k < k1; ++k) {
-                src[k] = make_int2(hp.csc_ptr[col_order_[k]], 0);
-                inv[(size_t)m + col_order_[k]] = (int)k;
-            }
-        });
-        parallel_for(m, [&](int64_t k0, int64_t k1) {
-            for (int64_t k = k0; k < k1; ++k) {
-                src[(size_t)n + k] = make_int2(hp.csr_ptr[row_order_[k]], m);
-                inv[row_order_[k]] = (int)k;
-            }
-        });
-        DevMem staging;  // the pairs of both sides, each segment's source, the new numbers
-        SIHG_TRY(staging.alloc(sizeof(Pair) * 2 * (size_t)nnz + sizeof(int2) * src.size() + sizeof(int) * inv.size()));
-        int2* raw = staging.as<int2>();
-        int2* seg = raw + 2 * (size_t)nnz;
-        int* map = reinterpret_cast<int*>(seg + src.size());
-        SIHG_CUDA(cudaMemcpyAsync(raw, hp.csc.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
-        SIHG_CUDA(cudaMemcpyAsync(raw + nnz, hp.csr.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
-        SIHG_CUDA(cudaMemcpyAsync(seg, src.data(), sizeof(int2) * src.size(), cudaMemcpyHostToDevice, s));
-        SIHG_CUDA(cudaMemcpyAsync(map, inv.data(), sizeof(int) * inv.size(), cudaMemcpyHostToDevice, s));
-        k_renumber_pairs<<<sm_count_ * 8, 256, 0, s>>>(n, csc_ptr_.as<int>(), seg, raw, map, csc_pairs_.as<int2>());
-        k_renumber_pairs<<<sm_count_ * 8, 256, 0, s>>>(m, csr_ptr_.as<int>(), seg + n, raw + nnz, map,
-                                                       csr_pairs_.as<int2>());
-        SIHG_LAUNCH_CHECK();
-        SIHG_CUDA(cudaStreamSynchronize(s));  // the staging buffers are released at scope end
-    }
     float* cv = colvec_.as<float>();
     float* rv = rowvec_.as<float>();
     // column vectors: c l u tau x xbar best_x (7 used of 8 slots)
@@ -304,24 +272,49 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
     vec_.ru = rv + 1 * (size_t)m;
     vec_.sigma = rv + 2 * (size_t)m;
     vec_.y = rv + 3 * (size_t)m;
-    std::vector<float> host((size_t)3 * n + 2 * (size_t)m);  // c l u | rl ru in device order
-    parallel_for(n, [&](int64_t k0, int64_t k1) {
-        for (int64_t k = k0; k < k1; ++k) {
-            const int64_t j = packs ? col_order_[k] : k;
-            host[k] = hp.c[j];
-            host[(size_t)n + k] = hp.l[j];
-            host[2 * (size_t)n + k] = hp.u[j];
+    // c l u, then rl ru
+    const float* cols[3] = {hp.c.data(), hp.l.data(), hp.u.data()};
+    const float* rows[2] = {hp.rl.data(), hp.ru.data()};
+    if (!packs) {
+        if (nnz > 0) {
+            SIHG_CUDA(cudaMemcpyAsync(csc_pairs_.as<Pair>(), hp.csc.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
+            SIHG_CUDA(cudaMemcpyAsync(csr_pairs_.as<Pair>(), hp.csr.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
         }
-    });
-    parallel_for(m, [&](int64_t k0, int64_t k1) {
-        for (int64_t k = k0; k < k1; ++k) {
-            const int64_t i = packs ? row_order_[k] : k;
-            host[3 * (size_t)n + k] = hp.rl[i];
-            host[3 * (size_t)n + m + k] = hp.ru[i];
+        for (int k = 0; k < 3; ++k)
+            SIHG_CUDA(cudaMemcpyAsync(cv + k * (size_t)n, cols[k], sizeof(float) * n, cudaMemcpyHostToDevice, s));
+        for (int k = 0; k < 2; ++k)
+            SIHG_CUDA(cudaMemcpyAsync(rv + k * (size_t)m, rows[k], sizeof(float) * m, cudaMemcpyHostToDevice, s));
+    } else {  // everything as it is, brought into the new order on the device
+        const size_t N = n, M = m;
+        DevMem staging;  // pairs of both sides | sources | orders, pointers, new numbers | vectors
+        SIHG_TRY(staging.alloc(sizeof(Pair) * 2 * (size_t)nnz + sizeof(int2) * (N + M) + sizeof(int) * (3 * (N + M) + 2) +
+                               sizeof(float) * (3 * N + 2 * M)));
+        int2* raw = staging.as<int2>();
+        int2* src = raw + 2 * (size_t)nnz;
+        int* order = reinterpret_cast<int*>(src + N + M);  // columns, rows
+        int* ptr = order + N + M;                          // of the columns, of the rows
+        int* inv = ptr + N + M + 2;                        // rows' new numbers, then columns'
+        float* vec = reinterpret_cast<float*>(inv + N + M);
+        SIHG_CUDA(cudaMemcpyAsync(order, col_order_.data(), sizeof(int) * N, cudaMemcpyHostToDevice, s));
+        SIHG_CUDA(cudaMemcpyAsync(order + N, row_order_.data(), sizeof(int) * M, cudaMemcpyHostToDevice, s));
+        SIHG_CUDA(cudaMemcpyAsync(ptr, hp.csc_ptr.data(), sizeof(int) * (N + 1), cudaMemcpyHostToDevice, s));
+        SIHG_CUDA(cudaMemcpyAsync(ptr + N + 1, hp.csr_ptr.data(), sizeof(int) * (M + 1), cudaMemcpyHostToDevice, s));
+        for (int k = 0; k < 3; ++k)
+            SIHG_CUDA(cudaMemcpyAsync(vec + k * N, cols[k], sizeof(float) * N, cudaMemcpyHostToDevice, s));
+        for (int k = 0; k < 2; ++k)
+            SIHG_CUDA(cudaMemcpyAsync(vec + 3 * N + k * M, rows[k], sizeof(float) * M, cudaMemcpyHostToDevice, s));
+        plain_order_kernel<<<sm_count_ * 8, 256, 0, s>>>(n, order, ptr, 0, vec, 3, cv, src, inv + M);
+        plain_order_kernel<<<sm_count_ * 8, 256, 0, s>>>(m, order + N, ptr + N + 1, m, vec + 3 * N, 2, rv, src + N, inv);
+        if (nnz > 0) {
+            SIHG_CUDA(cudaMemcpyAsync(raw, hp.csc.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
+            SIHG_CUDA(cudaMemcpyAsync(raw + nnz, hp.csr.data(), sizeof(Pair) * nnz, cudaMemcpyHostToDevice, s));
+            k_renumber_pairs<<<sm_count_ * 8, 256, 0, s>>>(n, csc_ptr_.as<int>(), src, raw, inv, csc_pairs_.as<int2>());
+            k_renumber_pairs<<<sm_count_ * 8, 256, 0, s>>>(m, csr_ptr_.as<int>(), src + N, raw + nnz, inv,
+                                                           csr_pairs_.as<int2>());
         }
-    });
-    SIHG_CUDA(cudaMemcpyAsync(cv, host.data(), sizeof(float) * 3 * (size_t)n, cudaMemcpyHostToDevice, s));
-    SIHG_CUDA(cudaMemcpyAsync(rv, host.data() + 3 * (size_t)n, sizeof(float) * 2 * (size_t)m, cudaMemcpyHostToDevice, s));
+        SIHG_LAUNCH_CHECK();
+        SIHG_CUDA(cudaStreamSynchronize(s));  // the staging buffer is released at scope end
+    }
 
     // plans and heavy lists
     std::vector<int> heavy_c, heavy_r;
@@ -368,11 +361,13 @@ int PlainSolver::setup(const HostProblem& hp, const sih_pdhg_config& cfg, const 
     }
     // initial point x = clip(0, l, u) (gpu_solver.cpp:192-196), x_bar = x, y = 0
     x0_.resize(n);
-    for (int k = 0; k < n; ++k) {
-        const int j = packs ? col_order_[k] : k;
-        const float up0 = (0.0f < hp.u[j]) ? 0.0f : hp.u[j];   // std::min(u, 0)
-        x0_[k] = (hp.l[j] < up0) ? up0 : hp.l[j];              // std::max(l, .)
-    }
+    parallel_for(n, [&](int64_t k0, int64_t k1) {
+        for (int64_t k = k0; k < k1; ++k) {
+            const int64_t j = packs ? col_order_[k] : k;
+            const float up0 = (0.0f < hp.u[j]) ? 0.0f : hp.u[j];   // std::min(u, 0)
+            x0_[k] = (hp.l[j] < up0) ? up0 : hp.l[j];              // std::max(l, .)
+        }
+    });
     // max |c| and max |b| over finite bounds (gpu_solver.cpp:112-126)
     max_abs_c_ = 1.0f;
     for (int j = 0; j < n; ++j) max_abs_c_ = (max_abs_c_ < std::fabs(hp.c[j])) ? std::fabs(hp.c[j]) : max_abs_c_;
