@@ -24,12 +24,14 @@ __device__ __forceinline__ float split_dot(const int* __restrict__ idx, const fl
     return s0 + s1;
 }
 
-// Segments summed in place by groups of L lanes (few or long segments).
+// Segments summed in place by groups of L lanes (few or long segments), by the
+// first `blocks` blocks.
 __device__ __forceinline__ void spmv_by_groups(int nseg, const int* __restrict__ ptr, const int* __restrict__ idx,
                                                const float* __restrict__ val, const float* __restrict__ vec,
-                                               float* __restrict__ out, int L) {
+                                               float* __restrict__ out, int L, int blocks) {
+    if (blockIdx.x >= blocks) return;
     const int lane = threadIdx.x & 31, sub = lane & (L - 1), gpw = 32 / L;
-    const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (blocks * blockDim.x) >> 5;
     for (unsigned base = wid * gpw; base < (unsigned)nseg; base += nw * gpw) {  // unsigned: nseg + a turn may pass 2^31
         const unsigned r = base + lane / L;
         float s = 0.f;
@@ -140,16 +142,16 @@ __device__ __forceinline__ void spmv_by_stream(int nseg, const int* __restrict__
 // on the device, so that no launch has to ask the host for it.  By stream from
 // kStreamSegs segments on, where every SM has several warps of 32, and below a
 // mean of 32 (L < 16), where equal lengths are no slower by it at any count.  us by
-// groups / by stream for segments of 20, 28, 36 and 56 entries (L2 flushed): 60,000
-// equal ones 15 / 15, 17 / 17, 19 / 21, 23 / 54; 400,000 equal ones 64 / 42, 76 / 52,
-// 108 / 66, 134 / 191 (past kLong the warp sums each alone); 400,000 by a power law
-// 112 / 55, 146 / 74, 146 / 95, 216 / 160.
+// groups / by stream for segments of 20, 28, 36 and 56 entries, back to back: 60,000
+// equal ones 8.7 / 8.9, 11.3 / 11.1, 11.9 / 13.9, 17 / 48; 400,000 equal ones 38 / 36,
+// 56 / 47, 74 / 59, 104 / 186 (past kLong the warp sums each alone); by a power law 60,000
+// 35 / 22, 48 / 30, 40 / 42, 58 / 76 and 400,000 80 / 48, 124 / 68, 148 / 90, 224 / 154.
 __global__ void __launch_bounds__(kSplitThreads, 8) split_spmv_kernel(int nseg, const int* __restrict__ ptr,
                                                                       const int* __restrict__ idx,
                                                                       const float* __restrict__ val,
                                                                       const float* __restrict__ vec,
-                                                                      float* __restrict__ out) {
-    extern __shared__ float prod[];  // [warps][kWindow]
+                                                                      float* __restrict__ out, int group_blocks) {
+    extern __shared__ float prod[];  // [warps that have segments by stream][kWindow]
     chain_wait_for(ptr, idx, val, vec, out);
     const long long nnz = ptr[nseg];
     int L = 1;
@@ -157,7 +159,7 @@ __global__ void __launch_bounds__(kSplitThreads, 8) split_spmv_kernel(int nseg, 
     if (nseg >= kStreamSegs && L < 16)
         spmv_by_stream(nseg, ptr, idx, val, vec, out, prod + kWindow * (threadIdx.x >> 5));
     else
-        spmv_by_groups(nseg, ptr, idx, val, vec, out, L);
+        spmv_by_groups(nseg, ptr, idx, val, vec, out, L, group_blocks);
 }
 
 __global__ void compat_primal_kernel(int n, const float* __restrict__ tau, const float* __restrict__ c,
@@ -235,7 +237,7 @@ static int split_spmv(int nseg, const int* ptr, const int* idx, const float* val
     if (!ptr || !out || !vec) return fail(SIH_PDHG_ERR_INVALID_ARGUMENT, "NULL device pointer");
     const SplitLaunch g = split_launch(nseg, sm_count());
     SIHG_CUDA(launch_chained(split_spmv_kernel, g.blocks, g.threads, g.smem, static_cast<cudaStream_t>(stream), nseg, ptr,
-                             idx, val, vec, out));
+                             idx, val, vec, out, g.group_blocks));
     return SIH_PDHG_OK;
 }
 

@@ -147,8 +147,10 @@ static int check_norms_noalloc_impl(int m, int n, int nnz, const int* d_row_ptr,
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     noalloc_clear_kernel<<<1, 32, 0, s>>>(words);
     const SplitLaunch gr = split_launch(m, sms), gc = split_launch(n, sms);
-    split_spmv_kernel<<<gr.blocks, gr.threads, gr.smem, s>>>(m, d_row_ptr, d_col_ind, d_csr_values, d_x, ax);
-    split_spmv_kernel<<<gc.blocks, gc.threads, gc.smem, s>>>(n, d_col_ptr, d_row_ind, d_csc_values, d_y, aty);
+    split_spmv_kernel<<<gr.blocks, gr.threads, gr.smem, s>>>(m, d_row_ptr, d_col_ind, d_csr_values, d_x, ax,
+                                                             gr.group_blocks);
+    split_spmv_kernel<<<gc.blocks, gc.threads, gc.smem, s>>>(n, d_col_ptr, d_row_ind, d_csc_values, d_y, aty,
+                                                             gc.group_blocks);
     compat_residuals_kernel<<<grid_for(std::max(m, n), 256, sms), 256, 0, s>>>(
         m, n, ax, d_row_l, d_row_u, row_map, d_x, d_c, aty, d_l, d_u, d_tau, col_map);
     noalloc_max_kernel<<<grid_for(m, 256, sms), 256, 0, s>>>(m, row_map, words, 0);
