@@ -115,7 +115,7 @@ typedef struct sih_pdhg_options {
                                   one thread-block cluster instead); 0 = launch kernel by kernel */
     int32_t autotune;          /* mixed: 1 = at creation, time the step kernels' launch shapes (task size, lanes
                                   per segment of each side, staged gathers, and with persistent < 0 the step
-                                  form) on this batch and keep the fastest, once per batch shape (instances,
+                                  form, a resident one too) on this batch and keep the fastest, once per batch shape (instances,
                                   rows, columns, nonzeros; cached per process); 0 = off; -1 = on for batches
                                   of two or more LPs that are not resident (see persistent; default) */
     int32_t verbose;           /* 0 */
@@ -150,7 +150,8 @@ typedef struct sih_pdhg_options {
                                   0 = one kernel per phase, replayed as CUDA graphs; -1 = automatic (default):
                                   the resident forms where they hold the LP (every instance of a batch in the
                                   shared memory of a thread-block cluster, reported as 2 for one LP and 1 for
-                                  a batch; one LP over the shared memory of every SM, 2), else 0 for one LP
+                                  a batch, unless the clusters' turns would take longer than the other forms;
+                                  one LP over the shared memory of every SM, 2), else 0 for one LP
                                   and the autotuner's choice for a batch.  2 takes the resident forms too. */
     int32_t packed;            /* mixed, kernels per phase: 1 = two kernels per step, the elementwise primal
                                   step folded into the SpMVs (the lanes that gather x' compute it from a packed

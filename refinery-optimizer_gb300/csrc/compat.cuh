@@ -19,14 +19,14 @@ constexpr int kWindow = 512;  // products of a warp at a time, there
 // lanes a segment would need (it takes fewer where the mean length says so), as
 // far as the SMs hold them, 64 warps each, and no more: further blocks would make
 // a second wave (400,000 equal segments of 33 / 70 entries 88 / 169 us with it, 70 / 140
-// without; by a power law 122 / 196 and 134 / 181).  By stream a warp per 32 segments: with more of those than the SMs hold,
-// blocks of four warps, which the hardware hands out as others end (columns of Zipf
-// lengths); below, what the groups want, in blocks of eight, of which the stream
-// leaves some warps idle: only the others have a window, because the shared memory
-// that it takes is missing in the groups' L1.  40,000 / 100,000
-// / 250,000 segments of 70 entries (groups) with a warp per 32 segments everywhere
-// 38.2 / 48.1 / 105, with a window for every warp 14.8 / 33.0 / 86.5, so 13.8 / 32.3 / 85.0
-// us; of 24 (stream) 8.7 / 14.8 / 31.9, 8.1 / 14.7 / 28.1 and 7.9 / 13.8 / 27.6 us.
+// without; by a power law 122 / 196 and 134 / 181).  By stream a warp per 32
+// segments: with more of those than the SMs hold, blocks of four warps, which the
+// hardware hands out as others end (columns of Zipf lengths); below, what the groups
+// want, in blocks of eight, of which the stream leaves some warps idle: only the
+// others have a window, because its shared memory is missing in the groups' L1.
+// 40,000 / 100,000 / 250,000 segments of 70 entries (groups) with a warp per 32 segments
+// everywhere 38.2 / 48.1 / 105, with a window for every warp 14.8 / 33.0 / 86.5, so 13.8 /
+// 32.3 / 85.0 us; of 24 (stream) 8.7 / 14.8 / 31.9, 8.1 / 14.7 / 28.1 and 7.9 / 13.8 / 27.6.
 struct SplitLaunch {
     int blocks, threads, smem;
     int group_blocks;  // that the groups use

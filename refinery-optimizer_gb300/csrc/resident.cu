@@ -21,20 +21,17 @@
 //
 // What bounds it: with one or two passes per warp the chains of dependent
 // instructions (cycle counters around each phase, 2,000 x 5,000 LP on 16 blocks,
-// 14,100 cycles a step before the last line of the measurements below: the x'
-// phase 1,050, its barrier with the average updates 2,100, A x' 2,200, barrier
-// 1,150, A^T y' 3,250, barrier 1,400, the controller 2,550, of which one FP64
-// division 550 and a dozen dependent FP64 operations of 65 each); with four and
-// more the number of instructions as well.  Measured per step, whole solves:
-// 317 x 803 13.7 -> 5.2 us (1, 2, 4, 8 blocks: 8.7, 6.6, 5.2, 5.2), 2,000 x 5,000
-// 13.7 -> 7.4 us (8 blocks: 9.9), 64 of the latter as a batch 84 -> 43 us, with
-// 12 bytes a pair of entries (four blocks an instance, two rounds of clusters) ->
-// 20.8 us.  Fewer instructions from there, steps alone: 16 warps with passes
-// instead of 20 and as few as do the passes in the same rounds, x' by a thread per
-// column instead of the lanes of its passes, the rest of a pass by code of its
-// length: the batch 20.8 -> 18.7 us, 64 of 1,000 x 2,500 by a power law 16.0 ->
-// 13.5, 2,000 x 5,000 6.9 -> 6.4, 317 x 803 4.5 -> 4.3 (26 and 30 warps: 23.0 and
-// 22.5 on the batch, 13: 23.2).
+// 14,100 cycles a step then, 12,400 now: the x' phase 1,050, its barrier with the average
+// updates 2,100, A x' 2,200, barrier 1,150, A^T y' 3,250, barrier 1,400, the controller
+// 2,550, of which one FP64 division 550 and a dozen dependent FP64 operations of
+// 65 each); with four and more the number of instructions as well.  Microseconds
+// per step, k_solo_steps (task engine for the batches) and here: 317 x 803 13.7 and
+// 4.3, 2,000 x 5,000 13.7 and 6.4 (on 8 blocks 9.9), 64 of the latter as a batch 84 and
+// 18.7 (clusters of four blocks, two rounds of them; with 16 bytes a pair of entries
+// 43).  1, 2, 4 and 8 blocks for 317 x 803: 8.7, 6.6, 5.2 and 5.2 in an earlier state.  Why 16
+// warps with passes at most: with 20 the batch 10 %, with 26, 30 or 13 20 % more; why
+// x' by a thread per column and a pass's rest by code of its length: fewer
+// instructions, 3 to 10 % each.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

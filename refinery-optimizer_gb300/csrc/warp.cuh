@@ -464,19 +464,20 @@ __device__ __forceinline__ void spmv_engine(const Side& side, State* st, Epi& ep
 // not wait for a segment's pointers, a counter or a task record, and an L1
 // that holds a line for every miss (shared memory takes its space).
 // The epilogue's operands load behind the gathers, when the pairs' registers
-// are free (before them: 64 registers spill, 2 % slower); packs of up to 128
-// short segments, four per lane, spill as well (6 to 15 % slower).  The entries
-// of one segment of 32 lanes are on their chains' lanes as they load and need no
-// window (500k x 1M, 12M entries below: 137.5 -> 129.0, the mixed step 150.2 ->
-// 147.9); there Epi::kPreFirst says whether the operands load first (plain
-// algorithm 142.7 -> 129.0) or, where that spills, last (the mixed step 152.9 ->
-// 147.9).
-// Microseconds per iteration of the plain algorithm (two kernels) with tasks from
-// a counter, with one run of neighbouring packs per warp and with packs in turn:
-// 20k x 50k, 0.5M entries 15.7 / 10.7 / 9.6; 60k x 130k, 1M entries 24.1 / 15.8 /
-// 14.9; 250k x 500k, 3M, lengths by a power law 60.8 / 49.2 / 41.0; 500k x 1M, 12M,
-// likewise 139.9 / 145.8 / 129.0.  The gathers' way through L1 (a line a cycle and
-// SM) is 70 % busy there, 80 % while the SM has work.
+// are free; before them, or with packs of up to 128 short segments, four per
+// lane, more of the 64 registers spill (2 %, and 6 to 15 % slower).  As it is
+// the kernels store 12 to 96 bytes a thread to local memory, outside the loads
+// in flight.  The entries of one segment of 32 lanes are on their chains' lanes
+// as they load and need no window (500k x 1M, 12M entries: 6 % of the plain
+// iteration, 1.5 % of the mixed step); there Epi::kPreFirst says whether the
+// operands load first (plain algorithm, 10 % faster) or last (the mixed step,
+// where first spills more: 3 % slower).
+// Microseconds per iteration of the plain algorithm (two kernels, a check every 25)
+// with tasks from a counter and with packs in turn: 20k x 50k, 0.5M entries 15.7
+// and 10.3; 60k x 130k, 1M entries 23.6 and 15.9; 150k x 300k, 2.7M 49.0 and 28.9;
+// 500k x 1M, 12M, lengths by a power law 131 and 120.  One run of neighbouring packs
+// per warp instead of turns: 6 to 20 % more.  The gathers' way through L1 (a line a
+// cycle and SM) is 70 % busy on the last, 80 % while the SM has work.
 template <bool COMP, class Epi>
 __device__ __forceinline__ void spmv_packs(const PackSide& P, Epi& epi, float2* __restrict__ window) {
     constexpr int kU = kPackEntries / 32;
